@@ -284,9 +284,7 @@ struct Ctx {
   // slot was needed again), per stream: the first error code, the device
   // status bits.
   std::map<cudaStream_t, std::pair<int, uint32_t>> async_err;
-  DevBuf<int32_t> d_lorder;           // lookahead: claim order (per block shape), done flags, results
-  std::pair<int, int> lorder_shape{0, 0};
-  DevBuf<int32_t> d_ldone;
+  DevBuf<unsigned long long> d_lwords;  // lookahead: published vectors, claim counter, status; results
   DevBuf<uint32_t> d_lcost, d_lsad;
   DevBuf<rme_mv> d_lmv, d_lmv2;
   DevBuf<LowresDesc> d_lpairs;
@@ -1957,32 +1955,19 @@ int rme_lowres_search_batch(void* ctx, int32_t npairs, const int32_t* cur_ids, c
   }
   cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
   CK(cudaSetDevice(c->device));
-  const int bw = pairs[0].bw, bh = pairs[0].bh, n = bw * bh;
-  const int64_t total = (int64_t)n * npairs;
-  // Claim order: anti-diagonals, each block after its left and above ones.
-  if (c->lorder_shape != std::make_pair(bw, bh)) {
-    std::vector<int32_t> order;
-    order.reserve(n);
-    for (int d = 0; d <= bw + bh - 2; ++d)
-      for (int by = std::max(0, d - bw + 1); by <= std::min(d, bh - 1); ++by) order.push_back((by << 16) | (d - by));
-    CK(c->d_lorder.ensure(n));
-    CK(cudaMemcpy(c->d_lorder.p, order.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice));
-    c->lorder_shape = {bw, bh};
-  }
-  CK(c->d_ldone.ensure(total + 8));
+  const int64_t total = (int64_t)pairs[0].bw * pairs[0].bh * npairs;
+  CK(c->d_lwords.ensure(total + 2));
   CK(c->d_lcost.ensure(total));
   CK(c->d_lsad.ensure(total));
   CK(c->d_lmv.ensure(total));
   CK(c->d_lpairs.ensure(2 * (int64_t)npairs));
   CK(cudaMemcpyAsync(c->d_lpairs.p, pairs.data(), sizeof(LowresDesc) * pairs.size(), cudaMemcpyHostToDevice, s));
-  // done flags, then the claim counter and the status word (one memset).
-  CK(cudaMemsetAsync(c->d_ldone.p, 0, sizeof(int32_t) * (total + 8), s));
-  const int64_t ci = (total + 3) & ~int64_t(1);  // an 8-byte aligned word after the flags
-  unsigned long long* counter = reinterpret_cast<unsigned long long*>(c->d_ldone.p + ci);
-  uint32_t* status = reinterpret_cast<uint32_t*>(c->d_ldone.p + ci + 2);
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(c->nsm * 4, (total + 7) / 8));
-  CK(launch_lowres_search(c->d_lpairs.p, npairs, pairs[0], c->d_lorder.p, c->d_ldone.p, counter, status, c->d_lcost.p,
-                          c->d_lmv.p, c->d_lsad.p, grid, s));
+  // Published words, then the claim counter and the status word (one memset).
+  CK(cudaMemsetAsync(c->d_lwords.p, 0, sizeof(unsigned long long) * (total + 2), s));
+  unsigned long long* counter = c->d_lwords.p + total;
+  uint32_t* status = reinterpret_cast<uint32_t*>(counter + 1);
+  CK(launch_lowres_search(c->d_lpairs.p, npairs, pairs[0], c->d_lwords.p, counter, status, c->d_lcost.p, c->d_lmv.p,
+                          c->d_lsad.p, c->nsm * 4, s));
   uint32_t st = 0;
   CK(cudaMemcpyAsync(cost, c->d_lcost.p, sizeof(uint32_t) * total, cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(mv, c->d_lmv.p, sizeof(rme_mv) * total, cudaMemcpyDeviceToHost, s));

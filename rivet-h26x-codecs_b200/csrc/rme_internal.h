@@ -194,9 +194,9 @@ cudaError_t launch_wp_moments(const void* cur, const void* ref, int stride, int 
                               unsigned long long* out, cudaStream_t s);
 cudaError_t launch_weighted_sad(const void* cur, const void* ref, int stride, int bd, int w, int h, int weight,
                                 int shift, int offset, unsigned long long* out, cudaStream_t s);
-// A bounded dependency wait that runs out (rme_lookahead.cu's wait on a flag
-// nothing sets, `limit` polls): sets kStatusWaitTimeout in *status.
-cudaError_t launch_probe_wait(const int32_t* flag, uint32_t limit, uint32_t* status, cudaStream_t s);
+// A bounded dependency wait that runs out (rme_lookahead.cu's wait on a word
+// nothing publishes, `limit` polls): sets kStatusWaitTimeout in *status.
+cudaError_t launch_probe_wait(const unsigned long long* word, uint32_t limit, uint32_t* status, cudaStream_t s);
 // HEVC bi-prediction (rme_bi.cu): the jobs of a frame's source and
 // references; refine_bi targets are kBiBlock-wide blocks.
 constexpr int kBiBlock = 64;
@@ -234,10 +234,11 @@ struct LowresDesc {
 };
 cudaError_t launch_lowres_build(const DevPlanes& pic, int bd, int w, int h, const LowresDesc& L, cudaStream_t s);
 // `pairs`: device array of (cur, ref) descriptors of npairs pairs that share
-// the block grid of `first`; per-pair outputs and done flags npairs x blocks.
-cudaError_t launch_lowres_search(const LowresDesc* pairs, int npairs, const LowresDesc& first, const int32_t* order,
-                                 int32_t* done, unsigned long long* counter, uint32_t* status, uint32_t* cost,
-                                 rme_mv* mv, uint32_t* nsad, int grid, cudaStream_t s);
+// the block grid of `first`; per-pair outputs and published words (zeroed)
+// npairs x blocks; at most `max_ctas` CTAs, all resident at once.
+cudaError_t launch_lowres_search(const LowresDesc* pairs, int npairs, const LowresDesc& first,
+                                 unsigned long long* words, unsigned long long* counter, uint32_t* status,
+                                 uint32_t* cost, rme_mv* mv, uint32_t* nsad, int max_ctas, cudaStream_t s);
 cudaError_t launch_lowres_bi(const LowresDesc& cur, const LowresDesc& r0, const LowresDesc& r1, const rme_mv* m0,
                              const rme_mv* m1, uint32_t* cost, cudaStream_t s);
 

@@ -5,11 +5,16 @@
 // a reference and the SATD against the average of two displaced blocks.
 //
 // The search reads the left and above blocks' vectors as seeds, so its
-// blocks form a wavefront. Warps claim blocks in anti-diagonal order from
-// one counter and wait (bounded) for the two blocks they read: every block
-// a warp waits for was claimed earlier by a running warp, so the wait
-// always ends unless a wait bound runs out, which sets the status word.
+// blocks form a wavefront. A warp owns a row of blocks and searches it left
+// to right, its left seed in registers; each block's vector is published as
+// one word, and the row below waits (bounded) for that word only. Rows are
+// claimed top to bottom from one counter, so a row a warp waits for was
+// claimed earlier by a running warp: the wait always ends unless its bound
+// runs out, which sets the status word. The winners' SATDs, which no other
+// block reads, are a second launch over all blocks at once.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "rme_internal.h"
 
@@ -35,14 +40,9 @@ __global__ void lowres_build_kernel(const S* __restrict__ pic, int pstride, int 
   L.plane[(ptrdiff_t)Y * L.stride + X] = (uint8_t)min(((s + 2) >> 2) >> (bd - 8), 255);
 }
 
-// One 4x4 tile's Hadamard SATD, (sum + 1) >> 1 (dsp/distortion.rs:350-381).
-template <class S>
-__device__ __forceinline__ uint32_t satd4x4_tile(const S* a, int as, const S* b, int bs) {
-  int d[16];
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) d[r * 4 + c] = (int)a[(ptrdiff_t)r * as + c] - (int)b[(ptrdiff_t)r * bs + c];
+// The 4x4 Hadamard SATD of sixteen differences, (sum + 1) >> 1
+// (dsp/distortion.rs:350-381).
+__device__ __forceinline__ uint32_t hadamard_satd(int (&d)[16]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int p = d[i * 4], q = d[i * 4 + 1], u = d[i * 4 + 2], v = d[i * 4 + 3];
@@ -60,6 +60,17 @@ __device__ __forceinline__ uint32_t satd4x4_tile(const S* a, int as, const S* b,
     sum += abs(s0 + s1) + abs(s3 + s2) + abs(s0 - s1) + abs(s3 - s2);
   }
   return (sum + 1) >> 1;
+}
+
+// One 4x4 tile's SATD.
+template <class S>
+__device__ __forceinline__ uint32_t satd4x4_tile(const S* a, int as, const S* b, int bs) {
+  int d[16];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) d[r * 4 + c] = (int)a[(ptrdiff_t)r * as + c] - (int)b[(ptrdiff_t)r * bs + c];
+  return hadamard_satd(d);
 }
 
 template <class S>
@@ -97,26 +108,36 @@ __global__ void lowres_intra_kernel(LowresDesc L) {
   L.intra[b] = max(best, 16u);
 }
 
-__device__ __forceinline__ uint32_t ld_acquire32(const int32_t* p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+// A block's published vector: bit 32 set, the vector in the low half. The
+// word carries all a reader needs, so relaxed accesses suffice.
+__device__ __forceinline__ unsigned long long ld_word(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release32(int32_t* p, int32_t v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void st_word(unsigned long long* p, uint32_t mv) {
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(1ull << 32 | mv) : "memory");
 }
 
-// A bounded wait (lane 0) for block b to be done: at most `limit` polls,
-// then the status word records the timeout and the wait gives up.
-__device__ __forceinline__ bool wait_done(const int32_t* done, int b, uint32_t* status, uint32_t limit = kSpinLimit) {
+// A bounded wait for a published word, already loaded once (`w`): at most
+// `limit` polls (the first few back to back, the upper row being a block
+// ahead), then the status word records the timeout and the wait gives up
+// (false). A warp that gave up once waits no more (`lost`).
+__device__ __forceinline__ bool wait_word(const unsigned long long* p, unsigned long long& w, uint32_t* status,
+                                          bool lost = false, uint32_t limit = kSpinLimit) {
   uint32_t ns = 32;
-  for (uint32_t it = 0; it < limit; ++it) {
-    if (ld_acquire32(done + b)) return true;
-    __nanosleep(ns);
-    if (ns < 256) ns <<= 1;
+  for (uint32_t it = 0; (w >> 32) == 0ull; ++it) {
+    if (lost || it >= limit) {
+      if (!lost) atomicOr(status, kStatusWaitTimeout);
+      return false;
+    }
+    if (it >= 16) {
+      __nanosleep(ns);
+      if (ns < 256) ns <<= 1;
+    }
+    w = ld_word(p);
   }
-  atomicOr(status, kStatusWaitTimeout);
-  return false;
+  return true;
 }
 
 // Eight bytes of a row at any byte address (three aligned loads).
@@ -138,102 +159,197 @@ __device__ __forceinline__ Pick2 argmin(uint32_t c) {
   return {m, __ffs(__ballot_sync(kAll, c == m)) - 1};
 }
 
-// search (h265_cutree.rs:152-216), one warp per block: four candidates per
-// step (group g = lane / 8, lane sub = row), the first least cost taken when
-// strictly below the best, as the reference's in-order scoring.
-__global__ void __launch_bounds__(256) lowres_search_kernel(const LowresDesc* pairs, int npairs, const int32_t* order,
-                                                            int32_t* done_all, unsigned long long* counter,
-                                                            uint32_t* status, uint32_t* cost_all, rme_mv* mv_all,
-                                                            uint32_t* nsad_all) {
-  const int lane = threadIdx.x & 31, g = lane >> 3, sub = lane & 7;
-  const int n = pairs[0].bw * pairs[0].bh, lim = kLowresPad - 1;
-  for (;;) {
-    unsigned long long i = 0;
-    if (lane == 0) i = atomicAdd(counter, 1ull);
-    i = __shfl_sync(kAll, i, 0);
-    if (i >= (unsigned long long)n * npairs) break;
-    // Claims interleave the pairs in wavefront order: entry e of pair pi is
-    // claim e * npairs + pi, after every block it reads.
-    const int pi = (int)(i % npairs), e = (int)(i / npairs);
+// The row a warp claims next: row-major over the pairs (every pair's row 0,
+// then every row 1, ...), so that a claim's upper row was claimed before it.
+__device__ __forceinline__ bool claim_row(unsigned long long* counter, int npairs, int rows, int lane, int& pair,
+                                          int& row) {
+  unsigned long long c = 0;
+  if (lane == 0) c = atomicAdd(counter, 1ull);
+  c = __shfl_sync(kAll, c, 0);
+  if (c >= (unsigned long long)npairs * rows) return false;
+  row = (int)(c / npairs);
+  pair = (int)(c - (unsigned long long)row * npairs);
+  return true;
+}
+
+// search (h265_cutree.rs:152-216), a warp per row of blocks, two lanes per
+// candidate (four rows of the block each). The reference walks a 4-, a 2-
+// and a 1-sample ring of four points, a ring again after each move; the
+// three rings around a centre are known together, so a pass scores all
+// twelve points and resolves them in the reference's order (the first ring
+// with a point below the best moves there and the walk goes on at that
+// ring; the points counted are those the reference scores). The first pass
+// scores the seeds and, around the first of the neighbours' vectors, the
+// rings: where that seed wins, as it does in even motion, its rings are
+// known already.
+//
+// Bound by the chain of passes along the wavefront (bw + 2 bh blocks): a
+// load, one shuffle and one warp minimum each. Eight pairs of 1080p
+// pictures: 3,010 us when a warp took one block at a time (claim, two waits,
+// up to twelve passes, the SATD), 547 us this way, the SATDs included.
+constexpr int kLaWarps = 4;  // rows per CTA: few, so that a launch's rows spread over the SMs
+__global__ void __launch_bounds__(kLaWarps * 32) lowres_search_kernel(const LowresDesc* pairs, int npairs,
+                                                                      unsigned long long* words_all,
+                                                                      unsigned long long* counter, uint32_t* status,
+                                                                      rme_mv* mv_all, uint32_t* nsad_all) {
+  const int lane = threadIdx.x & 31, q = lane >> 1, half = lane & 1;
+  const int bw = pairs[0].bw, bh = pairs[0].bh, n = bw * bh, lim = kLowresPad - 1;
+  bool lost = false;
+  // This lane's ring point as the q-th candidate of a pass of rings (q in
+  // 0..11: ring 4, 2, 1, each (s,0), (-s,0), (0,s), (0,-s)).
+  auto ring_x = [](int k) { const int st = 4 >> (k >> 2), d = k & 3; return d == 0 ? st : d == 1 ? -st : 0; };
+  auto ring_y = [](int k) { const int st = 4 >> (k >> 2), d = k & 3; return d == 2 ? st : d == 3 ? -st : 0; };
+  for (int pi, by; claim_row(counter, npairs, bh, lane, pi, by);) {
     const LowresDesc cur = pairs[2 * pi], ref = pairs[2 * pi + 1];
-    int32_t* done = done_all + (size_t)pi * n;
-    uint32_t* cost = cost_all + (size_t)pi * n;
-    rme_mv* mv = mv_all + (size_t)pi * n;
-    uint32_t* nsad_out = nsad_all ? nsad_all + (size_t)pi * n : nullptr;
-    const int packed = __ldg(order + e), bx = packed & 0xffff, by = packed >> 16, b = by * cur.bw + bx;
-    if (lane == 0) {
-      if (bx > 0) wait_done(done, b - 1, status);
-      if (by > 0) wait_done(done, b - cur.bw, status);
-    }
-    __syncwarp();
-    const int x = bx * 8, y = by * 8;
-    const uint8_t* src = cur.plane + (ptrdiff_t)(y + kLowresPad) * cur.stride + x + kLowresPad;
-    const uint8_t* rb = ref.plane + (ptrdiff_t)(y + kLowresPad) * ref.stride + x + kLowresPad;
-    // This lane's source row (8-byte aligned: x, the pad and the stride
-    // are multiples of 8).
-    const uint32_t s0 = *reinterpret_cast<const uint32_t*>(src + (ptrdiff_t)sub * cur.stride);
-    const uint32_t s1 = *reinterpret_cast<const uint32_t*>(src + (ptrdiff_t)sub * cur.stride + 4);
-    auto inplane = [&](int dx, int dy) {
-      return x + dx >= -lim && y + dy >= -lim && x + dx + 8 <= ref.pw + lim && y + dy + 8 <= ref.ph + lim;
-    };
-    auto score = [&](bool ok, int dx, int dy) -> uint32_t {
-      uint32_t part = 0;
-      if (ok) {
-        uint32_t a, c;
-        ld8(rb + (ptrdiff_t)(dy + sub) * ref.stride + dx, a, c);
-        part = __vsadu4(s0, a) + __vsadu4(s1, c);
+    unsigned long long* words = words_all + (size_t)pi * n + (size_t)by * bw;
+    const unsigned long long* up = words - bw;
+    const int y = by * 8;
+    const uint8_t* srow = cur.plane + (ptrdiff_t)(y + kLowresPad + half * 4) * cur.stride + kLowresPad;
+    const uint8_t* rrow = ref.plane + (ptrdiff_t)(y + kLowresPad + half * 4) * ref.stride + kLowresPad;
+    // The first block's source rows and upper vector; later ones are loaded
+    // a block ahead (8-byte aligned: x, the pad and the stride are multiples
+    // of 8).
+    uint2 s[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) s[r] = __ldg(reinterpret_cast<const uint2*>(srow + (ptrdiff_t)r * cur.stride));
+    unsigned long long uw = by > 0 ? ld_word(up) : 0ull;
+    uint32_t lv = 0;
+    for (int bx = 0; bx < bw; ++bx) {
+      const int x = bx * 8;
+      const uint8_t* rb = rrow + x;
+      if (by > 0 && !wait_word(up + bx, uw, status, lost)) lost = true;
+      const uint32_t av = (uint32_t)uw;
+      uint2 sn[4] = {};
+      unsigned long long un = 0ull;
+      if (bx + 1 < bw) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          sn[r] = __ldg(reinterpret_cast<const uint2*>(srow + (ptrdiff_t)r * cur.stride + x + 8));
+        if (by > 0) un = ld_word(up + bx + 1);
       }
-      part += __shfl_xor_sync(kAll, part, 4);
-      part += __shfl_xor_sync(kAll, part, 2);
-      part += __shfl_xor_sync(kAll, part, 1);
-      return ok ? part + 2u * (uint32_t)min(abs(dx) + abs(dy), 32) : 0xffffffffu;
-    };
-    // Seeds: zero, the left block's vector, the above block's.
-    uint32_t lv = 0, av = 0;
-    if (bx > 0) lv = __ldcg(reinterpret_cast<const unsigned int*>(mv + b - 1));
-    if (by > 0) av = __ldcg(reinterpret_cast<const unsigned int*>(mv + b - cur.bw));
-    const int ns = 1 + (bx > 0) + (by > 0);
-    const uint32_t sv = g == 0 ? 0u : g == 1 ? (bx > 0 ? lv : av) : av;
-    int dx = (int)(int16_t)(sv & 0xffffu), dy = (int)(int16_t)(sv >> 16);
-    bool ok = g < ns && inplane(dx, dy);
-    uint32_t nsad = __popc(__ballot_sync(kAll, ok && sub == 0));
-    Pick2 p = argmin(score(ok, dx, dy));
-    uint32_t bc = p.cost;
-    int bxm = __shfl_sync(kAll, dx, p.lane), bym = __shfl_sync(kAll, dy, p.lane);
-    if (bc == 0xffffffffu) bxm = bym = 0;  // no seed in the plane
-    const int cx = bxm, cy = bym;
-    for (int step = 4; step >= 1; step >>= 1) {
-      for (;;) {
-        dx = bxm + (g == 0 ? step : g == 1 ? -step : 0);
-        dy = bym + (g == 2 ? step : g == 3 ? -step : 0);
-        ok = abs(dx - cx) <= kLowresRange && abs(dy - cy) <= kLowresRange && inplane(dx, dy);
-        nsad += __popc(__ballot_sync(kAll, ok && sub == 0));
-        p = argmin(score(ok, dx, dy));
-        if (!(p.cost < bc)) break;
+      auto inplane = [&](int dx, int dy) {
+        return x + dx >= -lim && y + dy >= -lim && x + dx + 8 <= ref.pw + lim && y + dy + 8 <= ref.ph + lim;
+      };
+      auto score = [&](bool ok, int dx, int dy) -> uint32_t {
+        uint32_t part = 0;
+        if (ok) {
+          uint32_t a[4], b[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) ld8(rb + (ptrdiff_t)(dy + r) * ref.stride + dx, a[r], b[r]);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) part += __vsadu4(s[r].x, a[r]) + __vsadu4(s[r].y, b[r]);
+        }
+        part += __shfl_xor_sync(kAll, part, 1);
+        return ok ? part + 2u * (uint32_t)min(abs(dx) + abs(dy), 32) : 0xffffffffu;
+      };
+      // Seeds: zero, the left block's vector, the above block's (candidates
+      // 0..2); rings around the first neighbour's (candidates 3..14).
+      const int ns = 1 + (bx > 0) + (by > 0);
+      const uint32_t v1 = bx > 0 ? lv : av;
+      const int gx = (int)(int16_t)(v1 & 0xffffu), gy = (int)(int16_t)(v1 >> 16);  // zero with no neighbour
+      int dx, dy;
+      bool ok;
+      if (q < 3) {
+        const uint32_t sv = q == 0 ? 0u : q == 1 ? v1 : av;
+        dx = (int)(int16_t)(sv & 0xffffu);
+        dy = (int)(int16_t)(sv >> 16);
+        ok = q < ns && inplane(dx, dy);
+      } else {
+        dx = gx + ring_x(q - 3);
+        dy = gy + ring_y(q - 3);
+        ok = q < 15 && inplane(dx, dy);
+      }
+      uint32_t cost = score(ok, dx, dy);
+      uint32_t nsad = __popc(__ballot_sync(kAll, ok && q < 3 && half == 0));
+      Pick2 p = argmin(q < 3 ? cost : 0xffffffffu);
+      uint32_t bc = p.cost;
+      int bxm = __shfl_sync(kAll, dx, p.lane), bym = __shfl_sync(kAll, dy, p.lane);
+      if (bc == 0xffffffffu) bxm = bym = 0;  // no seed in the plane
+      const int cx = bxm, cy = bym;
+      int k = q - 3;  // this lane's ring candidate (0..11 where there is one)
+      bool known = bxm == gx && bym == gy;
+      for (int ring = 0;;) {  // rings `ring`.. of 0, 1, 2 are left around the best
+        if (!known) {
+          k = q;
+          dx = bxm + ring_x(k);
+          dy = bym + ring_y(k);
+          ok = k < 12 && (k >> 2) >= ring && abs(dx - cx) <= kLowresRange && abs(dy - cy) <= kLowresRange &&
+               inplane(dx, dy);
+          cost = score(ok, dx, dy);
+        }
+        known = false;
+        const bool live = ok && k >= 0;
+        const uint32_t cnt = __ballot_sync(kAll, live && half == 0);
+        const uint32_t low = __ballot_sync(kAll, live && cost < bc);
+        if (low == 0u) {
+          nsad += __popc(cnt);
+          break;
+        }
+        // The first ring with a point below the best; the rings before it
+        // and it are the ones scored.
+        const int at = __shfl_sync(kAll, k, __ffs(low) - 1) >> 2;
+        nsad += __popc(__ballot_sync(kAll, live && half == 0 && (k >> 2) <= at));
+        p = argmin(live && (k >> 2) == at ? cost : 0xffffffffu);
         bc = p.cost;
         bxm = __shfl_sync(kAll, dx, p.lane);
         bym = __shfl_sync(kAll, dy, p.lane);
+        ring = at;
       }
+      lv = (uint32_t)(uint16_t)(int16_t)bxm | (uint32_t)(uint16_t)(int16_t)bym << 16;
+      if (lane == 0) {
+        st_word(words + bx, lv);
+        const size_t o = (size_t)pi * n + (size_t)by * bw + bx;
+        *reinterpret_cast<uint32_t*>(mv_all + o) = lv;
+        nsad_all[o] = nsad;
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) s[r] = sn[r];
+      uw = un;
     }
-    // The winner's SATD: tile `lane` of the four (lanes 0..3).
-    uint32_t sat = 0;
-    if (lane < 4) {
-      const int tx = lane & 1, ty = lane >> 1;
-      sat = satd4x4_tile<uint8_t>(src + (ptrdiff_t)(ty * 4) * cur.stride + tx * 4, cur.stride,
-                                  rb + (ptrdiff_t)(bym + ty * 4) * ref.stride + bxm + tx * 4, ref.stride);
-    }
-    sat += __shfl_xor_sync(kAll, sat, 1);
-    sat += __shfl_xor_sync(kAll, sat, 2);
-    if (lane == 0) {
-      cost[b] = sat;
-      mv[b].x = (int16_t)bxm;
-      mv[b].y = (int16_t)bym;
-      if (nsad_out) nsad_out[b] = nsad;
-      __threadfence();
-      st_release32(done + b, 1);
-    }
-    __syncwarp();
   }
+}
+
+// The found vectors' SATDs (both lookaheads), a thread per 4x4 tile, four
+// per block.
+template <class S>
+__global__ void __launch_bounds__(256) lowres_cost_kernel(const LowresDesc* pairs, int npairs, const rme_mv* mv_all,
+                                                          uint32_t* cost_all) {
+  const int bw = pairs[0].bw, n = bw * pairs[0].bh;
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, blk = i >> 2;
+  uint32_t sat = 0;
+  if (blk < (int64_t)n * npairs) {
+    const int pi = (int)(blk / n), b = (int)(blk - (int64_t)pi * n), by = b / bw, bx = b - by * bw;
+    const int x = bx * 8 + ((int)i & 1) * 4 + kLowresPad, y = by * 8 + ((int)(i >> 1) & 1) * 4 + kLowresPad;
+    const LowresDesc &cur = pairs[2 * pi], &ref = pairs[2 * pi + 1];
+    const rme_mv m = mv_all[blk];
+    const S* sp = reinterpret_cast<const S*>(cur.plane) + (ptrdiff_t)y * cur.stride + x;
+    const S* rp = reinterpret_cast<const S*>(ref.plane) + (ptrdiff_t)(y + m.y) * ref.stride + x + m.x;
+    constexpr int W = sizeof(S);  // words of a tile row
+    uint32_t a[4][W], c[4][W + 1];
+    const uintptr_t u = reinterpret_cast<uintptr_t>(rp);
+    const uint32_t sh = (uint32_t)(u & 3) * 8u;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(u & ~uintptr_t(3)) + (ptrdiff_t)r * ref.stride * (int)sizeof(S) / 4;
+#pragma unroll
+      for (int k = 0; k <= W; ++k) c[r][k] = __ldg(w + k);
+#pragma unroll
+      for (int k = 0; k < W; ++k) a[r][k] = __ldg(reinterpret_cast<const uint32_t*>(sp + (ptrdiff_t)r * cur.stride) + k);
+    }
+    int d[16];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int k = e * (int)sizeof(S) / 4, f = e * 8 * (int)sizeof(S) - 32 * k;
+        const uint32_t mask = sizeof(S) == 1 ? 0xffu : 0xffffu;
+        d[r * 4 + e] = (int)((a[r][k] >> f) & mask) - (int)((__funnelshift_r(c[r][k], c[r][k + 1], sh) >> f) & mask);
+      }
+    sat = hadamard_satd(d);
+  }
+  sat += __shfl_xor_sync(kAll, sat, 1);
+  sat += __shfl_xor_sync(kAll, sat, 2);
+  if ((i & 3) == 0 && blk < (int64_t)n * npairs) cost_all[blk] = sat;
 }
 
 // bi_cost (h265_cutree.rs:222-243), one thread per block.
@@ -353,147 +469,127 @@ struct Row8<uint16_t> {
   }
 };
 
-// search (h264_lookahead.rs:227-376), one warp per block, eight points per
-// pass (group g = lane / 4 scores one point, lane q = lane % 4 its rows q
-// and q + 4). The window is the reference's: 16 samples into the border,
-// at most 32 from the block. From the zero vector, the left and above
-// blocks' vectors (zero where there is no such block) clamped to the window,
-// each scored unless it is the best's point, then the hexagon (after a step
-// in direction k only k - 1, k and k + 1 are new), at most 16 steps, then
-// the eight-point square; the SAD + 2 * min(|mx| + |my|, 64) of each point,
-// the first least cost taken when strictly below the best (the reference's
-// in-order scoring), the winner's SATD.
+// search (h264_lookahead.rs:227-376), a warp per row of blocks, two lanes
+// per candidate (four rows each). The window is the reference's: 16 samples
+// into the border, at most 32 from the block. From the zero vector, the left
+// and above blocks' vectors (zero where there is no such block) clamped to
+// the window, each scored unless it is the best's point, then the hexagon
+// (after a step in direction k only k - 1, k and k + 1 are new), at most 16
+// steps, then the eight-point square; the SAD + 2 * min(|mx| + |my|, 64) of
+// each point, the first least cost taken when strictly below the best (the
+// reference's in-order scoring). A pass scores a hexagon step (candidates
+// 0..5) together with the square around the same centre (6..13), which is
+// the walk's last step when the hexagon has settled there.
 template <class S>
-__global__ void __launch_bounds__(256) lowres_search_h264_kernel(const LowresDesc* pairs, int npairs,
-                                                                 const int32_t* order, int32_t* done_all,
-                                                                 unsigned long long* counter, uint32_t* status,
-                                                                 uint32_t* cost_all, rme_mv* mv_all,
-                                                                 uint32_t* nsad_all) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  const int n = pairs[0].bw * pairs[0].bh, lim = kLowresPad - 8;
-  for (;;) {
-    unsigned long long i = 0;
-    if (lane == 0) i = atomicAdd(counter, 1ull);
-    i = __shfl_sync(kAll, i, 0);
-    if (i >= (unsigned long long)n * npairs) break;
-    const int pi = (int)(i % npairs), e = (int)(i / npairs);  // as lowres_search_kernel's claims
+__global__ void __launch_bounds__(kLaWarps * 32) lowres_search_h264_kernel(const LowresDesc* pairs, int npairs,
+                                                                           unsigned long long* words_all,
+                                                                           unsigned long long* counter,
+                                                                           uint32_t* status, rme_mv* mv_all,
+                                                                           uint32_t* nsad_all) {
+  const int lane = threadIdx.x & 31, q = lane >> 1, half = lane & 1;
+  const int bw = pairs[0].bw, bh = pairs[0].bh, n = bw * bh, lim = kLowresPad - 8;
+  // This lane's offset from the centre: a point of the hexagon or of the
+  // 3x3 square without its centre.
+  const int sk = q - 6 < 4 ? q - 6 : q - 5;
+  const int ofx = q == 0 ? -2 : q == 1 ? -1 : q == 2 ? 1 : q == 3 ? 2 : q == 4 ? 1 : q == 5 ? -1 : sk % 3 - 1;
+  const int ofy = q == 0 || q == 3 ? 0 : q < 3 ? -2 : q < 6 ? 2 : sk / 3 - 1;
+  bool lost = false;
+  for (int pi, by; claim_row(counter, npairs, bh, lane, pi, by);) {
     const LowresDesc cur = pairs[2 * pi], ref = pairs[2 * pi + 1];
-    const S* cplane = reinterpret_cast<const S*>(cur.plane);
-    const S* rplane = reinterpret_cast<const S*>(ref.plane);
-    int32_t* done = done_all + (size_t)pi * n;
-    uint32_t* cost = cost_all + (size_t)pi * n;
-    rme_mv* mv = mv_all + (size_t)pi * n;
-    uint32_t* nsad_out = nsad_all ? nsad_all + (size_t)pi * n : nullptr;
-    const int packed = __ldg(order + e), bx = packed & 0xffff, by = packed >> 16, b = by * cur.bw + bx;
-    if (lane == 0) {
-      if (bx > 0) wait_done(done, b - 1, status);
-      if (by > 0) wait_done(done, b - cur.bw, status);
-    }
-    __syncwarp();
-    const int x = bx * 8, y = by * 8;
-    const S* src = cplane + (ptrdiff_t)(y + kLowresPad) * cur.stride + x + kLowresPad;
-    const S* rb = rplane + (ptrdiff_t)(y + kLowresPad) * ref.stride + x + kLowresPad;
-    const int lx = max(-x - lim, -2 * kLowresRange), hx = min(cur.pw - 8 - x + lim, 2 * kLowresRange);
+    unsigned long long* words = words_all + (size_t)pi * n + (size_t)by * bw;
+    const unsigned long long* up = words - bw;
+    const int y = by * 8;
+    const S* srow = reinterpret_cast<const S*>(cur.plane) + (ptrdiff_t)(y + kLowresPad + half * 4) * cur.stride + kLowresPad;
+    const S* rrow = reinterpret_cast<const S*>(ref.plane) + (ptrdiff_t)(y + kLowresPad + half * 4) * ref.stride + kLowresPad;
     const int ly = max(-y - lim, -2 * kLowresRange), hy = min(cur.ph - 8 - y + lim, 2 * kLowresRange);
-    // This lane's two source rows (aligned: x, the pad and the stride are
-    // multiples of 8 samples).
-    Row8<S> s0, s1;
-    s0.load(src + (ptrdiff_t)q * cur.stride);
-    s1.load(src + (ptrdiff_t)(q + 4) * cur.stride);
-    auto score = [&](bool ok, int dx, int dy) -> uint32_t {
-      uint32_t part = 0;
-      if (ok) {
-        Row8<S> a, c;
-        a.load(rb + (ptrdiff_t)(dy + q) * ref.stride + dx);
-        c.load(rb + (ptrdiff_t)(dy + q + 4) * ref.stride + dx);
-        part = s0.sad(a) + s1.sad(c);
+    Row8<S> s[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) s[r].load(srow + (ptrdiff_t)r * cur.stride);
+    unsigned long long uw = by > 0 ? ld_word(up) : 0ull;
+    uint32_t lv = 0;
+    for (int bx = 0; bx < bw; ++bx) {
+      const int x = bx * 8;
+      const S* rb = rrow + x;
+      if (by > 0 && !wait_word(up + bx, uw, status, lost)) lost = true;
+      const uint32_t av = (uint32_t)uw;
+      Row8<S> sn[4];
+      unsigned long long un = 0ull;
+      const int xn = bx + 1 < bw ? x + 8 : x;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) sn[r].load(srow + (ptrdiff_t)r * cur.stride + xn);
+      if (by > 0 && bx + 1 < bw) un = ld_word(up + bx + 1);
+      const int lx = max(-x - lim, -2 * kLowresRange), hx = min(cur.pw - 8 - x + lim, 2 * kLowresRange);
+      auto score = [&](bool ok, int dx, int dy) -> uint32_t {
+        uint32_t part = 0;
+        if (ok) {
+          Row8<S> a[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) a[r].load(rb + (ptrdiff_t)(dy + r) * ref.stride + dx);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) part += s[r].sad(a[r]);
+        }
+        part += __shfl_xor_sync(kAll, part, 1);
+        return ok ? part + 2u * (uint32_t)min(abs(dx) + abs(dy), 64) : 0xffffffffu;
+      };
+      auto inwin = [&](int dx, int dy) { return dx >= lx && dx <= hx && dy >= ly && dy <= hy; };
+      // The zero vector and the two candidates, scored at once, resolved in
+      // the reference's order.
+      const int c0x = min(max((int)(int16_t)(lv & 0xffffu), lx), hx), c0y = min(max((int)(int16_t)(lv >> 16), ly), hy);
+      const int c1x = min(max((int)(int16_t)(av & 0xffffu), lx), hx), c1y = min(max((int)(int16_t)(av >> 16), ly), hy);
+      int dx = q == 1 ? c0x : q == 2 ? c1x : 0, dy = q == 1 ? c0y : q == 2 ? c1y : 0;
+      const uint32_t sc = score(q < 3, dx, dy);
+      const uint32_t z = __shfl_sync(kAll, sc, 0), k0 = __shfl_sync(kAll, sc, 2), k1 = __shfl_sync(kAll, sc, 4);
+      uint32_t bc = z, nsad = 1;
+      int bxm = 0, bym = 0;
+      if (c0x != 0 || c0y != 0) {
+        ++nsad;
+        if (k0 < bc) {
+          bc = k0;
+          bxm = c0x;
+          bym = c0y;
+        }
       }
-      part += __shfl_xor_sync(kAll, part, 2);
-      part += __shfl_xor_sync(kAll, part, 1);
-      return ok ? part + 2u * (uint32_t)min(abs(dx) + abs(dy), 64) : 0xffffffffu;
-    };
-    auto inwin = [&](int dx, int dy) { return dx >= lx && dx <= hx && dy >= ly && dy <= hy; };
-    // The zero vector and the two candidates, scored at once (groups 0..2),
-    // resolved in the reference's order.
-    uint32_t lv = 0, av = 0;
-    if (bx > 0) lv = __ldcg(reinterpret_cast<const unsigned int*>(mv + b - 1));
-    if (by > 0) av = __ldcg(reinterpret_cast<const unsigned int*>(mv + b - cur.bw));
-    const int c0x = min(max((int)(int16_t)(lv & 0xffffu), lx), hx), c0y = min(max((int)(int16_t)(lv >> 16), ly), hy);
-    const int c1x = min(max((int)(int16_t)(av & 0xffffu), lx), hx), c1y = min(max((int)(int16_t)(av >> 16), ly), hy);
-    int dx = g == 1 ? c0x : g == 2 ? c1x : 0, dy = g == 1 ? c0y : g == 2 ? c1y : 0;
-    const uint32_t sc = score(g < 3, dx, dy);
-    const uint32_t z = __shfl_sync(kAll, sc, 0), k0 = __shfl_sync(kAll, sc, 4), k1 = __shfl_sync(kAll, sc, 8);
-    uint32_t bc = z, nsad = 1;
-    int bxm = 0, bym = 0;
-    if (c0x != 0 || c0y != 0) {
-      ++nsad;
-      if (k0 < bc) {
-        bc = k0;
-        bxm = c0x;
-        bym = c0y;
+      if (c1x != bxm || c1y != bym) {
+        ++nsad;
+        if (k1 < bc) {
+          bc = k1;
+          bxm = c1x;
+          bym = c1y;
+        }
       }
-    }
-    if (c1x != bxm || c1y != bym) {
-      ++nsad;
-      if (k1 < bc) {
-        bc = k1;
-        bxm = c1x;
-        bym = c1y;
-      }
-    }
-    // The hexagon, its points in order around it.
-    const int hxo = g == 0 ? -2 : g == 1 ? -1 : g == 2 ? 1 : g == 3 ? 2 : g == 4 ? 1 : -1;
-    const int hyo = g == 0 ? 0 : g < 3 ? -2 : g == 3 ? 0 : 2;
-    int from = -1;
-    for (int it = 0; it < kLowresRange; ++it) {
-      uint32_t live = 0x3f;
-      if (from >= 0) {
-        const uint32_t r = 7u << (from + 5);
+      uint32_t live = 0x3f;  // the hexagon's new points
+      for (int it = 0;; ++it) {
+        dx = bxm + ofx;
+        dy = bym + ofy;
+        const bool ok = (q < 6 ? it < kLowresRange && ((live >> q) & 1) : q < 14) && inwin(dx, dy);
+        const uint32_t cost = score(ok, dx, dy);
+        nsad += __popc(__ballot_sync(kAll, ok && q < 6 && half == 0));
+        Pick2 p = argmin(q < 6 ? cost : 0xffffffffu);
+        const bool step = p.cost < bc;
+        if (!step) {  // settled: the square around the hexagon's centre
+          nsad += __popc(__ballot_sync(kAll, ok && q >= 6 && half == 0));
+          p = argmin(q >= 6 ? cost : 0xffffffffu);
+        }
+        if (p.cost < bc) {
+          bc = p.cost;
+          bxm = __shfl_sync(kAll, dx, p.lane);
+          bym = __shfl_sync(kAll, dy, p.lane);
+        }
+        if (!step) break;
+        const uint32_t r = 7u << ((p.lane >> 1) + 5);
         live = (r | r >> 6 | r >> 12) & 0x3f;
       }
-      dx = bxm + hxo;
-      dy = bym + hyo;
-      const bool ok = g < 6 && ((live >> g) & 1) && inwin(dx, dy);
-      nsad += __popc(__ballot_sync(kAll, ok && q == 0));
-      const Pick2 p = argmin(score(ok, dx, dy));
-      if (!(p.cost < bc)) break;
-      bc = p.cost;
-      bxm = __shfl_sync(kAll, dx, p.lane);
-      bym = __shfl_sync(kAll, dy, p.lane);
-      from = p.lane >> 2;
-    }
-    // The square around the hexagon's centre.
-    {
-      const int k = g < 4 ? g : g + 1;  // the 3x3 square without its centre
-      dx = bxm + k % 3 - 1;
-      dy = bym + k / 3 - 1;
-      const bool ok = inwin(dx, dy);
-      nsad += __popc(__ballot_sync(kAll, ok && q == 0));
-      const Pick2 p = argmin(score(ok, dx, dy));
-      if (p.cost < bc) {
-        bc = p.cost;
-        bxm = __shfl_sync(kAll, dx, p.lane);
-        bym = __shfl_sync(kAll, dy, p.lane);
+      lv = (uint32_t)(uint16_t)(int16_t)bxm | (uint32_t)(uint16_t)(int16_t)bym << 16;
+      if (lane == 0) {
+        st_word(words + bx, lv);
+        const size_t o = (size_t)pi * n + (size_t)by * bw + bx;
+        *reinterpret_cast<uint32_t*>(mv_all + o) = lv;
+        nsad_all[o] = nsad;
       }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) s[r] = sn[r];
+      uw = un;
     }
-    // The winner's SATD: tile `lane` of the four (lanes 0..3).
-    uint32_t sat = 0;
-    if (lane < 4) {
-      const int tx = lane & 1, ty = lane >> 1;
-      sat = satd4x4_tile<S>(src + (ptrdiff_t)(ty * 4) * cur.stride + tx * 4, cur.stride,
-                            rb + (ptrdiff_t)(bym + ty * 4) * ref.stride + bxm + tx * 4, ref.stride);
-    }
-    sat += __shfl_xor_sync(kAll, sat, 1);
-    sat += __shfl_xor_sync(kAll, sat, 2);
-    if (lane == 0) {
-      cost[b] = sat;
-      mv[b].x = (int16_t)bxm;
-      mv[b].y = (int16_t)bym;
-      if (nsad_out) nsad_out[b] = nsad;
-      __threadfence();
-      st_release32(done + b, 1);
-    }
-    __syncwarp();
   }
 }
 
@@ -518,16 +614,19 @@ __global__ void lowres_bi_h264_kernel(LowresDesc cur, LowresDesc r0, LowresDesc 
   cost[b] = satd8x8<S>(src, cur.stride, pred, 8);
 }
 
-// The wavefront's wait on a flag nothing sets, with a short poll limit:
+// The wavefront's wait on a word nothing publishes, with a short poll limit:
 // the failure path of a dependency that never completes, taken on purpose.
-__global__ void probe_wait_kernel(const int32_t* flag, uint32_t limit, uint32_t* status) {
-  if ((threadIdx.x & 31) == 0) wait_done(flag, 0, status, limit);
+__global__ void probe_wait_kernel(const unsigned long long* word, uint32_t limit, uint32_t* status) {
+  if ((threadIdx.x & 31) == 0) {
+    unsigned long long w = ld_word(word);
+    wait_word(word, w, status, false, limit);
+  }
 }
 
 }  // namespace
 
-cudaError_t launch_probe_wait(const int32_t* flag, uint32_t limit, uint32_t* status, cudaStream_t s) {
-  probe_wait_kernel<<<1, 32, 0, s>>>(flag, limit, status);
+cudaError_t launch_probe_wait(const unsigned long long* word, uint32_t limit, uint32_t* status, cudaStream_t s) {
+  probe_wait_kernel<<<1, 32, 0, s>>>(word, limit, status);
   return cudaGetLastError();
 }
 
@@ -554,17 +653,24 @@ cudaError_t launch_lowres_build(const DevPlanes& pic, int bd, int w, int h, cons
   return cudaGetLastError();
 }
 
-cudaError_t launch_lowres_search(const LowresDesc* pairs, int npairs, const LowresDesc& first, const int32_t* order,
-                                 int32_t* done, unsigned long long* counter, uint32_t* status, uint32_t* cost,
-                                 rme_mv* mv, uint32_t* nsad, int grid, cudaStream_t s) {
+cudaError_t launch_lowres_search(const LowresDesc* pairs, int npairs, const LowresDesc& first,
+                                 unsigned long long* words, unsigned long long* counter, uint32_t* status,
+                                 uint32_t* cost, rme_mv* mv, uint32_t* nsad, int max_ctas, cudaStream_t s) {
+  const int64_t rows = (int64_t)first.bh * npairs, tiles = (int64_t)first.bw * first.bh * npairs * 4;
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(max_ctas, (rows + kLaWarps - 1) / kLaWarps));
+  const unsigned cgrid = (unsigned)((tiles + 255) / 256);
   if (!first.h264)
-    lowres_search_kernel<<<grid, 256, 0, s>>>(pairs, npairs, order, done, counter, status, cost, mv, nsad);
+    lowres_search_kernel<<<grid, kLaWarps * 32, 0, s>>>(pairs, npairs, words, counter, status, mv, nsad);
   else if (first.bytes == 1)
-    lowres_search_h264_kernel<uint8_t>
-        <<<grid, 256, 0, s>>>(pairs, npairs, order, done, counter, status, cost, mv, nsad);
+    lowres_search_h264_kernel<uint8_t><<<grid, kLaWarps * 32, 0, s>>>(pairs, npairs, words, counter, status, mv, nsad);
   else
-    lowres_search_h264_kernel<uint16_t>
-        <<<grid, 256, 0, s>>>(pairs, npairs, order, done, counter, status, cost, mv, nsad);
+    lowres_search_h264_kernel<uint16_t><<<grid, kLaWarps * 32, 0, s>>>(pairs, npairs, words, counter, status, mv, nsad);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  if (first.bytes == 1)
+    lowres_cost_kernel<uint8_t><<<cgrid, 256, 0, s>>>(pairs, npairs, mv, cost);
+  else
+    lowres_cost_kernel<uint16_t><<<cgrid, 256, 0, s>>>(pairs, npairs, mv, cost);
   return cudaGetLastError();
 }
 

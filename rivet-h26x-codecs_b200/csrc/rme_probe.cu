@@ -54,7 +54,7 @@ extern "C" int rme_probe_int_peak(int32_t device, double* ops_per_s) {
 }
 
 // The failure path of the library's bounded waits, taken on purpose: a wait
-// on a flag that nothing sets gives up after `polls` polls and reports it in
+// on a word that nothing publishes gives up after `polls` polls and reports it in
 // the status word, and the device stays usable.
 extern "C" int rme_probe_wait_timeout(int32_t device, uint32_t polls, uint32_t* status, double* seconds) {
   if (!status || polls == 0 || polls > (1u << 22)) return RME_EINVAL;
@@ -68,7 +68,7 @@ extern "C" int rme_probe_wait_timeout(int32_t device, uint32_t polls, uint32_t* 
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0);
-    if (rme::launch_probe_wait(flag, polls, st, nullptr) == cudaSuccess && cudaEventRecord(e1) == cudaSuccess &&
+    if (rme::launch_probe_wait(reinterpret_cast<const unsigned long long*>(flag), polls, st, nullptr) == cudaSuccess && cudaEventRecord(e1) == cudaSuccess &&
         cudaMemcpy(status, st, sizeof(uint32_t), cudaMemcpyDeviceToHost) == cudaSuccess) {
       float ms = 0.0f;
       cudaEventElapsedTime(&ms, e0, e1);

@@ -38,3 +38,26 @@ def test_weighted_refine_part_edges(ms, bd, cross):
     ms.release(2200)
     ms.release(2201)
 
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("codec,bd", [(HEVC, 8), (HEVC, 12), (H264, 8), (H264, 12)])
+@pytest.mark.parametrize("w,h", [(16, 16), (16, 210), (403, 16), (83, 75)])
+def test_lowres_rows_of_every_shape(ms, codec, bd, w, h):
+    """One block, one column, one row of blocks, ragged sides; still, even
+    and torn motion (the first pass's rings known or not), several pairs."""
+    rng = np.random.default_rng(w * h + bd)
+    pics = [random_picture(rng, w, h, bd, smooth=2)]
+    pics.append(shifted(pics[0], 4, -2))
+    torn = shifted(pics[0], -7, 5, rng, 2.0)
+    torn[: h // 2] = shifted(pics[0], 12, 9)[: h // 2]
+    pics.append(torn)
+    for i, pic in enumerate(pics):
+        ms.upload(2400 + i, pic, codec, bd, as_ref=False)
+        ms.lowres_build(2400 + i)
+    pairs = [(1, 0), (2, 0), (0, 0), (2, 1), (0, 2)]
+    got = ms.lowres_search_batch([(2400 + a, 2400 + b) for a, b in pairs])
+    for (a, b), g in zip(pairs, got):
+        for x, y, name in zip(g, oracle.lowres_search(pics[a], pics[b], bd, codec), ("cost", "mv", "nsad")):
+            np.testing.assert_array_equal(x, y, f"{name} of {a} against {b}")
+    for i in range(3):
+        ms.release(2400 + i)
