@@ -186,7 +186,8 @@ struct Deps {  // the dependency structure of one frame shape
   std::vector<uint32_t> ready;   // tasks that read none, in order
   uint32_t* d_ready = nullptr;   // device copy of `ready` (the resident engine publishes from it)
   size_t ntasks = 0;
-  // The row form (HEVC without AMP): the rows a warp runs (16x16 and 8x8)
+  // The row form. H.264: the rows of macroblocks, top to bottom (`rows`).
+  // HEVC without AMP: the rows a warp runs (16x16 and 8x8)
   // and the rows a CTA runs (64x64 and 32x32), as row_entry words, each
   // list ordered by the row's first sample row, larger blocks first: every
   // row comes after the rows it reads (its upper row, its parents' rows).
@@ -257,6 +258,7 @@ struct Slot {
 struct Ctx {
   int device = 0, nsm = 0;
   int bps[kParts][kSearchVariants][2] = {};  // resident search blocks per SM, per part, variant, form
+  int hrow_bps[2][RME_MAX_REFS] = {};        // H.264's row form: per sample width and references
   // The tuner: per (part, form, log2 of its task count), each launch shape
   // of that class (kShapes) is timed on one real launch, then the fastest is
   // kept. Results do not depend on the shape.
@@ -450,6 +452,7 @@ const Deps* get_deps(Ctx* c, const rme_picture_desc& d, const rme_params* p, int
     for (int my = 0; my < mbh; ++my)
       for (int mx = 0; mx < mbw; ++mx)
         pend.push_back((mx > 0) + (my > 0) + (my > 0 && mx + 1 < mbw) + (mx > 0 && my > 0));
+    for (int my = 0; my < mbh; ++my) dp.rows.push_back((uint32_t)my);
   } else {
     int sizes[4];
     const int nl = level_sizes(p, sizes);
@@ -732,7 +735,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   CK(sl.d_misc.ensure(kMiscWords));
   if (!dev_out && !pinned_out) CK(sl.h_out.ensure(std::max<int64_t>(total, 1)));
   CK(sl.h_misc.ensure(kMiscWords));
-  if (sl.epoch == 0 || sl.epoch == 0xffffffffu) {
+  if (sl.epoch == 0 || sl.epoch >= 0x3fffffffu) {  // 30 bits: an H.264 word's tag holds a reference beside it
     CK(cudaMemsetAsync(sl.d_ready.p, 0, sl.d_ready.n * sizeof(unsigned long long), s));
     CK(cudaMemsetAsync(sl.d_mvf.p, 0, sl.d_mvf.n * sizeof(unsigned long long), s));
     sl.epoch = 0;
@@ -750,7 +753,19 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   // blocks of HEVC STANDALONE frames together.
   const bool spec = total <= kSpecTasks;
   int64_t part_tasks[kParts] = {0, 0, 0, 0};
-  for (int i = 0; i < n; ++i) part_tasks[part_of(sl.h_frames.p[i])] += ntask[i];
+  // H.264 parts whose frames are all STANDALONE run their row form whatever
+  // the launch's size: against the best shape of the dataflow form it took
+  // 0.53 against 1.60 ms for one CIF frame and 0.86 against 2.49 ms for a
+  // hundred, 9.6 against 14.7 ms for 64 720p frames of two references, 20.4
+  // against 27.4 ms for 24 1080p 10-bit frames of three.
+  bool hrows[kParts] = {false, true, false, true};
+  int hrows_nref[kParts] = {0, 0, 0, 0};
+  for (int i = 0; i < n; ++i) {
+    const int k = part_of(sl.h_frames.p[i]);
+    part_tasks[k] += ntask[i];
+    hrows[k] = hrows[k] && params[i].predictor_mode == RME_PRED_STANDALONE;
+    hrows_nref[k] = std::max(hrows_nref[k], (int)frames[i].nref);
+  }
   // Each part's launch shape: the tuned one for its class, or the next one
   // to time (a launch of one kind only, so that its time is the part's).
   int nparts_used = 0;
@@ -763,7 +778,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     const Shape* shapes = !spec ? kThroughputShapes : part_codec(k) == RME_CODEC_HEVC ? kLatencyHevcShapes : kLatencyShapes;
     const int nsh = kNumShapes[!spec ? 0 : part_codec(k) == RME_CODEC_HEVC ? 1 : 2];
     shape[k] = shapes[0];
-    if (part_tasks[k] > 0 && c->tune_on) {
+    if (part_tasks[k] > 0 && c->tune_on && !hrows[k]) {
       const int bucket = 63 - __builtin_clzll((unsigned long long)part_tasks[k]);
       Ctx::Tune& T = c->tune[{k * 2 + spec, bucket}];
       if (T.best >= 0) {
@@ -775,14 +790,14 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
       }
     }
     variant[k] = shape[k].variant;
-    if (part_tasks[k] > 0 && !c->bps[k][variant[k]][spec])
+    if (part_tasks[k] > 0 && !hrows[k] && !c->bps[k][variant[k]][spec])
       c->bps[k][variant[k]][spec] = search_blocks_per_sm(part_bytes(k), part_codec(k), variant[k], spec);
   }
-  // The row form, for a part of the latency form whose frames are all HEVC
-  // STANDALONE without AMP when its shape asks for it.
+  // The row form: H.264's, and, for a part of the latency form whose frames
+  // are all HEVC STANDALONE without AMP, HEVC's when its shape asks for it.
   bool rows[kParts] = {false, false, false, false};
   std::vector<const Deps*> fdeps(n, nullptr);
-  for (int k = 0; k < kParts; ++k) rows[k] = spec && part_tasks[k] > 0 && shape[k].rows;
+  for (int k = 0; k < kParts; ++k) rows[k] = part_tasks[k] > 0 && (hrows[k] || (spec && shape[k].rows));
   for (int i = 0; i < n; ++i) {
     const FrameDesc& fd = sl.h_frames.p[i];
     if (params[i].predictor_mode == RME_PRED_STANDALONE) {
@@ -792,7 +807,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
       fdeps[i] = get_deps(c, src->d, &params[i], frames[i].nref, &rc);
       if (!fdeps[i]) return rc;
     }
-    if (fd.codec != RME_CODEC_HEVC || params[i].predictor_mode != RME_PRED_STANDALONE || fd.amp != 0)
+    if (fd.codec == RME_CODEC_HEVC && (params[i].predictor_mode != RME_PRED_STANDALONE || fd.amp != 0))
       rows[part_of(fd)] = false;
   }
   int64_t rows_small[kParts] = {0, 0, 0, 0}, rows_large[kParts] = {0, 0, 0, 0};
@@ -818,7 +833,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
       // frames' rows below); a search of this buffer tags its words anew.
       const Deps* dp = fdeps[i];
       fd.mvf = sl.d_mvf.p + toff[i];
-      fd.tag = sl.epoch;
+      fd.tag = hrows[part] ? sl.epoch << 2 : sl.epoch;
       fd.nrows = (int32_t)(dp->rows.size() + dp->rows_big.size());
       rows_small[part] += (int64_t)dp->rows.size();
       rows_large[part] += (int64_t)dp->rows_big.size();
@@ -933,6 +948,13 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   int grid[kParts] = {0, 0, 0, 0};
   for (int k = 0; k < kParts; ++k) {
     if (part_tasks[k] == 0) continue;
+    if (hrows[k]) {
+      int& bps = c->hrow_bps[k / 2][hrows_nref[k] - 1];
+      if (!bps) bps = h264_row_blocks_per_sm(part_bytes(k), hrows_nref[k]);
+      grid[k] = (int)std::min<int64_t>(rows_small[k], (int64_t)c->nsm * bps);
+      sig.push_back(-2);
+      continue;
+    }
     const int cap = c->nsm * c->bps[k][variant[k]][spec];
     int64_t big = 0;
     if (spec && part_codec(k) == RME_CODEC_HEVC)
@@ -986,7 +1008,8 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
       cudaStream_t sk = j == 0 ? s : c->aux[j];
       if (j > 0) e = cudaStreamWaitEvent(sk, c->ev_fork, 0);
       if (e == cudaSuccess)
-        e = launch_search(Ls[k], part_bytes(k), part_codec(k), variant[k], grid[k], sk, spec);
+        e = hrows[k] ? launch_h264_rows(Ls[k], part_bytes(k), hrows_nref[k], grid[k], sk)
+                     : launch_search(Ls[k], part_bytes(k), part_codec(k), variant[k], grid[k], sk, spec);
       if (e == cudaSuccess && j > 0) e = cudaEventRecord(c->ev_join[j], sk);
     }
     for (int j = 1; j < nparts && e == cudaSuccess; ++j) e = cudaStreamWaitEvent(s, c->ev_join[j], 0);

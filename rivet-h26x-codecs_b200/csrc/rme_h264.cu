@@ -1,0 +1,527 @@
+// The H.264 STANDALONE search in its row form: a CTA owns a row of
+// macroblocks and searches it left to right, four warps per reference.
+//
+// What a macroblock's search computes is p_mb's search section
+// (h264_analyse.rs:1884-1975), as h264_task does it with one warp: the
+// neighbours' vectors as candidates, Search::int_search and Search::refine
+// (h264_hpel.rs:789-1021) per reference, the reference of least cost. Its
+// candidates, order, tie-breaks and counts are the same.
+//
+// Macroblocks form a wavefront (A, B, C and D neighbours), so a picture is a
+// chain of mbw + 2 mbh macroblocks and bound by one macroblock's latency.
+// Against one warp per macroblock (the dataflow form):
+//   - a reference has four warps, eight lanes per candidate: up to sixteen
+//     candidates of a step at once, two rows (SAD) or two 4x4 tiles (SATD) a
+//     lane, one named barrier a step;
+//   - references are searched side by side, each by its own four warps; the
+//     refine_ratio gate, the only tie between them, needs the whole-sample
+//     costs alone, one CTA barrier;
+//   - a hexagon step also scores the square around the same centre, which is
+//     the walk's last step when the hexagon has settled;
+//   - the UMH points are scored without a decision between them: no two of
+//     them coincide and none is the start, so the one point the reference
+//     leaves out, the best so far, is never among them, and the outcome is
+//     the least cost, first reached;
+//   - a neighbour's result is one published word (tag, reference, vector),
+//     loaded a macroblock ahead, and the next source block is staged behind
+//     the search.
+// Measured on one B200, the search kernel alone, the dataflow form first:
+// CIF, one reference, medium tier 1.60 -> 0.53 ms; 1080p, three references,
+// UMH +-24 28.3 -> 4.5 ms; 64 720p pictures of two references in one launch
+// 14.7 -> 9.6 ms.
+#include <algorithm>
+
+#include "rme_search_impl.cuh"
+
+namespace rme {
+namespace {
+
+constexpr int kRefThreads = 128;  // threads per reference
+constexpr int kSlots16 = 16;      // candidates a step scores at once
+
+struct RefResult {
+  uint32_t cost, satd, icost;
+  int mx, my, imx, imy;
+};
+
+template <class S>
+struct RowSmem {
+  uint32_t src[2][16 * 16 * sizeof(S) / 4];
+  uint32_t cost[RME_MAX_REFS][2][kSlots16];
+  uint32_t best[RME_MAX_REFS][4][2];  // UMH: each warp's least cost and its point
+  uint32_t icost[2][RME_MAX_REFS];    // whole-sample costs, reference cost included
+  RefResult fin[2][RME_MAX_REFS];
+  uint32_t nsad[2], nsatd[2];
+  uint32_t entry;
+};
+
+// A macroblock's published word: the launch's tag in bits 34..63, the
+// reference in 32..33, the vector in the low half.
+__device__ __forceinline__ bool row_word_ok(unsigned long long w, uint32_t tag) {
+  return ((uint32_t)(w >> 32) & ~3u) == tag;
+}
+// Waits (bounded, as wait_word) for a word already loaded once; false once
+// the wait has run out, after which the caller waits no more.
+__device__ __noinline__ bool wait_row_word(const LaunchDesc& L, const unsigned long long* p, uint32_t tag,
+                                           unsigned long long& w, bool lost) {
+  uint32_t ns = 32;
+  for (uint32_t it = 0; !row_word_ok(w, tag); ++it) {
+    if (lost || it >= kSpinLimit) {
+      if (!lost) atomicOr(L.status, kStatusWaitTimeout);
+      w = (unsigned long long)tag << 32;
+      return false;
+    }
+    if (it >= 16) {
+      __nanosleep(ns);
+      if (ns < 256) ns <<= 1;
+    }
+    w = ld_relaxed64(p);
+  }
+  return true;
+}
+
+// One reference's search of a macroblock, by the 128 threads of its group.
+template <class S>
+struct RefSearch {
+  static constexpr int WR = 16 * (int)sizeof(S) / 4;  // words of a source row
+  RowSmem<S>& sm;
+  const uint32_t* src;
+  const DevPlanes R;  // copies: the barriers between steps would have them read again
+  const uint16_t* tab;
+  const int range, umh, dia, qpel_diamond;
+  H264Blk B;
+  const S* org;
+  int g, warp, lane, sub, slot;  // group; warp in it; this lane's part of candidate `slot`
+  int buf = 0;
+  uint32_t nsad = 0, nsatd = 0;  // this warp's candidates
+
+  __device__ __forceinline__ void sync() { asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(kRefThreads) : "memory"); }
+
+  // The candidate's SAD over its eight lanes (rows sub and sub + 8).
+  __device__ __forceinline__ uint32_t sad(bool ok, int fx, int fy) {
+    uint32_t acc = 0;
+    if (ok) {
+      const S* rp = org + (ptrdiff_t)(fy + sub) * R.stride + fx;
+      uint32_t a[WR], b[WR];
+      ldwords<WR>(rp, a);
+      ldwords<WR>(rp + (ptrdiff_t)8 * R.stride, b);
+#pragma unroll
+      for (int k = 0; k < WR; ++k) acc += vsad(src[sub * WR + k], a[k], S()) + vsad(src[(sub + 8) * WR + k], b[k], S());
+    }
+    acc += __shfl_xor_sync(kFull, acc, 4);
+    acc += __shfl_xor_sync(kFull, acc, 2);
+    acc += __shfl_xor_sync(kFull, acc, 1);
+    return acc;
+  }
+  // Every slot's cost to every lane: lane l of each warp gets slot l's (none
+  // beyond the sixteenth).
+  __device__ __forceinline__ uint32_t share(uint32_t cost) {
+    uint32_t* c = sm.cost[g][buf];
+    buf ^= 1;
+    if (sub == 0) c[slot] = cost;
+    sync();
+    return lane < kSlots16 ? c[lane] : kInf;
+  }
+  __device__ __forceinline__ uint32_t rate(int qx, int qy) {
+    const int dx = min(max(qx - B.px, -kMvSpan), kMvSpan), dy = min(max(qy - B.py, -kMvSpan), kMvSpan);
+    return (uint32_t)__ldg(&tab[dx + kMvSpan]) + (uint32_t)__ldg(&tab[dy + kMvSpan]);
+  }
+  __device__ __forceinline__ uint32_t count(bool yes) { return __popc(__ballot_sync(kFull, yes && sub == 0)); }
+
+  // Search::int_search: lane k + 1 of every warp holds candidate k of ncand.
+  __device__ __forceinline__ void whole(int ncand, int cand_x, int cand_y, int& imx, int& imy, uint32_t& icost) {
+    const int pxr = min(max((B.px + 2) >> 2, B.lx), B.hx), pyr = min(max((B.py + 2) >> 2, B.ly), B.hy);
+    const int qx = lane == 0 ? pxr : min(max((cand_x + 2) >> 2, B.lx), B.hx);
+    const int qy = lane == 0 ? pyr : min(max((cand_y + 2) >> 2, B.ly), B.hy);
+    // A candidate on the predictor's point or an earlier candidate's is
+    // skipped (`tried`).
+    bool skip = lane > 0 && qx == pxr && qy == pyr;
+#pragma unroll
+    for (int j = 1; j <= 8; ++j) {
+      const int ox = __shfl_sync(kFull, qx, j), oy = __shfl_sync(kFull, qy, j);
+      skip |= j < lane && ox == qx && oy == qy;
+    }
+    const uint32_t keep = __ballot_sync(kFull, lane <= ncand && !skip);
+    int bx, by;
+    uint32_t bcost;
+    {
+      const bool ok = (keep >> slot) & 1u;
+      const int fx = __shfl_sync(kFull, qx, slot), fy = __shfl_sync(kFull, qy, slot);
+      const uint32_t s = sad(ok, fx, fy);
+      nsad += count(ok);
+      const Pick p = warp_min(share(ok ? s + rate(fx * 4, fy * 4) : kInf));
+      bcost = p.cost;
+      bx = __shfl_sync(kFull, qx, p.lane);
+      by = __shfl_sync(kFull, qy, p.lane);
+    }
+    const int x0 = max(bx - range, B.lx), x1 = min(bx + range, B.hx), y0 = max(by - range, B.ly),
+              y1 = min(by + range, B.hy);
+    auto inside = [&](int x, int y) { return x >= x0 && x <= x1 && y >= y0 && y <= y1; };
+    if (umh) {
+      const int cx = bx, cy = by, ncross = 4 * (range / 2), total = ncross + 12 * (range / 4);
+      auto point = [&](int i, int& x, int& y) {
+        if (i < ncross) {
+          const int rr = 2 * (i / 4 + 1), k = i & 3;
+          x = cx + (k == 0 ? -rr : k == 1 ? rr : 0);
+          y = cy + (k == 2 ? -rr : k == 3 ? rr : 0);
+        } else {
+          const int j = i - ncross, rr = 4 * (j / 12 + 1), k = j % 12;
+          x = cx + c_hex12[k][0] * rr / 2;
+          y = cy + c_hex12[k][1] * rr / 2;
+        }
+      };
+      uint32_t mc = kInf, mi = 0xffffffffu;  // this lane's least cost, its first point
+#pragma unroll 2
+      for (int i0 = 0; i0 < total; i0 += kSlots16) {
+        const int i = i0 + slot;
+        int x = 0, y = 0;
+        if (i < total) point(i, x, y);
+        const bool ok = i < total && inside(x, y);
+        const uint32_t s = sad(ok, x, y);
+        nsad += count(ok);
+        const uint32_t c = ok ? s + rate(x * 4, y * 4) : kInf;
+        if (c < mc) {
+          mc = c;
+          mi = (uint32_t)i;
+        }
+      }
+      uint32_t m = __reduce_min_sync(kFull, mc);
+      uint32_t at = __reduce_min_sync(kFull, mc == m ? mi : 0xffffffffu);
+      if (lane == 0) {
+        sm.best[g][warp][0] = m;
+        sm.best[g][warp][1] = at;
+      }
+      sync();
+      const uint32_t wm = lane < 4 ? sm.best[g][lane][0] : kInf, wi = lane < 4 ? sm.best[g][lane][1] : 0xffffffffu;
+      m = __reduce_min_sync(kFull, wm);
+      at = __reduce_min_sync(kFull, wm == m ? wi : 0xffffffffu);
+      if (m < bcost) {
+        bcost = m;
+        point((int)at, bx, by);
+      }
+    }
+    // A step's points around the best: offset of slot k.
+    if (dia) {
+      for (int it = 0; it < range; ++it) {
+        auto off = [](int k, int& ox, int& oy) {
+          ox = k == 0 ? -1 : k == 1 ? 1 : 0;
+          oy = k == 2 ? -1 : k == 3 ? 1 : 0;
+        };
+        int ox, oy;
+        off(slot, ox, oy);
+        const bool ok = slot < 4 && inside(bx + ox, by + oy);
+        const uint32_t s = sad(ok, bx + ox, by + oy);
+        nsad += count(ok);
+        const Pick p = warp_min(share(ok ? s + rate((bx + ox) * 4, (by + oy) * 4) : kInf));
+        if (!(p.cost < bcost)) break;
+        bcost = p.cost;
+        off(p.lane, ox, oy);
+        bx += ox;
+        by += oy;
+      }
+    } else {
+      // Slots 0..5 the hexagon (after a step in direction d only d - 1, d,
+      // d + 1 are new, in that order), 6..13 the square.
+      int dir = -1;
+      for (int it = 0;; ++it) {
+        auto off = [&](int k, int& ox, int& oy) {
+          if (k < 6) {
+            const int e = dir < 0 ? k : k == 0 ? (dir + 5) % 6 : k == 1 ? dir : (dir + 1) % 6;
+            ox = c_hex[e][0];
+            oy = c_hex[e][1];
+          } else {
+            ox = c_sq[k - 6][0];
+            oy = c_sq[k - 6][1];
+          }
+        };
+        const int nhex = it == 0 ? 6 : it < range ? 3 : 0;
+        int ox = 0, oy = 0;
+        if (slot < 14) off(slot, ox, oy);
+        const bool ok = (slot < 6 ? slot < nhex : slot < 14) && inside(bx + ox, by + oy);
+        const uint32_t s = sad(ok, bx + ox, by + oy);
+        nsad += count(ok && slot < 6);
+        const uint32_t c = share(ok ? s + rate((bx + ox) * 4, (by + oy) * 4) : kInf);
+        Pick p = warp_min(lane < 6 ? c : kInf);
+        const bool step = p.cost < bcost;
+        if (!step) {
+          nsad += count(ok && slot >= 6);
+          p = warp_min(lane >= 6 ? c : kInf);
+        }
+        if (p.cost < bcost) {
+          bcost = p.cost;
+          off(p.lane, ox, oy);
+          bx += ox;
+          by += oy;
+        }
+        if (!step) break;
+        dir = dir < 0 ? p.lane : p.lane == 0 ? (dir + 5) % 6 : p.lane == 1 ? dir : (dir + 1) % 6;
+      }
+    }
+    imx = bx * 4;
+    imy = by * 4;
+    icost = bcost;
+  }
+
+  // Search::refine from (smx, smy), as h264_refine: the start with the first
+  // ring in one step.
+  __device__ __forceinline__ void refine(int smx, int smy, int hpel, int qpel, int& omx, int& omy, uint32_t& osatd,
+                                         uint32_t& ocost) {
+    const int qlx = B.lx * 4, qhx = B.hx * 4, qly = B.ly * 4, qhy = B.hy * 4;
+    int bmx = smx, bmy = smy;
+    uint32_t bsatd = 0, bc = kInf;
+    bool first = true;
+    for (int s = 0; s < 2; ++s) {
+      const int step = s == 0 ? 2 : 1, iters = s == 0 ? hpel : qpel;
+      const int pts = (step == 1 && qpel_diamond) ? 4 : 8;
+      bool has_prev = false;
+      int prevx = 0, prevy = 0;
+      for (int it = 0; it < iters || first; ++it) {
+        const int cmx = bmx, cmy = bmy;
+        const bool ring = it < iters;
+        const int base = first ? 1 : 0, n = base + (ring ? pts : 0);
+        auto vec = [&](int c, int& mx, int& my) {  // slot c's vector
+          mx = cmx;
+          my = cmy;
+          if (c >= base) {
+            mx = (int)(int16_t)(cmx + c_ring[(c - base) & 7][0] * step);
+            my = (int)(int16_t)(cmy + c_ring[(c - base) & 7][1] * step);
+          }
+        };
+        int mx, my;
+        vec(slot, mx, my);
+        bool ok = slot < n;
+        if (slot >= base)
+          ok = ok && mx >= qlx && mx <= qhx && my >= qly && my <= qhy &&
+               !(has_prev && abs(mx - prevx) <= step && abs(my - prevy) <= step);
+        uint32_t sv = 0;
+        if (ok) {
+          const int xi = B.x + (mx >> 2), yi = B.y + (my >> 2);
+          const int8_t* q = c_h264_qpel[(my & 3) * 4 + (mx & 3)];
+          const S* p1 = plane_at<S>(R, q[0], xi + q[1], yi + q[2]);
+          const S* p2 = q[3] < 0 ? nullptr : plane_at<S>(R, q[3], xi + q[4], yi + q[5]);
+          sv = satd_strips<S, 2>(src, WR, 4, 4, p1, p2, R.stride, 8, sub);
+        }
+        sv += __shfl_xor_sync(kFull, sv, 4);
+        sv += __shfl_xor_sync(kFull, sv, 2);
+        sv += __shfl_xor_sync(kFull, sv, 1);
+        nsatd += count(ok);
+        const Pick p = warp_min(share(ok ? sv + rate(mx, my) : kInf));
+        if (p.cost < bc) {
+          bc = p.cost;
+          vec(p.lane, bmx, bmy);
+          bsatd = bc - rate(bmx, bmy);
+        }
+        first = false;
+        if (!ring) break;
+        if (bmx == cmx && bmy == cmy) break;
+        prevx = cmx;
+        prevy = cmy;
+        has_prev = true;
+      }
+    }
+    omx = bmx;
+    omy = bmy;
+    osatd = bsatd;
+    ocost = bc;
+  }
+};
+
+template <class S>
+__device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSmem<S>& sm, int tid, bool& lost,
+                         unsigned long long (&cnt)[3]) {
+  constexpr int WR = RefSearch<S>::WR, NSRC = 16 * WR;
+  const int lane = tid & 31, g = tid >> 7, warp = (tid >> 5) & 3;
+  const int mbw = F.width / 16, nref = F.nref;
+  const uint32_t tag = F.tag;
+  const unsigned long long* up = F.mvf + (ptrdiff_t)(my - 1) * mbw;
+  auto load_src = [&](int mx) -> uint32_t {  // word tid of the macroblock's rows (16-byte aligned rows)
+    const S* o = plane_at<S>(F.src, 0, mx * 16, my * 16 + tid / WR);
+    return RME_LD32(reinterpret_cast<const uint32_t*>(o) + tid % WR);
+  };
+  if (tid < NSRC) sm.src[0][tid] = load_src(0);
+  if (tid < 2) sm.nsad[tid] = sm.nsatd[tid] = 0u;
+  unsigned long long wd = 0, wb = 0, wc = 0;  // the D, B and C macroblocks' words
+  if (my > 0) {
+    wb = ld_relaxed64(up);
+    if (mbw > 1) wc = ld_relaxed64(up + 1);
+    if (!wait_row_word(L, up, tag, wb, lost)) lost = true;
+    __syncwarp();
+  }
+  Nb A{false, -1, 0, 0};
+  __syncthreads();
+  for (int mx = 0; mx < mbw; ++mx) {
+    const int par = mx & 1;
+    const bool has_c = my > 0 && mx + 1 < mbw;
+    if (has_c && !wait_row_word(L, up + mx + 1, tag, wc, lost)) lost = true;
+    __syncwarp();
+    // The next macroblock's C word and source, on their way during the search.
+    unsigned long long wn = 0;
+    if (my > 0 && mx + 2 < mbw) wn = ld_relaxed64(up + mx + 2);
+    uint32_t nsrc = 0;
+    if (tid < NSRC && mx + 1 < mbw) nsrc = load_src(mx + 1);
+    auto nb = [](bool avail, unsigned long long w) {
+      Nb m{false, -1, 0, 0};
+      if (avail) {
+        m.avail = true;
+        m.ref = (int)((w >> 32) & 3u);
+        m.x = mvx_of((uint32_t)w);
+        m.y = mvy_of((uint32_t)w);
+      }
+      return m;
+    };
+    const Nb Bn = nb(my > 0, wb), C = nb(has_c, wc), D = nb(my > 0 && mx > 0, wd);
+    const Nb Cc = C.avail ? C : D;
+    if (g < nref) {
+      // p_skip_mv, then cands = [skip_mv, 0, distinct A, B, C] and a further
+      // reference's own predictor: lane k + 1 holds candidate k.
+      int skx = 0, sky = 0;
+      if (A.avail && Bn.avail && !(A.ref == 0 && A.x == 0 && A.y == 0) && !(Bn.ref == 0 && Bn.x == 0 && Bn.y == 0))
+        median_mvp(A, Bn, Cc, 0, skx, sky);
+      auto same = [](const Nb& p, const Nb& q) { return p.x == q.x && p.y == q.y; };
+      const bool va = A.avail, vb = Bn.avail && !(va && same(A, Bn)),
+                 vc = C.avail && !(va && same(A, C)) && !(vb && same(Bn, C));
+      const int ia = 2, ib = ia + va, ic = ib + vb, nc = ic + vc, k = lane - 1;
+      int prx, pry;
+      median_mvp(A, Bn, Cc, g, prx, pry);
+      int cx = 0, cy = 0;
+      if (k == 0) {
+        cx = skx;
+        cy = sky;
+      } else if (va && k == ia) {
+        cx = A.x;
+        cy = A.y;
+      } else if (vb && k == ib) {
+        cx = Bn.x;
+        cy = Bn.y;
+      } else if (vc && k == ic) {
+        cx = C.x;
+        cy = C.y;
+      } else if (g > 0 && k == nc) {
+        cx = prx;
+        cy = pry;
+      }
+      RefSearch<S> q{sm, sm.src[par], F.ref[g], F.tab, F.range, F.umh, F.dia, F.qpel_diamond};
+      q.g = g;
+      q.warp = warp;
+      q.lane = lane;
+      q.sub = lane & 7;
+      q.slot = warp * 4 + (lane >> 3);
+      H264Blk& B = q.B;
+      B.x = mx * 16;
+      B.y = my * 16;
+      B.w = B.h = 16;
+      B.px = prx;
+      B.py = pry;
+      B.lx = 4 - F.pad - B.x;  // search_bounds (h264_hpel.rs:476-488)
+      B.hx = F.width + F.pad - 20 - B.x;
+      B.ly = max(4 - F.pad - B.y, -F.vr);
+      B.hy = min(F.height + F.pad - 20 - B.y, F.vr);
+      q.org = plane_at<S>(q.R, 0, B.x, B.y);
+      RefResult r;
+      uint32_t ic0;
+      q.whole(nc + (g > 0), cx, cy, r.imx, r.imy, ic0);
+      r.icost = ic0 + F.ref_cost[g];
+      bool gate = false;
+      if (nref > 1) {
+        // refine_ratio: a further reference whose whole-sample cost is that
+        // factor of the best before it is only scored.
+        if ((tid & (kRefThreads - 1)) == 0) sm.icost[par][g] = r.icost;
+        asm volatile("bar.sync 8, %0;" ::"r"(nref * kRefThreads) : "memory");
+        uint32_t before = kInf;
+        for (int p = 0; p < g; ++p) before = min(before, sm.icost[par][p]);
+        gate = g > 0 && F.refine_ratio > 0.0f &&
+               __uint2float_rn(r.icost) >= __fmul_rn(F.refine_ratio, __uint2float_rn(before));
+      }
+      q.refine(r.imx, r.imy, gate ? 0 : F.hpel_iters, gate ? 0 : F.qpel_iters, r.mx, r.my, r.satd, r.cost);
+      r.cost += F.ref_cost[g];
+      if ((tid & (kRefThreads - 1)) == 0) sm.fin[par][g] = r;
+      if (lane == 0) {
+        atomicAdd(&sm.nsad[par], q.nsad);
+        atomicAdd(&sm.nsatd[par], q.nsatd);
+      }
+    }
+    if (tid < NSRC) sm.src[par ^ 1][tid] = nsrc;
+    __syncthreads();
+    // The reference of least cost, the first reaching it (all threads).
+    int best = 0;
+    uint32_t c16 = sm.fin[par][0].cost;
+    for (int r = 1; r < nref; ++r)
+      if (sm.fin[par][r].cost < c16) {
+        c16 = sm.fin[par][r].cost;
+        best = r;
+      }
+    const RefResult& w = sm.fin[par][best];
+    A = Nb{true, best, (int)(int16_t)w.mx, (int)(int16_t)w.my};
+    if (tid == 0) {
+      const int t = my * mbw + mx;
+      st_relaxed64(F.mvf + t, mv_word(tag | (uint32_t)best, w.mx, w.my));
+      write_result(&F.out[t], w.mx, w.my, best, w.cost, w.satd, w.imx, w.imy, w.icost, sm.nsad[par], sm.nsatd[par], 0);
+      cnt[0] += 1;
+      cnt[1] += sm.nsad[par];
+      cnt[2] += sm.nsatd[par];
+      sm.nsad[par] = sm.nsatd[par] = 0u;
+    }
+    wd = wb;
+    wb = wc;
+    wc = wn;
+  }
+}
+
+// Rows are taken in the order the host pushed them (every frame's row 0,
+// then every row 1, ...), each after the row it reads, so a row's upper row
+// is always owned by a running CTA.
+template <class S>
+__global__ void __launch_bounds__(RME_MAX_REFS * kRefThreads) h264_row_kernel(LaunchDesc L) {
+  __shared__ RowSmem<S> sm;
+  const int tid = threadIdx.x;
+  const uint32_t epoch = __ldg(L.epoch);
+  bool lost = false;
+  unsigned long long cnt[3] = {0, 0, 0};
+  for (;;) {
+    __syncthreads();
+    if (tid == 0) {
+      const unsigned long long idx = atomicAdd(L.head, 1ull);
+      sm.entry = idx >= (unsigned long long)L.total ? kPopDone : pop_slot(L, idx, epoch);
+    }
+    __syncthreads();
+    const uint32_t e = sm.entry;
+    if (e == kPopDone) break;
+    if (e == 0xffffffffu) continue;  // the wait ran out (status set)
+    const FrameDesc& F = L.frames[e >> 24];
+    const int row = (int)(e & 0xffffffu);
+    if (F.codec != RME_CODEC_H264 || F.mode != RME_PRED_STANDALONE || (sizeof(S) == 1) != (F.bd == 8) ||
+        F.mvf == nullptr || row >= F.height / 16 || F.nref * kRefThreads > (int)blockDim.x) {
+      if (tid == 0) atomicOr(L.status, kStatusBadTask);
+      continue;
+    }
+    h264_row<S>(L, F, row, sm, tid, lost, cnt);
+  }
+  if (tid == 0) {
+    atomicAdd(&L.counters[0], cnt[0]);
+    atomicAdd(&L.counters[1], cnt[1]);
+    atomicAdd(&L.counters[2], cnt[2]);
+    atomicAdd(&L.counters[3], cnt[1] * 256ull);
+    atomicAdd(&L.counters[4], cnt[2] * 256ull);
+  }
+}
+
+}  // namespace
+
+int h264_row_blocks_per_sm(int bytes_per_sample, int nref) {
+  int n = 0;
+  const cudaError_t e =
+      bytes_per_sample == 1
+          ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, h264_row_kernel<uint8_t>, nref * kRefThreads, 0)
+          : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, h264_row_kernel<uint16_t>, nref * kRefThreads, 0);
+  return e == cudaSuccess && n > 0 ? n : 1;
+}
+
+cudaError_t launch_h264_rows(const LaunchDesc& L, int bytes_per_sample, int nref, int grid, cudaStream_t s) {
+  if (bytes_per_sample == 1)
+    h264_row_kernel<uint8_t><<<grid, nref * kRefThreads, 0, s>>>(L);
+  else
+    h264_row_kernel<uint16_t><<<grid, nref * kRefThreads, 0, s>>>(L);
+  return cudaGetLastError();
+}
+
+}  // namespace rme

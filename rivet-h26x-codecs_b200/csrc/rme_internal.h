@@ -68,10 +68,12 @@ struct FrameDesc {
   uint32_t gen;  // the resident engine: this frame's generation in its slot
   int32_t big_end;  // HEVC STANDALONE: tasks below big_end * nref are blocks of 32 or more
   // The row form (HEVC STANDALONE without AMP, latency kernels and the
-  // engine): a warp or a CTA owns a row of one level and reference and
-  // searches its blocks left to right; per task its motion vector is
-  // published as one word, (tag << 32) | mv, which the rows below and the
-  // next size's rows wait for. Null: the dataflow form.
+  // engine; H.264 STANDALONE, rme_h264.cu): a warp or a CTA owns a row of one
+  // level and reference (H.264: of macroblocks) and searches its blocks left
+  // to right; per task its motion vector is published as one word,
+  // (tag << 32) | mv (H.264: the reference in the tag's two low bits), which
+  // the rows below and the next size's rows wait for. Null: the dataflow
+  // form.
   unsigned long long* mvf;
   uint32_t tag;     // nonzero, new for every search of the buffer (the launch's epoch, the slot's generation)
   int32_t nrows;    // rows of the frame, both kinds (the engine counts them to completion)
@@ -251,6 +253,12 @@ constexpr int kSearchVariants = 3, kDefaultVariant = 1;
 cudaError_t launch_search(const LaunchDesc& L, int bytes_per_sample, int codec, int variant, int grid,
                           cudaStream_t s, bool spec = false);
 int search_blocks_per_sm(int bytes_per_sample, int codec, int variant, bool spec = false);
+// H.264 STANDALONE frames in their row form (rme_h264.cu): L's queue holds
+// rows of macroblocks (all pushed by the host, each after the row above it),
+// the frames have `mvf`, a tag with its low two bits clear, and at most
+// `nref` references.
+cudaError_t launch_h264_rows(const LaunchDesc& L, int bytes_per_sample, int nref, int grid, cudaStream_t s);
+int h264_row_blocks_per_sm(int bytes_per_sample, int nref);
 cudaError_t launch_chroma(const void* cb, const void* cr, int bd, int codec, int cw, int ch, int cstride,
                           int nblocks, const int32_t* blocks, const rme_mv* mvs, const int64_t* out_off, void* out,
                           cudaStream_t s);

@@ -61,3 +61,51 @@ def test_lowres_rows_of_every_shape(ms, codec, bd, w, h):
             np.testing.assert_array_equal(x, y, f"{name} of {a} against {b}")
     for i in range(3):
         ms.release(2400 + i)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h,bd,nref,kw", [
+    (16, 16, 8, 1, {}), (16, 80, 10, 2, {}), (176, 16, 8, 4, dict(h264_umh=1)), (33, 47, 8, 3, {}),
+    (208, 144, 12, 4, dict(h264_umh=1, h264_range=37)), (208, 144, 8, 2, dict(h264_dia=1, h264_qpel_diamond=1)),
+    (208, 144, 8, 3, dict(h264_range=0, h264_refine_ratio=0.0)), (208, 144, 8, 2, dict(h264_range=1, h264_umh=1)),
+    (112, 96, 10, 3, dict(h264_hpel_iters=0, h264_qpel_iters=0)), (112, 96, 8, 3, dict(h264_vertical_range=3)),
+    (112, 96, 8, 2, dict(h264_pad=8, h264_hpel_iters=5, h264_qpel_iters=1))])
+def test_h264_rows_of_every_shape(ms, w, h, bd, nref, kw):
+    """One macroblock, one row, one column, ragged sides, every pattern and
+    the settings' ends, one to four references."""
+    rng = np.random.default_rng(w + h + nref)
+    refs = [random_picture(rng, w, h, bd)]
+    for k in range(1, nref):
+        refs.append(shifted(refs[0], 3 * k, -2 * k, rng, 2.0))
+    src = shifted(refs[-1], -5, 6, rng, 2.0)
+    src[: h // 2] = shifted(refs[0], 9, 2, rng, 1.0)[: h // 2]
+    for i, pic in enumerate(refs + [src]):
+        ms.upload(2500 + i, pic, H264, bd, as_ref=i < nref)
+    p = oracle.params(H264, 29, **kw)
+    got = ms.search(2500 + nref, [2500 + i for i in range(nref)], p)
+    assert_results_equal(got, oracle.frame_search(H264, bd, src, refs, p), "H.264 rows")
+    for i in range(nref + 1):
+        ms.release(2500 + i)
+
+
+@pytest.mark.gpu
+def test_h264_rows_of_uneven_frames_together(ms):
+    """Frames of different sizes, settings and reference counts in one
+    launch, beside a GIVEN-free HEVC frame: as each by itself."""
+    rng = np.random.default_rng(77)
+    frames, params, want = [], [], []
+    for k, (codec, w, h, nref) in enumerate([(H264, 96, 64, 1), (H264, 160, 48, 3), (HEVC, 128, 96, 2), (H264, 16, 96, 2)]):
+        refs = [random_picture(rng, w, h, 8) for _ in range(nref)]
+        src = shifted(refs[0], 2, 1, rng, 2.0)
+        base = 2600 + 10 * k
+        for i, pic in enumerate(refs + [src]):
+            ms.upload(base + i, pic, codec, 8)
+        frames.append((base + nref, [base + i for i in range(nref)]))
+        params.append(oracle.params(codec, 28, h264_umh=k & 1))
+        want.append(oracle.frame_search(codec, 8, src, refs, params[-1]))
+    for _ in range(4):  # the first calls, the capture, its replays
+        for g, w_ in zip(ms.search_batch(frames, params), want):
+            assert_results_equal(g, w_, "mixed rows")
+    for s, r in frames:
+        for i in [s] + r:
+            ms.release(i)
