@@ -142,7 +142,7 @@ __device__ void engine_group_loop(const LaunchDesc& L, const EngineCtl& E, unsig
   uint32_t cached_gen = 0;
   for (;;) {
     uint32_t e;
-    if (cont >= 0) {
+    if (cont != -1) {
       e = (uint32_t)cont;
     } else {
       if (tid == 0) {
@@ -210,7 +210,7 @@ __global__ void __maxnreg__(kEngineMaxRegs) engine_kernel(LaunchDesc L, EngineCt
   uint32_t cached_gen = 0;
   for (;;) {
     uint32_t e;
-    if (cont >= 0) {
+    if (cont != -1) {
       e = (uint32_t)cont;  // a task of the same frame: its descriptor is here already
     } else {
       e = 0;

@@ -71,7 +71,7 @@ __device__ void group_loop(const LaunchDesc& L, unsigned char* smem_raw) {
   __syncthreads();
   for (;;) {
     uint32_t e;
-    if (cont >= 0) {
+    if (cont != -1) {
       e = (uint32_t)cont;
     } else {
       if (tid == 0) {
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, MINB) search_kernel(Launc
   int cont = -1;  // a task the last one made ready, run next by this warp
   for (;;) {
     uint32_t e;
-    if (cont >= 0) {
+    if (cont != -1) {
       e = (uint32_t)cont;
     } else {
       unsigned long long idx = 0;

@@ -312,7 +312,7 @@ __device__ __forceinline__ int release_lanes(const LaunchDesc& L, const FrameDes
   const uint32_t m = __ballot_sync(kFull, ready && big == group);
   if (__ballot_sync(kFull, ready) == 0u) return cont;
   int keep = -1;
-  if (m != 0u && cont < 0 && (L.done != nullptr || L.ring_shift)) {
+  if (m != 0u && cont == -1 && (L.done != nullptr || L.ring_shift)) {
     keep = __ffs(m) - 1;
     cont = (f << 24) | __shfl_sync(kFull, dtask, keep);
   }

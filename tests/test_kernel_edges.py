@@ -109,3 +109,20 @@ def test_h264_rows_of_uneven_frames_together(ms):
     for s, r in frames:
         for i in [s] + r:
             ms.release(i)
+
+
+@pytest.mark.gpu
+def test_a_launch_of_more_than_128_dataflow_frames(ms):
+    """A task kept by the warp that made it ready is named by frame and task
+    in 32 bits: frames 128 and up set the top one."""
+    rng = np.random.default_rng(5)
+    ref = random_picture(rng, 64, 32, 8)
+    src = shifted(ref, 1, -2, rng, 2.0)
+    ms.upload(2700, ref, HEVC, 8)
+    ms.upload(2701, src, HEVC, 8)
+    p = oracle.params(HEVC, 32, hevc_amp=1)
+    want = oracle.frame_search(HEVC, 8, src, [ref], p)
+    for got in ms.search_batch([(2701, [2700])] * 200, p):
+        assert_results_equal(got, want, "frame of 200")
+    ms.release(2700)
+    ms.release(2701)
