@@ -186,12 +186,14 @@ struct Deps {  // the dependency structure of one frame shape
   std::vector<uint32_t> ready;   // tasks that read none, in order
   uint32_t* d_ready = nullptr;   // device copy of `ready` (the resident engine publishes from it)
   size_t ntasks = 0;
-  // The row form. H.264: the rows of macroblocks, top to bottom (`rows`).
-  // HEVC without AMP: the rows a warp runs (16x16 and 8x8)
+  // The row form. H.264: the rows of macroblocks, top to bottom (`row_ctas`).
+  // HEVC without AMP: `row_ctas`, the rows a CTA of the row kernel takes at
+  // once (the first of them); and for the resident engine the rows a warp
+  // runs (16x16 and 8x8)
   // and the rows a CTA runs (64x64 and 32x32), as row_entry words, each
   // list ordered by the row's first sample row, larger blocks first: every
   // row comes after the rows it reads (its upper row, its parents' rows).
-  std::vector<uint32_t> rows, rows_big;
+  std::vector<uint32_t> row_ctas, rows, rows_big;
   uint32_t* d_rows = nullptr;    // device: rows, then rows_big
 };
 
@@ -200,21 +202,18 @@ struct Graph {
   int seen = 0;  // launches of this shape so far: captured on the second
 };
 
-// A launch shape the tuner chooses among: the search kernel's occupancy
-// variant (registers per thread against resident warps), in the latency form
-// the share of CTAs that search 32x32 and 64x64 HEVC blocks a CTA per block
-// (0, a quarter or half of the SMs), and whether 8x8 blocks refine from
-// staged phase patches (the search window's neighbourhood in shared memory)
-// or straight from the caches; and whether HEVC STANDALONE frames without
-// AMP run in the row form (a warp or a CTA per row of blocks; `groups` 3:
-// a CTA for every row of large blocks, up to half the grid).
+// A launch shape the tuner chooses among for a dataflow launch: the search
+// kernel's occupancy variant (registers per thread against resident warps),
+// in the latency form the share of CTAs that search 32x32 and 64x64 HEVC
+// blocks a CTA per block (0, a quarter or half of the SMs), and whether 8x8
+// blocks refine from staged phase patches (the search window's neighbourhood
+// in shared memory) or straight from the caches.
 struct Shape {
-  int variant, groups, patch, rows;
+  int variant, groups, patch;
 };
-constexpr Shape kThroughputShapes[] = {{1, 0, 0, 0}, {0, 0, 0, 0}, {2, 0, 0, 0}};
-constexpr Shape kLatencyHevcShapes[] = {{0, 3, 0, 1}, {0, 3, 1, 1}, {1, 3, 0, 1}, {1, 2, 1, 0},
-                                        {1, 2, 0, 0}, {1, 1, 1, 0}, {1, 0, 0, 0}, {0, 2, 1, 0}};
-constexpr Shape kLatencyShapes[] = {{1, 0, 0, 0}, {0, 0, 0, 0}, {2, 0, 0, 0}};
+constexpr Shape kThroughputShapes[] = {{1, 0, 0}, {0, 0, 0}, {2, 0, 0}};
+constexpr Shape kLatencyHevcShapes[] = {{1, 2, 1}, {1, 2, 0}, {1, 1, 1}, {1, 0, 0}, {0, 2, 1}};
+constexpr Shape kLatencyShapes[] = {{1, 0, 0}, {0, 0, 0}, {2, 0, 0}};
 constexpr int kTuneRounds = 2;  // timings per shape before the tuner chooses (launch times vary)
 constexpr int kNumShapes[3] = {(int)(sizeof(kThroughputShapes) / sizeof(Shape)),
                                (int)(sizeof(kLatencyHevcShapes) / sizeof(Shape)),
@@ -258,7 +257,7 @@ struct Slot {
 struct Ctx {
   int device = 0, nsm = 0;
   int bps[kParts][kSearchVariants][2] = {};  // resident search blocks per SM, per part, variant, form
-  int hrow_bps[2][RME_MAX_REFS] = {};        // H.264's row form: per sample width and references
+  int row_bps[kParts][RME_MAX_REFS] = {};    // the row forms', per part (H.264: and references)
   // The tuner: per (part, form, log2 of its task count), each launch shape
   // of that class (kShapes) is timed on one real launch, then the fastest is
   // kept. Results do not depend on the shape.
@@ -452,7 +451,7 @@ const Deps* get_deps(Ctx* c, const rme_picture_desc& d, const rme_params* p, int
     for (int my = 0; my < mbh; ++my)
       for (int mx = 0; mx < mbw; ++mx)
         pend.push_back((mx > 0) + (my > 0) + (my > 0 && mx + 1 < mbw) + (mx > 0 && my > 0));
-    for (int my = 0; my < mbh; ++my) dp.rows.push_back((uint32_t)my);
+    for (int my = 0; my < mbh; ++my) dp.row_ctas.push_back((uint32_t)my);
   } else {
     int sizes[4];
     const int nl = level_sizes(p, sizes);
@@ -494,7 +493,10 @@ const Deps* get_deps(Ctx* c, const rme_picture_desc& d, const rme_params* p, int
     std::stable_sort(all.begin(), all.end(), [](const Row& a, const Row& b) {
       return a.r != b.r ? a.r < b.r : a.y != b.y ? a.y < b.y : a.size > b.size;
     });
-    for (const Row& w : all) (w.size >= 32 ? dp.rows_big : dp.rows).push_back(w.entry);
+    for (const Row& w : all) {
+      (w.size >= 32 ? dp.rows_big : dp.rows).push_back(w.entry);
+      if ((w.y / w.size) % hevc_row_rows(w.size) == 0) dp.row_ctas.push_back(w.entry);
+    }
   }
   cudaError_t e = cudaMalloc(&dp.pending, std::max<size_t>(pend.size(), 1) * sizeof(int32_t));
   if (e == cudaSuccess)
@@ -753,18 +755,21 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   // blocks of HEVC STANDALONE frames together.
   const bool spec = total <= kSpecTasks;
   int64_t part_tasks[kParts] = {0, 0, 0, 0};
-  // H.264 parts whose frames are all STANDALONE run their row form whatever
-  // the launch's size: against the best shape of the dataflow form it took
+  // Parts whose frames are all STANDALONE run their row form: H.264 whatever
+  // the launch's size (against the best shape of the dataflow form it took
   // 0.53 against 1.60 ms for one CIF frame and 0.86 against 2.49 ms for a
   // hundred, 9.6 against 14.7 ms for 64 720p frames of two references, 20.4
-  // against 27.4 ms for 24 1080p 10-bit frames of three.
-  bool hrows[kParts] = {false, true, false, true};
-  int hrows_nref[kParts] = {0, 0, 0, 0};
+  // against 27.4 ms for 24 1080p 10-bit frames of three); HEVC without AMP
+  // units in a launch of the latency form (one 1080p frame 3.1 ms, on the
+  // dataflow form's best shape 7.3).
+  bool rows[kParts] = {spec, true, spec, true};
+  int rows_nref[kParts] = {0, 0, 0, 0};
   for (int i = 0; i < n; ++i) {
-    const int k = part_of(sl.h_frames.p[i]);
+    const FrameDesc& fd = sl.h_frames.p[i];
+    const int k = part_of(fd);
     part_tasks[k] += ntask[i];
-    hrows[k] = hrows[k] && params[i].predictor_mode == RME_PRED_STANDALONE;
-    hrows_nref[k] = std::max(hrows_nref[k], (int)frames[i].nref);
+    rows[k] = rows[k] && params[i].predictor_mode == RME_PRED_STANDALONE && fd.amp == 0;
+    rows_nref[k] = std::max(rows_nref[k], fd.nref);
   }
   // Each part's launch shape: the tuned one for its class, or the next one
   // to time (a launch of one kind only, so that its time is the part's).
@@ -778,7 +783,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     const Shape* shapes = !spec ? kThroughputShapes : part_codec(k) == RME_CODEC_HEVC ? kLatencyHevcShapes : kLatencyShapes;
     const int nsh = kNumShapes[!spec ? 0 : part_codec(k) == RME_CODEC_HEVC ? 1 : 2];
     shape[k] = shapes[0];
-    if (part_tasks[k] > 0 && c->tune_on && !hrows[k]) {
+    if (part_tasks[k] > 0 && c->tune_on && !rows[k]) {
       const int bucket = 63 - __builtin_clzll((unsigned long long)part_tasks[k]);
       Ctx::Tune& T = c->tune[{k * 2 + spec, bucket}];
       if (T.best >= 0) {
@@ -790,16 +795,11 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
       }
     }
     variant[k] = shape[k].variant;
-    if (part_tasks[k] > 0 && !hrows[k] && !c->bps[k][variant[k]][spec])
+    if (part_tasks[k] > 0 && !rows[k] && !c->bps[k][variant[k]][spec])
       c->bps[k][variant[k]][spec] = search_blocks_per_sm(part_bytes(k), part_codec(k), variant[k], spec);
   }
-  // The row form: H.264's, and, for a part of the latency form whose frames
-  // are all HEVC STANDALONE without AMP, HEVC's when its shape asks for it.
-  bool rows[kParts] = {false, false, false, false};
   std::vector<const Deps*> fdeps(n, nullptr);
-  for (int k = 0; k < kParts; ++k) rows[k] = part_tasks[k] > 0 && (hrows[k] || (spec && shape[k].rows));
   for (int i = 0; i < n; ++i) {
-    const FrameDesc& fd = sl.h_frames.p[i];
     if (params[i].predictor_mode == RME_PRED_STANDALONE) {
       Picture* src;
       picture_of(c, frames[i].src_id, &src);
@@ -807,10 +807,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
       fdeps[i] = get_deps(c, src->d, &params[i], frames[i].nref, &rc);
       if (!fdeps[i]) return rc;
     }
-    if (fd.codec == RME_CODEC_HEVC && (params[i].predictor_mode != RME_PRED_STANDALONE || fd.amp != 0))
-      rows[part_of(fd)] = false;
   }
-  int64_t rows_small[kParts] = {0, 0, 0, 0}, rows_large[kParts] = {0, 0, 0, 0};
   std::vector<std::pair<const int32_t*, int>> pend_copies;  // (template, frame)
   for (int i = 0; i < n; ++i) {
     FrameDesc& fd = sl.h_frames.p[i];
@@ -831,12 +828,8 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     } else if (rows[part]) {
       // Every row of the frame is pushed now (interleaved with the other
       // frames' rows below); a search of this buffer tags its words anew.
-      const Deps* dp = fdeps[i];
       fd.mvf = sl.d_mvf.p + toff[i];
-      fd.tag = hrows[part] ? sl.epoch << 2 : sl.epoch;
-      fd.nrows = (int32_t)(dp->rows.size() + dp->rows_big.size());
-      rows_small[part] += (int64_t)dp->rows.size();
-      rows_large[part] += (int64_t)dp->rows_big.size();
+      fd.tag = fd.codec == RME_CODEC_H264 ? sl.epoch << 2 : sl.epoch;
       sig.push_back(fd.bd);
       sig.push_back(fd.codec);
       sig.push_back(fd.width);
@@ -867,20 +860,14 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   // own order kept).
   for (int k = 0; k < kParts; ++k) {
     if (!rows[k]) continue;
-    for (int big = 0; big < 2; ++big) {
-      auto list = [&](int i) -> const std::vector<uint32_t>& { return big ? fdeps[i]->rows_big : fdeps[i]->rows; };
-      size_t most = 0;
-      for (int i = 0; i < n; ++i)
-        if (part_of(sl.h_frames.p[i]) == k) most = std::max(most, list(i).size());
-      for (size_t j = 0; j < most; ++j)
-        for (int i = 0; i < n; ++i) {
-          if (part_of(sl.h_frames.p[i]) != k) continue;
-          const std::vector<uint32_t>& v = list(i);
-          if (j < v.size())
-            (big ? init_big : init)[k].push_back(((unsigned long long)sl.epoch << 32) |
-                                                 ((unsigned long long)i << 24) | v[j]);
-        }
-    }
+    size_t most = 0;
+    for (int i = 0; i < n; ++i)
+      if (part_of(sl.h_frames.p[i]) == k) most = std::max(most, fdeps[i]->row_ctas.size());
+    for (size_t j = 0; j < most; ++j)
+      for (int i = 0; i < n; ++i) {
+        if (part_of(sl.h_frames.p[i]) != k || j >= fdeps[i]->row_ctas.size()) continue;
+        init[k].push_back(((unsigned long long)sl.epoch << 32) | ((unsigned long long)i << 24) | fdeps[i]->row_ctas[j]);
+      }
   }
   // h_init: [the launch header (kMiscWords) | entries | the CTAs' entries]
   size_t ninit = 0, init_off[kParts], init_big_off[kParts];
@@ -919,9 +906,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     L.tail_big = sl.d_misc.p + kMiscBig + 2 * k + 1;
     L.group_ctas = 0;
     if (rows[k]) {
-      L.rows = 1;
-      L.total = rows_small[k];
-      L.total_big = rows_large[k];
+      L.total = (int64_t)init[k].size();
       L.done = nullptr;
     }
     slot0 += part_tasks[k];
@@ -948,10 +933,11 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   int grid[kParts] = {0, 0, 0, 0};
   for (int k = 0; k < kParts; ++k) {
     if (part_tasks[k] == 0) continue;
-    if (hrows[k]) {
-      int& bps = c->hrow_bps[k / 2][hrows_nref[k] - 1];
-      if (!bps) bps = h264_row_blocks_per_sm(part_bytes(k), hrows_nref[k]);
-      grid[k] = (int)std::min<int64_t>(rows_small[k], (int64_t)c->nsm * bps);
+    if (rows[k]) {
+      const bool h264 = part_codec(k) == RME_CODEC_H264;
+      int& bps = c->row_bps[k][h264 ? rows_nref[k] - 1 : 0];
+      if (!bps) bps = h264 ? h264_row_blocks_per_sm(part_bytes(k), rows_nref[k]) : hevc_row_blocks_per_sm(part_bytes(k));
+      grid[k] = (int)std::max<int64_t>(1, std::min<int64_t>(Ls[k].total, (int64_t)c->nsm * bps));
       sig.push_back(-2);
       continue;
     }
@@ -961,20 +947,9 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
       for (int i = 0; i < n; ++i)
         if (part_of(sl.h_frames.p[i]) == k && params[i].predictor_mode == RME_PRED_STANDALONE)
           big += (int64_t)sl.h_frames.p[i].big_end * sl.h_frames.p[i].nref;
-    const int share = shape[k].groups == 3 ? cap / 2
-                      : shape[k].groups == 2 ? c->nsm / 2
-                      : shape[k].groups == 1 ? c->nsm / 4
-                                             : 0;
-    int g = big > 0 && share > 0 ? (int)std::min<int64_t>({(int64_t)share, big, (int64_t)cap - 1}) : 0;
-    int64_t small = part_tasks[k] - big;
-    if (rows[k]) {
-      // A CTA per row of large blocks (at least one when there are any), a
-      // warp per row of small ones.
-      g = rows_large[k] > 0
-              ? (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)std::max(share, 1), rows_large[k], (int64_t)cap - 1}))
-              : 0;
-      small = rows_small[k];
-    }
+    const int share = shape[k].groups == 2 ? c->nsm / 2 : shape[k].groups == 1 ? c->nsm / 4 : 0;
+    const int g = big > 0 && share > 0 ? (int)std::min<int64_t>({(int64_t)share, big, (int64_t)cap - 1}) : 0;
+    const int64_t small = part_tasks[k] - big;
     const int solo = (int)std::max<int64_t>(1, std::min<int64_t>(cap - g, (small + kWarpsPerBlock - 1) / kWarpsPerBlock));
     Ls[k].group_ctas = g;
     grid[k] = g + solo;
@@ -1008,8 +983,9 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
       cudaStream_t sk = j == 0 ? s : c->aux[j];
       if (j > 0) e = cudaStreamWaitEvent(sk, c->ev_fork, 0);
       if (e == cudaSuccess)
-        e = hrows[k] ? launch_h264_rows(Ls[k], part_bytes(k), hrows_nref[k], grid[k], sk)
-                     : launch_search(Ls[k], part_bytes(k), part_codec(k), variant[k], grid[k], sk, spec);
+        e = !rows[k] ? launch_search(Ls[k], part_bytes(k), part_codec(k), variant[k], grid[k], sk, spec)
+            : part_codec(k) == RME_CODEC_H264 ? launch_h264_rows(Ls[k], part_bytes(k), rows_nref[k], grid[k], sk)
+                                              : launch_hevc_rows(Ls[k], part_bytes(k), grid[k], sk);
       if (e == cudaSuccess && j > 0) e = cudaEventRecord(c->ev_join[j], sk);
     }
     for (int j = 1; j < nparts && e == cudaSuccess; ++j) e = cudaStreamWaitEvent(s, c->ev_join[j], 0);

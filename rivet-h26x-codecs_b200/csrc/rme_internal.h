@@ -110,8 +110,6 @@ struct LaunchDesc {
   int32_t patch8;                // the latency form: 8x8 blocks refine from staged phase patches
   int32_t ring_shift;            // nonzero: the resident engine's ring of
                                  // 2^ring_shift slots (ring_entry)
-  int32_t rows;                  // the row form: the queues hold rows, all pushed by the host
-  int64_t total_big;             // the row form: rows in the CTAs' queue
 };
 
 // The resident engine (rme_engine.cu): one search kernel that stays on the
@@ -253,6 +251,12 @@ constexpr int kSearchVariants = 3, kDefaultVariant = 1;
 cudaError_t launch_search(const LaunchDesc& L, int bytes_per_sample, int codec, int variant, int grid,
                           cudaStream_t s, bool spec = false);
 int search_blocks_per_sm(int bytes_per_sample, int codec, int variant, bool spec = false);
+// HEVC STANDALONE frames without AMP in their row form (rme_rows.cu): L's
+// queue holds row_entry words, each the first of hevc_row_rows(size)
+// consecutive rows, all pushed by the host, each after the rows it reads.
+cudaError_t launch_hevc_rows(const LaunchDesc& L, int bytes_per_sample, int grid, cudaStream_t s);
+int hevc_row_blocks_per_sm(int bytes_per_sample);
+int hevc_row_rows(int size);  // rows a CTA takes at once
 // H.264 STANDALONE frames in their row form (rme_h264.cu): L's queue holds
 // rows of macroblocks (all pushed by the host, each after the row above it),
 // the frames have `mvf`, a tag with its low two bits clear, and at most

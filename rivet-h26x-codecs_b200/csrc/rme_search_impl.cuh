@@ -1150,6 +1150,13 @@ __device__ int hevc_task(const LaunchDesc& L, const FrameDesc& F, int f, int t, 
 // search's.
 constexpr int kGroupThreads = kWarpsPerBlock * 32;
 
+// A barrier of the T threads that share a block's search: the whole CTA
+// (barrier 0) or one of the groups a CTA is split into.
+template <int T>
+__device__ __forceinline__ void group_sync(int bar) {
+  asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(T) : "memory");
+}
+
 template <class S>
 struct alignas(16) GroupSmem {
   unsigned long long cnt[6];
@@ -1174,9 +1181,10 @@ __device__ __forceinline__ bool group_task_of(const LaunchDesc& L, const FrameDe
 // coalesced along the row; the word after a lane's comes from its neighbour,
 // the row's last lane loads it), four such passes' loads in flight; each
 // warp's sum is added into cost[b][c].
-template <class S, int N, class Pos>
-__device__ __forceinline__ void cta_sad(GroupSmem<S>& gs, int b, const S* org, int stride, int nc, Pos pos, int tid) {
-  constexpr int SPW = 4 / sizeof(S), WR = N / SPW, RPW = 32 / WR, K = 4, STEP = kWarpsPerBlock * RPW;
+template <class S, int N, int T, class Pos>
+__device__ __forceinline__ void cta_sad(GroupSmem<S>& gs, int b, const S* org, int stride, int nc, Pos pos, int tid,
+                                        int bar) {
+  constexpr int SPW = 4 / sizeof(S), WR = N / SPW, RPW = 32 / WR, K = 4, STEP = T / 32 * RPW;
   const int lane = tid & 31, warp = tid >> 5, wd = lane % WR, rsub = lane / WR;
   if (tid < 32) gs.cost[(b + 1) % 3][tid] = 0u;
   const int rows = nc * N;
@@ -1215,7 +1223,7 @@ __device__ __forceinline__ void cta_sad(GroupSmem<S>& gs, int b, const S* org, i
       if (lane == 0 && ok[k]) atomicAdd(&gs.cost[b][cc[k]], acc);
     }
   }
-  __syncthreads();
+  group_sync<T>(bar);
 }
 
 // The diamond's window: the reference's integer plane around a staging
@@ -1241,28 +1249,29 @@ static_assert(sizeof(GroupSmem<uint16_t>) + WinGeo<uint16_t, 64>::ROWS * WinGeo<
 // Stage the window around (scx, scy); returns the byte offset of its first
 // sample within the first word (the same on every row: rows are whole words
 // apart). All threads call; ends with a barrier.
-template <class S, int N>
-__device__ __forceinline__ uint32_t stage_window(uint32_t* win, const S* org, int stride, int scx, int scy, int tid) {
+template <class S, int N, int T>
+__device__ __forceinline__ uint32_t stage_window(uint32_t* win, const S* org, int stride, int scx, int scy, int tid,
+                                                 int bar) {
   using W = WinGeo<S, N>;
   const uintptr_t a0 = reinterpret_cast<uintptr_t>(org + (ptrdiff_t)(scy - kWinR) * stride + (scx - kWinR));
   const uint32_t* w0 = reinterpret_cast<const uint32_t*>(a0 & ~uintptr_t(3));
   const int rstep = stride * (int)sizeof(S) / 4;
-  for (int i = tid; i < W::ROWS * W::WRW; i += kGroupThreads) {
+  for (int i = tid; i < W::ROWS * W::WRW; i += T) {
     const int row = i / W::WRW, wd = i - row * W::WRW;
     win[i] = RME_LD32(w0 + (ptrdiff_t)row * rstep + wd);
   }
-  __syncthreads();
+  group_sync<T>(bar);
   return (uint32_t)(a0 & 3);
 }
 
 // The SADs of `nc` candidates, all within kWinR of the window's centre, from
 // the window (a lane per word of a candidate row, each thread's words of a
 // candidate summed, each warp's sum added into cost[b][c]).
-template <class S, int N, class Pos>
+template <class S, int N, int T, class Pos>
 __device__ __forceinline__ void cta_sad_win(GroupSmem<S>& gs, int b, const uint32_t* win, uint32_t off0, int scx,
-                                            int scy, int nc, Pos pos, int tid) {
+                                            int scy, int nc, Pos pos, int tid, int bar) {
   using W = WinGeo<S, N>;
-  constexpr int SPW = 4 / sizeof(S), WR = N / SPW, JOBS = N * WR, PER = JOBS / kGroupThreads;
+  constexpr int SPW = 4 / sizeof(S), WR = N / SPW, JOBS = N * WR, PER = JOBS / T;
   if (tid < 32) gs.cost[(b + 1) % 3][tid] = 0u;
   for (int c = 0; c < nc; ++c) {
     int fx, fy;
@@ -1272,7 +1281,7 @@ __device__ __forceinline__ void cta_sad_win(GroupSmem<S>& gs, int b, const uint3
     uint32_t acc = 0;
 #pragma unroll
     for (int m = 0; m < PER; ++m) {
-      const int j = tid + m * kGroupThreads, row = j / WR, k = j - row * WR;
+      const int j = tid + m * T, row = j / WR, k = j - row * WR;
       const uint32_t bb = b0 + 4u * k, wi = bb >> 2, sh = (bb & 3u) * 8u;
       const uint32_t* wr = win + (r0 + row) * W::WRW;
       acc += vsad(gs.src[row * WR + k], __funnelshift_r(wr[wi], wr[wi + 1], sh), S());
@@ -1280,20 +1289,20 @@ __device__ __forceinline__ void cta_sad_win(GroupSmem<S>& gs, int b, const uint3
     acc = __reduce_add_sync(kFull, acc);
     if ((tid & 31) == 0) atomicAdd(&gs.cost[b][c], acc);
   }
-  __syncthreads();
+  group_sync<T>(bar);
 }
 
 // The SATDs of `nc` candidates (quarter-sample vectors from pos), 4x4 tiles
 // split over the CTA (a warp's lanes on adjacent tiles of a tile row:
 // coalesced), each warp's sum added into cost[b][c].
-template <class S, int N, class Pos>
+template <class S, int N, int T, class Pos>
 __device__ __forceinline__ void cta_satd(GroupSmem<S>& gs, int b, const DevPlanes& R, int x, int y, int nc, Pos pos,
-                                         int tid) {
+                                         int tid, int bar) {
   constexpr int SPW = 4 / sizeof(S), WPT = 4 / SPW, TW = N / 4, NT = TW * TW, WR = N / SPW;
   if (tid < 32) gs.cost[(b + 1) % 3][tid] = 0u;
   const int jobs = nc * NT;
 #pragma unroll 3
-  for (int j0 = 0; j0 < jobs; j0 += kGroupThreads) {
+  for (int j0 = 0; j0 < jobs; j0 += T) {
     const int j = j0 + tid;
     uint32_t acc = 0;
     int c = 0;
@@ -1329,14 +1338,15 @@ __device__ __forceinline__ void cta_satd(GroupSmem<S>& gs, int b, const DevPlane
     acc = __reduce_add_sync(kFull, acc);  // a warp's 32 jobs are tiles of one candidate (NT >= 64)
     if ((tid & 31) == 0 && ok) atomicAdd(&gs.cost[b][c], acc);
   }
-  __syncthreads();
+  group_sync<T>(bar);
 }
 
 // search_full + refine_subpel of one STANDALONE square block of N in {32, 64}
 // by the whole CTA (all threads call). Returns a task it made ready to run
 // next (frame << 24 | task; another group task) or -1.
-template <class S, int N, bool ROW = false>
-__device__ int hevc_group_task(const LaunchDesc& L, const FrameDesc& F, int f, int t, GroupSmem<S>& gs, int tid) {
+template <class S, int N, bool ROW = false, int T = kGroupThreads>
+__device__ int hevc_group_task(const LaunchDesc& L, const FrameDesc& F, int f, int t, GroupSmem<S>& gs, int tid,
+                               int bar = 0) {
   constexpr int SPW = 4 / sizeof(S), WR = N / SPW;
   const int lane = tid & 31;
   const int r = t % F.nref, blk = t / F.nref;
@@ -1365,13 +1375,13 @@ __device__ int hevc_group_task(const LaunchDesc& L, const FrameDesc& F, int f, i
   if (tid < 64) gs.cost[tid >> 5][tid & 31] = 0u;  // the first step's buffer (and the next)
   {
     const S* so = plane_at<S>(F.src, 0, x, y);
-    for (int i = tid; i < WR * N; i += kGroupThreads) {
+    for (int i = tid; i < WR * N; i += T) {
       const int row = i / WR, wd = i - row * WR;
       gs.src[i] = ldw(so + (ptrdiff_t)row * F.src.stride + wd * SPW);
     }
   }
   if (ROW && tid < 3) gs.bc[tid] = didx >= 0 ? (uint32_t)wait_word(L, F.mvf + didx, F.tag, dw) : 0u;
-  __syncthreads();
+  group_sync<T>(bar);
   int p0x = 0, p0y = 0, p1x = 0, p1y = 0, na = 0;
   if (gs.bc[3]) {
     p0x = mvx_of(gs.bc[0]);
@@ -1422,7 +1432,7 @@ __device__ int hevc_group_task(const LaunchDesc& L, const FrameDesc& F, int f, i
   };
   int bx = 0, by = 0;
   uint32_t bcost = kInf;
-  cta_sad<S, N>(gs, buf, org, stride, 4, spos, tid);
+  cta_sad<S, N, T>(gs, buf, org, stride, 4, spos, tid, bar);
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     int fx, fy;
@@ -1459,10 +1469,10 @@ __device__ int hevc_group_task(const LaunchDesc& L, const FrameDesc& F, int f, i
       if (!staged || abs(cbx - scx) > kWinR - 1 || abs(cby - scy) > kWinR - 1) {
         scx = cbx;
         scy = cby;
-        woff = stage_window<S, N>(win, org, stride, scx, scy, tid);
+        woff = stage_window<S, N, T>(win, org, stride, scx, scy, tid, bar);
         staged = true;
       }
-      cta_sad_win<S, N>(gs, buf, win, woff, scx, scy, 4, pos, tid);
+      cta_sad_win<S, N, T>(gs, buf, win, woff, scx, scy, 4, pos, tid, bar);
       bool improved = false;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -1490,7 +1500,7 @@ __device__ int hevc_group_task(const LaunchDesc& L, const FrameDesc& F, int f, i
       fy = cyr + ((k8 == 2 || k8 == 4 || k8 == 5) ? rr : (k8 == 3 || k8 == 6 || k8 == 7) ? -rr : 0);
       return inside(fx, fy);
     };
-    cta_sad<S, N>(gs, buf, org, stride, 24, rpos, tid);
+    cta_sad<S, N, T>(gs, buf, org, stride, 24, rpos, tid, bar);
     bool moved = false;
     for (int c = 0; c < 24; ++c) {
       int fx, fy;
@@ -1517,7 +1527,7 @@ __device__ int hevc_group_task(const LaunchDesc& L, const FrameDesc& F, int f, i
     my = imy + (q / 3 - 1) * 2;
     return true;
   };
-  cta_satd<S, N>(gs, buf, R, x, y, 9, hpos, tid);
+  cta_satd<S, N, T>(gs, buf, R, x, y, 9, hpos, tid, bar);
   int bmx = imx, bmy = imy;
   uint32_t bc = kInf, bsatd = 0;
   for (int c = 0; c < 9; ++c) {
@@ -1539,7 +1549,7 @@ __device__ int hevc_group_task(const LaunchDesc& L, const FrameDesc& F, int f, i
     my = (int)(int16_t)(hmy + dy);
     return !(cross != 0 && dx != 0 && dy != 0);
   };
-  cta_satd<S, N>(gs, buf, R, x, y, 8, qpos, tid);
+  cta_satd<S, N, T>(gs, buf, R, x, y, 8, qpos, tid, bar);
   for (int c = 0; c < 8; ++c) {
     int mx, my;
     if (!qpos(c, mx, my)) continue;
@@ -1563,7 +1573,7 @@ __device__ int hevc_group_task(const LaunchDesc& L, const FrameDesc& F, int f, i
     gs.cnt[4] += (unsigned long long)nsatd * N * N;
     if (ROW) st_relaxed64(F.mvf + t, mv_word(F.tag, bmx, bmy));
   }
-  __syncthreads();
+  group_sync<T>(bar);
   if (ROW) return -1;
   // The tasks reading this result (warp 0 releases them, one per lane):
   // right and lower neighbours, the next size's blocks inside this one,
@@ -1598,7 +1608,7 @@ __device__ int hevc_group_task(const LaunchDesc& L, const FrameDesc& F, int f, i
     }
     if (tid == 0) gs.bc[6] = (uint32_t)cont;
   }
-  __syncthreads();
+  group_sync<T>(bar);
   return (int)gs.bc[6];
 }
 
