@@ -106,7 +106,7 @@ struct RefSearch {
       ldwords<WR>(rp, a);
       ldwords<WR>(rp + (ptrdiff_t)8 * R.stride, b);
 #pragma unroll
-      for (int k = 0; k < WR; ++k) acc += vsad(src[sub * WR + k], a[k], S()) + vsad(src[(sub + 8) * WR + k], b[k], S());
+      for (int k = 0; k < WR; ++k) acc = vsad(src[(sub + 8) * WR + k], b[k], vsad(src[sub * WR + k], a[k], acc, S()), S());
     }
     acc += __shfl_xor_sync(kFull, acc, 4);
     acc += __shfl_xor_sync(kFull, acc, 2);

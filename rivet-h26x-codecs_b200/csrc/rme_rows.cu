@@ -179,14 +179,14 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
 #pragma unroll
           for (int k = 0; k < RPL; ++k)
 #pragma unroll
-            for (int c = 0; c < WR; ++c) acc += vsad(src[(sub + k * LPC) * WR + c], a[k][c], S());
+            for (int c = 0; c < WR; ++c) acc = vsad(src[(sub + k * LPC) * WR + c], a[k][c], acc, S());
         } else {
 #pragma unroll 2
           for (int k = 0; k < RPL; ++k) {
             uint32_t a[WR];
             ldwords<WR>(rp + (ptrdiff_t)k * LPC * stride, a);
 #pragma unroll
-            for (int c = 0; c < WR; ++c) acc += vsad(src[(sub + k * LPC) * WR + c], a[c], S());
+            for (int c = 0; c < WR; ++c) acc = vsad(src[(sub + k * LPC) * WR + c], a[c], acc, S());
           }
         }
       }
@@ -283,20 +283,12 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
         uint32_t pw4[4][WPT];
 #pragma unroll
         for (int rr = 0; rr < 4; ++rr) ldwords<WPT>(q + (ptrdiff_t)rr * stride, pw4[rr]);
-        int d[16];
+        uint32_t sw[4][WPT];
 #pragma unroll
         for (int rr = 0; rr < 4; ++rr)
 #pragma unroll
-          for (int w = 0; w < WPT; ++w) {
-            const uint32_t sw = src[(ty * 4 + rr) * WR + tx * WPT + w], qw = pw4[rr][w];
-#pragma unroll
-            for (int e = 0; e < SPW; ++e) {
-              const int sh = e * (32 / SPW);
-              const uint32_t m = SPW == 4 ? 0xffu : 0xffffu;
-              d[rr * 4 + w * SPW + e] = (int)((sw >> sh) & m) - (int)((qw >> sh) & m);
-            }
-          }
-        v = satd4x4(d);
+          for (int w = 0; w < WPT; ++w) sw[rr][w] = src[(ty * 4 + rr) * WR + tx * WPT + w];
+        v = satd4x4<WPT>(sw, pw4);
       }
 #pragma unroll
       for (int o = NT >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);

@@ -75,30 +75,84 @@ __device__ __forceinline__ uint32_t ldw(const uint16_t* p) {
   uint32_t lo = RME_LD32(q), hi = RME_LD32(q + 1);
   return __funnelshift_r(lo, hi, (uint32_t)(a & 2) * 8u);
 }
-__device__ __forceinline__ uint32_t vsad(uint32_t a, uint32_t b, uint8_t) { return __vsadu4(a, b); }
-__device__ __forceinline__ uint32_t vsad(uint32_t a, uint32_t b, uint16_t) { return __vsadu2(a, b); }
+// acc plus the absolute differences of two words' samples. 8 bits: the
+// four-byte absolute difference and sum is one instruction (2 cycles of a
+// scheduler a warp; __vsadu4 and an add 2.2). 16 bits: __vsadu2 is emulated
+// (18 cycles); the larger less the smaller half, then their sum by a dot
+// product with ones, is four instructions (8 cycles).
+__device__ __forceinline__ uint32_t vsad(uint32_t a, uint32_t b, uint32_t acc, uint8_t) {
+  uint32_t r;
+  asm("vabsdiff4.u32.u32.u32.add %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(acc));
+  return r;
+}
+__device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {  // per 16-bit half
+  uint32_t r;
+  asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t min2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t vsad(uint32_t a, uint32_t b, uint32_t acc, uint16_t) {
+  return __dp2a_lo(max2(a, b) - min2(a, b), 0x0101u, acc);
+}
 __device__ __forceinline__ uint32_t vavg(uint32_t a, uint32_t b, uint8_t) { return __vavgu4(a, b); }
 __device__ __forceinline__ uint32_t vavg(uint32_t a, uint32_t b, uint16_t) { return __vavgu2(a, b); }
 
-// 4x4 Hadamard SATD of one tile (dsp/distortion.rs:326-381).
-__device__ __forceinline__ uint32_t satd4x4(int d[16]) {
+// A 4x4 tile's row of samples as two words of two 16-bit halves: samples 0
+// and 2, samples 1 and 3.
+__device__ __forceinline__ void tile_row(const uint32_t (&w)[1], uint32_t& even, uint32_t& odd) {
+  even = w[0] & 0x00ff00ffu;
+  odd = __byte_perm(w[0], 0u, 0x4341);
+}
+__device__ __forceinline__ void tile_row(const uint32_t (&w)[2], uint32_t& even, uint32_t& odd) {
+  even = __byte_perm(w[0], w[1], 0x5410);
+  odd = __byte_perm(w[0], w[1], 0x7632);
+}
+
+// 4x4 Hadamard SATD of one tile, (sum + 1) >> 1 (dsp/distortion.rs:326-381),
+// from its rows as words (one of 8-bit, two of 16-bit samples a row).
+//
+// Two differences share a word, as hi * 65536 + lo: sums and differences of
+// such words are those of their halves, so three of the four butterfly
+// stages run on eight words instead of sixteen values. The last stage, lo + hi
+// and lo - hi, is only needed as |lo + hi| + |lo - hi| = 2 max(|lo|, |hi|),
+// so the sum of the tile's absolute values is twice the sum of those maxima,
+// and the SATD is that sum itself. The halves are at most 8 * 4095 before it,
+// inside 16 bits at every depth: biased by 0x8000 they are unsigned, and
+// max(|a|, |b|) + 0x8000 = max(max(a, b), 0x10000 - min(a, b)) of biased
+// values. 90 cycles of a scheduler a warp and tile, 148 with the sixteen
+// differences in words of their own; alone on a scheduler 152 against 214.
+template <int WPT>
+__device__ __forceinline__ uint32_t satd4x4(const uint32_t (&s)[4][WPT], const uint32_t (&p)[4][WPT]) {
+  uint32_t e[4], o[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    int a = d[i * 4], b = d[i * 4 + 1], c = d[i * 4 + 2], e = d[i * 4 + 3];
-    int s0 = a + e, s1 = b + c, s2 = b - c, s3 = a - e;
-    d[i * 4] = s0 + s1;
-    d[i * 4 + 1] = s3 + s2;
-    d[i * 4 + 2] = s0 - s1;
-    d[i * 4 + 3] = s3 - s2;
+  for (int r = 0; r < 4; ++r) {
+    uint32_t se, so, pe, po;
+    tile_row(s[r], se, so);
+    tile_row(p[r], pe, po);
+    e[r] = se - pe;
+    o[r] = so - po;
   }
-  uint32_t sum = 0;
+  auto columns = [](uint32_t (&v)[4]) {
+    const uint32_t a = v[0] + v[1], b = v[0] - v[1], c = v[2] + v[3], d = v[2] - v[3];
+    v[0] = a + c;
+    v[1] = b + d;
+    v[2] = a - c;
+    v[3] = b - d;
+  };
+  columns(e);
+  columns(o);
+  uint32_t acc = 0;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    int a = d[j], b = d[4 + j], c = d[8 + j], e = d[12 + j];
-    int s0 = a + e, s1 = b + c, s2 = b - c, s3 = a - e;
-    sum += abs(s0 + s1) + abs(s3 + s2) + abs(s0 - s1) + abs(s3 - s2);
+  for (int r = 0; r < 4; ++r) {
+    const uint32_t x = e[r] + o[r] + 0x80008000u, y = e[r] - o[r] + 0x80008000u;
+    const uint32_t a = __byte_perm(x, y, 0x5410), b = __byte_perm(x, y, 0x7632);
+    acc = __dp2a_lo(max2(max2(a, b), 0x00010000u - min2(a, b)), 0x0101u, acc);
   }
-  return (sum + 1) >> 1;
+  return acc - 8u * 0x8000u;
 }
 
 // Lanes per candidate for a step of n candidates: as many candidates per
@@ -158,10 +212,10 @@ __device__ __forceinline__ uint32_t sad_chunks(const uint32_t* src, int wr, int 
     ldwords<CW>(rp + (ptrdiff_t)row * stride + col * CW * SPW, a);
     if (two) ldwords<CW>(rp + (ptrdiff_t)row2 * stride + col2 * CW * SPW, b);
 #pragma unroll
-    for (int k = 0; k < CW; ++k) acc += vsad(src[row * wr + col * CW + k], a[k], S());
+    for (int k = 0; k < CW; ++k) acc = vsad(src[row * wr + col * CW + k], a[k], acc, S());
     if (two) {
 #pragma unroll
-      for (int k = 0; k < CW; ++k) acc += vsad(src[row2 * wr + col2 * CW + k], b[k], S());
+      for (int k = 0; k < CW; ++k) acc = vsad(src[row2 * wr + col2 * CW + k], b[k], acc, S());
     }
     row = row2 + rs;
     col = col2 + cs;
@@ -192,8 +246,7 @@ __device__ __forceinline__ uint32_t group_sad(const uint32_t* src, int wr, int h
 template <class S, int TS>
 __device__ __forceinline__ uint32_t satd_strips(const uint32_t* src, int wr, int tw, int th, const S* p1,
                                                 const S* p2, int stride, int lpc, int sub) {
-  constexpr int SPW = 4 / sizeof(S);
-  constexpr int WPT = 4 / SPW;       // words per tile row
+  constexpr int WPT = (int)sizeof(S);  // words per tile row
   constexpr int WPS = TS * WPT;      // words per strip row
   const int nspr = tw / TS, items = nspr * th;
   uint32_t acc = 0;
@@ -213,22 +266,15 @@ __device__ __forceinline__ uint32_t satd_strips(const uint32_t* src, int wr, int
     }
 #pragma unroll
     for (int t = 0; t < TS; ++t) {
-      int d[16];
+      uint32_t sw[4][WPT], qw[4][WPT];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const uint32_t* srow = &src[(ty * 4 + r) * wr + (sx * TS + t) * WPT];
+      for (int r = 0; r < 4; ++r)
 #pragma unroll
         for (int k = 0; k < WPT; ++k) {
-          const uint32_t sw = srow[k], qw = pw[r][t * WPT + k];
-#pragma unroll
-          for (int e = 0; e < SPW; ++e) {
-            const int sh = e * (32 / SPW);
-            const uint32_t m = SPW == 4 ? 0xffu : 0xffffu;
-            d[r * 4 + k * SPW + e] = (int)((sw >> sh) & m) - (int)((qw >> sh) & m);
-          }
+          sw[r][k] = src[(ty * 4 + r) * wr + (sx * TS + t) * WPT + k];
+          qw[r][k] = pw[r][t * WPT + k];
         }
-      }
-      acc += satd4x4(d);
+      acc += satd4x4<WPT>(sw, qw);
     }
   }
   return acc;
@@ -435,19 +481,24 @@ __device__ __forceinline__ void write_result(rme_result* o, int mvx, int mvy, in
 
 // ---- HEVC -------------------------------------------------------------------
 
-// mvd_component_bits (h265_search.rs:212-247) in closed form: 1 at zero,
-// else 3 + 2 * floor(log2 |d|) (the loop of mvd_bits_of counts
-// floor(log2 |d|) - 1 Exp-Golomb prefix steps past the first).
-__device__ __forceinline__ uint32_t hevc_cbits(int d) {
-  uint32_t a = (uint32_t)abs(d);
-  return a == 0 ? 1u : 3u + 2u * (31u - __clz(a));
+// mvd_component_bits (h265_search.rs:212-247) in closed form: the loop of
+// mvd_bits_of counts Exp-Golomb prefix steps, so |d| costs 1 at zero, else
+// 3 + 2 * floor(log2 |d|), which is 1 + 2 * floor(log2(2 |d| + 1)) for every
+// |d|. The logarithm is the exponent of 2 |d| + 1 as a float (exact: |d| is
+// below 2^22): an addition to a float's bits, a subtraction, a multiply-add
+// and a mask, where counting leading zeros takes the slow pipe (8 cycles a
+// warp). Returns the exponent in place, (floor(log2) + 127) << 23.
+__device__ __forceinline__ uint32_t hevc_log(int d) {
+  const float f = __int_as_float(0x4b400000 + d) - 12582912.0f;  // d as a float
+  return __float_as_uint(fmaf(fabsf(f), 2.0f, 1.0f)) & 0x7f800000u;
 }
 // (lam * mv_bits as f32) as u32 (h265_me.rs:3776, 3890): one IEEE
-// round-to-nearest multiply, truncated.
+// round-to-nearest multiply, truncated. mv_bits: the cheaper predictor's two
+// components and one bit more.
 __device__ __forceinline__ uint32_t hevc_rate(float lam, int mx, int my, int p0x, int p0y, int p1x, int p1y) {
-  uint32_t b0 = hevc_cbits(mx - p0x) + hevc_cbits(my - p0y);
-  uint32_t b1 = hevc_cbits(mx - p1x) + hevc_cbits(my - p1y);
-  return __float2uint_rz(__fmul_rn(lam, __uint2float_rn(min(b0, b1) + 1u)));
+  const uint32_t b0 = hevc_log(mx - p0x) + hevc_log(my - p0y), b1 = hevc_log(mx - p1x) + hevc_log(my - p1y);
+  const uint32_t bits = 2u * (min(b0, b1) >> 23) - 505u;  // two biases of 127: 2 * (sum + 254) - 508 + 2 + 1
+  return __float2uint_rz(__fmul_rn(lam, __uint_as_float(0x4b000000u + bits) - 8388608.0f));
 }
 
 // ---- HEVC scoring: one lane's part of a candidate ----------------------------
@@ -472,7 +523,7 @@ __device__ __forceinline__ uint32_t sad_rows_fixed(const uint32_t* src, const S*
       uint32_t a[CW];
       ldwords<CW>(rr + c * SPW, a);
 #pragma unroll
-      for (int j = 0; j < CW; ++j) acc += vsad(sr[c + j], a[j], S());
+      for (int j = 0; j < CW; ++j) acc = vsad(sr[c + j], a[j], acc, S());
     }
   }
   return acc;
@@ -490,7 +541,7 @@ __device__ __forceinline__ uint32_t sad_part(const uint32_t* src, int w, int h, 
   const int wr = w / SPW;
   uint32_t acc = 0;
   for (int row = sub; row < h; row += 8)
-    for (int k = 0; k < wr; ++k) acc += vsad(src[row * wr + k], ldw(rp + (ptrdiff_t)row * stride + k * SPW), S());
+    for (int k = 0; k < wr; ++k) acc = vsad(src[row * wr + k], ldw(rp + (ptrdiff_t)row * stride + k * SPW), acc, S());
   return acc;
 }
 
@@ -508,7 +559,7 @@ __device__ __forceinline__ uint32_t sad16_half(const uint32_t* src, const S* rp,
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int k = 0; k < WR; ++k) acc += vsad(src[(half * 8 + r0 + r) * WR + k], a[r][k], S());
+      for (int k = 0; k < WR; ++k) acc = vsad(src[(half * 8 + r0 + r) * WR + k], a[r][k], acc, S());
   }
   return acc;
 }
@@ -524,7 +575,7 @@ __device__ __forceinline__ uint32_t sad8_half(const uint32_t* src, const S* rp, 
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int k = 0; k < WR; ++k) acc += vsad(src[(half * 4 + r) * WR + k], a[r][k], S());
+    for (int k = 0; k < WR; ++k) acc = vsad(src[(half * 4 + r) * WR + k], a[r][k], acc, S());
   return acc;
 }
 
@@ -534,7 +585,7 @@ __device__ __forceinline__ uint32_t sad8_half(const uint32_t* src, const S* rp, 
 template <class S>
 __device__ __forceinline__ uint32_t satd_part(const uint32_t* src, int wr, int tw, int ntiles, const S* pp, int stride,
                                               int sub, int G) {
-  constexpr int SPW = 4 / sizeof(S), WPT = 4 / SPW;  // words per tile row
+  constexpr int WPT = (int)sizeof(S);  // words per tile row
   const bool pow2 = (tw & (tw - 1)) == 0;
   const int sh = __ffs(tw) - 1;
   uint32_t acc = 0;
@@ -544,22 +595,12 @@ __device__ __forceinline__ uint32_t satd_part(const uint32_t* src, int wr, int t
     uint32_t pw[4][WPT];
 #pragma unroll
     for (int r = 0; r < 4; ++r) ldwords<WPT>(pp + (ptrdiff_t)(ty * 4 + r) * stride + tx * 4, pw[r]);
-    int d[16];
+    uint32_t sw[4][WPT];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const uint32_t* srow = &src[(ty * 4 + r) * wr + tx * WPT];
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int k = 0; k < WPT; ++k) {
-        const uint32_t sw = srow[k], qw = pw[r][k];
-#pragma unroll
-        for (int e = 0; e < SPW; ++e) {
-          const int shf = e * (32 / SPW);
-          const uint32_t m = SPW == 4 ? 0xffu : 0xffffu;
-          d[r * 4 + k * SPW + e] = (int)((sw >> shf) & m) - (int)((qw >> shf) & m);
-        }
-      }
-    }
-    acc += satd4x4(d);
+      for (int k = 0; k < WPT; ++k) sw[r][k] = src[(ty * 4 + r) * wr + tx * WPT + k];
+    acc += satd4x4<WPT>(sw, pw);
   }
   return acc;
 }
@@ -632,25 +673,19 @@ __device__ __forceinline__ uint32_t patch_tile_satd(const uint32_t* src, const u
                                                     int sy, int tx, int ty) {
   using G = PatchGeo<S>;
   constexpr int SPW = 4 / sizeof(S), WPT = 4 / SPW, SWR = 8 / SPW;
-  int d[16];
+  uint32_t sw[4][WPT], qw[4][WPT];
   const uint32_t bit0 = (off + (uint32_t)((sx + tx * 4) * sizeof(S))) * 8u;
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const uint32_t* prow = pp + (sy + ty * 4 + r) * G::WR;
-    const uint32_t* srow = src + (ty * 4 + r) * SWR + tx * WPT;
 #pragma unroll
     for (int k = 0; k < WPT; ++k) {
       const uint32_t b = bit0 + 32u * k, wi = b >> 5, sh = b & 31u;
-      const uint32_t qw = __funnelshift_r(prow[wi], prow[wi + 1], sh), sw = srow[k];
-#pragma unroll
-      for (int e = 0; e < SPW; ++e) {
-        const int shf = e * (32 / SPW);
-        const uint32_t m = SPW == 4 ? 0xffu : 0xffffu;
-        d[r * 4 + k * SPW + e] = (int)((sw >> shf) & m) - (int)((qw >> shf) & m);
-      }
+      qw[r][k] = __funnelshift_r(prow[wi], prow[wi + 1], sh);
+      sw[r][k] = src[(ty * 4 + r) * SWR + tx * WPT + k];
     }
   }
-  return satd4x4(d);
+  return satd4x4<WPT>(sw, qw);
 }
 
 // refine_subpel of an 8x8 block around whole-sample (bx, by) from staged
@@ -1218,7 +1253,7 @@ __device__ __forceinline__ void cta_sad(GroupSmem<S>& gs, int b, const S* org, i
     for (int k = 0; k < K; ++k) {
       const uint32_t nx = __shfl_down_sync(kFull, lo[k], 1);
       if (wd != WR - 1) hi[k] = nx;
-      uint32_t acc = ok[k] ? vsad(gs.src[rw[k] * WR + wd], __funnelshift_r(lo[k], hi[k], sh[k]), S()) : 0u;
+      uint32_t acc = ok[k] ? vsad(gs.src[rw[k] * WR + wd], __funnelshift_r(lo[k], hi[k], sh[k]), 0u, S()) : 0u;
       acc = __reduce_add_sync(kFull, acc);
       if (lane == 0 && ok[k]) atomicAdd(&gs.cost[b][cc[k]], acc);
     }
@@ -1284,7 +1319,7 @@ __device__ __forceinline__ void cta_sad_win(GroupSmem<S>& gs, int b, const uint3
       const int j = tid + m * T, row = j / WR, k = j - row * WR;
       const uint32_t bb = b0 + 4u * k, wi = bb >> 2, sh = (bb & 3u) * 8u;
       const uint32_t* wr = win + (r0 + row) * W::WRW;
-      acc += vsad(gs.src[row * WR + k], __funnelshift_r(wr[wi], wr[wi + 1], sh), S());
+      acc = vsad(gs.src[row * WR + k], __funnelshift_r(wr[wi], wr[wi + 1], sh), acc, S());
     }
     acc = __reduce_add_sync(kFull, acc);
     if ((tid & 31) == 0) atomicAdd(&gs.cost[b][c], acc);
@@ -1317,22 +1352,12 @@ __device__ __forceinline__ void cta_satd(GroupSmem<S>& gs, int b, const DevPlane
         uint32_t pw[4][WPT];
 #pragma unroll
         for (int r = 0; r < 4; ++r) ldwords<WPT>(pp + (ptrdiff_t)r * R.stride, pw[r]);
-        int d[16];
+        uint32_t sw[4][WPT];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const uint32_t* srow = &gs.src[(ty * 4 + r) * WR + tx * WPT];
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
-          for (int k = 0; k < WPT; ++k) {
-            const uint32_t sw = srow[k], qw = pw[r][k];
-#pragma unroll
-            for (int e = 0; e < SPW; ++e) {
-              const int shf = e * (32 / SPW);
-              const uint32_t m = SPW == 4 ? 0xffu : 0xffffu;
-              d[r * 4 + k * SPW + e] = (int)((sw >> shf) & m) - (int)((qw >> shf) & m);
-            }
-          }
-        }
-        acc = satd4x4(d);
+          for (int k = 0; k < WPT; ++k) sw[r][k] = gs.src[(ty * 4 + r) * WR + tx * WPT + k];
+        acc = satd4x4<WPT>(sw, pw);
       }
     }
     acc = __reduce_add_sync(kFull, acc);  // a warp's 32 jobs are tiles of one candidate (NT >= 64)

@@ -126,3 +126,24 @@ def test_a_launch_of_more_than_128_dataflow_frames(ms):
         assert_results_equal(got, want, "frame of 200")
     ms.release(2700)
     ms.release(2701)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("codec,bd", [(HEVC, 8), (HEVC, 12), (H264, 8), (H264, 12)])
+@pytest.mark.parametrize("kw", [{}, dict(hevc_amp=15, hevc_lambda_scale=1024.0)])
+def test_distortion_and_rate_at_their_ends(ms, codec, bd, kw):
+    """Samples at the depth's ends only, in stripes, squares and noise, so
+    that Hadamard sums reach their largest magnitudes; the largest rates."""
+    rng = np.random.default_rng(bd + len(kw))
+    w, h, top = 144, 80, (1 << bd) - 1
+    yy, xx = np.mgrid[0:h, 0:w]
+    fields = [xx % 2, yy % 2, (xx + yy) % 2, rng.integers(0, 2, (h, w)), np.zeros((h, w)), (xx // 2 + yy // 2) % 2]
+    pics = [(np.asarray(f) * top).astype(np.uint8 if bd == 8 else np.uint16) for f in fields]
+    for i, pic in enumerate(pics):
+        ms.upload(2800 + i, pic, codec, bd)
+    p = oracle.params(codec, 63 if kw else 12, **kw)
+    for a, b in [(0, 1), (2, 4), (3, 2), (5, 3), (1, 5)]:
+        got = ms.search(2800 + a, [2800 + b], p)
+        assert_results_equal(got, oracle.frame_search(codec, bd, pics[a], [pics[b]], p), f"fields {a} against {b}")
+    for i in range(len(pics)):
+        ms.release(2800 + i)
