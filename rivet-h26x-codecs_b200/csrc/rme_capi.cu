@@ -760,9 +760,11 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   // 0.53 against 1.60 ms for one CIF frame and 0.86 against 2.49 ms for a
   // hundred, 9.6 against 14.7 ms for 64 720p frames of two references, 20.4
   // against 27.4 ms for 24 1080p 10-bit frames of three); HEVC without AMP
-  // units in a launch of the latency form (one 1080p frame 3.1 ms, on the
-  // dataflow form's best shape 7.3).
-  bool rows[kParts] = {spec, true, spec, true};
+  // units too (against the dataflow form with the same arithmetic: one 1080p
+  // frame 1.8 against 6 ms, twelve 8.4 against 10.8, 24 of 10 bits 25.0
+  // against 26.2, 100 360p frames 6.6 against 6.8; only forty 1080p frames
+  // are 4 % slower, 25.3 against 24.2).
+  bool rows[kParts] = {true, true, true, true};
   int rows_nref[kParts] = {0, 0, 0, 0};
   for (int i = 0; i < n; ++i) {
     const FrameDesc& fd = sl.h_frames.p[i];

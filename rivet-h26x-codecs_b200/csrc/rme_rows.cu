@@ -10,18 +10,30 @@
 //   - no queue between blocks: a finished block publishes its vector as one
 //     word (tag, vector), and a block waits (bounded) for its upper and
 //     parent words only, loaded a block ahead; its left vector is at hand;
-//   - many threads a block and few steps: an 8x8 block has 128 threads, a
-//     16x16 or 32x32 block 256, a 64x64 block 512, so that a step is a
-//     handful of loads a thread, one shuffle sum and one barrier;
-//   - speculation instead of dependence for 8x8 and 16x16 blocks: every
-//     seed's SAD and those of the twelve points two diamond rounds around it
-//     can reach are scored together;
-//   - the next block's source is on its way while a block is searched.
+//   - several warps a block and few steps: an 8x8 block has 64 threads, a
+//     16x16 or 32x32 block 128, a 64x64 block 256, so that a step is a few
+//     loads a thread, a short sum and one barrier. More threads would repeat
+//     the decisions, which every warp of a group takes, for less: 128 threads
+//     an 8x8 block or 256 a 16x16 block gain 0 to 4 % on one 1080p frame and
+//     lose 8 to 20 % on launches of two to forty; half as many threads lose
+//     10 to 60 %;
+//   - speculation instead of dependence: the first step of an 8x8 or 16x16
+//     block scores all seeds and, around the two likeliest, the twelve points
+//     two diamond rounds can reach; later steps, and those of larger blocks,
+//     score two rounds at once;
+//   - a 32x32 or 64x64 block's diamond reads a window staged in shared memory
+//     while the seeds are scored, a thread its words' twelve candidates;
+//   - the next block's source is on its way while a block is searched;
+//   - 128 registers a thread, two CTAs an SM: three (80 registers) lose 8 to
+//     25 % at every launch size.
 // Which candidates are scored, in which order they win and how many are
 // counted is the reference's walk (h265_me.rs:3749-3922), as hevc_task runs
-// it with one warp.
+// it with one warp. Search kernel, one B200, before (dataflow or a warp a
+// row, the faster) and now: one 1080p frame of two references 3.8 -> 1.8 ms,
+// 850x478 1.59 -> 0.70 ms, twelve 1080p frames 13.4 -> 8.4 ms, one 2160p
+// 10-bit frame of four references 33 -> 11.7 ms.
 //
-// A CTA is 512 threads: one row of 64x64 blocks, two of 32x32 or 16x16, four
+// A CTA is 256 threads: one row of 64x64 blocks, two of 32x32 or 16x16, four
 // of 8x8. Rows are taken in the order the host pushed them, each after the
 // rows it reads, so the owner of a row that is waited for is always running.
 #include <algorithm>
@@ -31,19 +43,20 @@
 namespace rme {
 namespace {
 
-constexpr int kRowThreads = 512;
+constexpr int kRowThreads = 256;
 
 // Threads that share a block of N x N samples.
-constexpr int row_group(int n) { return n == 64 ? 512 : n == 8 ? 128 : 256; }
+constexpr int row_group(int n) { return n == 64 ? 256 : n == 8 ? 64 : 128; }
 
-constexpr int kSeeds = 4;          // zero, the AMVP pair, the parent
-constexpr int kAround = 16;        // slots per centre: the centre, its 12 points, three empty
-constexpr int kSlotCosts = kSeeds * kAround;
+// A step's candidates of an 8x8 or 16x16 block: 32 slots.
+constexpr int kSlots = 32;
+constexpr uint32_t kNoKey = 0xffffffffu;  // a slot without a candidate
 
 template <class S, int N>
 struct SmallSmem {
   uint32_t src[2][N * N * sizeof(S) / 4];
-  uint32_t cost[2][kSlotCosts];
+  uint32_t key[2][kSlots];  // cost << 5 | slot (a cost is below 2^26: at most 64 * 64 * 4095 and the largest rate)
+  uint32_t satd[2][16];     // half, quarter
 };
 
 // The points two rounds of the small diamond can reach, in an order in
@@ -85,7 +98,7 @@ __device__ __forceinline__ RowInfo<S> row_info(const FrameDesc& F, int l, int r,
 
 // The totals of a thread's rows (thread 0 of each group counts).
 struct RowCount {
-  unsigned long long tasks = 0, sad = 0, satd = 0, sad_samples = 0, satd_samples = 0;
+  uint32_t tasks = 0, sad = 0, satd = 0, area = 0;
 };
 
 // A row of 8x8 or 16x16 blocks by T threads.
@@ -93,27 +106,43 @@ template <class S, int N, int T>
 __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, int row, SmallSmem<S, N>& sm, int tid,
                           int bar, RowCount& cnt) {
   constexpr int SPW = 4 / (int)sizeof(S), WR = N / SPW, NSRC = N * WR, TW = N / 4, NT = TW * TW, WPT = 4 / SPW;
+  constexpr int PS = (NSRC + T - 1) / T;  // source words a thread stages
   const int y = row * N, lane = tid & 31;
   const RowInfo<S> I = row_info<S>(F, l, r, y);
   const unsigned long long* const up = I.mvf + ((ptrdiff_t)(I.base + (row - 1) * I.nbx)) * I.nref + I.r;
   const unsigned long long* const par = I.mvf + (ptrdiff_t)I.pbase * I.nref + I.r;
-  const int stride = I.ref.stride;
+  const int stride = I.ref.stride, range = I.range;
   const float lam = I.lam;
   // The word of the parent of the block at x, or null where there is none.
   auto parent_of = [&](int x) -> const unsigned long long* {
     const int px = I.psize ? x / I.psize : 0;
     return I.psize && px < I.pnbx ? par + (ptrdiff_t)px * I.nref : nullptr;
   };
-  auto load_src = [&](int bx) -> uint32_t {  // word tid of the block (aligned: N and the pad are whole words)
-    return RME_LD32(reinterpret_cast<const uint32_t*>(plane_at<S>(I.src, 0, bx * N, y + tid / WR)) + tid % WR);
+  auto load_src = [&](int bx, uint32_t (&v)[PS]) {  // aligned: N and the pad are whole words
+#pragma unroll
+    for (int k = 0; k < PS; ++k) {
+      const int i = tid + k * T;
+      v[k] = i < NSRC ? RME_LD32(reinterpret_cast<const uint32_t*>(plane_at<S>(I.src, 0, bx * N, y + i / WR)) + i % WR)
+                      : 0u;
+    }
   };
-  if (tid < NSRC) sm.src[0][tid] = load_src(0);
+  auto store_src = [&](uint32_t* dst, const uint32_t (&v)[PS]) {
+#pragma unroll
+    for (int k = 0; k < PS; ++k)
+      if (tid + k * T < NSRC) dst[tid + k * T] = v[k];
+  };
+  uint32_t nsrc[PS];
+  load_src(0, nsrc);
+  store_src(sm.src[0], nsrc);
   unsigned long long uw = row > 0 ? ld_relaxed64(up) : 0ull, pw = 0ull;
   if (const unsigned long long* p = parent_of(0)) pw = ld_relaxed64(p);
   uint32_t lv = 0;
-  int buf = 0;  // the cost buffer of the next step
-  const int slot = tid / (T / kSlotCosts), aq = slot & (kAround - 1), ax = around_x(aq), ay = around_y(aq);
-  const int slot16 = tid / (T / kAround), bx16 = around_x(slot16), by16 = around_y(slot16);
+  int buf = 0;  // the key buffer of the next step
+  // This thread's slot of a step, and its place around a centre: as one of
+  // the first step's two (slots 1..13 and 16..28), as the only one (0..12).
+  const int slot = tid / (T / kSlots), q2 = slot < 16 ? slot - 1 : slot - 16;
+  const bool in2 = q2 >= 0 && q2 < 13;
+  const int ax = around_x(max(q2, 0)), ay = around_y(max(q2, 0)), cxo = around_x(slot), cyo = around_y(slot);
   group_sync<T>(bar);
   for (int bx = 0; bx < I.nbx; ++bx) {
     const int x = bx * N;
@@ -124,229 +153,212 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
     __syncwarp();
     const uint32_t uv = (uint32_t)uw, pv = pp ? (uint32_t)pw : 0u;
     // The next block's words and source, on their way during the search.
-    uint32_t nsrc = 0;
     if (bx + 1 < I.nbx) {
       if (row > 0) uw = ld_relaxed64(up + (ptrdiff_t)(bx + 1) * I.nref);
       if (const unsigned long long* p = parent_of(x + N)) pw = ld_relaxed64(p);
-      if (tid < NSRC) nsrc = load_src(bx + 1);
+      load_src(bx + 1, nsrc);
     }
     // The AMVP pair (left, upper when another; zero-filled) and the seeds
     // [zero, mvp0, mvp1, parent], floored to whole samples and clamped.
-    int p0x = 0, p0y = 0, p1x = 0, p1y = 0;
+    uint32_t m0 = 0, m1 = 0;
     if (bx > 0) {
-      p0x = mvx_of(lv);
-      p0y = mvy_of(lv);
-      if (row > 0 && uv != lv) {
-        p1x = mvx_of(uv);
-        p1y = mvy_of(uv);
-      }
+      m0 = lv;
+      if (row > 0 && uv != lv) m1 = uv;
     } else if (row > 0) {
-      p0x = mvx_of(uv);
-      p0y = mvy_of(uv);
+      m0 = uv;
     }
+    const int p0x = mvx_of(m0), p0y = mvy_of(m0), p1x = mvx_of(m1), p1y = mvy_of(m1);
     const int lox = -I.padm - x, hix = I.width + I.padm - N - x, loy = -I.padm - y, hiy = I.height + I.padm - N - y;
-    int kx[kSeeds], ky[kSeeds];
-    uint32_t kept = 0;
-    {
-      const int sx[kSeeds] = {0, p0x, p1x, mvx_of(pv)}, sy[kSeeds] = {0, p0y, p1y, mvy_of(pv)};
-#pragma unroll
-      for (int i = 0; i < kSeeds; ++i) {
-        kx[i] = min(max(sx[i] >> 2, lox), hix);
-        ky[i] = min(max(sy[i] >> 2, loy), hiy);
-        bool dup = i == 3 && !pp;
-#pragma unroll
-        for (int j = 0; j < i; ++j) dup |= kx[j] == kx[i] && ky[j] == ky[i];
-        kept |= (dup ? 0u : 1u) << i;
-      }
-    }
-    auto seed_x = [&](int i) { return i == 0 ? kx[0] : i == 1 ? kx[1] : i == 2 ? kx[2] : kx[3]; };
-    auto seed_y = [&](int i) { return i == 0 ? ky[0] : i == 1 ? ky[1] : i == 2 ? ky[2] : ky[3]; };
+    auto to_x = [&](int v) { return min(max(v >> 2, lox), hix); };
+    auto to_y = [&](int v) { return min(max(v >> 2, loy), hiy); };
+    const int zx = to_x(0), zy = to_y(0), ux = to_x(p0x), uy = to_y(p0y), vx = to_x(p1x), vy = to_y(p1y);
+    const int wx = to_x(mvx_of(pv)), wy = to_y(mvy_of(pv));
+    // A seed on an earlier one's point is not scored again (`tried`).
+    const bool k1 = ux != zx || uy != zy, k2 = (vx != zx || vy != zy) && (vx != ux || vy != uy);
+    const bool k3 = pp && (wx != zx || wy != zy) && (wx != ux || wy != uy) && (wx != vx || wy != vy);
+    uint32_t nsad = 1u + k1 + k2 + k3, nsatd = 9;
     const S* const org = plane_at<S>(I.ref, 0, x, y);
-    uint32_t nsad = __popc(kept), nsatd = 9;
-    // A candidate's SAD over LPC lanes (rows sub, sub + LPC, ...) and its
-    // cost into its slot, then the barrier: every cost in `costs`.
-    const uint32_t* costs = nullptr;
-    auto score = [&](auto lanes, int at, bool ok, int fx, int fy) {
-      constexpr int LPC = decltype(lanes)::value, RPL = N / LPC;
+    auto inside = [&](int fx, int fy) { return fx >= lox && fx <= hix && fy >= loy && fy <= hiy; };
+    // A candidate's SAD over its slot's LPC lanes (rows sub, sub + LPC, ...)
+    // and its key into the slot `at`, then the barrier; lane i of every warp
+    // gets slot i's key.
+    auto score = [&](auto lanes, int at, bool ok, int fx, int fy) -> uint32_t {
+      constexpr int LPC = decltype(lanes)::value, RPL = N / LPC, UN = RPL * WR <= 16 ? RPL : 16 / WR;
       const int sub = tid % LPC;
       uint32_t acc = 0;
       if (ok) {
         const S* rp = org + (ptrdiff_t)(fy + sub) * stride + fx;
-        if constexpr (RPL * WR <= 16) {  // every load before any use
-          uint32_t a[RPL][WR];
 #pragma unroll
-          for (int k = 0; k < RPL; ++k) ldwords<WR>(rp + (ptrdiff_t)k * LPC * stride, a[k]);
+        for (int k0 = 0; k0 < RPL; k0 += UN) {
+          uint32_t a[UN][WR];
 #pragma unroll
-          for (int k = 0; k < RPL; ++k)
+          for (int k = 0; k < UN; ++k) ldwords<WR>(rp + (ptrdiff_t)(k0 + k) * LPC * stride, a[k]);
 #pragma unroll
-            for (int c = 0; c < WR; ++c) acc = vsad(src[(sub + k * LPC) * WR + c], a[k][c], acc, S());
-        } else {
-#pragma unroll 2
-          for (int k = 0; k < RPL; ++k) {
-            uint32_t a[WR];
-            ldwords<WR>(rp + (ptrdiff_t)k * LPC * stride, a);
+          for (int k = 0; k < UN; ++k)
 #pragma unroll
-            for (int c = 0; c < WR; ++c) acc = vsad(src[(sub + k * LPC) * WR + c], a[c], acc, S());
-          }
+            for (int c = 0; c < WR; ++c) acc = vsad(src[(sub + (k0 + k) * LPC) * WR + c], a[k][c], acc, S());
         }
       }
 #pragma unroll
       for (int o = LPC >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
-      uint32_t* c = sm.cost[buf];
+      uint32_t* c = sm.key[buf];
       buf ^= 1;
-      if (sub == 0) c[at] = ok ? acc + hevc_rate(lam, fx * 4, fy * 4, p0x, p0y, p1x, p1y) : kInf;
+      if (sub == 0)
+        c[at] = ok ? (acc + hevc_rate(lam, fx * 4, fy * 4, p0x, p0y, p1x, p1y)) << 5 | (uint32_t)at : kNoKey;
       group_sync<T>(bar);
-      costs = c;
+      return c[lane];
     };
-    // Every seed with the points two rounds around it.
-    const int range = I.range;
+    // First step. Slot 0 the zero seed; 1..13 mvp0 with the points around
+    // it; 14 mvp1 where the parent takes 16..28, else 16..28 mvp1 with the
+    // points around it.
+    const int gx = pp ? wx : vx, gy = pp ? wy : vy;
+    uint32_t key;
     {
-      const int i = slot / kAround, sx = seed_x(i), sy = seed_y(i), fx = sx + ax, fy = sy + ay;
-      const bool ok = ((kept >> i) & 1u) && aq < 13 &&
-                      (aq == 0 || (abs(ax) <= range && abs(ay) <= range && fx >= lox && fx <= hix && fy >= loy && fy <= hiy));
-      score(std::integral_constant<int, T / kSlotCosts>{}, slot, ok, fx, fy);
+      const bool a = slot < 16;
+      int fx = (a ? ux : gx) + ax, fy = (a ? uy : gy) + ay;
+      bool ok = in2 && (ax | ay) != 0 ? abs(ax) <= range && abs(ay) <= range && inside(fx, fy) : in2;
+      if (slot == 0) {
+        fx = zx;
+        fy = zy;
+        ok = true;
+      } else if (slot == 14) {
+        fx = vx;
+        fy = vy;
+        ok = pp != nullptr;
+      }
+      key = score(std::integral_constant<int, T / kSlots>{}, slot, ok, fx, fy);
     }
-    int ox, oy, mxw, myw;  // the best seed; the best whole-sample point
-    uint32_t bcost, c;
-    {
-      const Pick p = warp_min(lane < kSeeds ? costs[lane * kAround] : kInf);
-      bcost = p.cost;
-      mxw = ox = seed_x(p.lane);
-      myw = oy = seed_y(p.lane);
-      c = lane < kAround ? costs[p.lane * kAround + lane] : kInf;
-    }
-    int it = 0, rings = 0;
-    for (bool known = true;;) {
-      // The diamond, two rounds a step, from the costs `c` of the points
-      // around the best (lane q: point q).
+    // The best seed, the first in order (slots 0, 1, 14, 16) of least cost.
+    uint32_t best = __reduce_min_sync(kFull, (0x14003u >> lane) & 1u ? key : kNoKey);
+    const int s0 = (int)(best & 31u);
+    const int ox = s0 == 0 ? zx : s0 == 1 ? ux : s0 == 14 ? vx : gx, oy = s0 == 0 ? zy : s0 == 1 ? uy : s0 == 14 ? vy : gy;
+    int fbx = ox, fby = oy;        // the best whole-sample point
+    uint32_t bcost = best >> 5;
+    int base = ox == ux && oy == uy ? 1 : ox == gx && oy == gy ? 16 : -1;  // its points' slots, where scored
+    // The diamond, two rounds a step.
+    for (int it = 0, rings = 0;;) {
       while (it < 2 * range) {
-        if (!known) {
-          const int fx = mxw + bx16, fy = myw + by16;
-          const bool ok = slot16 > 0 && slot16 < 13 && abs(fx - ox) <= range && abs(fy - oy) <= range && fx >= lox &&
-                          fx <= hix && fy >= loy && fy <= hiy;
-          score(std::integral_constant<int, T / kAround>{}, slot16, ok, fx, fy);
-          c = lane < kAround ? costs[lane] : kInf;
+        if (base < 0) {
+          const int fx = fbx + cxo, fy = fby + cyo;
+          const bool ok = slot > 0 && slot < 13 && abs(fx - ox) <= range && abs(fy - oy) <= range && inside(fx, fy);
+          key = score(std::integral_constant<int, T / kSlots>{}, slot, ok, fx, fy);
+          base = 0;
         }
-        known = false;
-        const uint32_t in1 = lane >= 1 && lane <= 4 ? c : kInf;
-        nsad += __popc(__ballot_sync(kFull, in1 != kInf));
-        Pick p = warp_min(in1);
-        if (!(p.cost < bcost)) break;
-        const int j = p.lane - 1;
-        bcost = p.cost;
-        mxw += around_x(p.lane);
-        myw += around_y(p.lane);
-        if (++it >= 2 * range) break;
-        const int cx = mxw - around_x(p.lane), cy = myw - around_y(p.lane);
-        const uint32_t in2 = (second_round(j) >> lane) & 1u ? c : kInf;
-        nsad += 1u + __popc(__ballot_sync(kFull, in2 != kInf));  // the fourth point is the old best
-        p = warp_min(in2);
-        if (!(p.cost < bcost)) break;
-        bcost = p.cost;
-        mxw = cx + around_x(p.lane);
-        myw = cy + around_y(p.lane);
+        const uint32_t there = __ballot_sync(kFull, key != kNoKey) >> base;  // bit q: point q is scored
+        const int q = lane - base;
+        nsad += __popc(there & 0x1eu);
+        uint32_t m = __reduce_min_sync(kFull, q >= 1 && q <= 4 ? key : kNoKey);
+        if (!(m >> 5 < bcost)) break;
+        const int q1 = (int)(m & 31u) - base;
+        bcost = m >> 5;
+        const int x1 = around_x(q1), y1 = around_y(q1);
+        const uint32_t second = second_round(q1 - 1);
+        if (++it >= 2 * range) {
+          fbx += x1;
+          fby += y1;
+          break;
+        }
+        nsad += 1u + __popc(there & second);  // the fourth point is the old best
+        m = __reduce_min_sync(kFull, q >= 0 && ((second >> q) & 1u) ? key : kNoKey);
+        if (!(m >> 5 < bcost)) {
+          fbx += x1;
+          fby += y1;
+          break;
+        }
+        bcost = m >> 5;
+        const int q3 = (int)(m & 31u) - base;
+        fbx += around_x(q3);
+        fby += around_y(q3);
         ++it;
+        base = -1;
       }
       if (rings >= I.rings) break;
       ++rings;
       // The 24 ring points at 4, 8, 16 around the settled point, in order;
       // a move restarts the diamond.
-      const int k = tid / (T / 32), rr = k < 8 ? 4 : k < 16 ? 8 : 16;
-      auto ring_x = [](int q, int d) { return q == 0 || q == 4 || q == 6 ? d : q == 1 || q == 5 || q == 7 ? -d : 0; };
-      auto ring_y = [](int q, int d) { return q == 2 || q == 4 || q == 5 ? d : q == 3 || q == 6 || q == 7 ? -d : 0; };
-      const int fx = mxw + ring_x(k & 7, rr), fy = myw + ring_y(k & 7, rr);
-      const bool ok = k < 24 && abs(fx - ox) <= range && abs(fy - oy) <= range && fx >= lox && fx <= hix && fy >= loy &&
-                      fy <= hiy;
-      score(std::integral_constant<int, T / 32>{}, k, ok, fx, fy);
-      c = lane < 24 ? costs[lane] : kInf;
-      nsad += __popc(__ballot_sync(kFull, c != kInf));
-      const Pick p = warp_min(c);
-      if (!(p.cost < bcost)) break;
-      bcost = p.cost;
-      const int pr = p.lane < 8 ? 4 : p.lane < 16 ? 8 : 16;
-      mxw += ring_x(p.lane & 7, pr);
-      myw += ring_y(p.lane & 7, pr);
+      auto ring_x = [](int k) {
+        const int d = k < 8 ? 4 : k < 16 ? 8 : 16, c = k & 7;
+        return c == 0 || c == 4 || c == 6 ? d : c == 1 || c == 5 || c == 7 ? -d : 0;
+      };
+      auto ring_y = [](int k) {
+        const int d = k < 8 ? 4 : k < 16 ? 8 : 16, c = k & 7;
+        return c == 2 || c == 4 || c == 5 ? d : c == 3 || c == 6 || c == 7 ? -d : 0;
+      };
+      const int fx = fbx + ring_x(slot), fy = fby + ring_y(slot);
+      const bool ok = slot < 24 && abs(fx - ox) <= range && abs(fy - oy) <= range && inside(fx, fy);
+      key = score(std::integral_constant<int, T / kSlots>{}, slot, ok, fx, fy);
+      nsad += __popc(__ballot_sync(kFull, key != kNoKey));
+      const uint32_t m = __reduce_min_sync(kFull, key);
+      if (!(m >> 5 < bcost)) break;
+      bcost = m >> 5;
+      fbx += ring_x((int)(m & 31u));
+      fby += ring_y((int)(m & 31u));
       it = 0;
+      base = -1;
     }
     const uint32_t int_cost = bcost;
-    const int imx = mxw * 4, imy = myw * 4;
+    const int imx = fbx * 4, imy = fby * 4;
 
     // refine_subpel: the start and the half ring in one step, then the
     // quarter ring around the winner; a thread per 4x4 tile, NT threads a
-    // candidate.
-    auto satd = [&](int nc, auto vec) {
-      const int k = tid / NT, tile = tid % NT, ty = tile / TW, tx = tile % TW;
-      int mx, my;
-      uint32_t v = 0;
-      if (k < nc && vec(k, mx, my)) {
-        const S* q = plane_at<S>(I.ref, (my & 3) * 4 + (mx & 3), x + (mx >> 2) + tx * 4, y + (my >> 2) + ty * 4);
-        uint32_t pw4[4][WPT];
-#pragma unroll
-        for (int rr = 0; rr < 4; ++rr) ldwords<WPT>(q + (ptrdiff_t)rr * stride, pw4[rr]);
-        uint32_t sw[4][WPT];
-#pragma unroll
-        for (int rr = 0; rr < 4; ++rr)
-#pragma unroll
-          for (int w = 0; w < WPT; ++w) sw[rr][w] = src[(ty * 4 + rr) * WR + tx * WPT + w];
-        v = satd4x4<WPT>(sw, pw4);
-      }
-#pragma unroll
-      for (int o = NT >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-      uint32_t* cb = sm.cost[buf];
+    // candidate. Returns lane i's candidate's key.
+    auto satd = [&](auto count, auto vec) -> uint32_t {
+      constexpr int NC = decltype(count)::value;
+      uint32_t* kb = sm.key[buf];
       buf ^= 1;
-      if (tile == 0 && k < nc) cb[k] = v;
+#pragma unroll
+      for (int j0 = 0; j0 < NC * NT; j0 += T) {
+        const int j = j0 + tid, k = j / NT, tile = j % NT, ty = tile / TW, tx = tile % TW;
+        if (j0 + (tid & ~31) >= NC * NT) break;  // none of the warp's
+        int mx = 0, my = 0;
+        uint32_t v = 0;
+        const bool ok = k < NC && vec(k, mx, my);
+        if (ok) {
+          const S* q = plane_at<S>(I.ref, (my & 3) * 4 + (mx & 3), x + (mx >> 2) + tx * 4, y + (my >> 2) + ty * 4);
+          uint32_t pr[4][WPT], sw[4][WPT];
+#pragma unroll
+          for (int rr = 0; rr < 4; ++rr) ldwords<WPT>(q + (ptrdiff_t)rr * stride, pr[rr]);
+#pragma unroll
+          for (int rr = 0; rr < 4; ++rr)
+#pragma unroll
+            for (int w = 0; w < WPT; ++w) sw[rr][w] = src[(ty * 4 + rr) * WR + tx * WPT + w];
+          v = satd4x4<WPT>(sw, pr);
+        }
+#pragma unroll
+        for (int o = NT >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+        if (tile == 0 && k < NC) {
+          sm.satd[NC == 8][k] = v;
+          kb[k] = ok ? (v + hevc_rate(lam, mx, my, p0x, p0y, p1x, p1y)) << 5 | (uint32_t)k : kNoKey;
+        }
+      }
       group_sync<T>(bar);
-      costs = cb;
+      return lane < NC ? kb[lane] : kNoKey;
     };
     auto half_vec = [&](int k, int& mx, int& my) {
-      const int q = k == 0 ? 4 : k <= 4 ? k - 1 : k;
-      mx = imx + (q % 3 - 1) * 2;
-      my = imy + (q / 3 - 1) * 2;
+      const int q = k == 0 ? 4 : k <= 4 ? k - 1 : k, qy = q / 3;
+      mx = imx + (q - qy * 3 - 1) * 2;
+      my = imy + (qy - 1) * 2;
       return true;
     };
-    satd(9, half_vec);
+    uint32_t m = __reduce_min_sync(kFull, satd(std::integral_constant<int, 9>{}, half_vec));
     int bmx, bmy;
-    uint32_t bc, bsatd;
-    {
-      int mx = imx, my = imy;
-      uint32_t v = 0, cost = kInf;
-      if (lane < 9) {
-        half_vec(lane, mx, my);
-        v = costs[lane];
-        cost = v + hevc_rate(lam, mx, my, p0x, p0y, p1x, p1y);
-      }
-      const Pick p = warp_min(cost);
-      bc = p.cost;
-      bsatd = __shfl_sync(kFull, v, p.lane);
-      bmx = __shfl_sync(kFull, mx, p.lane);
-      bmy = __shfl_sync(kFull, my, p.lane);
-    }
+    half_vec((int)(m & 31u), bmx, bmy);
+    uint32_t bc = m >> 5, bsatd = sm.satd[0][m & 31u];
     const int hmx = bmx, hmy = bmy, cross = I.cross;
     auto quarter_vec = [&](int k, int& mx, int& my) {
-      const int q = k < 4 ? k : k + 1, dx = q % 3 - 1, dy = q / 3 - 1;
+      const int q = k < 4 ? k : k + 1, qy = q / 3, dx = q - qy * 3 - 1, dy = qy - 1;
       mx = (int)(int16_t)(hmx + dx);
       my = (int)(int16_t)(hmy + dy);
       return !(cross != 0 && dx != 0 && dy != 0);
     };
-    if (tid < NSRC) sm.src[(bx + 1) & 1][tid] = nsrc;
-    satd(8, quarter_vec);
-    {
-      int mx = 0, my = 0;
-      uint32_t v = 0, cost = kInf;
-      bool ok = false;
-      if (lane < 8) ok = quarter_vec(lane, mx, my);
-      if (ok) {
-        v = costs[lane];
-        cost = v + hevc_rate(lam, mx, my, p0x, p0y, p1x, p1y);
-      }
-      nsatd += __popc(__ballot_sync(kFull, ok));
-      const Pick p = warp_min(cost);
-      if (p.cost < bc) {
-        bc = p.cost;
-        bsatd = __shfl_sync(kFull, v, p.lane);
-        bmx = __shfl_sync(kFull, mx, p.lane);
-        bmy = __shfl_sync(kFull, my, p.lane);
-      }
+    store_src(sm.src[(bx + 1) & 1], nsrc);
+    const uint32_t qkey = satd(std::integral_constant<int, 8>{}, quarter_vec);
+    nsatd += cross ? 4 : 8;
+    m = __reduce_min_sync(kFull, qkey);
+    if (m != kNoKey && m >> 5 < bc) {
+      bc = m >> 5;
+      bsatd = sm.satd[1][m & 31u];
+      quarter_vec((int)(m & 31u), bmx, bmy);
     }
     lv = (uint32_t)(uint16_t)(int16_t)bmx | (uint32_t)(uint16_t)(int16_t)bmy << 16;
     if (tid == 0) {
@@ -356,30 +368,347 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
       cnt.tasks += 1;
       cnt.sad += nsad;
       cnt.satd += nsatd;
-      cnt.sad_samples += (unsigned long long)nsad * (N * N);
-      cnt.satd_samples += (unsigned long long)nsatd * (N * N);
     }
   }
-  group_sync<T>(bar);  // the last block's costs and source are read: the buffers may be reused
+  cnt.area = N * N;
+  group_sync<T>(bar);  // the last block's keys and source are read: the buffers may be reused
 }
 
-// A row of 32x32 or 64x64 blocks by T threads: the group search (GroupSmem,
-// its window behind it), its counts in the GroupSmem.
+// A 32x32 or 64x64 block's window: the reference's integer plane around a
+// centre, kMargin samples beyond the block on every side, as the aligned
+// words that hold it. A diamond step from any point within kMargin - 2 of the
+// centre reads the window only.
+constexpr int kMargin = 8;
+template <class S, int N>
+struct BigSmem {
+  static constexpr int ROWS = N + 2 * kMargin, WRW = (N + 2 * kMargin) * (int)sizeof(S) / 4 + 1;
+  uint32_t src[2][N * N * sizeof(S) / 4];
+  uint32_t win[ROWS * WRW];
+  uint32_t cost[3][32];  // a step's distortions, summed over the warps; in turn, the next one cleared a step ahead
+};
+
+// A row of 32x32 or 64x64 blocks by T threads: a thread has PW words of the
+// block for the SADs (a warp's lanes side by side in a row) and a 4x4 tile
+// for the SATDs, and scores every candidate of a step on them; the warps'
+// sums meet in shared memory, one barrier a step.
 template <class S, int N, int T>
-__device__ void big_row(const LaunchDesc& L, const FrameDesc& F, int f, int l, int r, int row, GroupSmem<S>& gs,
-                        int tid, int bar) {
-  const int nbx = F.nbx[l], t0 = (F.base[l] + row * nbx) * F.nref + r;
-  for (int bx = 0; bx < nbx; ++bx) hevc_group_task<S, N, true, T>(L, F, f, t0 + bx * F.nref, gs, tid, bar);
+__device__ void big_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, int row, BigSmem<S, N>& sm, int tid,
+                        int bar, RowCount& cnt) {
+  constexpr int B = (int)sizeof(S), SPW = 4 / B, WR = N / SPW, NSRC = N * WR, PW = NSRC / T, RSTEP = T / WR;
+  constexpr int TW = N / 4, NT = TW * TW, WPT = 4 / SPW, WRW = BigSmem<S, N>::WRW, ROWS = BigSmem<S, N>::ROWS;
+  static_assert(NSRC % T == 0 && T % WR == 0 && T % NT == 0, "a thread's words and tile");
+  const int y = row * N, lane = tid & 31, wd = tid % WR, row0 = tid / WR;
+  const RowInfo<S> I = row_info<S>(F, l, r, y);
+  const unsigned long long* const up = I.mvf + ((ptrdiff_t)(I.base + (row - 1) * I.nbx)) * I.nref + I.r;
+  const unsigned long long* const par = I.mvf + (ptrdiff_t)I.pbase * I.nref + I.r;
+  const int stride = I.ref.stride, range = I.range, plane = (int)I.ref.plane_elems;
+  const float lam = I.lam;
+  auto parent_of = [&](int x) -> const unsigned long long* {
+    const int px = I.psize ? x / I.psize : 0;
+    return I.psize && px < I.pnbx ? par + (ptrdiff_t)px * I.nref : nullptr;
+  };
+  // This thread's words: word wd of rows row0, row0 + RSTEP, ...
+  auto load_src = [&](int bx, uint32_t (&v)[PW]) {
+    const uint32_t* o = reinterpret_cast<const uint32_t*>(plane_at<S>(I.src, 0, bx * N, y + row0)) + wd;
+#pragma unroll
+    for (int k = 0; k < PW; ++k) v[k] = RME_LD32(o + (ptrdiff_t)k * RSTEP * I.src.stride * B / 4);
+  };
+  uint32_t sw[PW];
+  load_src(0, sw);
+  unsigned long long uw = row > 0 ? ld_relaxed64(up) : 0ull, pw = 0ull;
+  if (const unsigned long long* p = parent_of(0)) pw = ld_relaxed64(p);
+  uint32_t lv = 0;
+  int buf = 0;
+  if (tid < 32) sm.cost[0][tid] = 0u;
+  group_sync<T>(bar);
+  // After a step's sums are in `mine` (lane k: candidate k's over this warp):
+  // the totals, lane k candidate k's.
+  auto total = [&](uint32_t mine, int nc) -> uint32_t {
+    uint32_t* c = sm.cost[buf];
+    const int nx = buf == 2 ? 0 : buf + 1;
+    if (lane < nc) atomicAdd(&c[lane], mine);
+    if (tid < 32) sm.cost[nx][tid] = 0u;
+    buf = nx;
+    group_sync<T>(bar);
+    return c[lane];
+  };
+  for (int bx = 0; bx < I.nbx; ++bx) {
+    const int x = bx * N;
+    uint32_t* const src = sm.src[bx & 1];
+#pragma unroll
+    for (int k = 0; k < PW; ++k) src[tid + k * T] = sw[k];
+    if (row > 0) uw = wait_word(L, up + (ptrdiff_t)bx * I.nref, I.tag, uw);
+    const unsigned long long* const pp = parent_of(x);
+    if (pp) pw = wait_word(L, pp, I.tag, pw);
+    __syncwarp();
+    const uint32_t uv = (uint32_t)uw, pv = pp ? (uint32_t)pw : 0u;
+    if (bx + 1 < I.nbx) {
+      if (row > 0) uw = ld_relaxed64(up + (ptrdiff_t)(bx + 1) * I.nref);
+      if (const unsigned long long* p = parent_of(x + N)) pw = ld_relaxed64(p);
+    }
+    uint32_t m0 = 0, m1 = 0;
+    if (bx > 0) {
+      m0 = lv;
+      if (row > 0 && uv != lv) m1 = uv;
+    } else if (row > 0) {
+      m0 = uv;
+    }
+    const int p0x = mvx_of(m0), p0y = mvy_of(m0), p1x = mvx_of(m1), p1y = mvy_of(m1);
+    const int lox = -I.padm - x, hix = I.width + I.padm - N - x, loy = -I.padm - y, hiy = I.height + I.padm - N - y;
+    const S* const org = plane_at<S>(I.ref, 0, x, y);
+    auto inside = [&](int fx, int fy) { return fx >= lox && fx <= hix && fy >= loy && fy <= hiy; };
+    auto rate = [&](int mx, int my) { return hevc_rate(lam, mx, my, p0x, p0y, p1x, p1y); };
+    // Seeds [zero, mvp0, mvp1, parent], lane i the i-th: floored, clamped, a
+    // seed on an earlier one's point left out.
+    const uint32_t sv = lane == 1 ? m0 : lane == 2 ? m1 : lane == 3 ? pv : 0u;
+    const int sx = min(max(mvx_of(sv) >> 2, lox), hix), sy = min(max(mvy_of(sv) >> 2, loy), hiy);
+    bool keep = lane < (pp ? 4 : 3);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int jx = __shfl_sync(kFull, sx, j), jy = __shfl_sync(kFull, sy, j);
+      keep = keep && !(j < lane && jx == sx && jy == sy);
+    }
+    const uint32_t kept = __ballot_sync(kFull, keep);
+    // The window around the likeliest seed is staged while the seeds are
+    // scored: plane words clamped to the plane (a point there is no candidate).
+    int scx, scy;
+    uint32_t woff;
+    auto stage = [&](int cx, int cy) {
+      scx = cx;
+      scy = cy;
+      const int e0 = I.ref.origin + (y + cy - kMargin) * stride + x + cx - kMargin;  // may lie before the plane
+      const int w0 = (e0 * B) >> 2;
+      woff = (uint32_t)(e0 * B) & 3u;
+      const uint32_t* base = reinterpret_cast<const uint32_t*>(I.ref.base);
+      const int rs = stride * B / 4, last = plane * B / 4 - 1;
+      for (int i = tid; i < ROWS * WRW; i += T) {
+        const int rr = i / WRW, ww = i - rr * WRW;
+        sm.win[i] = RME_LD32(base + min(max(w0 + rr * rs + ww, 0), last));
+      }
+    };
+    {
+      const int gl = pp ? 3 : 1;
+      stage(__shfl_sync(kFull, sx, gl), __shfl_sync(kFull, sy, gl));
+    }
+    uint32_t nsad = __popc(kept), nsatd = 9;
+    uint32_t mine = 0;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      if (!((kept >> s) & 1u)) continue;
+      const int fx = __shfl_sync(kFull, sx, s), fy = __shfl_sync(kFull, sy, s);
+      const S* rp = org + (ptrdiff_t)(fy + row0) * stride + fx + wd * SPW;
+      uint32_t a[PW], acc = 0;
+#pragma unroll
+      for (int k = 0; k < PW; ++k) a[k] = ldw(rp + (ptrdiff_t)k * RSTEP * stride);
+#pragma unroll
+      for (int k = 0; k < PW; ++k) acc = vsad(sw[k], a[k], acc, S());
+      acc = __reduce_add_sync(kFull, acc);
+      if (lane == s) mine = acc;
+    }
+    uint32_t c = total(mine, 4);
+    c = keep ? c + rate(sx * 4, sy * 4) : kInf;
+    Pick p = warp_min(c);
+    uint32_t bcost = p.cost;
+    int fbx = __shfl_sync(kFull, sx, p.lane), fby = __shfl_sync(kFull, sy, p.lane);
+    const int ox = fbx, oy = fby;
+    // The diamond, two rounds a step: the twelve points around the best from
+    // the window (lane q: point q + 1 of the order around_x has).
+    for (int it = 0, rings = 0;;) {
+      while (it < 2 * range) {
+        if (abs(fbx - scx) > kMargin - 2 || abs(fby - scy) > kMargin - 2) {
+          group_sync<T>(bar);  // the window's last readers are done
+          stage(fbx, fby);
+          group_sync<T>(bar);
+        }
+        uint32_t acc[12];
+#pragma unroll
+        for (int q = 0; q < 12; ++q) acc[q] = 0u;
+        // The byte offset of dx = -2 in a window row, and for each dx whether
+        // its samples begin in the first or the second word from there.
+        const uint32_t b0 = woff + (uint32_t)((fbx - scx + kMargin - 2) * B);
+        const int wi = (int)(b0 >> 2), r0 = fby - scy + kMargin;
+#pragma unroll
+        for (int k = 0; k < PW; ++k) {
+          const uint32_t* wp = sm.win + (r0 + row0 + k * RSTEP) * WRW + wi + wd;
+          uint32_t w[5][4];
+#pragma unroll
+          for (int dy = -2; dy <= 2; ++dy)
+#pragma unroll
+            for (int j = 0; j < (B == 1 ? 3 : 4); ++j) w[dy + 2][j] = wp[dy * WRW + j];
+          auto at = [&](int dx, int dy) {  // the four (two) samples at dx, dy
+            const uint32_t o = (b0 & 3u) + (uint32_t)((dx + 2) * B), sh = (o & 3u) * 8u;
+            const int j = (int)(o >> 2);
+            const uint32_t lo = B == 1 ? (j ? w[dy + 2][1] : w[dy + 2][0])
+                                       : (j == 0 ? w[dy + 2][0] : j == 1 ? w[dy + 2][1] : w[dy + 2][2]);
+            const uint32_t hi = B == 1 ? (j ? w[dy + 2][2] : w[dy + 2][1])
+                                       : (j == 0 ? w[dy + 2][1] : j == 1 ? w[dy + 2][2] : w[dy + 2][3]);
+            return __funnelshift_r(lo, hi, sh);
+          };
+          const uint32_t s = sw[k];
+          acc[0] = vsad(s, at(1, 0), acc[0], S());
+          acc[1] = vsad(s, at(-1, 0), acc[1], S());
+          acc[2] = vsad(s, at(0, 1), acc[2], S());
+          acc[3] = vsad(s, at(0, -1), acc[3], S());
+          acc[4] = vsad(s, at(2, 0), acc[4], S());
+          acc[5] = vsad(s, at(-2, 0), acc[5], S());
+          acc[6] = vsad(s, at(1, 1), acc[6], S());
+          acc[7] = vsad(s, at(1, -1), acc[7], S());
+          acc[8] = vsad(s, at(-1, 1), acc[8], S());
+          acc[9] = vsad(s, at(-1, -1), acc[9], S());
+          acc[10] = vsad(s, at(0, 2), acc[10], S());
+          acc[11] = vsad(s, at(0, -2), acc[11], S());
+        }
+        mine = 0;
+#pragma unroll
+        for (int q = 0; q < 12; ++q) {
+          const uint32_t v = __reduce_add_sync(kFull, acc[q]);
+          if (lane == q) mine = v;
+        }
+        c = total(mine, 12);
+        const int q = lane + 1, fx = fbx + around_x(q & 15), fy = fby + around_y(q & 15);
+        const bool ok = lane < 12 && abs(fx - ox) <= range && abs(fy - oy) <= range && inside(fx, fy);
+        c = ok ? c + rate(fx * 4, fy * 4) : kInf;
+        const uint32_t there = __ballot_sync(kFull, ok) << 1;  // bit q: point q is scored
+        nsad += __popc(there & 0x1eu);
+        p = warp_min(lane < 4 ? c : kInf);
+        if (!(p.cost < bcost)) break;
+        bcost = p.cost;
+        const int q1 = p.lane + 1;
+        const uint32_t second = second_round(q1 - 1);
+        if (++it >= 2 * range) {
+          fbx += around_x(q1);
+          fby += around_y(q1);
+          break;
+        }
+        nsad += 1u + __popc(there & second);  // the fourth point is the old best
+        p = warp_min((second >> q) & 1u ? c : kInf);
+        if (!(p.cost < bcost)) {
+          fbx += around_x(q1);
+          fby += around_y(q1);
+          break;
+        }
+        bcost = p.cost;
+        fbx += around_x(p.lane + 1);
+        fby += around_y(p.lane + 1);
+        ++it;
+      }
+      if (rings >= I.rings) break;
+      ++rings;
+      // The 24 ring points at 4, 8, 16 around the settled point, in order.
+      auto ring_x = [](int k) {
+        const int d = k < 8 ? 4 : k < 16 ? 8 : 16, e = k & 7;
+        return e == 0 || e == 4 || e == 6 ? d : e == 1 || e == 5 || e == 7 ? -d : 0;
+      };
+      auto ring_y = [](int k) {
+        const int d = k < 8 ? 4 : k < 16 ? 8 : 16, e = k & 7;
+        return e == 2 || e == 4 || e == 5 ? d : e == 3 || e == 6 || e == 7 ? -d : 0;
+      };
+      auto allowed = [&](int fx, int fy) {
+        return abs(fx - ox) <= range && abs(fy - oy) <= range && inside(fx, fy);
+      };
+      mine = 0;
+      for (int k = 0; k < 24; ++k) {
+        const int fx = fbx + ring_x(k), fy = fby + ring_y(k);
+        if (!allowed(fx, fy)) continue;
+        const S* rp = org + (ptrdiff_t)(fy + row0) * stride + fx + wd * SPW;
+        uint32_t acc = 0;
+#pragma unroll
+        for (int j = 0; j < PW; ++j) acc = vsad(sw[j], ldw(rp + (ptrdiff_t)j * RSTEP * stride), acc, S());
+        acc = __reduce_add_sync(kFull, acc);
+        if (lane == k) mine = acc;
+      }
+      c = total(mine, 24);
+      const int fx = fbx + ring_x(min(lane, 23)), fy = fby + ring_y(min(lane, 23));
+      const bool ok = lane < 24 && allowed(fx, fy);
+      nsad += __popc(__ballot_sync(kFull, ok));
+      p = warp_min(ok ? c + rate(fx * 4, fy * 4) : kInf);
+      if (!(p.cost < bcost)) break;
+      bcost = p.cost;
+      fbx += ring_x(p.lane);
+      fby += ring_y(p.lane);
+      it = 0;
+    }
+    const uint32_t int_cost = bcost;
+    const int imx = fbx * 4, imy = fby * 4;
+    // The next block's source, on its way during the refinement.
+    if (bx + 1 < I.nbx) load_src(bx + 1, sw);
+
+    // refine_subpel: T / NT candidates at a time, a thread per 4x4 tile.
+    const int tile = tid % NT, ty = tile / TW, tx = tile % TW, cg = tid / NT;
+    uint32_t st[4][WPT];
+#pragma unroll
+    for (int rr = 0; rr < 4; ++rr)
+#pragma unroll
+      for (int w = 0; w < WPT; ++w) st[rr][w] = src[(ty * 4 + rr) * WR + tx * WPT + w];
+    auto satd = [&](auto count, auto vec) -> uint32_t {
+      constexpr int NC = decltype(count)::value, CG = T / NT;
+      uint32_t got = 0;
+#pragma unroll 2
+      for (int k0 = 0; k0 < NC; k0 += CG) {
+        const int k = k0 + cg;
+        int mx, my;
+        uint32_t v = 0;
+        if (k < NC && vec(k, mx, my)) {  // the same for a warp's lanes
+          const S* q = plane_at<S>(I.ref, (my & 3) * 4 + (mx & 3), x + (mx >> 2) + tx * 4, y + (my >> 2) + ty * 4);
+          uint32_t pr[4][WPT];
+#pragma unroll
+          for (int rr = 0; rr < 4; ++rr) ldwords<WPT>(q + (ptrdiff_t)rr * stride, pr[rr]);
+          v = satd4x4<WPT>(st, pr);
+        }
+        v = __reduce_add_sync(kFull, v);
+        if (lane == k) got = v;
+      }
+      return total(got, NC);
+    };
+    auto half_vec = [&](int k, int& mx, int& my) {
+      const int q = k == 0 ? 4 : k <= 4 ? k - 1 : k, qy = q / 3;
+      mx = imx + (q - qy * 3 - 1) * 2;
+      my = imy + (qy - 1) * 2;
+      return true;
+    };
+    uint32_t v = satd(std::integral_constant<int, 9>{}, half_vec);
+    int mx, my;
+    half_vec(min(lane, 8), mx, my);
+    p = warp_min(lane < 9 ? v + rate(mx, my) : kInf);
+    uint32_t bc = p.cost, bsatd = __shfl_sync(kFull, v, p.lane);
+    int bmx, bmy;
+    half_vec(p.lane, bmx, bmy);
+    const int hmx = bmx, hmy = bmy, cross = I.cross;
+    auto quarter_vec = [&](int k, int& ax, int& ay) {
+      const int q = k < 4 ? k : k + 1, qy = q / 3, dx = q - qy * 3 - 1, dy = qy - 1;
+      ax = (int)(int16_t)(hmx + dx);
+      ay = (int)(int16_t)(hmy + dy);
+      return !(cross != 0 && dx != 0 && dy != 0);
+    };
+    v = satd(std::integral_constant<int, 8>{}, quarter_vec);
+    const bool ok = quarter_vec(min(lane, 7), mx, my) && lane < 8;
+    nsatd += cross ? 4 : 8;
+    p = warp_min(ok ? v + rate(mx, my) : kInf);
+    if (p.cost < bc) {
+      bc = p.cost;
+      bsatd = __shfl_sync(kFull, v, p.lane);
+      quarter_vec(p.lane, bmx, bmy);
+    }
+    lv = (uint32_t)(uint16_t)(int16_t)bmx | (uint32_t)(uint16_t)(int16_t)bmy << 16;
+    if (tid == 0) {
+      const ptrdiff_t t = (ptrdiff_t)(I.base + row * I.nbx + bx) * I.nref + I.r;
+      st_relaxed64(I.mvf + t, (unsigned long long)I.tag << 32 | lv);
+      write_result(I.out + t, bmx, bmy, I.r, bc, bsatd, imx, imy, int_cost, nsad, nsatd, 0);
+      cnt.tasks += 1;
+      cnt.sad += nsad;
+      cnt.satd += nsatd;
+    }
+  }
+  cnt.area = N * N;
   group_sync<T>(bar);
 }
 
-template <class S, int N>
-constexpr size_t big_bytes() {
-  return (sizeof(GroupSmem<S>) + (size_t)WinGeo<S, N>::ROWS * WinGeo<S, N>::WRW * 4 + 15) / 16 * 16;
-}
 template <class S>
 constexpr size_t row_smem_bytes() {
-  return std::max({big_bytes<S, 64>(), 2 * big_bytes<S, 32>(), 2 * sizeof(SmallSmem<S, 16>), 4 * sizeof(SmallSmem<S, 8>)});
+  return std::max({(size_t)(kRowThreads / row_group(64)) * sizeof(BigSmem<S, 64>),
+                   (size_t)(kRowThreads / row_group(32)) * sizeof(BigSmem<S, 32>),
+                   (size_t)(kRowThreads / row_group(16)) * sizeof(SmallSmem<S, 16>),
+                   (size_t)(kRowThreads / row_group(8)) * sizeof(SmallSmem<S, 8>)});
 }
 
 template <class S>
@@ -388,7 +717,6 @@ __global__ void __launch_bounds__(kRowThreads, 2) hevc_row_kernel(LaunchDesc L) 
   __shared__ uint32_t entry;
   const int tid = threadIdx.x;
   const uint32_t epoch = __ldg(L.epoch);
-  RowCount cnt;
   for (;;) {
     __syncthreads();
     if (tid == 0) {
@@ -409,24 +737,22 @@ __global__ void __launch_bounds__(kRowThreads, 2) hevc_row_kernel(LaunchDesc L) 
     // The entry's row and the rows after it, a group each.
     const int N = F.size[l], T = row_group(N), g = tid / T, gt = tid % T, mine = row + g, bar = 1 + g;
     if (mine >= F.nby[l]) continue;
-    if (N == 8) {
+    RowCount cnt;
+    if (N == 8)
       small_row<S, 8, row_group(8)>(L, F, l, r, mine, reinterpret_cast<SmallSmem<S, 8>*>(smem_raw)[g], gt, bar, cnt);
-    } else if (N == 16) {
+    else if (N == 16)
       small_row<S, 16, row_group(16)>(L, F, l, r, mine, reinterpret_cast<SmallSmem<S, 16>*>(smem_raw)[g], gt, bar, cnt);
-    } else {
-      GroupSmem<S>& gs = *reinterpret_cast<GroupSmem<S>*>(smem_raw + (N == 32 ? g * big_bytes<S, 32>() : 0));
-      if (gt < 6) gs.cnt[gt] = 0;
-      if (N == 32) big_row<S, 32, row_group(32)>(L, F, f, l, r, mine, gs, gt, bar);
-      else big_row<S, 64, row_group(64)>(L, F, f, l, r, mine, gs, gt, bar);
-      if (gt < 5) atomicAdd(&L.counters[gt], gs.cnt[gt]);
+    else if (N == 32)
+      big_row<S, 32, row_group(32)>(L, F, l, r, mine, reinterpret_cast<BigSmem<S, 32>*>(smem_raw)[g], gt, bar, cnt);
+    else
+      big_row<S, 64, row_group(64)>(L, F, l, r, mine, reinterpret_cast<BigSmem<S, 64>*>(smem_raw)[g], gt, bar, cnt);
+    if (gt == 0) {
+      atomicAdd(&L.counters[0], (unsigned long long)cnt.tasks);
+      atomicAdd(&L.counters[1], (unsigned long long)cnt.sad);
+      atomicAdd(&L.counters[2], (unsigned long long)cnt.satd);
+      atomicAdd(&L.counters[3], (unsigned long long)cnt.sad * cnt.area);
+      atomicAdd(&L.counters[4], (unsigned long long)cnt.satd * cnt.area);
     }
-  }
-  if (cnt.tasks != 0) {
-    atomicAdd(&L.counters[0], cnt.tasks);
-    atomicAdd(&L.counters[1], cnt.sad);
-    atomicAdd(&L.counters[2], cnt.satd);
-    atomicAdd(&L.counters[3], cnt.sad_samples);
-    atomicAdd(&L.counters[4], cnt.satd_samples);
   }
 }
 
