@@ -96,11 +96,9 @@ namespace {
 // part = 2 * (deeper than 8 bits) + (H.264).
 constexpr int kParts = 4;
 // The launch header in device memory (u64 words): head and tail of each
-// part's queue, then the counters, the status word and the epoch.
-// The launch header: head and tail of each part's queue (0..7), the
-// counters (8..12), status, epoch, then each part's finished-task count.
-constexpr int64_t kSpecTasks = 200000;  // about two 1080p frames of 2Nx2N PUs, 2 references
-constexpr int kMiscCounters = 8, kMiscStatus = 13, kMiscEpoch = 14, kMiscDone = 16, kMiscBig = 20, kMiscWords = 32;
+// part's row queue (0..7), the counters (8..12), the status word, the epoch,
+// then each part's next GIVEN job and next AMP unit.
+constexpr int kMiscCounters = 8, kMiscStatus = 13, kMiscEpoch = 14, kMiscGiven = 16, kMiscAmp = 20, kMiscWords = 24;
 
 int part_of(const FrameDesc& fd) { return 2 * (fd.bd > 8) + (fd.codec == RME_CODEC_H264); }
 int part_bytes(int k) { return k >= 2 ? 2 : 1; }
@@ -187,9 +185,9 @@ struct Deps {  // the dependency structure of one frame shape
   uint32_t* d_ready = nullptr;   // device copy of `ready` (the resident engine publishes from it)
   size_t ntasks = 0;
   // The row form. H.264: the rows of macroblocks, top to bottom (`row_ctas`).
-  // HEVC without AMP: `row_ctas`, the rows a CTA of the row kernel takes at
-  // once (the first of them); and for the resident engine the rows a warp
-  // runs (16x16 and 8x8)
+  // HEVC: `row_ctas`, the rows of 2Nx2N blocks a CTA of the row kernel takes
+  // at once (the first of them); and for the resident engine (frames without
+  // AMP) the rows a warp runs (16x16 and 8x8)
   // and the rows a CTA runs (64x64 and 32x32), as row_entry words, each
   // list ordered by the row's first sample row, larger blocks first: every
   // row comes after the rows it reads (its upper row, its parents' rows).
@@ -202,22 +200,7 @@ struct Graph {
   int seen = 0;  // launches of this shape so far: captured on the second
 };
 
-// A launch shape the tuner chooses among for a dataflow launch: the search
-// kernel's occupancy variant (registers per thread against resident warps),
-// in the latency form the share of CTAs that search 32x32 and 64x64 HEVC
-// blocks a CTA per block (0, a quarter or half of the SMs), and whether 8x8
-// blocks refine from staged phase patches (the search window's neighbourhood
-// in shared memory) or straight from the caches.
-struct Shape {
-  int variant, groups, patch;
-};
-constexpr Shape kThroughputShapes[] = {{1, 0, 0}, {0, 0, 0}, {2, 0, 0}};
-constexpr Shape kLatencyHevcShapes[] = {{1, 2, 1}, {1, 2, 0}, {1, 1, 1}, {1, 0, 0}, {0, 2, 1}};
-constexpr Shape kLatencyShapes[] = {{1, 0, 0}, {0, 0, 0}, {2, 0, 0}};
 constexpr int kTuneRounds = 2;  // timings per shape before the tuner chooses (launch times vary)
-constexpr int kNumShapes[3] = {(int)(sizeof(kThroughputShapes) / sizeof(Shape)),
-                               (int)(sizeof(kLatencyHevcShapes) / sizeof(Shape)),
-                               (int)(sizeof(kLatencyShapes) / sizeof(Shape))};
 
 // One search launch's buffers and events. A context keeps kSlots of them and
 // takes them in turn: a synchronous search finishes its launch before it
@@ -226,9 +209,8 @@ constexpr int kNumShapes[3] = {(int)(sizeof(kThroughputShapes) / sizeof(Shape)),
 constexpr int kSlots = 4;
 struct Slot {
   DevBuf<FrameDesc> d_frames;
-  DevBuf<unsigned long long> d_ready;  // the dataflow queue's slots
+  DevBuf<unsigned long long> d_ready;  // the launch's queues: rows, GIVEN jobs
   DevBuf<rme_result> d_out;
-  DevBuf<int32_t> d_pending;
   DevBuf<rme_job> d_jobs;
   DevBuf<unsigned long long> d_misc;  // the launch header (kMisc*)
   DevBuf<unsigned long long> d_mvf;   // the row form's published vectors (tagged with the epoch)
@@ -244,7 +226,6 @@ struct Slot {
   cudaStream_t stream = nullptr;
   int64_t total = 0;
   void* tuning = nullptr;
-  int tune_shapes = 0;
   rme_result* host_out = nullptr;
   std::vector<int64_t> host_off, host_count, dev_off;
   ~Slot() {
@@ -256,14 +237,15 @@ struct Slot {
 
 struct Ctx {
   int device = 0, nsm = 0;
-  int bps[kParts][kSearchVariants][2] = {};  // resident search blocks per SM, per part, variant, form
-  int row_bps[kParts][RME_MAX_REFS] = {};    // the row forms', per part (H.264: and references)
-  // The tuner: per (part, form, log2 of its task count), each launch shape
-  // of that class (kShapes) is timed on one real launch, then the fastest is
-  // kept. Results do not depend on the shape.
+  int bps[kParts][kSearchVariants] = {};   // resident blocks per SM of H.264's GIVEN search, per part and variant
+  int row_bps[kParts][RME_MAX_REFS] = {};  // the row forms', per part (H.264: and references)
+  // The tuner: per (part, log2 of its job count) of H.264 GIVEN launches,
+  // each occupancy variant of the kernel (registers per thread against
+  // resident warps) is timed on real launches, then the fastest is kept.
+  // Results do not depend on the variant.
   struct Tune {
     int best = -1, tried = 0;
-    float ms[8] = {};  // per shape, its best time so far
+    float ms[kSearchVariants] = {};  // per variant, its best time so far
   };
   std::map<std::pair<int, int>, Tune> tune;
   bool tune_on = true;
@@ -474,7 +456,7 @@ const Deps* get_deps(Ctx* c, const rme_picture_desc& d, const rme_params* p, int
   for (size_t t = 0; t < pend.size(); ++t)
     if (pend[t] == 0) dp.ready.push_back((uint32_t)t);
   dp.ntasks = pend.size();
-  if (d.codec == RME_CODEC_HEVC && p->hevc_amp == 0) {
+  if (d.codec == RME_CODEC_HEVC) {
     // Reference-major: a block's warps take consecutive rows of one
     // reference, whose reference bands overlap in the SM's L1.
     struct Row {
@@ -644,12 +626,12 @@ int finish_launch(Ctx* c, Slot& sl, bool wait_planes = true) {
   if (sl.tuning) {
     auto* T = (Ctx::Tune*)sl.tuning;
     sl.tuning = nullptr;
-    if (T->best < 0 && T->tried < kTuneRounds * sl.tune_shapes) {
-      // Each shape is timed kTuneRounds times (in turn); its best time counts.
-      const int i = T->tried % sl.tune_shapes;
-      T->ms[i] = T->tried < sl.tune_shapes ? ms : std::min(T->ms[i], ms);
-      if (++T->tried == kTuneRounds * sl.tune_shapes)
-        T->best = (int)(std::min_element(T->ms, T->ms + sl.tune_shapes) - T->ms);
+    if (T->best < 0 && T->tried < kTuneRounds * kSearchVariants) {
+      // Each variant is timed kTuneRounds times (in turn); its best time counts.
+      const int i = T->tried % kSearchVariants;
+      T->ms[i] = T->tried < kSearchVariants ? ms : std::min(T->ms[i], ms);
+      if (++T->tried == kTuneRounds * kSearchVariants)
+        T->best = (int)(std::min_element(T->ms, T->ms + kSearchVariants) - T->ms);
     }
   }
   c->last.planes_ms = 0.0f;
@@ -725,10 +707,9 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     if (ntask[i] >= (1 << 24)) return fail(c, RME_EINVAL, "more than 2^24 tasks in one frame");
   CK(sl.d_frames.ensure(n));
   if (!dev_out) CK(sl.d_out.ensure(std::max<int64_t>(total, 1)));
-  CK(sl.d_pending.ensure(std::max<int64_t>(total, 1)));
   unsigned long long* old_ready = sl.d_ready.p;
   unsigned long long* old_mvf = sl.d_mvf.p;
-  CK(sl.d_ready.ensure(2 * std::max<int64_t>(total, 1)));  // the warps' queues, then the CTAs' queues
+  CK(sl.d_ready.ensure(2 * std::max<int64_t>(total, 1)));  // the parts' rows, then their GIVEN jobs
   CK(sl.d_mvf.ensure(std::max<int64_t>(total, 1)));
   // Fresh slot memory may hold any word, an epoch's among them: zero it
   // (epochs start at 1).
@@ -743,236 +724,185 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     sl.epoch = 0;
   }
   ++sl.epoch;
-  // Pass 2: device pointers; the queue's initial entries (8-bit frames'
-  // tasks first, then deeper ones: each part is one kernel launch of its
-  // own sample width, with its own part of the slots).
+  // Pass 2: device pointers and the parts' queues. A part (one sample width
+  // and codec) is up to three launches in turn, each over its own queue:
+  //   - its STANDALONE frames' rows (HEVC: their 2Nx2N blocks): against the
+  //     dataflow form that ran one task a warp with dependency counts, H.264
+  //     took 0.53 against 1.60 ms for one CIF frame, 0.86 against 2.49 ms for
+  //     a hundred and 9.6 against 14.7 ms for 64 720p frames of two
+  //     references; HEVC, with the same arithmetic, 1.8 against 6 ms for one
+  //     1080p frame, 8.4 against 10.8 for twelve, 25.0 against 26.2 for 24 of
+  //     10 bits (only forty 8-bit ones 25.3 against 24.2);
+  //   - HEVC frames' AMP units, which read those blocks' results;
+  //   - GIVEN jobs, largest blocks first.
   std::vector<int64_t> sig;
   sig.push_back(n);
   sig.push_back(dev_out + 2 * pinned_out);
-  std::vector<unsigned long long> init[kParts], init_big[kParts];
-  // A launch of a frame or two is latency-bound: it runs the latency form
-  // of the search kernel (same results), where CTAs run the 32x32 and 64x64
-  // blocks of HEVC STANDALONE frames together.
-  const bool spec = total <= kSpecTasks;
-  int64_t part_tasks[kParts] = {0, 0, 0, 0};
-  // Parts whose frames are all STANDALONE run their row form: H.264 whatever
-  // the launch's size (against the best shape of the dataflow form it took
-  // 0.53 against 1.60 ms for one CIF frame and 0.86 against 2.49 ms for a
-  // hundred, 9.6 against 14.7 ms for 64 720p frames of two references, 20.4
-  // against 27.4 ms for 24 1080p 10-bit frames of three); HEVC without AMP
-  // units too (against the dataflow form with the same arithmetic: one 1080p
-  // frame 1.8 against 6 ms, twelve 8.4 against 10.8, 24 of 10 bits 25.0
-  // against 26.2, 100 360p frames 6.6 against 6.8; only forty 1080p frames
-  // are 4 % slower, 25.3 against 24.2).
-  bool rows[kParts] = {true, true, true, true};
+  std::vector<unsigned long long> rows[kParts], given[kParts];
+  int64_t part_tasks[kParts] = {0, 0, 0, 0}, amp_tasks[kParts] = {0, 0, 0, 0};
   int rows_nref[kParts] = {0, 0, 0, 0};
-  for (int i = 0; i < n; ++i) {
-    const FrameDesc& fd = sl.h_frames.p[i];
-    const int k = part_of(fd);
-    part_tasks[k] += ntask[i];
-    rows[k] = rows[k] && params[i].predictor_mode == RME_PRED_STANDALONE && fd.amp == 0;
-    rows_nref[k] = std::max(rows_nref[k], fd.nref);
-  }
-  // Each part's launch shape: the tuned one for its class, or the next one
-  // to time (a launch of one kind only, so that its time is the part's).
-  int nparts_used = 0;
-  for (int k = 0; k < kParts; ++k) nparts_used += part_tasks[k] > 0;
-  Shape shape[kParts];
-  int variant[kParts];
-  Ctx::Tune* tuning = nullptr;  // the class this launch times, if any
-  int tune_shapes = 0;
-  for (int k = 0; k < kParts; ++k) {
-    const Shape* shapes = !spec ? kThroughputShapes : part_codec(k) == RME_CODEC_HEVC ? kLatencyHevcShapes : kLatencyShapes;
-    const int nsh = kNumShapes[!spec ? 0 : part_codec(k) == RME_CODEC_HEVC ? 1 : 2];
-    shape[k] = shapes[0];
-    if (part_tasks[k] > 0 && c->tune_on && !rows[k]) {
-      const int bucket = 63 - __builtin_clzll((unsigned long long)part_tasks[k]);
-      Ctx::Tune& T = c->tune[{k * 2 + spec, bucket}];
-      if (T.best >= 0) {
-        shape[k] = shapes[T.best];
-      } else if (nparts_used == 1 && !async) {
-        shape[k] = shapes[T.tried % nsh];
-        tuning = &T;
-        tune_shapes = nsh;
-      }
-    }
-    variant[k] = shape[k].variant;
-    if (part_tasks[k] > 0 && !rows[k] && !c->bps[k][variant[k]][spec])
-      c->bps[k][variant[k]][spec] = search_blocks_per_sm(part_bytes(k), part_codec(k), variant[k], spec);
-  }
   std::vector<const Deps*> fdeps(n, nullptr);
   for (int i = 0; i < n; ++i) {
-    if (params[i].predictor_mode == RME_PRED_STANDALONE) {
-      Picture* src;
-      picture_of(c, frames[i].src_id, &src);
-      int rc = 0;
-      fdeps[i] = get_deps(c, src->d, &params[i], frames[i].nref, &rc);
-      if (!fdeps[i]) return rc;
-    }
-  }
-  std::vector<std::pair<const int32_t*, int>> pend_copies;  // (template, frame)
-  for (int i = 0; i < n; ++i) {
     FrameDesc& fd = sl.h_frames.p[i];
-    const int part = part_of(fd);
+    const int k = part_of(fd);
+    part_tasks[k] += ntask[i];
     fd.out = dev_out ? out + (offsets ? offsets[i] : toff[i]) : sl.d_out.p + toff[i];
-    fd.pending = sl.d_pending.p + toff[i];
-    const unsigned long long tag = ((unsigned long long)sl.epoch << 32) | ((unsigned long long)i << 24);
+    fd.amp_first[0] = amp_tasks[0];
+    fd.amp_first[1] = amp_tasks[2];
+    sig.push_back(fd.bd);
+    sig.push_back(fd.codec);
     if (params[i].predictor_mode == RME_PRED_GIVEN) {
       fd.jobs = sl.d_jobs.p + jobs_off[i];
       if (i == 0) fd.bi_src = bi_src;
       if (frames[i].njobs > 0)
         CK(cudaMemcpyAsync(sl.d_jobs.p + jobs_off[i], frames[i].jobs, sizeof(rme_job) * frames[i].njobs,
                            cudaMemcpyHostToDevice, s));
-      for (int t = 0; t < ntask[i]; ++t) init[part].push_back(tag | (uint32_t)t);
       sig.push_back(-1);
       sig.push_back(frames[i].njobs);
-      sig.push_back(fd.bd);
-    } else if (rows[part]) {
-      // Every row of the frame is pushed now (interleaved with the other
-      // frames' rows below); a search of this buffer tags its words anew.
-      fd.mvf = sl.d_mvf.p + toff[i];
-      fd.tag = fd.codec == RME_CODEC_H264 ? sl.epoch << 2 : sl.epoch;
-      sig.push_back(fd.bd);
-      sig.push_back(fd.codec);
-      sig.push_back(fd.width);
-      sig.push_back(fd.height);
-      sig.push_back(fd.nref);
-      sig.push_back(params[i].hevc_pu_mask);
-    } else {
-      const Deps* dp = fdeps[i];
-      pend_copies.emplace_back(dp->pending, i);
-      const bool groups = spec && fd.codec == RME_CODEC_HEVC && shape[part].groups > 0;
-      for (uint32_t t : dp->ready)
-        (groups && (int)(t / fd.nref) < fd.big_end ? init_big : init)[part].push_back(tag | t);
-      sig.push_back(fd.bd);
-      sig.push_back(fd.codec);
-      sig.push_back(fd.width);
-      sig.push_back(fd.height);
-      sig.push_back(fd.nref);
-      sig.push_back(params[i].hevc_pu_mask);
+      continue;
     }
+    Picture* src;
+    picture_of(c, frames[i].src_id, &src);
+    int rc = 0;
+    fdeps[i] = get_deps(c, src->d, &params[i], frames[i].nref, &rc);
+    if (!fdeps[i]) return rc;
+    // A search of this buffer tags its published words anew.
+    fd.mvf = sl.d_mvf.p + toff[i];
+    fd.tag = fd.codec == RME_CODEC_H264 ? sl.epoch << 2 : sl.epoch;
+    if (fd.amp) amp_tasks[k] += ntask[i] - (int64_t)fd.base[fd.nlevels] * fd.nref;
+    rows_nref[k] = std::max(rows_nref[k], fd.nref);
+    sig.push_back(fd.width);
+    sig.push_back(fd.height);
+    sig.push_back(fd.nref);
+    sig.push_back(params[i].hevc_pu_mask);
+    sig.push_back(params[i].hevc_amp);
   }
-  // Frames' first tasks interleaved, so every frame starts at once.
-  for (int k = 0; k < kParts; ++k)
-    for (auto* v : {&init[k], &init_big[k]})
-      std::stable_sort(v->begin(), v->end(), [](unsigned long long a, unsigned long long b) {
-        return (a & 0xffffffu) < (b & 0xffffffu);
-      });
-  // Row-form parts: the frames' rows interleaved row for row (each frame's
-  // own order kept).
+  // The frames' rows, interleaved row for row so that every frame starts at
+  // once (each frame's own order kept: a row comes after the rows it reads).
   for (int k = 0; k < kParts; ++k) {
-    if (!rows[k]) continue;
     size_t most = 0;
     for (int i = 0; i < n; ++i)
-      if (part_of(sl.h_frames.p[i]) == k) most = std::max(most, fdeps[i]->row_ctas.size());
+      if (fdeps[i] && part_of(sl.h_frames.p[i]) == k) most = std::max(most, fdeps[i]->row_ctas.size());
     for (size_t j = 0; j < most; ++j)
       for (int i = 0; i < n; ++i) {
-        if (part_of(sl.h_frames.p[i]) != k || j >= fdeps[i]->row_ctas.size()) continue;
-        init[k].push_back(((unsigned long long)sl.epoch << 32) | ((unsigned long long)i << 24) | fdeps[i]->row_ctas[j]);
+        if (!fdeps[i] || part_of(sl.h_frames.p[i]) != k || j >= fdeps[i]->row_ctas.size()) continue;
+        rows[k].push_back(((unsigned long long)sl.epoch << 32) | ((unsigned long long)i << 24) | fdeps[i]->row_ctas[j]);
       }
   }
-  // h_init: [the launch header (kMiscWords) | entries | the CTAs' entries]
-  size_t ninit = 0, init_off[kParts], init_big_off[kParts];
+  // GIVEN jobs by their block's area, in 4x4 tiles (1..256), largest first:
+  // the jobs that run last are short ones.
   for (int k = 0; k < kParts; ++k) {
-    init_off[k] = ninit;
-    ninit += init[k].size();
+    size_t at[257] = {0}, nk = 0;
+    auto tiles = [](const rme_job& j) { return 256 - (j.w >> 2) * (j.h >> 2); };
+    for (int i = 0; i < n; ++i)
+      if (!fdeps[i] && part_of(sl.h_frames.p[i]) == k)
+        for (int t = 0; t < ntask[i]; ++t, ++nk) ++at[tiles(frames[i].jobs[t]) + 1];
+    if (nk == 0) continue;
+    for (int q = 0; q < 256; ++q) at[q + 1] += at[q];
+    given[k].resize(nk);
+    for (int i = 0; i < n; ++i)
+      if (!fdeps[i] && part_of(sl.h_frames.p[i]) == k)
+        for (int t = 0; t < ntask[i]; ++t)
+          given[k][at[tiles(frames[i].jobs[t])]++] =
+              ((unsigned long long)sl.epoch << 32) | ((unsigned long long)i << 24) | (unsigned long long)t;
+  }
+  // H.264 GIVEN launches: the tuned occupancy variant, or the next one to
+  // time (a launch of such jobs only, so that its time is theirs).
+  int variant[kParts];
+  Ctx::Tune* tuning = nullptr;  // the class this launch times, if any
+  for (int k = 0; k < kParts; ++k) {
+    variant[k] = kDefaultVariant;
+    if (part_codec(k) != RME_CODEC_H264 || given[k].empty()) continue;
+    if (c->tune_on) {
+      Ctx::Tune& T = c->tune[{k, 63 - __builtin_clzll((unsigned long long)given[k].size())}];
+      if (T.best >= 0) {
+        variant[k] = T.best;
+      } else if ((int64_t)given[k].size() == total && !async) {
+        variant[k] = T.tried % kSearchVariants;
+        tuning = &T;
+      }
+    }
+    if (!c->bps[k][variant[k]]) c->bps[k][variant[k]] = h264_given_blocks_per_sm(part_bytes(k), variant[k]);
+  }
+  // h_init: [the launch header (kMiscWords) | rows | GIVEN jobs]
+  size_t ninit = 0, rows_off[kParts], given_off[kParts];
+  for (int k = 0; k < kParts; ++k) {
+    rows_off[k] = ninit;
+    ninit += rows[k].size();
   }
   for (int k = 0; k < kParts; ++k) {
-    init_big_off[k] = ninit;
-    ninit += init_big[k].size();
+    given_off[k] = ninit;
+    ninit += given[k].size();
   }
   CK(sl.h_init.ensure(kMiscWords + ninit));
   unsigned long long* hi = sl.h_init.p;
   std::memset(hi, 0, kMiscWords * sizeof(unsigned long long));
   hi[kMiscEpoch] = sl.epoch;
-  LaunchDesc Ls[kParts] = {};
+  LaunchDesc Ls[kParts] = {}, Lgiven[kParts] = {};
   int64_t slot0 = 0, slot_off[kParts];
+  int grid[kParts] = {0, 0, 0, 0}, nparts = 0, order[kParts];
   for (int k = 0; k < kParts; ++k) {
-    hi[2 * k + 1] = init[k].size();
-    hi[kMiscBig + 2 * k + 1] = init_big[k].size();
-    std::memcpy(hi + kMiscWords + init_off[k], init[k].data(), init[k].size() * sizeof(unsigned long long));
-    std::memcpy(hi + kMiscWords + init_big_off[k], init_big[k].data(), init_big[k].size() * sizeof(unsigned long long));
+    hi[2 * k + 1] = rows[k].size();
+    std::copy(rows[k].begin(), rows[k].end(), hi + kMiscWords + rows_off[k]);
+    std::copy(given[k].begin(), given[k].end(), hi + kMiscWords + given_off[k]);
     slot_off[k] = slot0;
     LaunchDesc& L = Ls[k];
     L.frames = sl.d_frames.p;
     L.ready = sl.d_ready.p + slot0;
-    L.total = part_tasks[k];
+    L.total = (int64_t)rows[k].size();
     L.head = sl.d_misc.p + 2 * k;
     L.tail = sl.d_misc.p + 2 * k + 1;
     L.counters = sl.d_misc.p + kMiscCounters;
     L.status = reinterpret_cast<uint32_t*>(sl.d_misc.p + kMiscStatus);
     L.epoch = reinterpret_cast<const uint32_t*>(sl.d_misc.p + kMiscEpoch);
-    L.done = sl.d_misc.p + kMiscDone + k;
-    L.ready_big = sl.d_ready.p + total + slot0;
-    L.head_big = sl.d_misc.p + kMiscBig + 2 * k;
-    L.tail_big = sl.d_misc.p + kMiscBig + 2 * k + 1;
-    L.group_ctas = 0;
-    if (rows[k]) {
-      L.total = (int64_t)init[k].size();
-      L.done = nullptr;
-    }
+    Lgiven[k] = L;
+    Lgiven[k].ready = sl.d_ready.p + total + slot0;
+    Lgiven[k].total = (int64_t)given[k].size();
+    Lgiven[k].head = sl.d_misc.p + kMiscGiven + k;
     slot0 += part_tasks[k];
-  }
-  for (int k = 0; k < kParts; ++k) {
-    sig.push_back(variant[k]);
-    sig.push_back(shape[k].patch);
-    sig.push_back(rows[k]);
-    Ls[k].patch8 = shape[k].patch;
-  }
-  int nparts = 0, order[kParts];
-  for (int k = 0; k < kParts; ++k)
     if (part_tasks[k] > 0) order[nparts++] = k;
+    if (!rows[k].empty()) {
+      const bool h264 = part_codec(k) == RME_CODEC_H264;
+      int& bps = c->row_bps[k][h264 ? rows_nref[k] - 1 : 0];
+      if (!bps) bps = h264 ? h264_row_blocks_per_sm(part_bytes(k), rows_nref[k]) : hevc_row_blocks_per_sm(part_bytes(k));
+      grid[k] = (int)std::min<int64_t>(L.total, (int64_t)c->nsm * bps);
+    }
+  }
   for (int j = 1; j < nparts; ++j) {
     if (!c->aux[j]) CK(cudaStreamCreateWithFlags(&c->aux[j], cudaStreamNonBlocking));
     if (!c->ev_join[j]) CK(cudaEventCreateWithFlags(&c->ev_join[j], cudaEventDisableTiming));
   }
   if (nparts > 1 && !c->ev_fork) CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
-  sig.push_back(nparts);
-  // Grids: in the latency form a part with large HEVC blocks gives them up
-  // to half the SMs' worth of CTAs (one block at a time each) and the rest to
-  // the warps; all CTAs fit on the GPU at once, so neither kind waits for
-  // the other to be scheduled.
-  int grid[kParts] = {0, 0, 0, 0};
-  for (int k = 0; k < kParts; ++k) {
-    if (part_tasks[k] == 0) continue;
-    if (rows[k]) {
-      const bool h264 = part_codec(k) == RME_CODEC_H264;
-      int& bps = c->row_bps[k][h264 ? rows_nref[k] - 1 : 0];
-      if (!bps) bps = h264 ? h264_row_blocks_per_sm(part_bytes(k), rows_nref[k]) : hevc_row_blocks_per_sm(part_bytes(k));
-      grid[k] = (int)std::max<int64_t>(1, std::min<int64_t>(Ls[k].total, (int64_t)c->nsm * bps));
-      sig.push_back(-2);
-      continue;
+  // One part's launches, in turn on `sk`.
+  auto launch_part = [&](int k, cudaStream_t sk) -> cudaError_t {
+    const bool h264 = part_codec(k) == RME_CODEC_H264;
+    const int bytes = part_bytes(k);
+    cudaError_t e = cudaSuccess;
+    if (!rows[k].empty())
+      e = h264 ? launch_h264_rows(Ls[k], bytes, rows_nref[k], grid[k], sk) : launch_hevc_rows(Ls[k], bytes, grid[k], sk);
+    if (e == cudaSuccess && amp_tasks[k] > 0) {
+      LaunchDesc A = Ls[k];
+      A.head = sl.d_misc.p + kMiscAmp + k;
+      A.total = amp_tasks[k];
+      e = launch_hevc_flat(A, bytes, true, true, n, c->nsm, sk);
     }
-    const int cap = c->nsm * c->bps[k][variant[k]][spec];
-    int64_t big = 0;
-    if (spec && part_codec(k) == RME_CODEC_HEVC)
-      for (int i = 0; i < n; ++i)
-        if (part_of(sl.h_frames.p[i]) == k && params[i].predictor_mode == RME_PRED_STANDALONE)
-          big += (int64_t)sl.h_frames.p[i].big_end * sl.h_frames.p[i].nref;
-    const int share = shape[k].groups == 2 ? c->nsm / 2 : shape[k].groups == 1 ? c->nsm / 4 : 0;
-    const int g = big > 0 && share > 0 ? (int)std::min<int64_t>({(int64_t)share, big, (int64_t)cap - 1}) : 0;
-    const int64_t small = part_tasks[k] - big;
-    const int solo = (int)std::max<int64_t>(1, std::min<int64_t>(cap - g, (small + kWarpsPerBlock - 1) / kWarpsPerBlock));
-    Ls[k].group_ctas = g;
-    grid[k] = g + solo;
-    sig.push_back(g);
-  }
+    if (e == cudaSuccess && !given[k].empty())
+      e = h264 ? launch_h264_given(Lgiven[k], bytes, variant[k], c->nsm * c->bps[k][variant[k]], sk)
+               : launch_hevc_flat(Lgiven[k], bytes, false, true, n, c->nsm, sk);
+    return e;
+  };
   auto enqueue = [&](bool capturing) -> cudaError_t {
     const unsigned rec = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
     cudaError_t e = cudaMemcpyAsync(sl.d_frames.p, sl.h_frames.p, sizeof(FrameDesc) * n, cudaMemcpyHostToDevice, s);
-    for (auto& pc : pend_copies)
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(sl.d_pending.p + toff[pc.second], pc.first, sizeof(int32_t) * ntask[pc.second],
-                            cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(sl.d_misc.p, hi, kMiscWords * sizeof(unsigned long long), cudaMemcpyHostToDevice, s);
     for (int k = 0; k < kParts; ++k) {
-      if (e == cudaSuccess && !init[k].empty())
-        e = cudaMemcpyAsync(sl.d_ready.p + slot_off[k], hi + kMiscWords + init_off[k],
-                            init[k].size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, s);
-      if (e == cudaSuccess && !init_big[k].empty())
-        e = cudaMemcpyAsync(sl.d_ready.p + total + slot_off[k], hi + kMiscWords + init_big_off[k],
-                            init_big[k].size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, s);
+      if (e == cudaSuccess && !rows[k].empty())
+        e = cudaMemcpyAsync(sl.d_ready.p + slot_off[k], hi + kMiscWords + rows_off[k],
+                            rows[k].size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, s);
+      if (e == cudaSuccess && !given[k].empty())
+        e = cudaMemcpyAsync(sl.d_ready.p + total + slot_off[k], hi + kMiscWords + given_off[k],
+                            given[k].size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, s);
     }
     // Under capture the records are external ones: they become event-record
     // nodes, so the kernels' device time is measured on every replay.
@@ -984,10 +914,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
       const int k = order[j];
       cudaStream_t sk = j == 0 ? s : c->aux[j];
       if (j > 0) e = cudaStreamWaitEvent(sk, c->ev_fork, 0);
-      if (e == cudaSuccess)
-        e = !rows[k] ? launch_search(Ls[k], part_bytes(k), part_codec(k), variant[k], grid[k], sk, spec)
-            : part_codec(k) == RME_CODEC_H264 ? launch_h264_rows(Ls[k], part_bytes(k), rows_nref[k], grid[k], sk)
-                                              : launch_hevc_rows(Ls[k], part_bytes(k), grid[k], sk);
+      if (e == cudaSuccess) e = launch_part(k, sk);
       if (e == cudaSuccess && j > 0) e = cudaEventRecord(c->ev_join[j], sk);
     }
     for (int j = 1; j < nparts && e == cudaSuccess; ++j) e = cudaStreamWaitEvent(s, c->ev_join[j], 0);
@@ -1003,7 +930,6 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   if (use_graph && !has_given) {
     std::vector<int64_t> gsig = sig;
     gsig.push_back(total);
-    for (int k = 0; k < kParts; ++k) gsig.push_back((int64_t)init[k].size());
     gsig.push_back((int64_t)(uintptr_t)s);
     gsig.push_back((int64_t)(&sl - c->slots));
     gsig.push_back((int64_t)g_buffer_generation);
@@ -1047,7 +973,6 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   sl.stream = s;
   sl.total = total;
   sl.tuning = tuning;
-  sl.tune_shapes = tune_shapes;
   if (!dev_out && !pinned_out) {
     sl.host_out = out;
     sl.host_off.resize(n);

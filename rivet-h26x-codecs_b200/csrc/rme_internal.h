@@ -50,6 +50,7 @@ struct FrameDesc {
   // (the first amp_nlev: sizes of 16 or more), and per such level the block
   // index of its first AMP unit (amp_base[0] = base[nlevels]).
   int32_t amp, amp_nmodes, amp_nlev;
+  int64_t amp_first[2];  // a batched launch: AMP units of the 8-bit, of the deeper frames before this one
   int32_t amp_base[kMaxLevels + 1];
   // H.264
   const uint16_t* tab;       // MvCostTable
@@ -242,16 +243,20 @@ cudaError_t launch_lowres_search(const LowresDesc* pairs, int npairs, const Lowr
 cudaError_t launch_lowres_bi(const LowresDesc& cur, const LowresDesc& r0, const LowresDesc& r1, const rme_mv* m0,
                              const rme_mv* m1, uint32_t* cost, cudaStream_t s);
 
-// The search over one kind of task (sample width, codec): `grid` persistent
-// blocks pulling from L's queue. `variant` picks the kernel's occupancy
-// bound: 0, 1, 2 for 2, 3, 4 resident blocks per SM (1 is the default).
+// H.264 GIVEN jobs, a warp each (rme_search.cu): L's queue holds (frame, job)
+// entries; `grid` blocks at most. `variant` picks the kernel's occupancy
+// bound: 0, 1, 2 for 2, 3, 4 resident blocks per SM.
 constexpr int kSearchVariants = 3, kDefaultVariant = 1;
-// `spec` picks the latency form (HEVC: 8x8 diamonds two rounds per step)
-// for launches of a frame or two; results are the same.
-cudaError_t launch_search(const LaunchDesc& L, int bytes_per_sample, int codec, int variant, int grid,
-                          cudaStream_t s, bool spec = false);
-int search_blocks_per_sm(int bytes_per_sample, int codec, int variant, bool spec = false);
-// HEVC STANDALONE frames without AMP in their row form (rme_rows.cu): L's
+cudaError_t launch_h264_given(const LaunchDesc& L, int bytes_per_sample, int variant, int grid, cudaStream_t s);
+int h264_given_blocks_per_sm(int bytes_per_sample, int variant);
+// HEVC searches without dependencies, a warp each (rme_flat.cu): `amp`, the
+// AMP units of L's frames (L.total of them, FrameDesc::amp_first giving each
+// frame's); else the (frame, job) entries of L's queue. L.head counts the
+// searches taken. `words`: rows, planes and origins of every picture are
+// whole 32-bit words apart (true of the library's own).
+cudaError_t launch_hevc_flat(const LaunchDesc& L, int bytes_per_sample, bool amp, bool words, int nframes, int nsm,
+                             cudaStream_t s);
+// HEVC STANDALONE frames' 2Nx2N blocks in their row form (rme_rows.cu): L's
 // queue holds row_entry words, each the first of hevc_row_rows(size)
 // consecutive rows, all pushed by the host, each after the rows it reads.
 cudaError_t launch_hevc_rows(const LaunchDesc& L, int bytes_per_sample, int grid, cudaStream_t s);

@@ -169,13 +169,22 @@ extern "C" int rme_search_given_noalloc(const rme_picture_desc* d, const rme_par
   L.counters = d_misc + 4;
   L.status = reinterpret_cast<uint32_t*>(d_misc + 9);
   L.epoch = reinterpret_cast<const uint32_t*>(d_misc + 10);
-  L.done = nullptr;  // GIVEN jobs only: no task makes another ready
   const int bytes = d->bit_depth == 8 ? 1 : 2;
   int nsm = 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return RME_ECUDA;
-  const int64_t want = ((int64_t)njobs + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)nsm * search_blocks_per_sm(bytes, d->codec, kDefaultVariant), want));
-  if (launch_search(L, bytes, d->codec, kDefaultVariant, grid, s) != cudaSuccess) return RME_ECUDA;
+  if (h264) {
+    if (launch_h264_given(L, bytes, kDefaultVariant, nsm * h264_given_blocks_per_sm(bytes, kDefaultVariant), s) !=
+        cudaSuccess)
+      return RME_ECUDA;
+  } else {
+    // The caller's rows may lie at any sample offset from one another.
+    auto whole = [&](const DevPlanes& q) {
+      return ((int64_t)q.stride * bytes & 3) == 0 && ((int64_t)q.origin * bytes & 3) == 0 && (q.plane_elems * bytes & 3) == 0;
+    };
+    bool words = whole(fd.src);
+    for (int r = 0; r < nref; ++r) words = words && whole(fd.ref[r]);
+    if (launch_hevc_flat(L, bytes, false, words, 1, nsm, s) != cudaSuccess) return RME_ECUDA;
+  }
   if (cudaMemcpyAsync(misc, d_misc, sizeof(misc), cudaMemcpyDeviceToHost, s) != cudaSuccess) return RME_ECUDA;
   if (cudaStreamSynchronize(s) != cudaSuccess) return RME_ECUDA;
   if ((uint32_t)misc[9] != 0 || misc[4] != (unsigned long long)njobs) return RME_EDEVICE;

@@ -730,7 +730,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) hevc_row_kernel(LaunchDesc L) 
     const int f = (int)(e >> 24);
     const FrameDesc& F = L.frames[f];
     int l, r, row;
-    if ((sizeof(S) == 1) != (F.bd == 8) || !row_ok(F, e & 0xffffffu, l, r, row)) {
+    if ((sizeof(S) == 1) != (F.bd == 8) || !row_ok(F, e & 0xffffffu, l, r, row, true)) {
       if (tid == 0) atomicOr(L.status, kStatusBadTask);
       continue;
     }

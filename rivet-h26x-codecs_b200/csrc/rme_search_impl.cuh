@@ -1645,11 +1645,11 @@ __device__ int hevc_group_task(const LaunchDesc& L, const FrameDesc& F, int f, i
 // which its owner started earlier and runs ahead of this one) and of its
 // parent one size up; its left neighbour is this row's previous block. No
 // dependency counts, no queue traffic between the blocks of a row.
-__device__ __forceinline__ bool row_ok(const FrameDesc& F, uint32_t e, int& l, int& r, int& row) {
+__device__ __forceinline__ bool row_ok(const FrameDesc& F, uint32_t e, int& l, int& r, int& row, bool amp = false) {
   l = (int)((e >> 22) & 3u);
   r = (int)((e >> 20) & 3u);
   row = (int)(e & 0xfffffu);
-  return F.mvf != nullptr && F.codec == RME_CODEC_HEVC && F.mode == RME_PRED_STANDALONE && F.amp == 0 &&
+  return F.mvf != nullptr && F.codec == RME_CODEC_HEVC && F.mode == RME_PRED_STANDALONE && (amp || F.amp == 0) &&
          l < F.nlevels && r < F.nref && row < F.nby[l];
 }
 

@@ -147,3 +147,94 @@ def test_distortion_and_rate_at_their_ends(ms, codec, bd, kw):
         assert_results_equal(got, oracle.frame_search(codec, bd, pics[a], [pics[b]], p), f"fields {a} against {b}")
     for i in range(len(pics)):
         ms.release(2800 + i)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bd,kw", [(8, {}), (10, dict(hevc_search_rings=2, hevc_quarter_cross=1)),
+                                   (12, dict(hevc_search_range=1)), (8, dict(hevc_search_range=0, hevc_pad=8))])
+def test_given_jobs_of_every_shape(ms, bd, kw):
+    """Every block shape, no seed to ten, seeds far outside, blocks at the
+    picture's edges."""
+    rng = np.random.default_rng(bd + len(kw))
+    w, h = 150, 102
+    ref = random_picture(rng, w, h, bd)
+    src = shifted(ref, -4, 3, rng, 2.0)
+    ms.upload(2900, src, HEVC, bd)
+    ms.upload(2901, ref, HEVC, bd)
+    jobs = np.zeros(512, capi.JOB_DTYPE)
+    for i, j in enumerate(jobs):
+        bw, bh = 4 * (i % 16) + 4, 4 * (i // 16 % 16) + 4
+        j["w"], j["h"] = bw, bh
+        j["x"] = rng.choice([0, w - bw, rng.integers(0, w - bw + 1)])
+        j["y"] = rng.choice([0, h - bh, rng.integers(0, h - bh + 1)])
+        j["nseeds"] = i % 11
+        spread = 40 if i % 3 else 2000
+        j["mvp"] = rng.integers(-spread, spread + 1, (2, 2))
+        j["seeds"] = rng.integers(-spread, spread + 1, (capi.RME_MAX_SEEDS, 2))
+    p = oracle.params(HEVC, 31, predictor_mode=capi.RME_PRED_GIVEN, **kw)
+    got = ms.search(2900, [2901], p, jobs)
+    assert_results_equal(got, oracle.frame_search(HEVC, bd, src, [ref], p, jobs), "GIVEN shapes")
+    ms.release(2900)
+    ms.release(2901)
+
+
+@pytest.mark.gpu
+def test_amp_frames_of_both_depths_with_given_frames(ms):
+    """AMP units of several frames of two depths in one launch, frames
+    without units and H.264 frames among them: each as by itself."""
+    rng = np.random.default_rng(91)
+    frames, params, want = [], [], []
+    shapes = [(HEVC, 10, 130, 70, 2, 5), (HEVC, 8, 64, 64, 1, 0), (HEVC, 8, 96, 48, 2, 15), (H264, 8, 64, 48, 1, 0),
+              (HEVC, 10, 72, 136, 1, 8), (HEVC, 8, 16, 16, 3, 2)]
+    for k, (codec, bd, w, h, nref, amp) in enumerate(shapes):
+        refs = [random_picture(rng, w, h, bd) for _ in range(nref)]
+        src = shifted(refs[0], -2, 3, rng, 2.0)
+        base = 3000 + 10 * k
+        for i, pic in enumerate(refs + [src]):
+            ms.upload(base + i, pic, codec, bd)
+        frames.append((base + nref, [base + i for i in range(nref)]))
+        params.append(oracle.params(codec, 30, hevc_amp=amp))
+        want.append(oracle.frame_search(codec, bd, src, refs, params[-1]))
+    for _ in range(4):  # the first calls, the capture, its replays
+        for g, w_ in zip(ms.search_batch(frames, params), want):
+            assert_results_equal(g, w_, "AMP among others")
+    for s, r in frames:
+        for i in [s] + r:
+            ms.release(i)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bd,extra", [(8, 0), (8, 1), (8, 2), (8, 3), (10, 1), (10, 2)])
+def test_no_alloc_search_on_rows_at_any_offset(ms, bd, extra):
+    """A caller's planes whose rows lie whole words apart, and not."""
+    import ctypes as C
+    import torch
+    rng = np.random.default_rng(bd + extra)
+    w, h, pad = 96, 72, 80
+    ref = random_picture(rng, w, h, bd)
+    src = shifted(ref, 3, -2, rng, 2.0)
+    for i, pic in enumerate((src, ref)):
+        ms.upload(3100 + i, pic, HEVC, bd)
+    p = oracle.params(HEVC, 30, predictor_mode=capi.RME_PRED_GIVEN)
+    from _common import random_jobs
+    jobs = random_jobs(rng, HEVC, w, h, 1, 120, spread=200)
+    want = oracle.frame_search(HEVC, bd, src, [ref], p, jobs)
+    sets, keep = [], []
+    for i in range(2):
+        planes = np.stack([ms.plane(3100 + i, k) for k in range(16)])
+        wide = np.zeros(planes.shape[:2] + (planes.shape[2] + extra,), planes.dtype)
+        wide[:, :, :planes.shape[2]] = planes
+        buf = torch.zeros(wide.nbytes + 16, dtype=torch.uint8, device="cuda")
+        buf[:wide.nbytes].copy_(torch.from_numpy(wide.view(np.uint8).ravel()))
+        keep.append(buf)
+        sets.append(capi.PlaneSet(buf.data_ptr(), wide.shape[1] * wide.shape[2], wide.shape[2], pad))
+    d_jobs = torch.from_numpy(jobs.view(np.uint8).copy()).cuda()
+    d_out = torch.zeros(len(jobs) * capi.RESULT_DTYPE.itemsize, dtype=torch.uint8, device="cuda")
+    d = capi.PictureDesc(HEVC, bd, w, h, w)
+    refs = (capi.PlaneSet * 1)(sets[1])
+    rc = capi.lib().rme_search_given_noalloc(C.byref(d), C.byref(p), C.byref(sets[0]), refs, 1,
+                                             C.c_void_p(d_jobs.data_ptr()), len(jobs), C.c_void_p(d_out.data_ptr()), None)
+    assert rc == capi.RME_OK, rc
+    assert_results_equal(d_out.cpu().numpy().view(capi.RESULT_DTYPE), want, f"rows {extra} samples further apart")
+    ms.release(3100)
+    ms.release(3101)
