@@ -332,7 +332,7 @@ class MotionSearch:
         d = self._desc[ref_id]
         blocks = np.ascontiguousarray(blocks, np.int32)
         mvs = np.ascontiguousarray(mvs, np.int16)
-        n = int(sum((b[2] // 2) * (b[3] // 2) * 2 for b in blocks))
+        n = int(np.sum((blocks[:, 2] // 2).astype(np.int64) * (blocks[:, 3] // 2)) * 2) if blocks.size else 0
         out = np.zeros(n, np.uint8 if d.bit_depth == 8 else np.uint16)
         self._check(self._lib.rme_chroma_predict(self.ctx, ref_id, len(blocks),
                                                  blocks.ctypes.data_as(C.POINTER(C.c_int32)),
