@@ -238,3 +238,43 @@ def test_no_alloc_search_on_rows_at_any_offset(ms, bd, extra):
     assert_results_equal(d_out.cpu().numpy().view(capi.RESULT_DTYPE), want, f"rows {extra} samples further apart")
     ms.release(3100)
     ms.release(3101)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bd", [8, 9, 10, 12])
+@pytest.mark.parametrize("w,h", [(16, 16), (17, 31), (97, 45), (130, 70)])
+def test_phase_planes_at_tile_edges(ms, bd, w, h):
+    """Every phase over pictures whose padded planes end inside a tile, a
+    lane's columns and a strip's rows; noise and rails."""
+    rng = np.random.default_rng(w + bd)
+    top = (1 << bd) - 1
+    pic = np.where(rng.random((h, w)) < 0.5, rng.integers(0, 2, (h, w)) * top, rng.integers(0, top + 1, (h, w)))
+    pic = pic.astype(np.uint8 if bd == 8 else np.uint16)
+    ms.upload(3200, pic, HEVC, bd)
+    base, _ = oracle.hevc_planes(pic, bd)
+    want, ext = oracle.hevc_planes(pic, bd, force_quarter=True)
+    np.testing.assert_array_equal(ms.plane(3200, 0), base[0])
+    sl = (slice(80 - ext, 80 + h + ext), slice(80 - ext, 80 + w + ext))
+    for k in range(1, 16):
+        np.testing.assert_array_equal(ms.plane(3200, k)[sl], want[k][sl], err_msg=f"phase {k}")
+    # The whole padded plane is the interpolation of the replicated picture.
+    taps = np.array([[0, 0, 0, 64, 0, 0, 0, 0], [-1, 4, -10, 58, 17, -5, 1, 0], [-1, 4, -11, 40, 40, -11, 4, -1],
+                     [0, 1, -5, 17, 58, -10, 4, -1]], np.int64)
+    full = np.pad(pic.astype(np.int64), 80 + 4, mode="edge")
+    rows, cols = h + 160, w + 160
+    for fy in range(4):
+        for fx in range(4):
+            if not fx and not fy:
+                continue
+            if fx:
+                t = sum(taps[fx][k] * full[:, k + 1:k + 1 + cols] for k in range(8)) >> (min(bd, 12) - 8)
+            else:
+                t = full[:, 4:4 + cols]
+            if fy:
+                t = sum(taps[fy][k] * t[k + 1:k + 1 + rows] for k in range(8)) >> (6 if fx else min(bd, 12) - 8)
+            else:
+                t = t[4:4 + rows]
+            sh = 14 - bd
+            np.testing.assert_array_equal(ms.plane(3200, fy * 4 + fx), np.clip((t + (1 << (sh - 1))) >> sh, 0, top),
+                                          err_msg=f"padded phase {fx}, {fy}")
+    ms.release(3200)
