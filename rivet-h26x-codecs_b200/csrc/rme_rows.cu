@@ -186,6 +186,9 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
       constexpr int LPC = decltype(lanes)::value, RPL = N / LPC, UN = RPL * WR <= 16 ? RPL : 16 / WR;
       const int sub = tid % LPC;
       uint32_t acc = 0;
+      // The key but for the distortion, worked out while the loads are on
+      // their way (behind the sum it would lengthen the step).
+      const uint32_t low = hevc_rate(lam, fx * 4, fy * 4, p0x, p0y, p1x, p1y) << 5 | (uint32_t)at;
       if (ok) {
         const S* rp = org + (ptrdiff_t)(fy + sub) * stride + fx;
 #pragma unroll
@@ -203,8 +206,7 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
       for (int o = LPC >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
       uint32_t* c = sm.key[buf];
       buf ^= 1;
-      if (sub == 0)
-        c[at] = ok ? (acc + hevc_rate(lam, fx * 4, fy * 4, p0x, p0y, p1x, p1y)) << 5 | (uint32_t)at : kNoKey;
+      if (sub == 0) c[at] = ok ? (acc << 5) + low : kNoKey;
       group_sync<T>(bar);
       return c[lane];
     };
@@ -244,32 +246,34 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
           key = score(std::integral_constant<int, T / kSlots>{}, slot, ok, fx, fy);
           base = 0;
         }
+        // The first round's minimum and, for each way it can move, the
+        // second's: five minima that wait for nothing but the keys. (A step
+        // begins at an even round and their number is even, so both rounds
+        // are always allowed.)
         const uint32_t there = __ballot_sync(kFull, key != kNoKey) >> base;  // bit q: point q is scored
         const int q = lane - base;
+        const uint32_t bit = q >= 0 && q < 13 ? 1u << q : 0u;
+        const uint32_t m1 = __reduce_min_sync(kFull, bit & 0x1eu ? key : kNoKey);
+        uint32_t m2 = kNoKey, second = 0;
+        {
+          uint32_t mj[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) mj[j] = __reduce_min_sync(kFull, bit & second_round(j) ? key : kNoKey);
+          const int j = (int)(m1 & 31u) - base - 1;
+          m2 = j == 0 ? mj[0] : j == 1 ? mj[1] : j == 2 ? mj[2] : mj[3];
+          second = second_round(j);
+        }
+        const bool moved = m1 >> 5 < bcost, again = moved && m2 < m1 && m2 >> 5 < m1 >> 5;
         nsad += __popc(there & 0x1eu);
-        uint32_t m = __reduce_min_sync(kFull, q >= 1 && q <= 4 ? key : kNoKey);
-        if (!(m >> 5 < bcost)) break;
-        const int q1 = (int)(m & 31u) - base;
-        bcost = m >> 5;
-        const int x1 = around_x(q1), y1 = around_y(q1);
-        const uint32_t second = second_round(q1 - 1);
-        if (++it >= 2 * range) {
-          fbx += x1;
-          fby += y1;
-          break;
-        }
+        if (!moved) break;
         nsad += 1u + __popc(there & second);  // the fourth point is the old best
-        m = __reduce_min_sync(kFull, q >= 0 && ((second >> q) & 1u) ? key : kNoKey);
-        if (!(m >> 5 < bcost)) {
-          fbx += x1;
-          fby += y1;
-          break;
-        }
-        bcost = m >> 5;
-        const int q3 = (int)(m & 31u) - base;
-        fbx += around_x(q3);
-        fby += around_y(q3);
-        ++it;
+        const uint32_t won = again ? m2 : m1;
+        const int qw = (int)(won & 31u) - base;
+        bcost = won >> 5;
+        fbx += around_x(qw);
+        fby += around_y(qw);
+        it += 2;
+        if (!again) break;
         base = -1;
       }
       if (rings >= I.rings) break;
@@ -301,8 +305,11 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
 
     // refine_subpel: the start and the half ring in one step, then the
     // quarter ring around the winner; a thread per 4x4 tile, NT threads a
-    // candidate. Returns lane i's candidate's key.
-    auto satd = [&](auto count, auto vec) -> uint32_t {
+    // candidate. at(k, dx, dy): candidate k's offset from the whole-sample
+    // point in quarter samples, and whether it is scored. Returns lane i's
+    // candidate's key.
+    const S* const whole = org + (ptrdiff_t)fby * stride + fbx;
+    auto satd = [&](auto count, auto at) -> uint32_t {
       constexpr int NC = decltype(count)::value;
       uint32_t* kb = sm.key[buf];
       buf ^= 1;
@@ -310,14 +317,16 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
       for (int j0 = 0; j0 < NC * NT; j0 += T) {
         const int j = j0 + tid, k = j / NT, tile = j % NT, ty = tile / TW, tx = tile % TW;
         if (j0 + (tid & ~31) >= NC * NT) break;  // none of the warp's
-        int mx = 0, my = 0;
-        uint32_t v = 0;
-        const bool ok = k < NC && vec(k, mx, my);
+        int dx = 0, dy = 0;
+        uint32_t v = 0, low = 0;
+        const bool ok = k < NC && at(k, dx, dy);
         if (ok) {
-          const S* q = plane_at<S>(I.ref, (my & 3) * 4 + (mx & 3), x + (mx >> 2) + tx * 4, y + (my >> 2) + ty * 4);
+          const S* q = whole + (int64_t)((dy & 3) * 4 + (dx & 3)) * I.ref.plane_elems +
+                       (ptrdiff_t)((dy >> 2) + ty * 4) * stride + ((dx >> 2) + tx * 4);
           uint32_t pr[4][WPT], sw[4][WPT];
 #pragma unroll
           for (int rr = 0; rr < 4; ++rr) ldwords<WPT>(q + (ptrdiff_t)rr * stride, pr[rr]);
+          low = hevc_rate(lam, imx + dx, imy + dy, p0x, p0y, p1x, p1y);
 #pragma unroll
           for (int rr = 0; rr < 4; ++rr)
 #pragma unroll
@@ -327,38 +336,42 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
 #pragma unroll
         for (int o = NT >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
         if (tile == 0 && k < NC) {
+          kb[k] = ok ? (v + low) << 5 | (uint32_t)k : kNoKey;
           sm.satd[NC == 8][k] = v;
-          kb[k] = ok ? (v + hevc_rate(lam, mx, my, p0x, p0y, p1x, p1y)) << 5 | (uint32_t)k : kNoKey;
         }
       }
       group_sync<T>(bar);
       return lane < NC ? kb[lane] : kNoKey;
     };
-    auto half_vec = [&](int k, int& mx, int& my) {
+    auto half_at = [](int k, int& dx, int& dy) {
       const int q = k == 0 ? 4 : k <= 4 ? k - 1 : k, qy = q / 3;
-      mx = imx + (q - qy * 3 - 1) * 2;
-      my = imy + (qy - 1) * 2;
+      dx = (q - qy * 3 - 1) * 2;
+      dy = (qy - 1) * 2;
       return true;
     };
-    uint32_t m = __reduce_min_sync(kFull, satd(std::integral_constant<int, 9>{}, half_vec));
-    int bmx, bmy;
-    half_vec((int)(m & 31u), bmx, bmy);
+    uint32_t m = __reduce_min_sync(kFull, satd(std::integral_constant<int, 9>{}, half_at));
+    int hdx, hdy;
+    half_at((int)(m & 31u), hdx, hdy);
+    int bmx = imx + hdx, bmy = imy + hdy;
     uint32_t bc = m >> 5, bsatd = sm.satd[0][m & 31u];
-    const int hmx = bmx, hmy = bmy, cross = I.cross;
-    auto quarter_vec = [&](int k, int& mx, int& my) {
-      const int q = k < 4 ? k : k + 1, qy = q / 3, dx = q - qy * 3 - 1, dy = qy - 1;
-      mx = (int)(int16_t)(hmx + dx);
-      my = (int)(int16_t)(hmy + dy);
-      return !(cross != 0 && dx != 0 && dy != 0);
+    const int cross = I.cross;
+    auto quarter_at = [&](int k, int& dx, int& dy) {
+      const int q = k < 4 ? k : k + 1, qy = q / 3, ex = q - qy * 3 - 1, ey = qy - 1;
+      dx = hdx + ex;
+      dy = hdy + ey;
+      return !(cross != 0 && ex != 0 && ey != 0);
     };
     store_src(sm.src[(bx + 1) & 1], nsrc);
-    const uint32_t qkey = satd(std::integral_constant<int, 8>{}, quarter_vec);
+    const uint32_t qkey = satd(std::integral_constant<int, 8>{}, quarter_at);
     nsatd += cross ? 4 : 8;
     m = __reduce_min_sync(kFull, qkey);
     if (m != kNoKey && m >> 5 < bc) {
+      int dx, dy;
       bc = m >> 5;
       bsatd = sm.satd[1][m & 31u];
-      quarter_vec((int)(m & 31u), bmx, bmy);
+      quarter_at((int)(m & 31u), dx, dy);
+      bmx = imx + dx;
+      bmy = imy + dy;
     }
     lv = (uint32_t)(uint16_t)(int16_t)bmx | (uint32_t)(uint16_t)(int16_t)bmy << 16;
     if (tid == 0) {
