@@ -20,7 +20,7 @@
 //   - speculation instead of dependence: the first step of an 8x8 or 16x16
 //     block scores all seeds and, around the two likeliest, the twelve points
 //     two diamond rounds can reach; later steps, and those of larger blocks,
-//     score two rounds at once;
+//     score two or three rounds at once;
 //   - a 32x32 or 64x64 block's diamond reads a window staged in shared memory
 //     while the seeds are scored, a thread its words' twelve candidates;
 //   - the next block's source is on its way while a block is searched;
@@ -59,18 +59,31 @@ struct SmallSmem {
   uint32_t satd[2][16];     // half, quarter
 };
 
-// The points two rounds of the small diamond can reach, in an order in
-// which, whichever way the first round moves, the second round's new points
-// come in the reference's order ((1,0), (-1,0), (0,1), (0,-1) around the new
-// best): the centre, the first round, (2,0), (-2,0), (1,1), (1,-1), (-1,1),
-// (-1,-1), (0,2), (0,-2). Offsets + 2 as hex digits, slot 0 the lowest.
-constexpr unsigned long long kAroundX = 0x2211330422132ull, kAroundY = 0x0413132213222ull;
-__device__ __forceinline__ int around_x(int q) { return (int)((kAroundX >> (4 * q)) & 15u) - 2; }
-__device__ __forceinline__ int around_y(int q) { return (int)((kAroundY >> (4 * q)) & 15u) - 2; }
+// The points three rounds of the small diamond can reach, in an order in
+// which, whichever way the rounds before moved, a round's new points come in
+// the reference's order ((1,0), (-1,0), (0,1), (0,-1) around the new best):
+// the centre, the first round (1..4), then (2,0), (-2,0), (1,1), (1,-1),
+// (-1,1), (-1,-1), (0,2), (0,-2) (5..12), then (3,0), (-3,0), (2,1), (2,-1),
+// (-2,1), (-2,-1), (1,2), (1,-2), (-1,2), (-1,-2), (0,3), (0,-3) (13..24).
+// Offsets + 3 as hex digits, 16 points a word, the lowest digit first.
+__device__ __forceinline__ int around_x(int q) {
+  return (int)(((q < 16 ? 0x5063322441533243ull : 0x332244115ull) >> (4 * (q & 15))) & 15u) - 3;
+}
+__device__ __forceinline__ int around_y(int q) {
+  return (int)(((q < 16 ? 0x4331524243324333ull : 0x061515242ull) >> (4 * (q & 15))) & 15u) - 3;
+}
 // The second round's new points after the first moved in direction j.
-__device__ __forceinline__ uint32_t second_round(int j) {
+__device__ __forceinline__ constexpr uint32_t second_round(int j) {
   return j == 0 ? 0x1a0u : j == 1 ? 0x640u : j == 2 ? 0xa80u : 0x1500u;
 }
+// The third round's points after the second moved to point 5 + k: all four
+// (the first round's points among them, which cannot win: they cost no less
+// than the point the first round moved to), and the new ones.
+__constant__ uint32_t c_third[8] = {
+    1u << 13 | 1u << 1 | 1u << 15 | 1u << 16, 1u << 14 | 1u << 2 | 1u << 17 | 1u << 18,
+    1u << 15 | 1u << 3 | 1u << 19 | 1u << 1,  1u << 16 | 1u << 4 | 1u << 1 | 1u << 20,
+    1u << 3 | 1u << 17 | 1u << 21 | 1u << 2,  1u << 4 | 1u << 18 | 1u << 2 | 1u << 22,
+    1u << 19 | 1u << 21 | 1u << 23 | 1u << 3, 1u << 20 | 1u << 22 | 1u << 4 | 1u << 24};
 
 // What a row's blocks share, read once.
 template <class S>
@@ -80,7 +93,7 @@ struct RowInfo {
   rme_result* out;
   const uint32_t tag;
   const int nref, r, nbx, base;          // this level
-  const int pnbx, pbase, psize;          // the parents' level (psize 0: none over this row)
+  const int pnbx, pbase, pshift;         // the parents' level, log2 of its size (pnbx 0: none over this row)
   const int width, height, padm, range, rings, cross;
   const float lam;
 };
@@ -91,7 +104,7 @@ __device__ __forceinline__ RowInfo<S> row_info(const FrameDesc& F, int l, int r,
   return RowInfo<S>{F.src,    F.ref[r],  F.mvf,
                     F.out,    F.tag,     F.nref,
                     r,        F.nbx[l],  F.base[l],
-                    psize ? F.nbx[l - 1] : 0, psize ? F.base[l - 1] + (y / psize) * F.nbx[l - 1] : 0, psize,
+                    psize ? F.nbx[l - 1] : 0, psize ? F.base[l - 1] + (y / psize) * F.nbx[l - 1] : 0, 31 - __clz(psize | 1),
                     F.width,  F.height,  F.pad - 4,
                     F.search_range, F.search_rings, F.quarter_cross, F.lam};
 }
@@ -115,8 +128,8 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
   const float lam = I.lam;
   // The word of the parent of the block at x, or null where there is none.
   auto parent_of = [&](int x) -> const unsigned long long* {
-    const int px = I.psize ? x / I.psize : 0;
-    return I.psize && px < I.pnbx ? par + (ptrdiff_t)px * I.nref : nullptr;
+    const int px = x >> I.pshift;
+    return px < I.pnbx ? par + (ptrdiff_t)px * I.nref : nullptr;
   };
   auto load_src = [&](int bx, uint32_t (&v)[PS]) {  // aligned: N and the pad are whole words
 #pragma unroll
@@ -142,7 +155,7 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
   // the first step's two (slots 1..13 and 16..28), as the only one (0..12).
   const int slot = tid / (T / kSlots), q2 = slot < 16 ? slot - 1 : slot - 16;
   const bool in2 = q2 >= 0 && q2 < 13;
-  const int ax = around_x(max(q2, 0)), ay = around_y(max(q2, 0)), cxo = around_x(slot), cyo = around_y(slot);
+  const int ax = around_x(in2 ? q2 : 0), ay = around_y(in2 ? q2 : 0), cxo = around_x(slot), cyo = around_y(slot);
   group_sync<T>(bar);
   for (int bx = 0; bx < I.nbx; ++bx) {
     const int x = bx * N;
@@ -242,19 +255,17 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
       while (it < 2 * range) {
         if (base < 0) {
           const int fx = fbx + cxo, fy = fby + cyo;
-          const bool ok = slot > 0 && slot < 13 && abs(fx - ox) <= range && abs(fy - oy) <= range && inside(fx, fy);
+          const bool ok = slot > 0 && slot < 25 && abs(fx - ox) <= range && abs(fy - oy) <= range && inside(fx, fy);
           key = score(std::integral_constant<int, T / kSlots>{}, slot, ok, fx, fy);
           base = 0;
         }
         // The first round's minimum and, for each way it can move, the
-        // second's: five minima that wait for nothing but the keys. (A step
-        // begins at an even round and their number is even, so both rounds
-        // are always allowed.)
+        // second's: five minima that wait for nothing but the keys.
         const uint32_t there = __ballot_sync(kFull, key != kNoKey) >> base;  // bit q: point q is scored
         const int q = lane - base;
-        const uint32_t bit = q >= 0 && q < 13 ? 1u << q : 0u;
+        const uint32_t bit = q >= 0 && q < (base == 0 ? 25 : 13) ? 1u << q : 0u;
         const uint32_t m1 = __reduce_min_sync(kFull, bit & 0x1eu ? key : kNoKey);
-        uint32_t m2 = kNoKey, second = 0;
+        uint32_t m2, second;
         {
           uint32_t mj[4];
 #pragma unroll
@@ -263,17 +274,36 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
           m2 = j == 0 ? mj[0] : j == 1 ? mj[1] : j == 2 ? mj[2] : mj[3];
           second = second_round(j);
         }
-        const bool moved = m1 >> 5 < bcost, again = moved && m2 < m1 && m2 >> 5 < m1 >> 5;
+        const int left = 2 * range - it;  // rounds allowed, this one the first
         nsad += __popc(there & 0x1eu);
-        if (!moved) break;
-        nsad += 1u + __popc(there & second);  // the fourth point is the old best
-        const uint32_t won = again ? m2 : m1;
+        if (!(m1 >> 5 < bcost)) break;
+        uint32_t won = m1;
+        ++it;
+        bool more = left > 1;
+        if (more) {
+          nsad += 1u + __popc(there & second);  // the fourth point is the old best
+          more = m2 >> 5 < m1 >> 5;
+        }
+        if (more) {
+          won = m2;
+          ++it;
+          more = left > 2;
+          if (more && base == 0) {
+            const uint32_t third = c_third[(m2 & 31u) - 5u];
+            nsad += __popc(there & third);
+            const uint32_t m3 = __reduce_min_sync(kFull, bit & third & ~0x1eu ? key : kNoKey);
+            more = m3 >> 5 < m2 >> 5;
+            if (more) {
+              won = m3;
+              ++it;
+            }
+          }
+        }
         const int qw = (int)(won & 31u) - base;
         bcost = won >> 5;
         fbx += around_x(qw);
         fby += around_y(qw);
-        it += 2;
-        if (!again) break;
+        if (!more) break;
         base = -1;
       }
       if (rings >= I.rings) break;
@@ -417,8 +447,8 @@ __device__ void big_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, i
   const int stride = I.ref.stride, range = I.range, plane = (int)I.ref.plane_elems;
   const float lam = I.lam;
   auto parent_of = [&](int x) -> const unsigned long long* {
-    const int px = I.psize ? x / I.psize : 0;
-    return I.psize && px < I.pnbx ? par + (ptrdiff_t)px * I.nref : nullptr;
+    const int px = x >> I.pshift;
+    return px < I.pnbx ? par + (ptrdiff_t)px * I.nref : nullptr;
   };
   // This thread's words: word wd of rows row0, row0 + RSTEP, ...
   auto load_src = [&](int bx, uint32_t (&v)[PW]) {
