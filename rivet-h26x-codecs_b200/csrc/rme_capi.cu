@@ -97,8 +97,9 @@ namespace {
 constexpr int kParts = 4;
 // The launch header in device memory (u64 words): head and tail of each
 // part's row queue (0..7), the counters (8..12), the status word, the epoch,
-// then each part's next GIVEN job and next AMP unit.
-constexpr int kMiscCounters = 8, kMiscStatus = 13, kMiscEpoch = 14, kMiscGiven = 16, kMiscAmp = 20, kMiscWords = 24;
+// then per part the next big and
+// the next other GIVEN job (two words), and so the next AMP units.
+constexpr int kMiscCounters = 8, kMiscStatus = 13, kMiscEpoch = 14, kMiscGiven = 16, kMiscAmp = 24, kMiscWords = 32;
 
 int part_of(const FrameDesc& fd) { return 2 * (fd.bd > 8) + (fd.codec == RME_CODEC_H264); }
 int part_bytes(int k) { return k >= 2 ? 2 : 1; }
@@ -739,7 +740,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   sig.push_back(n);
   sig.push_back(dev_out + 2 * pinned_out);
   std::vector<unsigned long long> rows[kParts], given[kParts];
-  int64_t part_tasks[kParts] = {0, 0, 0, 0}, amp_tasks[kParts] = {0, 0, 0, 0};
+  int64_t part_tasks[kParts] = {0, 0, 0, 0}, amp_tasks[kParts][2] = {};
   int rows_nref[kParts] = {0, 0, 0, 0};
   std::vector<const Deps*> fdeps(n, nullptr);
   for (int i = 0; i < n; ++i) {
@@ -747,8 +748,8 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     const int k = part_of(fd);
     part_tasks[k] += ntask[i];
     fd.out = dev_out ? out + (offsets ? offsets[i] : toff[i]) : sl.d_out.p + toff[i];
-    fd.amp_first[0] = amp_tasks[0];
-    fd.amp_first[1] = amp_tasks[2];
+    for (int big = 0; big < 2; ++big)
+      for (int deep = 0; deep < 2; ++deep) fd.amp_first[big][deep] = amp_tasks[2 * deep][big];
     sig.push_back(fd.bd);
     sig.push_back(fd.codec);
     if (params[i].predictor_mode == RME_PRED_GIVEN) {
@@ -769,7 +770,11 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     // A search of this buffer tags its published words anew.
     fd.mvf = sl.d_mvf.p + toff[i];
     fd.tag = fd.codec == RME_CODEC_H264 ? sl.epoch << 2 : sl.epoch;
-    if (fd.amp) amp_tasks[k] += ntask[i] - (int64_t)fd.base[fd.nlevels] * fd.nref;
+    if (fd.amp) {
+      const int64_t big = fd.size[0] == 64 ? (int64_t)(fd.amp_base[1] - fd.amp_base[0]) * fd.nref : 0;
+      amp_tasks[k][1] += big;
+      amp_tasks[k][0] += ntask[i] - (int64_t)fd.base[fd.nlevels] * fd.nref - big;
+    }
     rows_nref[k] = std::max(rows_nref[k], fd.nref);
     sig.push_back(fd.width);
     sig.push_back(fd.height);
@@ -791,6 +796,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   }
   // GIVEN jobs by their block's area, in 4x4 tiles (1..256), largest first:
   // the jobs that run last are short ones.
+  int64_t given_big[kParts] = {0, 0, 0, 0};
   for (int k = 0; k < kParts; ++k) {
     size_t at[257] = {0}, nk = 0;
     auto tiles = [](const rme_job& j) { return 256 - (j.w >> 2) * (j.h >> 2); };
@@ -799,6 +805,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
         for (int t = 0; t < ntask[i]; ++t, ++nk) ++at[tiles(frames[i].jobs[t]) + 1];
     if (nk == 0) continue;
     for (int q = 0; q < 256; ++q) at[q + 1] += at[q];
+    given_big[k] = (int64_t)at[256 - kFlatBigTiles + 1];
     given[k].resize(nk);
     for (int i = 0; i < n; ++i)
       if (!fdeps[i] && part_of(sl.h_frames.p[i]) == k)
@@ -858,7 +865,8 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     Lgiven[k] = L;
     Lgiven[k].ready = sl.d_ready.p + total + slot0;
     Lgiven[k].total = (int64_t)given[k].size();
-    Lgiven[k].head = sl.d_misc.p + kMiscGiven + k;
+    Lgiven[k].head = sl.d_misc.p + kMiscGiven + 2 * k;
+    Lgiven[k].tail = sl.d_misc.p + kMiscGiven + 2 * k + 1;
     slot0 += part_tasks[k];
     if (part_tasks[k] > 0) order[nparts++] = k;
     if (!rows[k].empty()) {
@@ -880,15 +888,16 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     cudaError_t e = cudaSuccess;
     if (!rows[k].empty())
       e = h264 ? launch_h264_rows(Ls[k], bytes, rows_nref[k], grid[k], sk) : launch_hevc_rows(Ls[k], bytes, grid[k], sk);
-    if (e == cudaSuccess && amp_tasks[k] > 0) {
+    if (e == cudaSuccess && amp_tasks[k][0] + amp_tasks[k][1] > 0) {
       LaunchDesc A = Ls[k];
-      A.head = sl.d_misc.p + kMiscAmp + k;
-      A.total = amp_tasks[k];
-      e = launch_hevc_flat(A, bytes, true, true, n, c->nsm, sk);
+      A.head = sl.d_misc.p + kMiscAmp + 2 * k;
+      A.tail = sl.d_misc.p + kMiscAmp + 2 * k + 1;
+      A.total = amp_tasks[k][0] + amp_tasks[k][1];
+      e = launch_hevc_flat(A, bytes, true, true, n, amp_tasks[k][1], c->nsm, sk);
     }
     if (e == cudaSuccess && !given[k].empty())
       e = h264 ? launch_h264_given(Lgiven[k], bytes, variant[k], c->nsm * c->bps[k][variant[k]], sk)
-               : launch_hevc_flat(Lgiven[k], bytes, false, true, n, c->nsm, sk);
+               : launch_hevc_flat(Lgiven[k], bytes, false, true, n, given_big[k], c->nsm, sk);
     return e;
   };
   auto enqueue = [&](bool capturing) -> cudaError_t {

@@ -1,6 +1,6 @@
-// HEVC searches that wait for no other search of their launch, a warp each:
-// GIVEN jobs (any block, the caller's predictors and seeds) and the AMP units
-// of STANDALONE frames, which start from their CU's finished 2Nx2N result.
+// HEVC searches that wait for no other search of their launch: GIVEN jobs
+// (any block, the caller's predictors and seeds) and the AMP units of
+// STANDALONE frames, which start from their CU's finished 2Nx2N result.
 //
 // What a search computes is search_full and refine_subpel
 // (h265_me.rs:3749-3922): candidates, order, tie-breaks and counts as
@@ -13,13 +13,18 @@
 //     (16 bits: four) words give all twelve.
 //   - SATD: a lane per 4x4 tile; a block of fewer than 32 tiles has several
 //     candidates side by side.
-// Jobs come largest first, so the last ones running are short. Bound by issue
-// and by cache reads; one warp's 64x64 search is the shortest a launch takes.
+// Blocks of kFlatBigTiles 4x4 tiles and more are searched by a CTA's four warps
+// together, smaller ones by a warp each: jobs come largest first, and a
+// 64x64 block is then a quarter as long for the launch to wait for. (It also
+// keeps a lane's words at sixteen, which sad_add's halves hold.) Bound by
+// issue and by cache reads.
 // Against a warp per task of the dataflow kernel (blocks but the square ones
 // went a word at a time; AMP units waited in its queue): the 680,160 AMP units
 // of a 2160p 10-bit frame, four references, 7.4 ms, with the frame's 2Nx2N
-// rows 19 ms for 45; 6,000 mixed 10-bit GIVEN jobs 0.76 -> 0.58 ms; 8,040
-// 16x16 units of bi refinement 155 -> 119 us.
+// rows 19 ms for 45; 6,000 mixed 10-bit GIVEN jobs 0.76 -> 0.34 ms (a warp
+// each: 0.60), 600 of 8 bits 0.07 (0.21), 20,000 of 8 bits 0.57 (0.54);
+// 8,040 16x16 units of bi refinement 155 -> 119 us. Five or six CTAs an SM
+// (spills) gain at most 2 % and lose up to 7.
 #include <algorithm>
 
 #include "rme_search_impl.cuh"
@@ -54,9 +59,27 @@ struct FlatBlock {
 // caller's own planes) the diamond is scored a point at a time. SRC: every
 // row of the source block begins on a word (a GIVEN block may lie at any
 // sample); otherwise its reads find their words by themselves.
-template <class S, bool WORDS, bool SRC>
-__device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_result* out, int lane, uint32_t& nsad,
-                            uint32_t& nsatd) {
+// W: the warps that share the search (1, or all of the CTA's, which then
+// exchange their sums through `part`).
+template <class S, bool WORDS, bool SRC, int W>
+__device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_result* out, uint32_t (*part)[W][32],
+                            uint32_t& nsad, uint32_t& nsatd) {
+  const int lane = threadIdx.x & 31, warp = W == 1 ? 0 : (int)(threadIdx.x >> 5), tid = warp * 32 + lane;
+  int buf = 0;
+  // Lane k's sum over this warp to lane k's sum over the search's warps.
+  auto total = [&](uint32_t mine) -> uint32_t {
+    if constexpr (W == 1) {
+      return mine;
+    } else {
+      part[buf][warp][lane] = mine;
+      __syncthreads();
+      uint32_t v = 0;
+#pragma unroll
+      for (int i = 0; i < W; ++i) v += part[buf][i][lane];
+      buf ^= 1;
+      return v;
+    }
+  };
   constexpr int B = (int)sizeof(S), SPW = 4 / B, WPT = 4 / SPW, NW = B == 1 ? 3 : 4;
   const DevPlanes R = F.ref[K.r];
   const int x = K.x, y = K.y, w = K.w, h = K.h, stride = R.stride, wr = w / SPW, items = wr * h;
@@ -65,8 +88,9 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
   const int range = F.search_range;
   const S* const org = plane_at<S>(R, 0, x, y);
   auto rate = [&](int mx, int my) { return hevc_rate(K.lam, mx, my, K.p0x, K.p0y, K.p1x, K.p1y); };
-  // This lane's first item and the step of 32 items.
-  const int row0 = lane / wr, wd0 = lane - row0 * wr, rstep = 32 / wr, wstep = 32 - rstep * wr;
+  // This lane's first item and the step from one to the next.
+  constexpr int STEP = 32 * W;
+  const int row0 = tid / wr, wd0 = tid - row0 * wr, rstep = STEP / wr, wstep = STEP - rstep * wr;
   auto source = [&](const S* q) -> uint32_t {
     return SRC ? RME_LD32(reinterpret_cast<const uint32_t*>(q)) : ldw(q);
   };
@@ -74,7 +98,7 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
   auto items_do = [&](auto f) {
     int row = row0, wd = wd0;
 #pragma unroll 2
-    for (int i = lane; i < items; i += 32) {
+    for (int i = tid; i < items; i += STEP) {
       f(source(K.src + (ptrdiff_t)row * K.src_stride + wd * SPW), row, wd);
       row += rstep;
       wd += wstep;
@@ -84,19 +108,22 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
       }
     }
   };
-  // One candidate's SAD.
+  // A CTA's lanes have at most sixteen words of a block; a lone warp's may
+  // have more (a caller's own job list is not sorted by size).
+  auto add = [](uint32_t a, uint32_t b, uint32_t acc) { return W > 1 ? sad_add(a, b, acc, S()) : vsad(a, b, acc, S()); };
+  auto sum_of = [](uint32_t acc) { return W > 1 ? sad_sum(acc, S()) : acc; };
+  // One candidate's SAD over this warp.
   auto sad1 = [&](int fx, int fy) -> uint32_t {
     uint32_t acc = 0;
     const S* rp = org + (ptrdiff_t)fy * stride + fx;
-    items_do([&](uint32_t s, int row, int wd) { acc = vsad(s, ldw(rp + (ptrdiff_t)row * stride + wd * SPW), acc, S()); });
-    return __reduce_add_sync(kFull, acc);
+    items_do([&](uint32_t s, int row, int wd) { acc = add(s, ldw(rp + (ptrdiff_t)row * stride + wd * SPW), acc); });
+    return __reduce_add_sync(kFull, sum_of(acc));
   };
 
   // Seeds: >> 2, clamp_pos, deduplicated (`tried`), scored in order.
   const int qx = min(max(K.sx >> 2, lox), hix), qy = min(max(K.sy >> 2, loy), hiy);
   bool dup = false;
-#pragma unroll
-  for (int j = 0; j < RME_MAX_SEEDS - 1; ++j) {
+  for (int j = 0; j + 1 < K.ns; ++j) {
     const int jx = __shfl_sync(kFull, qx, j), jy = __shfl_sync(kFull, qy, j);
     dup |= j < lane && jx == qx && jy == qy;
   }
@@ -109,6 +136,7 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
     const uint32_t v = sad1(__shfl_sync(kFull, qx, s), __shfl_sync(kFull, qy, s));
     if (lane == s) c = v;
   }
+  c = total(c);
   Pick p = warp_min((kept >> lane) & 1u ? c + rate(qx * 4, qy * 4) : kInf);
   uint32_t bcost = p.cost;
   int fbx = 0, fby = 0;
@@ -155,22 +183,22 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
                                        : (j == 0 ? v[dy + 2][1] : j == 1 ? v[dy + 2][2] : v[dy + 2][NW - 1]);
             return __funnelshift_r(lo, hi, sh);
           };
-          acc[0] = vsad(s, at(1, 0), acc[0], S());
-          acc[1] = vsad(s, at(-1, 0), acc[1], S());
-          acc[2] = vsad(s, at(0, 1), acc[2], S());
-          acc[3] = vsad(s, at(0, -1), acc[3], S());
-          acc[4] = vsad(s, at(2, 0), acc[4], S());
-          acc[5] = vsad(s, at(-2, 0), acc[5], S());
-          acc[6] = vsad(s, at(1, 1), acc[6], S());
-          acc[7] = vsad(s, at(1, -1), acc[7], S());
-          acc[8] = vsad(s, at(-1, 1), acc[8], S());
-          acc[9] = vsad(s, at(-1, -1), acc[9], S());
-          acc[10] = vsad(s, at(0, 2), acc[10], S());
-          acc[11] = vsad(s, at(0, -2), acc[11], S());
+          acc[0] = add(s, at(1, 0), acc[0]);
+          acc[1] = add(s, at(-1, 0), acc[1]);
+          acc[2] = add(s, at(0, 1), acc[2]);
+          acc[3] = add(s, at(0, -1), acc[3]);
+          acc[4] = add(s, at(2, 0), acc[4]);
+          acc[5] = add(s, at(-2, 0), acc[5]);
+          acc[6] = add(s, at(1, 1), acc[6]);
+          acc[7] = add(s, at(1, -1), acc[7]);
+          acc[8] = add(s, at(-1, 1), acc[8]);
+          acc[9] = add(s, at(-1, -1), acc[9]);
+          acc[10] = add(s, at(0, 2), acc[10]);
+          acc[11] = add(s, at(0, -2), acc[11]);
         });
 #pragma unroll
         for (int q = 0; q < 12; ++q) {
-          const uint32_t v = __reduce_add_sync(kFull, acc[q]);
+          const uint32_t v = __reduce_add_sync(kFull, sum_of(acc[q]));
           if (lane == q) mine = v;
         }
       } else {
@@ -180,6 +208,7 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
           if (lane == q) mine = v;
         }
       }
+      mine = total(mine);
       c = ok ? mine + rate(fx * 4, fy * 4) : kInf;
       nsad += __popc(there & 0xfu);
       p = warp_min(lane < 4 ? c : kInf);
@@ -225,6 +254,7 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
       const uint32_t v = sad1(__shfl_sync(kFull, fx, s), __shfl_sync(kFull, fy, s));
       if (lane == s) mine = v;
     }
+    mine = total(mine);
     nsad += __popc(there);
     p = warp_min(ok ? mine + rate(fx * 4, fy * 4) : kInf);
     if (!(p.cost < bcost)) break;
@@ -237,17 +267,17 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
   const int imx = fbx * 4, imy = fby * 4;
 
   // refine_subpel: P lanes a candidate (the tiles, rounded up to a power of
-  // two, at most 32), 32 / P candidates side by side; lane k gets candidate
-  // k's SATD.
-  const int tw = w >> 2, nt = tw * (h >> 2), lp = nt >= 32 ? 5 : 32 - __clz(nt - 1), P = 1 << lp;
-  const int t0 = lane & (P - 1), g = lane >> lp;
+  // two, at most 32 a warp), 32 / P candidates side by side; lane k gets
+  // candidate k's SATD.
+  const int tw = w >> 2, nt = tw * (h >> 2), lp = W > 1 || nt >= 32 ? 5 : 32 - __clz(nt - 1), P = 1 << lp;
+  const int t0 = W > 1 ? tid : lane & (P - 1), g = lane >> lp, tstep = W > 1 ? STEP : P;
   const bool pow2 = (tw & (tw - 1)) == 0;
   const int tsh = __ffs(tw) - 1;
   auto tile_sum = [&](int mx, int my) -> uint32_t {  // over this lane's tiles
     const S* const pp = plane_at<S>(R, (my & 3) * 4 + (mx & 3), x + (mx >> 2), y + (my >> 2));
     uint32_t acc = 0;
 #pragma unroll 2
-    for (int t = t0; t < nt; t += P) {
+    for (int t = t0; t < nt; t += tstep) {
       const int ty = pow2 ? t >> tsh : t / tw, tx = t - ty * tw;
       uint32_t pr[4][WPT], sw[4][WPT];
 #pragma unroll
@@ -276,7 +306,7 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
       const uint32_t u = __shfl_sync(kFull, v, from & 31);
       if (lane >= k0 && from < 32) got = u;
     }
-    return got;
+    return total(got);
   };
   auto half_vec = [&](int k, int& mx, int& my) {
     const int q = k == 0 ? 4 : k <= 4 ? k - 1 : k, qr = q / 3;
@@ -307,7 +337,7 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
     bsatd = __shfl_sync(kFull, v, p.lane);
     quarter_vec(p.lane, bmx, bmy);
   }
-  write_result(out, bmx, bmy, K.r, bc, bsatd, imx, imy, int_cost, nsad, nsatd, lane);
+  write_result(out, bmx, bmy, K.r, bc, bsatd, imx, imy, int_cost, nsad, nsatd, tid);
 }
 
 // A GIVEN job; false (and the status bit) for one that fails the check.
@@ -383,69 +413,95 @@ __device__ void amp_block(const FrameDesc& F, int t, int lane, FlatBlock<S>& K) 
   K.lam = F.lam;
 }
 
-// Warps take `chunk` consecutive searches at a time.
+// Searches are taken from L.head: the first `nbig` by CTAs, one at a time,
+// the others by warps, `chunk` consecutive ones at a time. GIVEN: entry i of
+// L's queue. AMP: the frames' AMP units one frame after another; those of a
+// frame's 64x64 CUs are its big ones (their halves of 1024 samples and more),
+// numbered first over all frames.
 template <class S, bool AMP, bool WORDS>
-__global__ void __launch_bounds__(kFlatWarps * 32, kFlatBlocks) hevc_flat_kernel(LaunchDesc L, int nframes, int chunk) {
+__global__ void __launch_bounds__(kFlatWarps * 32, kFlatBlocks) hevc_flat_kernel(LaunchDesc L, int nframes, int64_t nbig,
+                                                                                 int chunk) {
+  __shared__ uint32_t part[2][kFlatWarps][32];
+  __shared__ unsigned long long next;
   const int lane = threadIdx.x & 31;
+  constexpr int D = sizeof(S) == 1 ? 0 : 1;  // the frames' counts of this depth
   unsigned long long cnt[5] = {0, 0, 0, 0, 0};
-  constexpr int D = sizeof(S) == 1 ? 0 : 1;  // amp_first's depth
   int f = 0;
+  // Search i (or false): by the whole CTA, or by this warp.
+  auto search = [&](int64_t i, auto warps) {
+    constexpr int W = decltype(warps)::value;
+    int t;
+    if (AMP) {
+      const int64_t j = W > 1 ? i : i - nbig;
+      while (f + 1 < nframes && j >= L.frames[f + 1].amp_first[W > 1][D]) ++f;
+    } else {
+      const uint32_t e = (uint32_t)L.ready[i];
+      f = (int)(e >> 24);
+      t = (int)(e & 0xffffffu);
+    }
+    const FrameDesc& F = L.frames[f];
+    if (AMP) {
+      // The first level's units are the big ones where its blocks are 64x64.
+      const int big = F.size[0] == 64 ? F.amp_base[1] : F.amp_base[0];
+      t = (W > 1 ? F.amp_base[0] : big) * F.nref + (int)((W > 1 ? i : i - nbig) - F.amp_first[W > 1][D]);
+    }
+    if ((sizeof(S) == 1) != (F.bd == 8) || F.codec != RME_CODEC_HEVC || t >= F.ntasks) {
+      if (lane == 0) atomicOr(L.status, kStatusBadTask);
+      return;
+    }
+    FlatBlock<S> K;
+    if (AMP) amp_block<S>(F, t, lane, K);
+    else if (!given_block<S>(L, F, t, lane, K)) return;
+    uint32_t nsad, nsatd;
+    auto* const shared = reinterpret_cast<uint32_t(*)[W][32]>(part);
+    if (AMP || ((reinterpret_cast<uintptr_t>(K.src) & 3) == 0 && (K.src_stride * (int)sizeof(S) & 3) == 0))
+      flat_search<S, WORDS, true, W>(F, K, &F.out[t], shared, nsad, nsatd);
+    else
+      flat_search<S, WORDS, false, W>(F, K, &F.out[t], shared, nsad, nsatd);
+    if (W > 1 && threadIdx.x >= 32) return;
+    cnt[0] += 1;
+    cnt[1] += nsad;
+    cnt[2] += nsatd;
+    cnt[3] += (unsigned long long)nsad * (K.w * K.h);
+    cnt[4] += (unsigned long long)nsatd * (K.w * K.h);
+  };
+  while (nbig > 0) {
+    __syncthreads();  // the last search's sums, and its place, are read
+    if (threadIdx.x == 0) next = atomicAdd(L.head, 1ull);
+    __syncthreads();
+    const unsigned long long i = next;
+    if ((int64_t)i >= nbig) break;
+    search((int64_t)i, std::integral_constant<int, kFlatWarps>{});
+  }
+  f = 0;
   for (;;) {
     unsigned long long i0 = 0;
-    if (lane == 0) i0 = atomicAdd(L.head, (unsigned long long)chunk);
-    i0 = __shfl_sync(kFull, i0, 0);
+    if (lane == 0) i0 = atomicAdd(L.tail, (unsigned long long)chunk);
+    i0 = __shfl_sync(kFull, i0, 0) + (unsigned long long)nbig;
     if ((int64_t)i0 >= L.total) break;
     const int64_t end = min((int64_t)i0 + chunk, L.total);
-    for (int64_t i = (int64_t)i0; i < end; ++i) {
-      int t;
-      if (AMP) {
-        while (f + 1 < nframes && i >= L.frames[f + 1].amp_first[D]) ++f;
-      } else {
-        const uint32_t e = (uint32_t)L.ready[i];
-        f = (int)(e >> 24);
-        t = (int)(e & 0xffffffu);
-      }
-      const FrameDesc& F = L.frames[f];
-      if (AMP) t = F.amp_base[0] * F.nref + (int)(i - F.amp_first[D]);
-      if ((sizeof(S) == 1) != (F.bd == 8) || F.codec != RME_CODEC_HEVC || t >= F.ntasks) {
-        if (lane == 0) atomicOr(L.status, kStatusBadTask);
-        continue;
-      }
-      FlatBlock<S> K;
-      if (AMP) amp_block<S>(F, t, lane, K);
-      else if (!given_block<S>(L, F, t, lane, K)) continue;
-      uint32_t nsad, nsatd;
-      if (AMP || ((reinterpret_cast<uintptr_t>(K.src) & 3) == 0 && (K.src_stride * (int)sizeof(S) & 3) == 0))
-        flat_search<S, WORDS, true>(F, K, &F.out[t], lane, nsad, nsatd);
-      else
-        flat_search<S, WORDS, false>(F, K, &F.out[t], lane, nsad, nsatd);
-      cnt[0] += 1;
-      cnt[1] += nsad;
-      cnt[2] += nsatd;
-      cnt[3] += (unsigned long long)nsad * (K.w * K.h);
-      cnt[4] += (unsigned long long)nsatd * (K.w * K.h);
-    }
+    for (int64_t i = (int64_t)i0; i < end; ++i) search(i, std::integral_constant<int, 1>{});
   }
   if (lane < 5) atomicAdd(&L.counters[lane], lane == 0 ? cnt[0] : lane == 1 ? cnt[1] : lane == 2 ? cnt[2] : lane == 3 ? cnt[3] : cnt[4]);
 }
 
 }  // namespace
 
-cudaError_t launch_hevc_flat(const LaunchDesc& L, int bytes_per_sample, bool amp, bool words, int nframes, int nsm,
-                             cudaStream_t s) {
-  const int64_t most = (int64_t)nsm * kFlatBlocks;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((L.total + kFlatWarps - 1) / kFlatWarps, most));
+cudaError_t launch_hevc_flat(const LaunchDesc& L, int bytes_per_sample, bool amp, bool words, int nframes, int64_t nbig,
+                             int nsm, cudaStream_t s) {
+  const int64_t most = (int64_t)nsm * kFlatBlocks, small = L.total - nbig;
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nbig + (small + kFlatWarps - 1) / kFlatWarps, most));
   // Few takes from the counter while many searches are left for every warp.
-  const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(16, L.total / (most * kFlatWarps * 16)));
+  const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(16, small / (most * kFlatWarps * 16)));
   constexpr int T = kFlatWarps * 32;
   if (bytes_per_sample == 1) {
-    if (amp) hevc_flat_kernel<uint8_t, true, true><<<grid, T, 0, s>>>(L, nframes, chunk);
-    else if (words) hevc_flat_kernel<uint8_t, false, true><<<grid, T, 0, s>>>(L, nframes, chunk);
-    else hevc_flat_kernel<uint8_t, false, false><<<grid, T, 0, s>>>(L, nframes, chunk);
+    if (amp) hevc_flat_kernel<uint8_t, true, true><<<grid, T, 0, s>>>(L, nframes, nbig, chunk);
+    else if (words) hevc_flat_kernel<uint8_t, false, true><<<grid, T, 0, s>>>(L, nframes, nbig, chunk);
+    else hevc_flat_kernel<uint8_t, false, false><<<grid, T, 0, s>>>(L, nframes, nbig, chunk);
   } else {
-    if (amp) hevc_flat_kernel<uint16_t, true, true><<<grid, T, 0, s>>>(L, nframes, chunk);
-    else if (words) hevc_flat_kernel<uint16_t, false, true><<<grid, T, 0, s>>>(L, nframes, chunk);
-    else hevc_flat_kernel<uint16_t, false, false><<<grid, T, 0, s>>>(L, nframes, chunk);
+    if (amp) hevc_flat_kernel<uint16_t, true, true><<<grid, T, 0, s>>>(L, nframes, nbig, chunk);
+    else if (words) hevc_flat_kernel<uint16_t, false, true><<<grid, T, 0, s>>>(L, nframes, nbig, chunk);
+    else hevc_flat_kernel<uint16_t, false, false><<<grid, T, 0, s>>>(L, nframes, nbig, chunk);
   }
   return cudaGetLastError();
 }

@@ -50,7 +50,9 @@ struct FrameDesc {
   // (the first amp_nlev: sizes of 16 or more), and per such level the block
   // index of its first AMP unit (amp_base[0] = base[nlevels]).
   int32_t amp, amp_nmodes, amp_nlev;
-  int64_t amp_first[2];  // a batched launch: AMP units of the 8-bit, of the deeper frames before this one
+  // A batched launch: the AMP units of the 8-bit, of the deeper frames before
+  // this one; [1] those of 64x64 CUs, [0] the others.
+  int64_t amp_first[2][2];
   int32_t amp_base[kMaxLevels + 1];
   // H.264
   const uint16_t* tab;       // MvCostTable
@@ -249,13 +251,16 @@ cudaError_t launch_lowres_bi(const LowresDesc& cur, const LowresDesc& r0, const 
 constexpr int kSearchVariants = 3, kDefaultVariant = 1;
 cudaError_t launch_h264_given(const LaunchDesc& L, int bytes_per_sample, int variant, int grid, cudaStream_t s);
 int h264_given_blocks_per_sm(int bytes_per_sample, int variant);
-// HEVC searches without dependencies, a warp each (rme_flat.cu): `amp`, the
-// AMP units of L's frames (L.total of them, FrameDesc::amp_first giving each
-// frame's); else the (frame, job) entries of L's queue. L.head counts the
-// searches taken. `words`: rows, planes and origins of every picture are
-// whole 32-bit words apart (true of the library's own).
-cudaError_t launch_hevc_flat(const LaunchDesc& L, int bytes_per_sample, bool amp, bool words, int nframes, int nsm,
-                             cudaStream_t s);
+// HEVC searches without dependencies (rme_flat.cu): `amp`, the AMP units of
+// L's frames (L.total of them, FrameDesc::amp_first giving each frame's);
+// else the (frame, job) entries of L's queue. The first `nbig` searches are
+// the units of 64x64 CUs, the jobs of kFlatBigTiles 4x4 tiles and more, each
+// searched by a CTA. L.head and L.tail count the big and the other searches
+// taken. `words`: rows, planes and origins of every picture are whole 32-bit
+// words apart (true of the library's own).
+constexpr int kFlatBigTiles = 64;
+cudaError_t launch_hevc_flat(const LaunchDesc& L, int bytes_per_sample, bool amp, bool words, int nframes, int64_t nbig,
+                             int nsm, cudaStream_t s);
 // HEVC STANDALONE frames' 2Nx2N blocks in their row form (rme_rows.cu): L's
 // queue holds row_entry words, each the first of hevc_row_rows(size)
 // consecutive rows, all pushed by the host, each after the rows it reads.

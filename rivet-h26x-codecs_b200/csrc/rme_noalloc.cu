@@ -183,7 +183,10 @@ extern "C" int rme_search_given_noalloc(const rme_picture_desc* d, const rme_par
     };
     bool words = whole(fd.src);
     for (int r = 0; r < nref; ++r) words = words && whole(fd.ref[r]);
-    if (launch_hevc_flat(L, bytes, false, words, 1, nsm, s) != cudaSuccess) return RME_ECUDA;
+    // The jobs are in device memory, in the caller's order: their sizes are
+    // not known here, so a warp searches each.
+    L.tail = d_misc + 2;
+    if (launch_hevc_flat(L, bytes, false, words, 1, 0, nsm, s) != cudaSuccess) return RME_ECUDA;
   }
   if (cudaMemcpyAsync(misc, d_misc, sizeof(misc), cudaMemcpyDeviceToHost, s) != cudaSuccess) return RME_ECUDA;
   if (cudaStreamSynchronize(s) != cudaSuccess) return RME_ECUDA;
