@@ -5,12 +5,13 @@
 // What a search computes is search_full and refine_subpel
 // (h265_me.rs:3749-3922): candidates, order, tie-breaks and counts as
 // hevc_task has them. Blocks are any multiple of 4 up to 64x64, so a lane
-// takes whole words of the block wherever they lie: item i is word i % wr of
-// row i / wr, lanes on consecutive items, and every candidate of a step is
-// scored on the lane's words at once.
-//   - Seeds: one after another, a word and its neighbour per item.
-//   - Diamond: the twelve points of two rounds; per item five rows of three
-//     (16 bits: four) words give all twelve.
+// takes one word column of a run of rows, and every candidate of a step is
+// scored on its words at once.
+//   - Seeds: one after another, a word and its neighbour per row.
+//   - Diamond: the twelve points of two rounds; five rows of three (16 bits:
+//     four) words give all twelve, and each row is read once: the L1's
+//     wavefronts, not the arithmetic, bound the kernel (60 % of their peak
+//     when every word read its five rows).
 //   - SATD: a lane per 4x4 tile; a block of fewer than 32 tiles has several
 //     candidates side by side.
 // Blocks of kFlatBigTiles 4x4 tiles and more are searched by a CTA's four warps
@@ -20,11 +21,10 @@
 // issue and by cache reads.
 // Against a warp per task of the dataflow kernel (blocks but the square ones
 // went a word at a time; AMP units waited in its queue): the 680,160 AMP units
-// of a 2160p 10-bit frame, four references, 7.4 ms, with the frame's 2Nx2N
-// rows 19 ms for 45; 6,000 mixed 10-bit GIVEN jobs 0.76 -> 0.34 ms (a warp
-// each: 0.60), 600 of 8 bits 0.07 (0.21), 20,000 of 8 bits 0.57 (0.54);
-// 8,040 16x16 units of bi refinement 155 -> 119 us. Five or six CTAs an SM
-// (spills) gain at most 2 % and lose up to 7.
+// of a 2160p 10-bit frame, four references, 7.0 ms, with the frame's 2Nx2N
+// rows 17.5 ms for 45; 6,000 mixed 10-bit GIVEN jobs 0.76 -> 0.27 ms (a warp
+// each: 0.60), 600 of 8 bits 0.06 (0.21), 20,000 of 8 bits 0.48. Five or six
+// CTAs an SM (spills) gain at most 2 % and lose up to 7.
 #include <algorithm>
 
 #include "rme_search_impl.cuh"
@@ -82,31 +82,19 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
   };
   constexpr int B = (int)sizeof(S), SPW = 4 / B, WPT = 4 / SPW, NW = B == 1 ? 3 : 4;
   const DevPlanes R = F.ref[K.r];
-  const int x = K.x, y = K.y, w = K.w, h = K.h, stride = R.stride, wr = w / SPW, items = wr * h;
+  const int x = K.x, y = K.y, w = K.w, h = K.h, stride = R.stride, wr = w / SPW;
   const int padm = F.pad - 4;
   const int lox = -padm - x, hix = F.width + padm - w - x, loy = -padm - y, hiy = F.height + padm - h - y;
   const int range = F.search_range;
   const S* const org = plane_at<S>(R, 0, x, y);
   auto rate = [&](int mx, int my) { return hevc_rate(K.lam, mx, my, K.p0x, K.p0y, K.p1x, K.p1y); };
-  // This lane's first item and the step from one to the next.
+  // This lane's words: word wd of `rows` rows from row0 (none for the lanes
+  // left over). Rows follow one another, so the diamond reads each once.
   constexpr int STEP = 32 * W;
-  const int row0 = tid / wr, wd0 = tid - row0 * wr, rstep = STEP / wr, wstep = STEP - rstep * wr;
+  const int segs = min(STEP / wr, h), each = (h + segs - 1) / segs;
+  const int seg = tid / wr, wd = tid - seg * wr, row0 = seg * each, rows = seg < segs ? min(each, h - row0) : 0;
   auto source = [&](const S* q) -> uint32_t {
     return SRC ? RME_LD32(reinterpret_cast<const uint32_t*>(q)) : ldw(q);
-  };
-  // f(source word, row, word) over the lane's items.
-  auto items_do = [&](auto f) {
-    int row = row0, wd = wd0;
-#pragma unroll 2
-    for (int i = tid; i < items; i += STEP) {
-      f(source(K.src + (ptrdiff_t)row * K.src_stride + wd * SPW), row, wd);
-      row += rstep;
-      wd += wstep;
-      if (wd >= wr) {
-        wd -= wr;
-        ++row;
-      }
-    }
   };
   // A CTA's lanes have at most sixteen words of a block; a lone warp's may
   // have more (a caller's own job list is not sorted by size).
@@ -115,8 +103,10 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
   // One candidate's SAD over this warp.
   auto sad1 = [&](int fx, int fy) -> uint32_t {
     uint32_t acc = 0;
-    const S* rp = org + (ptrdiff_t)fy * stride + fx;
-    items_do([&](uint32_t s, int row, int wd) { acc = add(s, ldw(rp + (ptrdiff_t)row * stride + wd * SPW), acc); });
+    const S* rp = org + (ptrdiff_t)(fy + row0) * stride + fx + wd * SPW;
+    const S* sp = K.src + (ptrdiff_t)row0 * K.src_stride + wd * SPW;
+#pragma unroll 4
+    for (int k = 0; k < rows; ++k) acc = add(source(sp + (ptrdiff_t)k * K.src_stride), ldw(rp + (ptrdiff_t)k * stride), acc);
     return __reduce_add_sync(kFull, sum_of(acc));
   };
 
@@ -167,13 +157,14 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
         const uint32_t off = (uint32_t)(a0 & 3);
         const uint32_t* const q0 = reinterpret_cast<const uint32_t*>(a0 & ~uintptr_t(3));
         const int rs = stride * B / 4;  // rows are whole words apart
-        items_do([&](uint32_t s, int row, int wd) {
-          const uint32_t* wp = q0 + (ptrdiff_t)row * rs + wd;
+        const uint32_t* wp = q0 + (ptrdiff_t)(row0 - 2) * rs + wd;
+        const S* sp = K.src + (ptrdiff_t)row0 * K.src_stride + wd * SPW;
+        if (rows > 0) {
           uint32_t v[5][NW];
 #pragma unroll
-          for (int dy = -2; dy <= 2; ++dy)
+          for (int i = 0; i < 4; ++i, wp += rs)
 #pragma unroll
-            for (int j = 0; j < NW; ++j) v[dy + 2][j] = RME_LD32(wp + (ptrdiff_t)dy * rs + j);
+            for (int j = 0; j < NW; ++j) v[i][j] = RME_LD32(wp + j);
           auto at = [&](int dx, int dy) {  // the word of samples at (dx, dy)
             const uint32_t o = off + (uint32_t)((dx + 2) * B), sh = (o & 3u) * 8u;
             const int j = (int)(o >> 2);
@@ -183,19 +174,29 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
                                        : (j == 0 ? v[dy + 2][1] : j == 1 ? v[dy + 2][2] : v[dy + 2][NW - 1]);
             return __funnelshift_r(lo, hi, sh);
           };
-          acc[0] = add(s, at(1, 0), acc[0]);
-          acc[1] = add(s, at(-1, 0), acc[1]);
-          acc[2] = add(s, at(0, 1), acc[2]);
-          acc[3] = add(s, at(0, -1), acc[3]);
-          acc[4] = add(s, at(2, 0), acc[4]);
-          acc[5] = add(s, at(-2, 0), acc[5]);
-          acc[6] = add(s, at(1, 1), acc[6]);
-          acc[7] = add(s, at(1, -1), acc[7]);
-          acc[8] = add(s, at(-1, 1), acc[8]);
-          acc[9] = add(s, at(-1, -1), acc[9]);
-          acc[10] = add(s, at(0, 2), acc[10]);
-          acc[11] = add(s, at(0, -2), acc[11]);
-        });
+#pragma unroll 2
+          for (int k = 0; k < rows; ++k, wp += rs, sp += K.src_stride) {
+#pragma unroll
+            for (int j = 0; j < NW; ++j) v[4][j] = RME_LD32(wp + j);
+            const uint32_t s = source(sp);
+            acc[0] = add(s, at(1, 0), acc[0]);
+            acc[1] = add(s, at(-1, 0), acc[1]);
+            acc[2] = add(s, at(0, 1), acc[2]);
+            acc[3] = add(s, at(0, -1), acc[3]);
+            acc[4] = add(s, at(2, 0), acc[4]);
+            acc[5] = add(s, at(-2, 0), acc[5]);
+            acc[6] = add(s, at(1, 1), acc[6]);
+            acc[7] = add(s, at(1, -1), acc[7]);
+            acc[8] = add(s, at(-1, 1), acc[8]);
+            acc[9] = add(s, at(-1, -1), acc[9]);
+            acc[10] = add(s, at(0, 2), acc[10]);
+            acc[11] = add(s, at(0, -2), acc[11]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+              for (int j = 0; j < NW; ++j) v[i][j] = v[i + 1][j];
+          }
+        }
 #pragma unroll
         for (int q = 0; q < 12; ++q) {
           const uint32_t v = __reduce_add_sync(kFull, sum_of(acc[q]));
@@ -273,21 +274,31 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
   const int t0 = W > 1 ? tid : lane & (P - 1), g = lane >> lp, tstep = W > 1 ? STEP : P;
   const bool pow2 = (tw & (tw - 1)) == 0;
   const int tsh = __ffs(tw) - 1;
+  auto source_tile = [&](int t, uint32_t (&sw)[4][WPT]) {
+    const int ty = pow2 ? t >> tsh : t / tw, tx = t - ty * tw;
+#pragma unroll
+    for (int rr = 0; rr < 4; ++rr) {
+      const S* sp = K.src + (ptrdiff_t)(ty * 4 + rr) * K.src_stride + tx * 4;
+#pragma unroll
+      for (int q = 0; q < WPT; ++q) sw[rr][q] = source(sp + q * SPW);
+    }
+  };
+  uint32_t first[4][WPT] = {};  // the lane's first tile, most blocks' only one
+  if (t0 < nt) source_tile(t0, first);
   auto tile_sum = [&](int mx, int my) -> uint32_t {  // over this lane's tiles
     const S* const pp = plane_at<S>(R, (my & 3) * 4 + (mx & 3), x + (mx >> 2), y + (my >> 2));
-    uint32_t acc = 0;
-#pragma unroll 2
-    for (int t = t0; t < nt; t += tstep) {
+    auto tile = [&](int t, const uint32_t (&sw)[4][WPT]) {
       const int ty = pow2 ? t >> tsh : t / tw, tx = t - ty * tw;
-      uint32_t pr[4][WPT], sw[4][WPT];
+      uint32_t pr[4][WPT];
 #pragma unroll
-      for (int rr = 0; rr < 4; ++rr) {
-        ldwords<WPT>(pp + (ptrdiff_t)(ty * 4 + rr) * stride + tx * 4, pr[rr]);
-        const S* sp = K.src + (ptrdiff_t)(ty * 4 + rr) * K.src_stride + tx * 4;
-#pragma unroll
-        for (int q = 0; q < WPT; ++q) sw[rr][q] = source(sp + q * SPW);
-      }
-      acc += satd4x4<WPT>(sw, pr);
+      for (int rr = 0; rr < 4; ++rr) ldwords<WPT>(pp + (ptrdiff_t)(ty * 4 + rr) * stride + tx * 4, pr[rr]);
+      return satd4x4<WPT>(sw, pr);
+    };
+    uint32_t acc = t0 < nt ? tile(t0, first) : 0u;
+    for (int t = t0 + tstep; t < nt; t += tstep) {
+      uint32_t sw[4][WPT];
+      source_tile(t, sw);
+      acc += tile(t, sw);
     }
     return acc;
   };

@@ -437,10 +437,10 @@ struct BigSmem {
 template <class S, int N, int T>
 __device__ void big_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, int row, BigSmem<S, N>& sm, int tid,
                         int bar, RowCount& cnt) {
-  constexpr int B = (int)sizeof(S), SPW = 4 / B, WR = N / SPW, NSRC = N * WR, PW = NSRC / T, RSTEP = T / WR;
+  constexpr int B = (int)sizeof(S), SPW = 4 / B, WR = N / SPW, NSRC = N * WR, PW = NSRC / T, NW = B == 1 ? 3 : 4;
   constexpr int TW = N / 4, NT = TW * TW, WPT = 4 / SPW, WRW = BigSmem<S, N>::WRW, ROWS = BigSmem<S, N>::ROWS;
-  static_assert(NSRC % T == 0 && T % WR == 0 && T % NT == 0, "a thread's words and tile");
-  const int y = row * N, lane = tid & 31, wd = tid % WR, row0 = tid / WR;
+  static_assert(NSRC % T == 0 && T % WR == 0 && T % NT == 0 && PW <= 16, "a thread's words and tile");
+  const int y = row * N, lane = tid & 31, wd = tid % WR, row0 = tid / WR * PW;
   const RowInfo<S> I = row_info<S>(F, l, r, y);
   const unsigned long long* const up = I.mvf + ((ptrdiff_t)(I.base + (row - 1) * I.nbx)) * I.nref + I.r;
   const unsigned long long* const par = I.mvf + (ptrdiff_t)I.pbase * I.nref + I.r;
@@ -450,11 +450,11 @@ __device__ void big_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, i
     const int px = x >> I.pshift;
     return px < I.pnbx ? par + (ptrdiff_t)px * I.nref : nullptr;
   };
-  // This thread's words: word wd of rows row0, row0 + RSTEP, ...
+  // This thread's words: word wd of rows row0 .. row0 + PW - 1.
   auto load_src = [&](int bx, uint32_t (&v)[PW]) {
     const uint32_t* o = reinterpret_cast<const uint32_t*>(plane_at<S>(I.src, 0, bx * N, y + row0)) + wd;
 #pragma unroll
-    for (int k = 0; k < PW; ++k) v[k] = RME_LD32(o + (ptrdiff_t)k * RSTEP * I.src.stride * B / 4);
+    for (int k = 0; k < PW; ++k) v[k] = RME_LD32(o + (ptrdiff_t)k * I.src.stride * B / 4);
   };
   uint32_t sw[PW];
   load_src(0, sw);
@@ -479,7 +479,7 @@ __device__ void big_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, i
     const int x = bx * N;
     uint32_t* const src = sm.src[bx & 1];
 #pragma unroll
-    for (int k = 0; k < PW; ++k) src[tid + k * T] = sw[k];
+    for (int k = 0; k < PW; ++k) src[(row0 + k) * WR + wd] = sw[k];
     if (row > 0) uw = wait_word(L, up + (ptrdiff_t)bx * I.nref, I.tag, uw);
     const unsigned long long* const pp = parent_of(x);
     if (pp) pw = wait_word(L, pp, I.tag, pw);
@@ -542,10 +542,10 @@ __device__ void big_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, i
       const S* rp = org + (ptrdiff_t)(fy + row0) * stride + fx + wd * SPW;
       uint32_t a[PW], acc = 0;
 #pragma unroll
-      for (int k = 0; k < PW; ++k) a[k] = ldw(rp + (ptrdiff_t)k * RSTEP * stride);
+      for (int k = 0; k < PW; ++k) a[k] = ldw(rp + (ptrdiff_t)k * stride);
 #pragma unroll
-      for (int k = 0; k < PW; ++k) acc = vsad(sw[k], a[k], acc, S());
-      acc = __reduce_add_sync(kFull, acc);
+      for (int k = 0; k < PW; ++k) acc = sad_add(sw[k], a[k], acc, S());
+      acc = __reduce_add_sync(kFull, sad_sum(acc, S()));
       if (lane == s) mine = acc;
     }
     uint32_t c = total(mine, 4);
@@ -569,42 +569,44 @@ __device__ void big_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, i
         // The byte offset of dx = -2 in a window row, and for each dx whether
         // its samples begin in the first or the second word from there.
         const uint32_t b0 = woff + (uint32_t)((fbx - scx + kMargin - 2) * B);
-        const int wi = (int)(b0 >> 2), r0 = fby - scy + kMargin;
+        // The thread's rows follow one another: five rows of words are kept,
+        // each row read once.
+        const uint32_t* const wp = sm.win + (fby - scy + kMargin + row0) * WRW + (b0 >> 2) + wd;
+        uint32_t w[5][NW];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < NW; ++j) w[i][j] = wp[(i - 2) * WRW + j];
 #pragma unroll
         for (int k = 0; k < PW; ++k) {
-          const uint32_t* wp = sm.win + (r0 + row0 + k * RSTEP) * WRW + wi + wd;
-          uint32_t w[5][4];
 #pragma unroll
-          for (int dy = -2; dy <= 2; ++dy)
-#pragma unroll
-            for (int j = 0; j < (B == 1 ? 3 : 4); ++j) w[dy + 2][j] = wp[dy * WRW + j];
+          for (int j = 0; j < NW; ++j) w[(k + 4) % 5][j] = wp[(k + 2) * WRW + j];
           auto at = [&](int dx, int dy) {  // the four (two) samples at dx, dy
+            const uint32_t (&v)[NW] = w[(k + dy + 2) % 5];
             const uint32_t o = (b0 & 3u) + (uint32_t)((dx + 2) * B), sh = (o & 3u) * 8u;
             const int j = (int)(o >> 2);
-            const uint32_t lo = B == 1 ? (j ? w[dy + 2][1] : w[dy + 2][0])
-                                       : (j == 0 ? w[dy + 2][0] : j == 1 ? w[dy + 2][1] : w[dy + 2][2]);
-            const uint32_t hi = B == 1 ? (j ? w[dy + 2][2] : w[dy + 2][1])
-                                       : (j == 0 ? w[dy + 2][1] : j == 1 ? w[dy + 2][2] : w[dy + 2][3]);
+            const uint32_t lo = B == 1 ? (j ? v[1] : v[0]) : (j == 0 ? v[0] : j == 1 ? v[1] : v[2]);
+            const uint32_t hi = B == 1 ? (j ? v[2] : v[1]) : (j == 0 ? v[1] : j == 1 ? v[2] : v[NW - 1]);
             return __funnelshift_r(lo, hi, sh);
           };
           const uint32_t s = sw[k];
-          acc[0] = vsad(s, at(1, 0), acc[0], S());
-          acc[1] = vsad(s, at(-1, 0), acc[1], S());
-          acc[2] = vsad(s, at(0, 1), acc[2], S());
-          acc[3] = vsad(s, at(0, -1), acc[3], S());
-          acc[4] = vsad(s, at(2, 0), acc[4], S());
-          acc[5] = vsad(s, at(-2, 0), acc[5], S());
-          acc[6] = vsad(s, at(1, 1), acc[6], S());
-          acc[7] = vsad(s, at(1, -1), acc[7], S());
-          acc[8] = vsad(s, at(-1, 1), acc[8], S());
-          acc[9] = vsad(s, at(-1, -1), acc[9], S());
-          acc[10] = vsad(s, at(0, 2), acc[10], S());
-          acc[11] = vsad(s, at(0, -2), acc[11], S());
+          acc[0] = sad_add(s, at(1, 0), acc[0], S());
+          acc[1] = sad_add(s, at(-1, 0), acc[1], S());
+          acc[2] = sad_add(s, at(0, 1), acc[2], S());
+          acc[3] = sad_add(s, at(0, -1), acc[3], S());
+          acc[4] = sad_add(s, at(2, 0), acc[4], S());
+          acc[5] = sad_add(s, at(-2, 0), acc[5], S());
+          acc[6] = sad_add(s, at(1, 1), acc[6], S());
+          acc[7] = sad_add(s, at(1, -1), acc[7], S());
+          acc[8] = sad_add(s, at(-1, 1), acc[8], S());
+          acc[9] = sad_add(s, at(-1, -1), acc[9], S());
+          acc[10] = sad_add(s, at(0, 2), acc[10], S());
+          acc[11] = sad_add(s, at(0, -2), acc[11], S());
         }
         mine = 0;
 #pragma unroll
         for (int q = 0; q < 12; ++q) {
-          const uint32_t v = __reduce_add_sync(kFull, acc[q]);
+          const uint32_t v = __reduce_add_sync(kFull, sad_sum(acc[q], S()));
           if (lane == q) mine = v;
         }
         c = total(mine, 12);
@@ -656,8 +658,8 @@ __device__ void big_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, i
         const S* rp = org + (ptrdiff_t)(fy + row0) * stride + fx + wd * SPW;
         uint32_t acc = 0;
 #pragma unroll
-        for (int j = 0; j < PW; ++j) acc = vsad(sw[j], ldw(rp + (ptrdiff_t)j * RSTEP * stride), acc, S());
-        acc = __reduce_add_sync(kFull, acc);
+        for (int j = 0; j < PW; ++j) acc = sad_add(sw[j], ldw(rp + (ptrdiff_t)j * stride), acc, S());
+        acc = __reduce_add_sync(kFull, sad_sum(acc, S()));
         if (lane == k) mine = acc;
       }
       c = total(mine, 24);
