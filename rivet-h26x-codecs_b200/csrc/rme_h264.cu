@@ -39,6 +39,24 @@ namespace {
 constexpr int kRefThreads = 128;  // threads per reference
 constexpr int kSlots16 = 16;      // candidates a step scores at once
 
+// Small tables as hex digits (the lowest first), so that lanes with entries of
+// their own do not queue at the constant cache: the hexagon's and the square's
+// offsets + 2, the UMH hexagon's + 2, the refinement ring's + 1.
+__device__ __forceinline__ int digit(unsigned long long t, int k) { return (int)((t >> (4 * k)) & 15u); }
+__device__ __forceinline__ int hex_x(int k) { return digit(0x134310ull, k) - 2; }
+__device__ __forceinline__ int hex_y(int k) { return digit(0x442002ull, k) - 2; }
+__device__ __forceinline__ int square_x(int k) { return digit(0x32131321ull, k) - 2; }
+__device__ __forceinline__ int square_y(int k) { return digit(0x33322111ull, k) - 2; }
+__device__ __forceinline__ int hex12_x(int k) { return digit(0x404031314400ull, k) - 2; }
+__device__ __forceinline__ int hex12_y(int k) { return digit(0x4400441313ull, k) - 2; }
+__device__ __forceinline__ int ring_x(int k) { return digit(0x20201201ull, k) - 1; }
+__device__ __forceinline__ int ring_y(int k) { return digit(0x22002110ull, k) - 1; }
+// The quarter-sample table (8.4.2.2.1): per position (fy * 4 + fx) a digit
+// plane * 4 + dy * 2 + dx of the first view and of the second; positions
+// 0, 2, 8 and 10 have one view.
+constexpr unsigned long long kView1 = 0x9c88cc8844404400ull, kView2 = 0x666290c09c881040ull;
+constexpr uint32_t kTwoViews = 0xfafau;
+
 struct RefResult {
   uint32_t cost, satd, icost;
   int mx, my, imx, imy;
@@ -147,9 +165,9 @@ struct RefSearch {
     {
       const bool ok = (keep >> slot) & 1u;
       const int fx = __shfl_sync(kFull, qx, slot), fy = __shfl_sync(kFull, qy, slot);
-      const uint32_t s = sad(ok, fx, fy);
+      const uint32_t rt = rate(fx * 4, fy * 4), s = sad(ok, fx, fy);
       nsad += count(ok);
-      const Pick p = warp_min(share(ok ? s + rate(fx * 4, fy * 4) : kInf));
+      const Pick p = warp_min(share(ok ? s + rt : kInf));
       bcost = p.cost;
       bx = __shfl_sync(kFull, qx, p.lane);
       by = __shfl_sync(kFull, qy, p.lane);
@@ -166,8 +184,8 @@ struct RefSearch {
           y = cy + (k == 2 ? -rr : k == 3 ? rr : 0);
         } else {
           const int j = i - ncross, rr = 4 * (j / 12 + 1), k = j % 12;
-          x = cx + c_hex12[k][0] * rr / 2;
-          y = cy + c_hex12[k][1] * rr / 2;
+          x = cx + hex12_x(k) * rr / 2;
+          y = cy + hex12_y(k) * rr / 2;
         }
       };
       uint32_t mc = kInf, mi = 0xffffffffu;  // this lane's least cost, its first point
@@ -177,9 +195,9 @@ struct RefSearch {
         int x = 0, y = 0;
         if (i < total) point(i, x, y);
         const bool ok = i < total && inside(x, y);
-        const uint32_t s = sad(ok, x, y);
+        const uint32_t rt = rate(x * 4, y * 4), s = sad(ok, x, y);
         nsad += count(ok);
-        const uint32_t c = ok ? s + rate(x * 4, y * 4) : kInf;
+        const uint32_t c = ok ? s + rt : kInf;
         if (c < mc) {
           mc = c;
           mi = (uint32_t)i;
@@ -210,9 +228,9 @@ struct RefSearch {
         int ox, oy;
         off(slot, ox, oy);
         const bool ok = slot < 4 && inside(bx + ox, by + oy);
-        const uint32_t s = sad(ok, bx + ox, by + oy);
+        const uint32_t rt = rate((bx + ox) * 4, (by + oy) * 4), s = sad(ok, bx + ox, by + oy);
         nsad += count(ok);
-        const Pick p = warp_min(share(ok ? s + rate((bx + ox) * 4, (by + oy) * 4) : kInf));
+        const Pick p = warp_min(share(ok ? s + rt : kInf));
         if (!(p.cost < bcost)) break;
         bcost = p.cost;
         off(p.lane, ox, oy);
@@ -227,20 +245,20 @@ struct RefSearch {
         auto off = [&](int k, int& ox, int& oy) {
           if (k < 6) {
             const int e = dir < 0 ? k : k == 0 ? (dir + 5) % 6 : k == 1 ? dir : (dir + 1) % 6;
-            ox = c_hex[e][0];
-            oy = c_hex[e][1];
+            ox = hex_x(e);
+            oy = hex_y(e);
           } else {
-            ox = c_sq[k - 6][0];
-            oy = c_sq[k - 6][1];
+            ox = square_x(k - 6);
+            oy = square_y(k - 6);
           }
         };
         const int nhex = it == 0 ? 6 : it < range ? 3 : 0;
         int ox = 0, oy = 0;
         if (slot < 14) off(slot, ox, oy);
         const bool ok = (slot < 6 ? slot < nhex : slot < 14) && inside(bx + ox, by + oy);
-        const uint32_t s = sad(ok, bx + ox, by + oy);
+        const uint32_t rt = rate((bx + ox) * 4, (by + oy) * 4), s = sad(ok, bx + ox, by + oy);
         nsad += count(ok && slot < 6);
-        const uint32_t c = share(ok ? s + rate((bx + ox) * 4, (by + oy) * 4) : kInf);
+        const uint32_t c = share(ok ? s + rt : kInf);
         Pick p = warp_min(lane < 6 ? c : kInf);
         const bool step = p.cost < bcost;
         if (!step) {
@@ -283,8 +301,8 @@ struct RefSearch {
           mx = cmx;
           my = cmy;
           if (c >= base) {
-            mx = (int)(int16_t)(cmx + c_ring[(c - base) & 7][0] * step);
-            my = (int)(int16_t)(cmy + c_ring[(c - base) & 7][1] * step);
+            mx = (int)(int16_t)(cmx + ring_x((c - base) & 7) * step);
+            my = (int)(int16_t)(cmy + ring_y((c - base) & 7) * step);
           }
         };
         int mx, my;
@@ -293,19 +311,20 @@ struct RefSearch {
         if (slot >= base)
           ok = ok && mx >= qlx && mx <= qhx && my >= qly && my <= qhy &&
                !(has_prev && abs(mx - prevx) <= step && abs(my - prevy) <= step);
+        const uint32_t rt = rate(mx, my);
         uint32_t sv = 0;
         if (ok) {
           const int xi = B.x + (mx >> 2), yi = B.y + (my >> 2);
-          const int8_t* q = c_h264_qpel[(my & 3) * 4 + (mx & 3)];
-          const S* p1 = plane_at<S>(R, q[0], xi + q[1], yi + q[2]);
-          const S* p2 = q[3] < 0 ? nullptr : plane_at<S>(R, q[3], xi + q[4], yi + q[5]);
+          const int pos = (my & 3) * 4 + (mx & 3), a = digit(kView1, pos), b = digit(kView2, pos);
+          const S* p1 = plane_at<S>(R, a >> 2, xi + (a & 1), yi + ((a >> 1) & 1));
+          const S* p2 = (kTwoViews >> pos) & 1u ? plane_at<S>(R, b >> 2, xi + (b & 1), yi + ((b >> 1) & 1)) : nullptr;
           sv = satd_strips<S, 2>(src, WR, 4, 4, p1, p2, R.stride, 8, sub);
         }
         sv += __shfl_xor_sync(kFull, sv, 4);
         sv += __shfl_xor_sync(kFull, sv, 2);
         sv += __shfl_xor_sync(kFull, sv, 1);
         nsatd += count(ok);
-        const Pick p = warp_min(share(ok ? sv + rate(mx, my) : kInf));
+        const Pick p = warp_min(share(ok ? sv + rt : kInf));
         if (p.cost < bc) {
           bc = p.cost;
           vec(p.lane, bmx, bmy);
