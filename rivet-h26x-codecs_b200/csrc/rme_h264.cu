@@ -57,6 +57,18 @@ __device__ __forceinline__ int ring_y(int k) { return digit(0x22002110ull, k) - 
 constexpr unsigned long long kView1 = 0x9c88cc8844404400ull, kView2 = 0x666290c09c881040ull;
 constexpr uint32_t kTwoViews = 0xfafau;
 
+// A reference's staged samples: its four planes kWinM samples around the seeds'
+// best point, in rows of an odd number of 16-byte chunks (eight rows on eight
+// different banks); the planes a chunk apart more, so that candidates of
+// different planes fall on different banks.
+constexpr int kWinM = 8, kWinRows = 16 + 2 * kWinM;
+template <class S>
+struct Win {
+  static constexpr int CH = sizeof(S) == 1 ? 3 : 5;  // chunks that hold kWinRows samples from any byte on
+  static constexpr int PITCH = CH * 4, PLANE = kWinRows * PITCH + 4, WORDS = 4 * PLANE;
+  static_assert((kWinRows * (int)sizeof(S) + 15 + 4) / 16 <= CH && CH % 2 == 1, "row width");
+};
+
 struct RefResult {
   uint32_t cost, satd, icost;
   int mx, my, imx, imy;
@@ -64,6 +76,7 @@ struct RefResult {
 
 template <class S>
 struct RowSmem {
+  alignas(16) uint32_t win[RME_MAX_REFS][Win<S>::WORDS];
   uint32_t src[2][16 * 16 * sizeof(S) / 4];
   uint32_t cost[RME_MAX_REFS][2][kSlots16];
   uint32_t best[RME_MAX_REFS][4][2];  // UMH: each warp's least cost and its point
@@ -110,6 +123,9 @@ struct RefSearch {
   H264Blk B;
   const S* org;
   int g, warp, lane, sub, slot;  // group; warp in it; this lane's part of candidate `slot`
+  int height;         // the plane's coded height
+  uint32_t* win;      // this reference's window
+  int wx = 0, wy = 0, wofs = 0;  // its centre; the centre's first byte in a row
   int buf = 0;
   uint32_t nsad = 0, nsatd = 0;  // this warp's candidates
 
@@ -123,13 +139,116 @@ struct RefSearch {
       uint32_t a[WR], b[WR];
       ldwords<WR>(rp, a);
       ldwords<WR>(rp + (ptrdiff_t)8 * R.stride, b);
-#pragma unroll
-      for (int k = 0; k < WR; ++k) acc = vsad(src[(sub + 8) * WR + k], b[k], vsad(src[sub * WR + k], a[k], acc, S()), S());
+      acc = sad2(a, b);
     }
     acc += __shfl_xor_sync(kFull, acc, 4);
     acc += __shfl_xor_sync(kFull, acc, 2);
     acc += __shfl_xor_sync(kFull, acc, 1);
     return acc;
+  }
+  // Copies rows of 16-byte chunks around whole-sample offset (x, y) into the
+  // window, unwaited. What lies outside the padded plane is clamped to it: no
+  // candidate reads it.
+  __device__ __forceinline__ void copy_chunk(uint32_t* dst, int plane, int row, int chunk) {
+    const int stride = R.stride * (int)sizeof(S);
+    row = min(max(row, -kH264Pad), height + kH264Pad - 1);
+    chunk = min(max(chunk, 0), stride / 16 - 1);
+    const char* p = reinterpret_cast<const char*>(plane_at<S>(R, plane, -kH264Pad, row)) + chunk * 16;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(p)
+                 : "memory");
+  }
+  // The four planes around (x, y): plane 0 as one copy group, the others the next.
+  __device__ __forceinline__ void stage(int x, int y) {
+    typedef Win<S> W;
+    wx = x;
+    wy = y;
+    const int byte = (B.x + x - kWinM + kH264Pad) * (int)sizeof(S), c0 = byte >> 4;
+    wofs = (byte & 15) + kWinM * (int)sizeof(S);
+    const int t = warp * 32 + lane, row0 = B.y + y - kWinM;
+    constexpr int N1 = kWinRows * W::CH;
+    for (int i = t; i < N1; i += kRefThreads)
+      copy_chunk(win + (i / W::CH) * W::PITCH + (i % W::CH) * 4, 0, row0 + i / W::CH, c0 + i % W::CH);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int i = t; i < 3 * N1; i += kRefThreads) {
+      const int q = i / W::CH, pl = 1 + q / kWinRows, row = q % kWinRows;
+      copy_chunk(win + pl * W::PLANE + row * W::PITCH + (i % W::CH) * 4, pl, row0 + row, c0 + i % W::CH);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // Whether points lo .. hi samples from (x, y) lie in the window.
+  __device__ __forceinline__ bool in_window(int x, int y, int lo, int hi) {
+    return min(x - wx, y - wy) >= lo - kWinM && max(x - wx, y - wy) <= kWinM - hi;
+  }
+  // N words of the window from byte `byte` of the row at `w`.
+  template <int N>
+  __device__ __forceinline__ void win_words(const uint32_t* w, int byte, uint32_t (&out)[N]) {
+    const uint32_t* p = w + (byte >> 2);
+    const uint32_t sh = (uint32_t)(byte & 3) * 8u;
+    uint32_t v[N + 1];
+#pragma unroll
+    for (int k = 0; k <= N; ++k) v[k] = p[k];
+#pragma unroll
+    for (int k = 0; k < N; ++k) out[k] = __funnelshift_r(v[k], v[k + 1], sh);
+  }
+  __device__ __forceinline__ uint32_t sad2(const uint32_t (&a)[WR], const uint32_t (&b)[WR]) {
+    uint32_t acc = 0;
+#pragma unroll
+    for (int k = 0; k < WR; ++k) acc = vsad(src[(sub + 8) * WR + k], b[k], vsad(src[sub * WR + k], a[k], acc, S()), S());
+    return acc;
+  }
+  // As sad, a point of the window.
+  __device__ __forceinline__ uint32_t win_sad(bool ok, int fx, int fy) {
+    uint32_t acc = 0;
+    if (ok) {
+      const uint32_t* w = win + (fy - wy + kWinM + sub) * Win<S>::PITCH;
+      const int byte = wofs + (fx - wx) * (int)sizeof(S);
+      uint32_t a[WR], b[WR];
+      win_words<WR>(w, byte, a);
+      win_words<WR>(w + 8 * Win<S>::PITCH, byte, b);
+      acc = sad2(a, b);
+    }
+    acc += __shfl_xor_sync(kFull, acc, 4);
+    acc += __shfl_xor_sync(kFull, acc, 2);
+    acc += __shfl_xor_sync(kFull, acc, 1);
+    return acc;
+  }
+  // Two 4x4 tiles of the window (tile row sub / 2, tile columns 2 * (sub & 1)
+  // and the next): SATD against one view or the average of two. The lower
+  // tiles' rows are taken in the order 2 3 0 1, for the banks' sake: a Hadamard
+  // sum of magnitudes is the same when row numbers are XORed with a constant.
+  __device__ __forceinline__ uint32_t win_satd(int mx, int my) {
+    constexpr int WPT = (int)sizeof(S), WPS = 2 * WPT;
+    const int pos = (my & 3) * 4 + (mx & 3), a = digit(kView1, pos), b = digit(kView2, pos);
+    const int ty = sub >> 1, sx = sub & 1, flip = ty & 2;
+    const int row = (my >> 2) - wy + kWinM + ty * 4, byte = wofs + ((mx >> 2) - wx + sx * 8) * (int)sizeof(S);
+    uint32_t pw[4][WPS];
+    const uint32_t* w = win + (a >> 2) * Win<S>::PLANE + (row + ((a >> 1) & 1)) * Win<S>::PITCH;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) win_words<WPS>(w + (r ^ flip) * Win<S>::PITCH, byte + (a & 1) * (int)sizeof(S), pw[r]);
+    if ((kTwoViews >> pos) & 1u) {
+      w = win + (b >> 2) * Win<S>::PLANE + (row + ((b >> 1) & 1)) * Win<S>::PITCH;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        uint32_t q[WPS];
+        win_words<WPS>(w + (r ^ flip) * Win<S>::PITCH, byte + (b & 1) * (int)sizeof(S), q);
+#pragma unroll
+        for (int k = 0; k < WPS; ++k) pw[r][k] = vavg(pw[r][k], q[k], S());
+      }
+    }
+    uint32_t v = 0;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      uint32_t sw[4][WPT], qw[4][WPT];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int k = 0; k < WPT; ++k) {
+          sw[r][k] = src[(ty * 4 + (r ^ flip)) * WR + (sx * 2 + t) * WPT + k];
+          qw[r][k] = pw[r][t * WPT + k];
+        }
+      v += satd4x4<WPT>(sw, qw);
+    }
+    return v;
   }
   // Every slot's cost to every lane: lane l of each warp gets slot l's (none
   // beyond the sixteenth).
@@ -188,17 +307,61 @@ struct RefSearch {
           y = cy + hex12_y(k) * rr / 2;
         }
       };
+      // The points' samples staged where they fit: a warp's four candidates lie
+      // on 32 lines of the plane, each a pass of its own through L1.
+      const int reach = max(2 * (range / 2), 4 * (range / 4)), wrows = 16 + 2 * reach;
+      const int byte0 = (B.x + cx - reach + kH264Pad) * (int)sizeof(S);
+      const int wch = ((wrows * (int)sizeof(S) + 15 + 4 + 15) / 16) | 1, wpitch = wch * 4;
+      const bool fit = wrows * wpitch <= Win<S>::WORDS;
+      if (fit) {
+        const int per = 32 / wch, lr = lane / wch, lc = lane - lr * wch;
+        for (int r = warp * per + lr; lr < per && r < wrows; r += 4 * per)
+          copy_chunk(win + r * wpitch + lc * 4, 0, B.y + cy - reach + r, (byte0 >> 4) + lc);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        sync();
+      }
       uint32_t mc = kInf, mi = 0xffffffffu;  // this lane's least cost, its first point
-#pragma unroll 2
-      for (int i0 = 0; i0 < total; i0 += kSlots16) {
-        const int i = i0 + slot;
-        int x = 0, y = 0;
+      // 128 points at a time, eight for each lane; then their sums are turned,
+      // so that each lane has one point's: slot's of pass `sub`.
+      for (int i0 = 0; i0 < total; i0 += 8 * kSlots16) {
+        uint32_t acc[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int i = i0 + u * kSlots16 + slot;
+          int x = cx, y = cy;
+          if (i < total) point(i, x, y);
+          acc[u] = 0;
+          if (i < total && inside(x, y)) {
+            uint32_t a[WR], b[WR];
+            if (fit) {
+              const uint32_t* w = win + (y - cy + reach + sub) * wpitch;
+              const int byte = (byte0 & 15) + (x - cx + reach) * (int)sizeof(S);
+              win_words<WR>(w, byte, a);
+              win_words<WR>(w + 8 * wpitch, byte, b);
+            } else {
+              const S* rp = org + (ptrdiff_t)(y + sub) * R.stride + x;
+              ldwords<WR>(rp, a);
+              ldwords<WR>(rp + (ptrdiff_t)8 * R.stride, b);
+            }
+            acc[u] = sad2(a, b);
+          }
+        }
+#pragma unroll
+        for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+          for (int u = 0; u < h; ++u) {
+            const bool up = sub & h;
+            const uint32_t give = up ? acc[u] : acc[u + h], keep = up ? acc[u + h] : acc[u];
+            acc[u] = keep + __shfl_xor_sync(kFull, give, h);
+          }
+        const int i = i0 + sub * kSlots16 + slot;
+        int x = cx, y = cy;
         if (i < total) point(i, x, y);
         const bool ok = i < total && inside(x, y);
-        const uint32_t rt = rate(x * 4, y * 4), s = sad(ok, x, y);
-        nsad += count(ok);
-        const uint32_t c = ok ? s + rt : kInf;
-        if (c < mc) {
+        nsad += __popc(__ballot_sync(kFull, ok));
+        const uint32_t c = acc[0] + rate(x * 4, y * 4);
+        if (ok && c < mc) {
           mc = c;
           mi = (uint32_t)i;
         }
@@ -218,6 +381,10 @@ struct RefSearch {
         point((int)at, bx, by);
       }
     }
+    // The steps' samples staged around the best point so far.
+    stage(bx, by);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    sync();
     // A step's points around the best: offset of slot k.
     if (dia) {
       for (int it = 0; it < range; ++it) {
@@ -228,7 +395,8 @@ struct RefSearch {
         int ox, oy;
         off(slot, ox, oy);
         const bool ok = slot < 4 && inside(bx + ox, by + oy);
-        const uint32_t rt = rate((bx + ox) * 4, (by + oy) * 4), s = sad(ok, bx + ox, by + oy);
+        const uint32_t rt = rate((bx + ox) * 4, (by + oy) * 4);
+        const uint32_t s = in_window(bx, by, 1, 1) ? win_sad(ok, bx + ox, by + oy) : sad(ok, bx + ox, by + oy);
         nsad += count(ok);
         const Pick p = warp_min(share(ok ? s + rt : kInf));
         if (!(p.cost < bcost)) break;
@@ -256,7 +424,8 @@ struct RefSearch {
         int ox = 0, oy = 0;
         if (slot < 14) off(slot, ox, oy);
         const bool ok = (slot < 6 ? slot < nhex : slot < 14) && inside(bx + ox, by + oy);
-        const uint32_t rt = rate((bx + ox) * 4, (by + oy) * 4), s = sad(ok, bx + ox, by + oy);
+        const uint32_t rt = rate((bx + ox) * 4, (by + oy) * 4);
+        const uint32_t s = in_window(bx, by, 2, 2) ? win_sad(ok, bx + ox, by + oy) : sad(ok, bx + ox, by + oy);
         nsad += count(ok && slot < 6);
         const uint32_t c = share(ok ? s + rt : kInf);
         Pick p = warp_min(lane < 6 ? c : kInf);
@@ -288,6 +457,18 @@ struct RefSearch {
     int bmx = smx, bmy = smy;
     uint32_t bsatd = 0, bc = kInf;
     bool first = true;
+    // No step leaves the start by more than `far` samples. A walk that went
+    // too far for the window has it staged anew.
+    const int far = (2 * hpel + qpel + 3) / 4;
+    bool staged = in_window(smx >> 2, smy >> 2, far, far + 1);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    sync();
+    if (!staged && far + 1 <= kWinM) {
+      stage(smx >> 2, smy >> 2);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      sync();
+      staged = true;
+    }
     for (int s = 0; s < 2; ++s) {
       const int step = s == 0 ? 2 : 1, iters = s == 0 ? hpel : qpel;
       const int pts = (step == 1 && qpel_diamond) ? 4 : 8;
@@ -313,7 +494,9 @@ struct RefSearch {
                !(has_prev && abs(mx - prevx) <= step && abs(my - prevy) <= step);
         const uint32_t rt = rate(mx, my);
         uint32_t sv = 0;
-        if (ok) {
+        if (ok && staged) {
+          sv = win_satd(mx, my);
+        } else if (ok) {
           const int xi = B.x + (mx >> 2), yi = B.y + (my >> 2);
           const int pos = (my & 3) * 4 + (mx & 3), a = digit(kView1, pos), b = digit(kView2, pos);
           const S* p1 = plane_at<S>(R, a >> 2, xi + (a & 1), yi + ((a >> 1) & 1));
@@ -425,6 +608,8 @@ __device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSme
       q.lane = lane;
       q.sub = lane & 7;
       q.slot = warp * 4 + (lane >> 3);
+      q.height = F.height;
+      q.win = sm.win[g];
       H264Blk& B = q.B;
       B.x = mx * 16;
       B.y = my * 16;
