@@ -12,7 +12,14 @@
 // Against one warp per macroblock (the dataflow form):
 //   - a reference has four warps, eight lanes per candidate: up to sixteen
 //     candidates of a step at once, two rows (SAD) or two 4x4 tiles (SATD) a
-//     lane, one named barrier a step;
+//     lane, one named barrier a step (a refinement step but the first has at
+//     most eight: sixteen lanes and a tile a lane);
+//   - the walk and the refinement read the four planes around the seeds' best
+//     point from shared memory, staged once a macroblock while it is needed;
+//     from the planes a step's candidates, on lines of their own, are up to 32
+//     passes through L1 a load: staging took the search of four 10-bit 720p
+//     references from 3.10 to 2.41 ms, the UMH points' samples that of 1080p
+//     from 3.92 to 2.61 ms;
 //   - references are searched side by side, each by its own four warps; the
 //     refine_ratio gate, the only tie between them, needs the whole-sample
 //     costs alone, one CTA barrier;
@@ -22,13 +29,16 @@
 //     them coincide and none is the start, so the one point the reference
 //     leaves out, the best so far, is never among them, and the outcome is
 //     the least cost, first reached;
+//   - a step is its instructions' latency more than its work: counts stay in
+//     the lanes, a lane's part of a sum goes to shared memory instead of three
+//     shuffles, offsets that do not change are kept (CIF 0.43 -> 0.36 ms);
 //   - a neighbour's result is one published word (tag, reference, vector),
 //     loaded a macroblock ahead, and the next source block is staged behind
 //     the search.
 // Measured on one B200, the search kernel alone, the dataflow form first:
-// CIF, one reference, medium tier 1.60 -> 0.53 ms; 1080p, three references,
-// UMH +-24 28.3 -> 4.5 ms; 64 720p pictures of two references in one launch
-// 14.7 -> 9.6 ms.
+// CIF, one reference, medium tier 1.60 -> 0.36 ms; 1080p, three references,
+// UMH +-24 28.3 -> 2.2 ms; 64 720p pictures of two references in one launch
+// 14.5 -> 5.9 ms.
 #include <algorithm>
 
 #include "rme_search_impl.cuh"
@@ -43,14 +53,15 @@ constexpr int kSlots16 = 16;      // candidates a step scores at once
 // their own do not queue at the constant cache: the hexagon's and the square's
 // offsets + 2, the UMH hexagon's + 2, the refinement ring's + 1.
 __device__ __forceinline__ int digit(unsigned long long t, int k) { return (int)((t >> (4 * k)) & 15u); }
-__device__ __forceinline__ int hex_x(int k) { return digit(0x134310ull, k) - 2; }
-__device__ __forceinline__ int hex_y(int k) { return digit(0x442002ull, k) - 2; }
-__device__ __forceinline__ int square_x(int k) { return digit(0x32131321ull, k) - 2; }
-__device__ __forceinline__ int square_y(int k) { return digit(0x33322111ull, k) - 2; }
+__device__ __forceinline__ int digit(uint32_t t, int k) { return (int)((t >> (4 * k)) & 15u); }
+__device__ __forceinline__ int hex_x(int k) { return digit(0x134310u, k) - 2; }
+__device__ __forceinline__ int hex_y(int k) { return digit(0x442002u, k) - 2; }
+__device__ __forceinline__ int square_x(int k) { return digit(0x32131321u, k) - 2; }
+__device__ __forceinline__ int square_y(int k) { return digit(0x33322111u, k) - 2; }
 __device__ __forceinline__ int hex12_x(int k) { return digit(0x404031314400ull, k) - 2; }
 __device__ __forceinline__ int hex12_y(int k) { return digit(0x4400441313ull, k) - 2; }
-__device__ __forceinline__ int ring_x(int k) { return digit(0x20201201ull, k) - 1; }
-__device__ __forceinline__ int ring_y(int k) { return digit(0x22002110ull, k) - 1; }
+__device__ __forceinline__ int ring_x(int k) { return digit(0x20201201u, k) - 1; }
+__device__ __forceinline__ int ring_y(int k) { return digit(0x22002110u, k) - 1; }
 // The quarter-sample table (8.4.2.2.1): per position (fy * 4 + fx) a digit
 // plane * 4 + dy * 2 + dx of the first view and of the second; positions
 // 0, 2, 8 and 10 have one view.
@@ -69,6 +80,34 @@ struct Win {
   static_assert((kWinRows * (int)sizeof(S) + 15 + 4) / 16 <= CH && CH % 2 == 1, "row width");
 };
 
+// The UMH points' offsets: the cross, then the twelve-point hexagons.
+__device__ __forceinline__ int umh_points(int range) { return 4 * (range / 2) + 12 * (range / 4); }
+__device__ __forceinline__ void umh_point(int i, int range, int& x, int& y) {
+  const int ncross = 4 * (range / 2);
+  if (i < ncross) {
+    const int r = 2 * (i / 4 + 1), k = i & 3;
+    x = k == 0 ? -r : k == 1 ? r : 0;
+    y = k == 2 ? -r : k == 3 ? r : 0;
+  } else {
+    const int j = i - ncross, r = 2 * (j / 12 + 1), k = j % 12;
+    x = hex12_x(k) * r;
+    y = hex12_y(k) * r;
+  }
+}
+// The UMH points' samples staged in the same memory, where they fit (ranges to
+// 25): rows of an odd number of chunks that hold the points from any byte on
+// and one word more.
+template <class S>
+struct UmhWindow {
+  int reach, rows, chunks;
+  bool fit;
+  __device__ __forceinline__ explicit UmhWindow(int range)
+      : reach(max(2 * (range / 2), 4 * (range / 4))),
+        rows(16 + 2 * reach),
+        chunks(((rows * (int)sizeof(S) + 31) / 16) | 1),
+        fit(range < 26 && rows * chunks * 4 <= Win<S>::WORDS) {}
+};
+
 struct RefResult {
   uint32_t cost, satd, icost;
   int mx, my, imx, imy;
@@ -78,7 +117,8 @@ template <class S>
 struct RowSmem {
   alignas(16) uint32_t win[RME_MAX_REFS][Win<S>::WORDS];
   uint32_t src[2][16 * 16 * sizeof(S) / 4];
-  uint32_t cost[RME_MAX_REFS][2][kSlots16];
+  alignas(16) uint32_t part[RME_MAX_REFS][2][kRefThreads];  // a step's partial sums, two steps in turn
+  uint32_t umh[128];                  // UMH: where each point's samples start in the window
   uint32_t best[RME_MAX_REFS][4][2];  // UMH: each warp's least cost and its point
   uint32_t icost[2][RME_MAX_REFS];    // whole-sample costs, reference cost included
   RefResult fin[2][RME_MAX_REFS];
@@ -127,24 +167,18 @@ struct RefSearch {
   uint32_t* win;      // this reference's window
   int wx = 0, wy = 0, wofs = 0;  // its centre; the centre's first byte in a row
   int buf = 0;
-  uint32_t nsad = 0, nsatd = 0;  // this warp's candidates
+  uint32_t nsad = 0, nsatd = 0;  // candidates scored: this lane's eighths, sixteenths
+  uint32_t s0[WR], s1[WR];       // source rows sub and sub + 8
 
   __device__ __forceinline__ void sync() { asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(kRefThreads) : "memory"); }
 
-  // The candidate's SAD over its eight lanes (rows sub and sub + 8).
-  __device__ __forceinline__ uint32_t sad(bool ok, int fx, int fy) {
-    uint32_t acc = 0;
-    if (ok) {
-      const S* rp = org + (ptrdiff_t)(fy + sub) * R.stride + fx;
-      uint32_t a[WR], b[WR];
-      ldwords<WR>(rp, a);
-      ldwords<WR>(rp + (ptrdiff_t)8 * R.stride, b);
-      acc = sad2(a, b);
-    }
-    acc += __shfl_xor_sync(kFull, acc, 4);
-    acc += __shfl_xor_sync(kFull, acc, 2);
-    acc += __shfl_xor_sync(kFull, acc, 1);
-    return acc;
+  // This lane's part of a candidate's SAD: rows sub and sub + 8.
+  __device__ __forceinline__ uint32_t sad(int fx, int fy) {
+    const S* rp = org + (ptrdiff_t)(fy + sub) * R.stride + fx;
+    uint32_t a[WR], b[WR];
+    ldwords<WR>(rp, a);
+    ldwords<WR>(rp + (ptrdiff_t)8 * R.stride, b);
+    return sad2(a, b);
   }
   // Copies rows of 16-byte chunks around whole-sample offset (x, y) into the
   // window, unwaited. What lies outside the padded plane is clamped to it: no
@@ -190,37 +224,34 @@ struct RefSearch {
 #pragma unroll
     for (int k = 0; k < N; ++k) out[k] = __funnelshift_r(v[k], v[k + 1], sh);
   }
+  // Two chains: one sum after the other is the longest of a step.
   __device__ __forceinline__ uint32_t sad2(const uint32_t (&a)[WR], const uint32_t (&b)[WR]) {
-    uint32_t acc = 0;
+    uint32_t lo = 0, hi = 0;
 #pragma unroll
-    for (int k = 0; k < WR; ++k) acc = vsad(src[(sub + 8) * WR + k], b[k], vsad(src[sub * WR + k], a[k], acc, S()), S());
-    return acc;
+    for (int k = 0; k < WR; ++k) {
+      lo = vsad(s0[k], a[k], lo, S());
+      hi = vsad(s1[k], b[k], hi, S());
+    }
+    return lo + hi;
   }
   // As sad, a point of the window.
-  __device__ __forceinline__ uint32_t win_sad(bool ok, int fx, int fy) {
-    uint32_t acc = 0;
-    if (ok) {
-      const uint32_t* w = win + (fy - wy + kWinM + sub) * Win<S>::PITCH;
-      const int byte = wofs + (fx - wx) * (int)sizeof(S);
-      uint32_t a[WR], b[WR];
-      win_words<WR>(w, byte, a);
-      win_words<WR>(w + 8 * Win<S>::PITCH, byte, b);
-      acc = sad2(a, b);
-    }
-    acc += __shfl_xor_sync(kFull, acc, 4);
-    acc += __shfl_xor_sync(kFull, acc, 2);
-    acc += __shfl_xor_sync(kFull, acc, 1);
-    return acc;
+  __device__ __forceinline__ uint32_t win_sad(int fx, int fy) {
+    const uint32_t* w = win + (fy - wy + kWinM + sub) * Win<S>::PITCH;
+    const int byte = wofs + (fx - wx) * (int)sizeof(S);
+    uint32_t a[WR], b[WR];
+    win_words<WR>(w, byte, a);
+    win_words<WR>(w + 8 * Win<S>::PITCH, byte, b);
+    return sad2(a, b);
   }
-  // Two 4x4 tiles of the window (tile row sub / 2, tile columns 2 * (sub & 1)
-  // and the next): SATD against one view or the average of two. The lower
-  // tiles' rows are taken in the order 2 3 0 1, for the banks' sake: a Hadamard
-  // sum of magnitudes is the same when row numbers are XORed with a constant.
-  __device__ __forceinline__ uint32_t win_satd(int mx, int my) {
-    constexpr int WPT = (int)sizeof(S), WPS = 2 * WPT;
-    const int pos = (my & 3) * 4 + (mx & 3), a = digit(kView1, pos), b = digit(kView2, pos);
-    const int ty = sub >> 1, sx = sub & 1, flip = ty & 2;
-    const int row = (my >> 2) - wy + kWinM + ty * 4, byte = wofs + ((mx >> 2) - wx + sx * 8) * (int)sizeof(S);
+  // NT 4x4 tiles of the window side by side (tile row ty, from tile column tx
+  // on): SATD against one view or the average of two. The lower tiles' rows
+  // are taken in the order 2 3 0 1, for the banks' sake: a Hadamard sum of
+  // magnitudes is the same when row numbers are XORed with a constant.
+  template <int NT>
+  __device__ __forceinline__ uint32_t win_satd(int mx, int my, int ty, int tx) {
+    constexpr int WPT = (int)sizeof(S), WPS = NT * WPT;
+    const int pos = (my & 3) * 4 + (mx & 3), a = digit(kView1, pos), b = digit(kView2, pos), flip = ty & 2;
+    const int row = (my >> 2) - wy + kWinM + ty * 4, byte = wofs + ((mx >> 2) - wx + tx * 4) * (int)sizeof(S);
     uint32_t pw[4][WPS];
     const uint32_t* w = win + (a >> 2) * Win<S>::PLANE + (row + ((a >> 1) & 1)) * Win<S>::PITCH;
 #pragma unroll
@@ -237,33 +268,57 @@ struct RefSearch {
     }
     uint32_t v = 0;
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
+    for (int t = 0; t < NT; ++t) {
       uint32_t sw[4][WPT], qw[4][WPT];
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
         for (int k = 0; k < WPT; ++k) {
-          sw[r][k] = src[(ty * 4 + (r ^ flip)) * WR + (sx * 2 + t) * WPT + k];
+          sw[r][k] = src[(ty * 4 + (r ^ flip)) * WR + (tx + t) * WPT + k];
           qw[r][k] = pw[r][t * WPT + k];
         }
       v += satd4x4<WPT>(sw, qw);
     }
     return v;
   }
-  // Every slot's cost to every lane: lane l of each warp gets slot l's (none
-  // beyond the sixteenth).
-  __device__ __forceinline__ uint32_t share(uint32_t cost) {
-    uint32_t* c = sm.cost[g][buf];
+  // A step's candidates, LANES threads each: every thread gives its part of
+  // its candidate's cost (kNone where there is no candidate, whose cost is
+  // then above any other's), and lane l gets cost << 4 | slot of slot l (mod
+  // the number of slots). A cost is below 2^23 at every depth (twelve bits:
+  // sixteen tiles' SATD of at most 262080 and two 16-bit rates).
+  static constexpr uint32_t kNone = 1u << 23;
+  template <int LANES>
+  __device__ __forceinline__ uint32_t share(uint32_t part) {
+    uint32_t* c = sm.part[g][buf];
     buf ^= 1;
-    if (sub == 0) c[slot] = cost;
+    c[warp * 32 + lane] = part;
     sync();
-    return lane < kSlots16 ? c[lane] : kInf;
+    const int k = lane & (kRefThreads / LANES - 1);
+    uint32_t v = 0;
+#pragma unroll
+    for (int i = 0; i < LANES / 4; ++i) {
+      // Each slot from another chunk on: eight lanes' loads on all banks.
+      const uint4 q = reinterpret_cast<const uint4*>(c + k * LANES)[(i + k * LANES / 32) & (LANES / 4 - 1)];
+      v += (q.x + q.y) + (q.z + q.w);
+    }
+    return v << 4 | (uint32_t)k;
   }
   __device__ __forceinline__ uint32_t rate(int qx, int qy) {
     const int dx = min(max(qx - B.px, -kMvSpan), kMvSpan), dy = min(max(qy - B.py, -kMvSpan), kMvSpan);
     return (uint32_t)__ldg(&tab[dx + kMvSpan]) + (uint32_t)__ldg(&tab[dy + kMvSpan]);
   }
-  __device__ __forceinline__ uint32_t count(bool yes) { return __popc(__ballot_sync(kFull, yes && sub == 0)); }
+
+  // This lane's part of the cost of the point (ox, oy), at most two samples
+  // each way, from (x, y).
+  __device__ __forceinline__ uint32_t score(int x, int y, int ox, int oy, bool ok) {
+    const uint32_t rt = rate((x + ox) * 4, (y + oy) * 4);
+    uint32_t v = 0;
+    if ((uint32_t)(x - wx + kWinM - 2) <= 2u * kWinM - 4 && (uint32_t)(y - wy + kWinM - 2) <= 2u * kWinM - 4)
+      v = win_sad(x + ox, y + oy);  // without a branch on ok: a point outside the box is in the window all the same
+    else if (ok)
+      v = sad(x + ox, y + oy);
+    return ok ? v + (sub == 0 ? rt : 0u) : kNone;
+  }
 
   // Search::int_search: lane k + 1 of every warp holds candidate k of ncand.
   __device__ __forceinline__ void whole(int ncand, int cand_x, int cand_y, int& imx, int& imy, uint32_t& icost) {
@@ -284,68 +339,43 @@ struct RefSearch {
     {
       const bool ok = (keep >> slot) & 1u;
       const int fx = __shfl_sync(kFull, qx, slot), fy = __shfl_sync(kFull, qy, slot);
-      const uint32_t rt = rate(fx * 4, fy * 4), s = sad(ok, fx, fy);
-      nsad += count(ok);
-      const Pick p = warp_min(share(ok ? s + rt : kInf));
-      bcost = p.cost;
-      bx = __shfl_sync(kFull, qx, p.lane);
-      by = __shfl_sync(kFull, qy, p.lane);
+      const uint32_t rt = rate(fx * 4, fy * 4);
+      const uint32_t m = __reduce_min_sync(kFull, share<8>(ok ? sad(fx, fy) + (sub == 0 ? rt : 0u) : kNone));
+      nsad += ok;
+      bcost = m >> 4;
+      bx = __shfl_sync(kFull, qx, m & 15);
+      by = __shfl_sync(kFull, qy, m & 15);
     }
     const int x0 = max(bx - range, B.lx), x1 = min(bx + range, B.hx), y0 = max(by - range, B.ly),
               y1 = min(by + range, B.hy);
-    auto inside = [&](int x, int y) { return x >= x0 && x <= x1 && y >= y0 && y <= y1; };
+    const uint32_t xr = (uint32_t)(x1 - x0), yr = (uint32_t)(y1 - y0);  // the start lies between them
+    auto inside = [&](int x, int y) { return (uint32_t)(x - x0) <= xr && (uint32_t)(y - y0) <= yr; };
     if (umh) {
-      const int cx = bx, cy = by, ncross = 4 * (range / 2), total = ncross + 12 * (range / 4);
-      auto point = [&](int i, int& x, int& y) {
-        if (i < ncross) {
-          const int rr = 2 * (i / 4 + 1), k = i & 3;
-          x = cx + (k == 0 ? -rr : k == 1 ? rr : 0);
-          y = cy + (k == 2 ? -rr : k == 3 ? rr : 0);
-        } else {
-          const int j = i - ncross, rr = 4 * (j / 12 + 1), k = j % 12;
-          x = cx + hex12_x(k) * rr / 2;
-          y = cy + hex12_y(k) * rr / 2;
-        }
-      };
-      // The points' samples staged where they fit: a warp's four candidates lie
-      // on 32 lines of the plane, each a pass of its own through L1.
-      const int reach = max(2 * (range / 2), 4 * (range / 4)), wrows = 16 + 2 * reach;
-      const int byte0 = (B.x + cx - reach + kH264Pad) * (int)sizeof(S);
-      const int wch = ((wrows * (int)sizeof(S) + 15 + 4 + 15) / 16) | 1, wpitch = wch * 4;
-      const bool fit = wrows * wpitch <= Win<S>::WORDS;
-      if (fit) {
-        const int per = 32 / wch, lr = lane / wch, lc = lane - lr * wch;
-        for (int r = warp * per + lr; lr < per && r < wrows; r += 4 * per)
-          copy_chunk(win + r * wpitch + lc * 4, 0, B.y + cy - reach + r, (byte0 >> 4) + lc);
+      const int cx = bx, cy = by, total = umh_points(range);
+      uint32_t mc = kInf, mi = 0xffffffffu;  // this lane's least cost, its first point
+      const UmhWindow<S> U(range);
+      if (U.fit) {
+        // The points' samples staged: a warp's four candidates lie on 32 lines
+        // of the plane, each a pass of its own through L1.
+        const int byte0 = (B.x + cx - U.reach + kH264Pad) * (int)sizeof(S), lr = lane / U.chunks,
+                  lc = lane - lr * U.chunks, per = 32 / U.chunks;
+        for (int r = warp * per + lr; lr < per && r < U.rows; r += 4 * per)
+          copy_chunk(win + (r * U.chunks + lc) * 4, 0, B.y + cy - U.reach + r, (byte0 >> 4) + lc);
         asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         sync();
-      }
-      uint32_t mc = kInf, mi = 0xffffffffu;  // this lane's least cost, its first point
-      // 128 points at a time, eight for each lane; then their sums are turned,
-      // so that each lane has one point's: slot's of pass `sub`.
-      for (int i0 = 0; i0 < total; i0 += 8 * kSlots16) {
+        // Eight points for each lane (those past the last and those outside the
+        // box count for nothing below); then the sums are turned, so that each
+        // lane has one point's: slot's of pass `sub`.
+        const uint32_t* w0 = win + sub * U.chunks * 4;
         uint32_t acc[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-          const int i = i0 + u * kSlots16 + slot;
-          int x = cx, y = cy;
-          if (i < total) point(i, x, y);
-          acc[u] = 0;
-          if (i < total && inside(x, y)) {
-            uint32_t a[WR], b[WR];
-            if (fit) {
-              const uint32_t* w = win + (y - cy + reach + sub) * wpitch;
-              const int byte = (byte0 & 15) + (x - cx + reach) * (int)sizeof(S);
-              win_words<WR>(w, byte, a);
-              win_words<WR>(w + 8 * wpitch, byte, b);
-            } else {
-              const S* rp = org + (ptrdiff_t)(y + sub) * R.stride + x;
-              ldwords<WR>(rp, a);
-              ldwords<WR>(rp + (ptrdiff_t)8 * R.stride, b);
-            }
-            acc[u] = sad2(a, b);
-          }
+          const int at = (int)sm.umh[u * kSlots16 + slot] + (byte0 & 15);
+          uint32_t a[WR], b[WR];
+          win_words<WR>(w0, at, a);
+          win_words<WR>(w0 + 8 * U.chunks * 4, at, b);
+          acc[u] = sad2(a, b);
         }
 #pragma unroll
         for (int h = 4; h > 0; h >>= 1)
@@ -355,15 +385,37 @@ struct RefSearch {
             const uint32_t give = up ? acc[u] : acc[u + h], keep = up ? acc[u + h] : acc[u];
             acc[u] = keep + __shfl_xor_sync(kFull, give, h);
           }
-        const int i = i0 + sub * kSlots16 + slot;
-        int x = cx, y = cy;
-        if (i < total) point(i, x, y);
+        const int i = sub * kSlots16 + slot;
+        int x, y;
+        umh_point(i, range, x, y);
+        x += cx;
+        y += cy;
         const bool ok = i < total && inside(x, y);
-        nsad += __popc(__ballot_sync(kFull, ok));
-        const uint32_t c = acc[0] + rate(x * 4, y * 4);
-        if (ok && c < mc) {
-          mc = c;
+        nsad += ok ? 8 : 0;
+        const uint32_t rt = rate(x * 4, y * 4);
+        if (ok) {
+          mc = acc[0] + rt;
           mi = (uint32_t)i;
+        }
+      } else {
+#pragma unroll 2
+        for (int i0 = 0; i0 < total; i0 += kSlots16) {
+          const int i = i0 + slot;
+          int x, y;
+          umh_point(i, range, x, y);
+          x += cx;
+          y += cy;
+          const bool ok = i < total && inside(x, y);
+          uint32_t v = ok ? sad(x, y) : 0u;
+          v += __shfl_xor_sync(kFull, v, 4);
+          v += __shfl_xor_sync(kFull, v, 2);
+          v += __shfl_xor_sync(kFull, v, 1);
+          nsad += ok;
+          const uint32_t c = v + rate(x * 4, y * 4);
+          if (ok && c < mc) {
+            mc = c;
+            mi = (uint32_t)i;
+          }
         }
       }
       uint32_t m = __reduce_min_sync(kFull, mc);
@@ -378,7 +430,9 @@ struct RefSearch {
       at = __reduce_min_sync(kFull, wm == m ? wi : 0xffffffffu);
       if (m < bcost) {
         bcost = m;
-        point((int)at, bx, by);
+        umh_point((int)at, range, bx, by);
+        bx += cx;
+        by += cy;
       }
     }
     // The steps' samples staged around the best point so far.
@@ -395,53 +449,49 @@ struct RefSearch {
         int ox, oy;
         off(slot, ox, oy);
         const bool ok = slot < 4 && inside(bx + ox, by + oy);
-        const uint32_t rt = rate((bx + ox) * 4, (by + oy) * 4);
-        const uint32_t s = in_window(bx, by, 1, 1) ? win_sad(ok, bx + ox, by + oy) : sad(ok, bx + ox, by + oy);
-        nsad += count(ok);
-        const Pick p = warp_min(share(ok ? s + rt : kInf));
-        if (!(p.cost < bcost)) break;
-        bcost = p.cost;
-        off(p.lane, ox, oy);
+        const uint32_t m = __reduce_min_sync(kFull, share<8>(score(bx, by, ox, oy, ok)));
+        nsad += ok;
+        if (!(m >> 4 < bcost)) break;
+        bcost = m >> 4;
+        off(m & 15, ox, oy);
         bx += ox;
         by += oy;
       }
     } else {
       // Slots 0..5 the hexagon (after a step in direction d only d - 1, d,
       // d + 1 are new, in that order), 6..13 the square.
-      int dir = -1;
+      auto turn = [](int d, int k) {  // direction d + k - 1 of the six
+        const int e = d + k - 1;
+        return e < 0 ? 5 : e > 5 ? 0 : e;
+      };
+      int ox = slot < 6 ? hex_x(slot) : slot < 14 ? square_x(slot - 6) : 0;
+      int oy = slot < 6 ? hex_y(slot) : slot < 14 ? square_y(slot - 6) : 0;
+      int dir = -1, nhex = 6;
       for (int it = 0;; ++it) {
-        auto off = [&](int k, int& ox, int& oy) {
-          if (k < 6) {
-            const int e = dir < 0 ? k : k == 0 ? (dir + 5) % 6 : k == 1 ? dir : (dir + 1) % 6;
-            ox = hex_x(e);
-            oy = hex_y(e);
-          } else {
-            ox = square_x(k - 6);
-            oy = square_y(k - 6);
-          }
-        };
-        const int nhex = it == 0 ? 6 : it < range ? 3 : 0;
-        int ox = 0, oy = 0;
-        if (slot < 14) off(slot, ox, oy);
         const bool ok = (slot < 6 ? slot < nhex : slot < 14) && inside(bx + ox, by + oy);
-        const uint32_t rt = rate((bx + ox) * 4, (by + oy) * 4);
-        const uint32_t s = in_window(bx, by, 2, 2) ? win_sad(ok, bx + ox, by + oy) : sad(ok, bx + ox, by + oy);
-        nsad += count(ok && slot < 6);
-        const uint32_t c = share(ok ? s + rt : kInf);
-        Pick p = warp_min(lane < 6 ? c : kInf);
-        const bool step = p.cost < bcost;
-        if (!step) {
-          nsad += count(ok && slot >= 6);
-          p = warp_min(lane >= 6 ? c : kInf);
+        const uint32_t c = share<8>(score(bx, by, ox, oy, ok));
+        uint32_t m = __reduce_min_sync(kFull, (lane & 15) < 6 ? c : kInf);
+        nsad += ok && slot < 6;
+        if (!(m >> 4 < bcost)) {  // the hexagon has settled: the square is the last step
+          nsad += ok && slot >= 6;
+          m = __reduce_min_sync(kFull, (lane & 15) < 6 ? kInf : c);
+          if (m >> 4 < bcost) {
+            bcost = m >> 4;
+            bx += square_x((int)(m & 15) - 6);
+            by += square_y((int)(m & 15) - 6);
+          }
+          break;
         }
-        if (p.cost < bcost) {
-          bcost = p.cost;
-          off(p.lane, ox, oy);
-          bx += ox;
-          by += oy;
+        bcost = m >> 4;
+        dir = dir < 0 ? (int)(m & 15) : turn(dir, m & 15);
+        bx += hex_x(dir);
+        by += hex_y(dir);
+        if (slot < 6) {
+          const int e = turn(dir, min(slot, 2));
+          ox = hex_x(e);
+          oy = hex_y(e);
         }
-        if (!step) break;
-        dir = dir < 0 ? p.lane : p.lane == 0 ? (dir + 5) % 6 : p.lane == 1 ? dir : (dir + 1) % 6;
+        nhex = it + 1 < range ? 3 : 0;
       }
     }
     imx = bx * 4;
@@ -455,15 +505,18 @@ struct RefSearch {
                                          uint32_t& ocost) {
     const int qlx = B.lx * 4, qhx = B.hx * 4, qly = B.ly * 4, qhy = B.hy * 4;
     int bmx = smx, bmy = smy;
-    uint32_t bsatd = 0, bc = kInf;
+    uint32_t bc = kInf;
     bool first = true;
     // No step leaves the start by more than `far` samples. A walk that went
     // too far for the window has it staged anew.
     const int far = (2 * hpel + qpel + 3) / 4;
     bool staged = in_window(smx >> 2, smy >> 2, far, far + 1);
+    // (A vector that wraps at 16 bits lies elsewhere: its samples are read from the plane.)
+    const bool near = max(abs(smx), abs(smy)) + 4 * far < 32768;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     sync();
-    if (!staged && far + 1 <= kWinM) {
+    staged = staged && near;
+    if (!staged && near && far + 1 <= kWinM) {
       stage(smx >> 2, smy >> 2);
       asm volatile("cp.async.wait_group 0;" ::: "memory");
       sync();
@@ -472,8 +525,7 @@ struct RefSearch {
     for (int s = 0; s < 2; ++s) {
       const int step = s == 0 ? 2 : 1, iters = s == 0 ? hpel : qpel;
       const int pts = (step == 1 && qpel_diamond) ? 4 : 8;
-      bool has_prev = false;
-      int prevx = 0, prevy = 0;
+      int prevx = 1 << 20, prevy = 1 << 20;  // none yet
       for (int it = 0; it < iters || first; ++it) {
         const int cmx = bmx, cmy = bmy;
         const bool ring = it < iters;
@@ -486,44 +538,49 @@ struct RefSearch {
             my = (int)(int16_t)(cmy + ring_y((c - base) & 7) * step);
           }
         };
+        // At most eight candidates, all but the first step's nine: sixteen
+        // threads each, a tile a thread.
+        const bool wide = staged && !first;
+        const int sl = wide ? warp * 2 + (lane >> 4) : slot, part = wide ? lane & 15 : sub;
         int mx, my;
-        vec(slot, mx, my);
-        bool ok = slot < n;
-        if (slot >= base)
+        vec(sl, mx, my);
+        bool ok = sl < n;
+        if (sl >= base)
           ok = ok && mx >= qlx && mx <= qhx && my >= qly && my <= qhy &&
-               !(has_prev && abs(mx - prevx) <= step && abs(my - prevy) <= step);
+               !((uint32_t)(mx - prevx + step) <= 2u * step && (uint32_t)(my - prevy + step) <= 2u * step);
         const uint32_t rt = rate(mx, my);
-        uint32_t sv = 0;
-        if (ok && staged) {
-          sv = win_satd(mx, my);
-        } else if (ok) {
-          const int xi = B.x + (mx >> 2), yi = B.y + (my >> 2);
-          const int pos = (my & 3) * 4 + (mx & 3), a = digit(kView1, pos), b = digit(kView2, pos);
-          const S* p1 = plane_at<S>(R, a >> 2, xi + (a & 1), yi + ((a >> 1) & 1));
-          const S* p2 = (kTwoViews >> pos) & 1u ? plane_at<S>(R, b >> 2, xi + (b & 1), yi + ((b >> 1) & 1)) : nullptr;
-          sv = satd_strips<S, 2>(src, WR, 4, 4, p1, p2, R.stride, 8, sub);
+        uint32_t v = kNone;
+        if (ok) {
+          if (wide) {
+            v = win_satd<1>(mx, my, part >> 2, part & 3);
+          } else if (staged) {
+            v = win_satd<2>(mx, my, part >> 1, (part & 1) * 2);
+          } else {
+            const int xi = B.x + (mx >> 2), yi = B.y + (my >> 2);
+            const int pos = (my & 3) * 4 + (mx & 3), a = digit(kView1, pos), b = digit(kView2, pos);
+            const S* p1 = plane_at<S>(R, a >> 2, xi + (a & 1), yi + ((a >> 1) & 1));
+            const S* p2 =
+                (kTwoViews >> pos) & 1u ? plane_at<S>(R, b >> 2, xi + (b & 1), yi + ((b >> 1) & 1)) : nullptr;
+            v = satd_strips<S, 2>(src, WR, 4, 4, p1, p2, R.stride, 8, sub);
+          }
+          v += part == 0 ? rt : 0u;
         }
-        sv += __shfl_xor_sync(kFull, sv, 4);
-        sv += __shfl_xor_sync(kFull, sv, 2);
-        sv += __shfl_xor_sync(kFull, sv, 1);
-        nsatd += count(ok);
-        const Pick p = warp_min(share(ok ? sv + rt : kInf));
-        if (p.cost < bc) {
-          bc = p.cost;
-          vec(p.lane, bmx, bmy);
-          bsatd = bc - rate(bmx, bmy);
+        const uint32_t m = __reduce_min_sync(kFull, wide ? share<16>(v) : share<8>(v));
+        nsatd += ok ? (wide ? 1 : 2) : 0;
+        if (m >> 4 < bc) {
+          bc = m >> 4;
+          vec(m & 15, bmx, bmy);
         }
         first = false;
         if (!ring) break;
         if (bmx == cmx && bmy == cmy) break;
         prevx = cmx;
         prevy = cmy;
-        has_prev = true;
       }
     }
     omx = bmx;
     omy = bmy;
-    osatd = bsatd;
+    osatd = bc - rate(bmx, bmy);
     ocost = bc;
   }
 };
@@ -541,6 +598,12 @@ __device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSme
     return RME_LD32(reinterpret_cast<const uint32_t*>(o) + tid % WR);
   };
   if (tid < NSRC) sm.src[0][tid] = load_src(0);
+  if (F.umh && tid < 128) {
+    const UmhWindow<S> U(F.range);
+    int x = 0, y = 0;
+    if (tid < umh_points(F.range)) umh_point(tid, F.range, x, y);
+    sm.umh[tid] = (uint32_t)((y + U.reach) * U.chunks * 16 + (x + U.reach) * (int)sizeof(S));
+  }
   if (tid < 2) sm.nsad[tid] = sm.nsatd[tid] = 0u;
   unsigned long long wd = 0, wb = 0, wc = 0;  // the D, B and C macroblocks' words
   if (my > 0) {
@@ -610,6 +673,11 @@ __device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSme
       q.slot = warp * 4 + (lane >> 3);
       q.height = F.height;
       q.win = sm.win[g];
+#pragma unroll
+      for (int i = 0; i < WR; ++i) {
+        q.s0[i] = q.src[q.sub * WR + i];
+        q.s1[i] = q.src[(q.sub + 8) * WR + i];
+      }
       H264Blk& B = q.B;
       B.x = mx * 16;
       B.y = my * 16;
@@ -639,9 +707,10 @@ __device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSme
       q.refine(r.imx, r.imy, gate ? 0 : F.hpel_iters, gate ? 0 : F.qpel_iters, r.mx, r.my, r.satd, r.cost);
       r.cost += F.ref_cost[g];
       if ((tid & (kRefThreads - 1)) == 0) sm.fin[par][g] = r;
+      const uint32_t nsad = __reduce_add_sync(kFull, q.nsad) / 8, nsatd = __reduce_add_sync(kFull, q.nsatd) / 16;
       if (lane == 0) {
-        atomicAdd(&sm.nsad[par], q.nsad);
-        atomicAdd(&sm.nsatd[par], q.nsatd);
+        atomicAdd(&sm.nsad[par], nsad);
+        atomicAdd(&sm.nsatd[par], nsatd);
       }
     }
     if (tid < NSRC) sm.src[par ^ 1][tid] = nsrc;

@@ -89,6 +89,33 @@ def test_h264_rows_of_every_shape(ms, w, h, bd, nref, kw):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("bd,kw", [
+    (8, dict(h264_range=40)), (10, dict(h264_range=40, h264_dia=1)), (8, dict(h264_range=24, h264_hpel_iters=13)),
+    (10, dict(h264_range=24, h264_hpel_iters=14, h264_qpel_iters=1)), (8, dict(h264_umh=1, h264_range=25)),
+    (10, dict(h264_umh=1, h264_range=25)), (8, dict(h264_umh=1, h264_range=26)), (10, dict(h264_umh=1, h264_range=3))])
+def test_h264_walks_beyond_the_staged_window(ms, bd, kw):
+    """Long walks over smooth pictures, which leave the samples staged around
+    their start; refinements too long to be staged; the UMH ranges on both
+    sides of the largest staged one."""
+    w, h = 144, 112
+    rng = np.random.default_rng(bd + kw["h264_range"])
+    yy, xx = np.mgrid[0:h + 64, 0:w + 64]
+    full = (1 << bd) - 1
+    wave = np.sin(xx / 23.0) + np.sin(yy / 19.0) + np.sin((xx + 2 * yy) / 41.0)
+    big = np.clip((wave / 6 + 0.5) * full + rng.normal(0, 1.0, wave.shape), 0, full)
+    big = big.astype(np.uint8 if bd == 8 else np.uint16)
+    ref = np.ascontiguousarray(big[32:32 + h, 32:32 + w])
+    src = np.ascontiguousarray(big[32 - 13:32 - 13 + h, 32 + 19:32 + 19 + w])
+    ms.upload(2560, ref, H264, bd)
+    ms.upload(2561, src, H264, bd, as_ref=False)
+    p = oracle.params(H264, 30, **kw)
+    got = ms.search(2561, [2560], p)
+    assert_results_equal(got, oracle.frame_search(H264, bd, src, [ref], p), "long walks")
+    ms.release(2560)
+    ms.release(2561)
+
+
+@pytest.mark.gpu
 def test_h264_rows_of_uneven_frames_together(ms):
     """Frames of different sizes, settings and reference counts in one
     launch, beside a GIVEN-free HEVC frame: as each by itself."""
