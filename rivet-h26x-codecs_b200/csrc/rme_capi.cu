@@ -1164,14 +1164,24 @@ int ctx_picture_upload(void* ctx, int32_t pic_id, const rme_picture_desc* d, con
   const bool h264 = d->codec == RME_CODEC_H264;
   const int bps = d->bit_depth == 8 ? 1 : 2, stride = pic->planes.stride;
   CK(take_buffer(c, pic_id, pic.get(), s));
-  // The visible picture straight into plane 0, then its border in place:
-  // nothing is staged, so nothing waits (a pageable source is consumed
-  // before the copy call returns; a pinned one is read on the stream).
+  // No host staging, so nothing waits (a pageable source is consumed before
+  // the copy call returns; a pinned one is read on the stream). A reference's
+  // packed picture goes in one piece into its second plane, which is built
+  // afterwards, and the padded plane is made from there: row by row the copy
+  // takes 0.1 us a row where rows are not whole lines (352x288 28 us, 850x478
+  // 58 us, in one piece 6 and 11). Any other picture goes straight into plane
+  // 0 and is padded in place.
   uint8_t* origin = (uint8_t*)pic->buf + (size_t)pic->planes.origin * bps;
   if (!c->planes_pending) CK(cudaEventRecord(c->evp0, s));
-  CK(cudaMemcpy2DAsync(origin, (size_t)stride * bps, luma, (size_t)d->stride * bps, (size_t)d->width * bps, d->height,
-                       cudaMemcpyHostToDevice, s));
-  CK(launch_pad_plane(origin, d->bit_depth, d->width, d->height, stride, pic->planes, pic->cw, pic->ch, pic->pad, s));
+  if (as_ref && d->stride == d->width) {
+    uint8_t* packed = (uint8_t*)pic->buf + (size_t)pic->planes.plane_elems * bps;
+    CK(cudaMemcpyAsync(packed, luma, (size_t)d->width * bps * d->height, cudaMemcpyHostToDevice, s));
+    CK(launch_pad_plane(packed, d->bit_depth, d->width, d->height, d->width, pic->planes, pic->ch, pic->pad, s));
+  } else {
+    CK(cudaMemcpy2DAsync(origin, (size_t)stride * bps, luma, (size_t)d->stride * bps, (size_t)d->width * bps,
+                         d->height, cudaMemcpyHostToDevice, s));
+    CK(launch_pad_plane(origin, d->bit_depth, d->width, d->height, stride, pic->planes, pic->ch, pic->pad, s));
+  }
   if (as_ref && build_planes) {
     if (h264) CK(launch_h264_hpel(pic->planes, d->bit_depth, pic->cw, pic->ch, pic->pad, s));
     else CK(launch_hevc_phases(pic->planes, d->bit_depth, pic->cw, pic->ch, pic->pad, s));

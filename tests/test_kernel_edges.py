@@ -305,3 +305,25 @@ def test_phase_planes_at_tile_edges(ms, bd, w, h):
             np.testing.assert_array_equal(ms.plane(3200, fy * 4 + fx), np.clip((t + (1 << (sh - 1))) >> sh, 0, top),
                                           err_msg=f"padded phase {fx}, {fy}")
     ms.release(3200)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("codec,bd,w,h,extra,as_ref", [
+    (HEVC, 8, 16, 16, 0, True), (HEVC, 8, 33, 17, 0, True), (HEVC, 8, 850, 21, 5, True), (HEVC, 10, 131, 40, 0, True),
+    (HEVC, 10, 130, 16, 2, False), (HEVC, 8, 47, 19, 0, False), (H264, 8, 31, 47, 0, True), (H264, 10, 99, 33, 0, True),
+    (H264, 8, 99, 33, 7, True), (H264, 8, 17, 16, 0, False)])
+def test_padded_plane_of_packed_and_of_strided_rows(ms, codec, bd, w, h, extra, as_ref):
+    """Plane 0 is the picture, its border replicated, whichever way the rows
+    came: chunks across the sides, odd addresses, in place or from a packed
+    picture."""
+    import ctypes as C
+    rng = np.random.default_rng(w * h + extra)
+    rows = rng.integers(0, 1 << bd, (h, w + extra)).astype(np.uint8 if bd == 8 else np.uint16)
+    d = capi.PictureDesc(codec, bd, w, h, w + extra)
+    ms.upload(3300, np.zeros((h, w), rows.dtype), codec, bd, as_ref=as_ref)  # registers the picture's shape
+    assert capi.lib().rme_picture_upload(ms.ctx, 3300, C.byref(d), capi.ptr(rows), int(as_ref), None) == capi.RME_OK
+    pad = 32 if codec == H264 else 80
+    cw, ch = ((w + 15) // 16 * 16, (h + 15) // 16 * 16) if codec == H264 else (w, h)
+    want = np.pad(rows[:, :w], ((pad, pad + ch - h), (pad, pad + cw - w)), mode="edge")
+    np.testing.assert_array_equal(ms.plane(3300, 0), want)
+    ms.release(3300)
