@@ -250,7 +250,7 @@ __device__ __forceinline__ void phase_columns(const S* g, S* planes, int64_t pla
   }
   RowWords<S> next = load_row<S>(row_of(y0 + 4), col);
   S* out = planes + (int64_t)y0 * stride + x;
-#pragma unroll 2
+#pragma unroll (sizeof(S) == 1 ? 2 : 1)
   for (int r = 0; r < rows; ++r) {
     int h[4];
     horizontal<FX>(next, shift1, h);
@@ -288,14 +288,16 @@ __device__ __forceinline__ void phase_columns(const S* g, S* planes, int64_t pla
 
 // The fifteen phases of every padded position: a CTA of two warps, two of the
 // horizontal fractions (grid z the other two), over a tile of 128 x
-// `strip` positions. 64 threads of at most 128 registers: one CTA fits in the
-// registers the resident engine leaves free on every SM, so a picture's
-// planes are built while the engine runs. Bound by issue: about 5 instructions an output sample, where a
-// multiply-add per tap and the passes' round trip through shared memory took
-// about 50. One 1080p reference 61 -> 20 us, one of
-// 2160p at 10 bits 203 -> 87 us (3.2 TB/s written), one of 360p 13 -> 8 us.
+// `strip` positions. At most 64 registers a thread: the resident engine leaves
+// 2,048 on each of an SM's four schedulers, one warp's at 64, so a picture's
+// planes are built while the engine runs (with more, no warp could start until
+// it left, and it waits for the planes). Bound by issue: about 5 instructions
+// an output sample, where a multiply-add per tap and the passes' round trip
+// through shared memory took about 50. One 1080p reference 61 -> 21 us, one of
+// 2160p at 10 bits 203 -> 86 us (3.2 TB/s written), one of 360p 13 -> 8 us; up
+// to 94 registers gave the same but at 1080p and 10 bits (26 us against 31).
 template <class S>
-__global__ void __launch_bounds__(64, 8) hevc_phase_kernel(const S* g, S* planes, int64_t plane_elems, int stride,
+__global__ void __launch_bounds__(64, 16) hevc_phase_kernel(const S* g, S* planes, int64_t plane_elems, int stride,
                                                             int prow, int pcol, int bd, int strip) {
   const int x = blockIdx.x * kPhaseTX + (threadIdx.x & 31) * 4, y0 = blockIdx.y * strip;
   if (x >= pcol) return;
