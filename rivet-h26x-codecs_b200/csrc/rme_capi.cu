@@ -209,16 +209,14 @@ constexpr int kTuneRounds = 2;  // timings per shape before the tuner chooses (l
 // until rme_sync (or until its slot comes round again, which waits for it).
 constexpr int kSlots = 4;
 struct Slot {
-  DevBuf<FrameDesc> d_frames;
-  DevBuf<unsigned long long> d_ready;  // the launch's queues: rows, GIVEN jobs
   DevBuf<rme_result> d_out;
   DevBuf<rme_job> d_jobs;
-  DevBuf<unsigned long long> d_misc;  // the launch header (kMisc*)
+  DevBuf<unsigned long long> d_init;  // what a launch reads: [header (kMisc*) | frames | queues]
   DevBuf<unsigned long long> d_mvf;   // the row form's published vectors (tagged with the epoch)
   PinBuf<FrameDesc> h_frames;
   PinBuf<rme_result> h_out;
   PinBuf<unsigned long long> h_misc;
-  PinBuf<unsigned long long> h_init;  // [misc header | initial queue entries]
+  PinBuf<unsigned long long> h_init;  // as d_init
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, done = nullptr;
   uint32_t epoch = 0;
   // The launch in flight: its stream, its task count, the tuner class it
@@ -706,21 +704,16 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   const int64_t total = toff[n];
   for (int i = 0; i < n; ++i)
     if (ntask[i] >= (1 << 24)) return fail(c, RME_EINVAL, "more than 2^24 tasks in one frame");
-  CK(sl.d_frames.ensure(n));
   if (!dev_out) CK(sl.d_out.ensure(std::max<int64_t>(total, 1)));
-  unsigned long long* old_ready = sl.d_ready.p;
   unsigned long long* old_mvf = sl.d_mvf.p;
-  CK(sl.d_ready.ensure(2 * std::max<int64_t>(total, 1)));  // the parts' rows, then their GIVEN jobs
   CK(sl.d_mvf.ensure(std::max<int64_t>(total, 1)));
   // Fresh slot memory may hold any word, an epoch's among them: zero it
   // (epochs start at 1).
-  if (sl.d_ready.p != old_ready || sl.d_mvf.p != old_mvf) sl.epoch = 0;
+  if (sl.d_mvf.p != old_mvf) sl.epoch = 0;
   CK(sl.d_jobs.ensure(std::max<int64_t>(jobs_off[n], 1)));
-  CK(sl.d_misc.ensure(kMiscWords));
   if (!dev_out && !pinned_out) CK(sl.h_out.ensure(std::max<int64_t>(total, 1)));
   CK(sl.h_misc.ensure(kMiscWords));
   if (sl.epoch == 0 || sl.epoch >= 0x3fffffffu) {  // 30 bits: an H.264 word's tag holds a reference beside it
-    CK(cudaMemsetAsync(sl.d_ready.p, 0, sl.d_ready.n * sizeof(unsigned long long), s));
     CK(cudaMemsetAsync(sl.d_mvf.p, 0, sl.d_mvf.n * sizeof(unsigned long long), s));
     sl.epoch = 0;
   }
@@ -831,8 +824,9 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     }
     if (!c->bps[k][variant[k]]) c->bps[k][variant[k]] = h264_given_blocks_per_sm(part_bytes(k), variant[k]);
   }
-  // h_init: [the launch header (kMiscWords) | rows | GIVEN jobs]
-  size_t ninit = 0, rows_off[kParts], given_off[kParts];
+  // One block, copied at once: [the launch header | frames | rows | GIVEN jobs].
+  static_assert(sizeof(FrameDesc) % sizeof(unsigned long long) == 0, "whole words");
+  size_t ninit = kMiscWords + sizeof(FrameDesc) / sizeof(unsigned long long) * n, rows_off[kParts], given_off[kParts];
   for (int k = 0; k < kParts; ++k) {
     rows_off[k] = ninit;
     ninit += rows[k].size();
@@ -841,33 +835,32 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     given_off[k] = ninit;
     ninit += given[k].size();
   }
-  CK(sl.h_init.ensure(kMiscWords + ninit));
-  unsigned long long* hi = sl.h_init.p;
+  CK(sl.h_init.ensure(ninit));
+  CK(sl.d_init.ensure(ninit));
+  unsigned long long *hi = sl.h_init.p, *di = sl.d_init.p;
   std::memset(hi, 0, kMiscWords * sizeof(unsigned long long));
+  std::memcpy(hi + kMiscWords, sl.h_frames.p, sizeof(FrameDesc) * n);
   hi[kMiscEpoch] = sl.epoch;
   LaunchDesc Ls[kParts] = {}, Lgiven[kParts] = {};
-  int64_t slot0 = 0, slot_off[kParts];
   int grid[kParts] = {0, 0, 0, 0}, nparts = 0, order[kParts];
   for (int k = 0; k < kParts; ++k) {
     hi[2 * k + 1] = rows[k].size();
-    std::copy(rows[k].begin(), rows[k].end(), hi + kMiscWords + rows_off[k]);
-    std::copy(given[k].begin(), given[k].end(), hi + kMiscWords + given_off[k]);
-    slot_off[k] = slot0;
+    std::copy(rows[k].begin(), rows[k].end(), hi + rows_off[k]);
+    std::copy(given[k].begin(), given[k].end(), hi + given_off[k]);
     LaunchDesc& L = Ls[k];
-    L.frames = sl.d_frames.p;
-    L.ready = sl.d_ready.p + slot0;
+    L.frames = reinterpret_cast<const FrameDesc*>(di + kMiscWords);
+    L.ready = di + rows_off[k];
     L.total = (int64_t)rows[k].size();
-    L.head = sl.d_misc.p + 2 * k;
-    L.tail = sl.d_misc.p + 2 * k + 1;
-    L.counters = sl.d_misc.p + kMiscCounters;
-    L.status = reinterpret_cast<uint32_t*>(sl.d_misc.p + kMiscStatus);
-    L.epoch = reinterpret_cast<const uint32_t*>(sl.d_misc.p + kMiscEpoch);
+    L.head = di + 2 * k;
+    L.tail = di + 2 * k + 1;
+    L.counters = di + kMiscCounters;
+    L.status = reinterpret_cast<uint32_t*>(di + kMiscStatus);
+    L.epoch = reinterpret_cast<const uint32_t*>(di + kMiscEpoch);
     Lgiven[k] = L;
-    Lgiven[k].ready = sl.d_ready.p + total + slot0;
+    Lgiven[k].ready = di + given_off[k];
     Lgiven[k].total = (int64_t)given[k].size();
-    Lgiven[k].head = sl.d_misc.p + kMiscGiven + 2 * k;
-    Lgiven[k].tail = sl.d_misc.p + kMiscGiven + 2 * k + 1;
-    slot0 += part_tasks[k];
+    Lgiven[k].head = di + kMiscGiven + 2 * k;
+    Lgiven[k].tail = di + kMiscGiven + 2 * k + 1;
     if (part_tasks[k] > 0) order[nparts++] = k;
     if (!rows[k].empty()) {
       const bool h264 = part_codec(k) == RME_CODEC_H264;
@@ -890,8 +883,8 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
       e = h264 ? launch_h264_rows(Ls[k], bytes, rows_nref[k], grid[k], sk) : launch_hevc_rows(Ls[k], bytes, grid[k], sk);
     if (e == cudaSuccess && amp_tasks[k][0] + amp_tasks[k][1] > 0) {
       LaunchDesc A = Ls[k];
-      A.head = sl.d_misc.p + kMiscAmp + 2 * k;
-      A.tail = sl.d_misc.p + kMiscAmp + 2 * k + 1;
+      A.head = di + kMiscAmp + 2 * k;
+      A.tail = di + kMiscAmp + 2 * k + 1;
       A.total = amp_tasks[k][0] + amp_tasks[k][1];
       e = launch_hevc_flat(A, bytes, true, true, n, amp_tasks[k][1], c->nsm, sk);
     }
@@ -902,17 +895,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   };
   auto enqueue = [&](bool capturing) -> cudaError_t {
     const unsigned rec = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
-    cudaError_t e = cudaMemcpyAsync(sl.d_frames.p, sl.h_frames.p, sizeof(FrameDesc) * n, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(sl.d_misc.p, hi, kMiscWords * sizeof(unsigned long long), cudaMemcpyHostToDevice, s);
-    for (int k = 0; k < kParts; ++k) {
-      if (e == cudaSuccess && !rows[k].empty())
-        e = cudaMemcpyAsync(sl.d_ready.p + slot_off[k], hi + kMiscWords + rows_off[k],
-                            rows[k].size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, s);
-      if (e == cudaSuccess && !given[k].empty())
-        e = cudaMemcpyAsync(sl.d_ready.p + total + slot_off[k], hi + kMiscWords + given_off[k],
-                            given[k].size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, s);
-    }
+    cudaError_t e = cudaMemcpyAsync(di, hi, ninit * sizeof(unsigned long long), cudaMemcpyHostToDevice, s);
     // Under capture the records are external ones: they become event-record
     // nodes, so the kernels' device time is measured on every replay.
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(sl.ev0, s, rec);
@@ -931,7 +914,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     if (e == cudaSuccess && !dev_out && !pinned_out)
       e = cudaMemcpyAsync(sl.h_out.p, sl.d_out.p, sizeof(rme_result) * total, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(sl.h_misc.p, sl.d_misc.p, kMiscWords * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
+      e = cudaMemcpyAsync(sl.h_misc.p, di, kMiscWords * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
     return e;
   };
   bool has_given = false;
