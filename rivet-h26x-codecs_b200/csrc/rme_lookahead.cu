@@ -159,6 +159,17 @@ __device__ __forceinline__ Pick2 argmin(uint32_t c) {
   return {m, __ffs(__ballot_sync(kAll, c == m)) - 1};
 }
 
+// |a - b| of four bytes, summed onto acc.
+__device__ __forceinline__ uint32_t sad4(uint32_t a, uint32_t b, uint32_t acc) {
+  uint32_t r;
+  asm("vabsdiff4.u32.u32.u32.add %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(acc));
+  return r;
+}
+// Point k of the rings (4, 2, 1 samples; each (s,0), (-s,0), (0,s), (0,-s)):
+// offsets + 4 as hex digits, the lowest first.
+__device__ __forceinline__ int ring_x(int k) { return (int)((0x443544264408ull >> (4 * k)) & 15u) - 4; }
+__device__ __forceinline__ int ring_y(int k) { return (int)((0x354426440844ull >> (4 * k)) & 15u) - 4; }
+
 // The row a warp claims next: row-major over the pairs (every pair's row 0,
 // then every row 1, ...), so that a claim's upper row was claimed before it.
 __device__ __forceinline__ bool claim_row(unsigned long long* counter, int npairs, int rows, int lane, int& pair,
@@ -183,10 +194,15 @@ __device__ __forceinline__ bool claim_row(unsigned long long* counter, int npair
 // rings: where that seed wins, as it does in even motion, its rings are
 // known already.
 //
-// Bound by the chain of passes along the wavefront (bw + 2 bh blocks): a
-// load, one shuffle and one warp minimum each. Eight pairs of 1080p
-// pictures: 3,010 us when a warp took one block at a time (claim, two waits,
-// up to twelve passes, the SATD), 547 us this way, the SATDs included.
+// Bound by the chain of passes along the wavefront (bw + bh blocks), each a
+// chain of dependent instructions: a load, one shuffle and one warp minimum,
+// over keys that order the points by ring, cost and place, so that the minimum
+// is the decision; what depends on the lane alone is kept. Eight pairs of
+// 1080p pictures: 3,010 us when a warp took one block at a time (claim, two
+// waits, up to twelve passes, the SATD), 547 us a row a warp with ballots and
+// shuffles to decide, 445 us this way, the SATDs included; a row of eight
+// bytes by two 8-byte loads instead of three words took 50 us of it (the
+// candidates lie on lines of their own, each a pass through L1 a load).
 constexpr int kLaWarps = 4;  // rows per CTA: few, so that a launch's rows spread over the SMs
 __global__ void __launch_bounds__(kLaWarps * 32) lowres_search_kernel(const LowresDesc* pairs, int npairs,
                                                                       unsigned long long* words_all,
@@ -195,17 +211,21 @@ __global__ void __launch_bounds__(kLaWarps * 32) lowres_search_kernel(const Lowr
   const int lane = threadIdx.x & 31, q = lane >> 1, half = lane & 1;
   const int bw = pairs[0].bw, bh = pairs[0].bh, n = bw * bh, lim = kLowresPad - 1;
   bool lost = false;
-  // This lane's ring point as the q-th candidate of a pass of rings (q in
-  // 0..11: ring 4, 2, 1, each (s,0), (-s,0), (0,s), (0,-s)).
-  auto ring_x = [](int k) { const int st = 4 >> (k >> 2), d = k & 3; return d == 0 ? st : d == 1 ? -st : 0; };
-  auto ring_y = [](int k) { const int st = 4 >> (k >> 2), d = k & 3; return d == 2 ? st : d == 3 ? -st : 0; };
+  // This lane's ring point in a first pass (candidates 3..14) and in a later
+  // one (0..11).
+  const int rx0 = ring_x(min(max(q - 3, 0), 11)), ry0 = ring_y(min(max(q - 3, 0), 11));
+  const int rx1 = ring_x(min(q, 11)), ry1 = ring_y(min(q, 11));
   for (int pi, by; claim_row(counter, npairs, bh, lane, pi, by);) {
     const LowresDesc cur = pairs[2 * pi], ref = pairs[2 * pi + 1];
     unsigned long long* words = words_all + (size_t)pi * n + (size_t)by * bw;
     const unsigned long long* up = words - bw;
     const int y = by * 8;
     const uint8_t* srow = cur.plane + (ptrdiff_t)(y + kLowresPad + half * 4) * cur.stride + kLowresPad;
-    const uint8_t* rrow = ref.plane + (ptrdiff_t)(y + kLowresPad + half * 4) * ref.stride + kLowresPad;
+    const uint32_t rstride = (uint32_t)ref.stride;  // a multiple of 8: a block's rows start alike
+    const uint32_t rrow = (uint32_t)(y + kLowresPad + half * 4) * rstride + kLowresPad;
+    const int ylo = -lim - y, yn = ref.ph + 2 * lim - 8;  // rows a block may be displaced to: ylo .. ylo + yn
+    const int xn = ref.pw + 2 * lim - 8;
+    uint32_t prev_n = 0;  // the block before's count, stored a block later
     // The first block's source rows and upper vector; later ones are loaded
     // a block ahead (8-byte aligned: x, the pad and the stride are multiples
     // of 8).
@@ -215,8 +235,8 @@ __global__ void __launch_bounds__(kLaWarps * 32) lowres_search_kernel(const Lowr
     unsigned long long uw = by > 0 ? ld_word(up) : 0ull;
     uint32_t lv = 0;
     for (int bx = 0; bx < bw; ++bx) {
-      const int x = bx * 8;
-      const uint8_t* rb = rrow + x;
+      const int x = bx * 8, xlo = -lim - x;
+      const uint32_t rb = rrow + x;
       if (by > 0 && !wait_word(up + bx, uw, status, lost)) lost = true;
       const uint32_t av = (uint32_t)uw;
       uint2 sn[4] = {};
@@ -228,71 +248,70 @@ __global__ void __launch_bounds__(kLaWarps * 32) lowres_search_kernel(const Lowr
         if (by > 0) un = ld_word(up + bx + 1);
       }
       auto inplane = [&](int dx, int dy) {
-        return x + dx >= -lim && y + dy >= -lim && x + dx + 8 <= ref.pw + lim && y + dy + 8 <= ref.ph + lim;
+        return (uint32_t)(dx - xlo) <= (uint32_t)xn && (uint32_t)(dy - ylo) <= (uint32_t)yn;
       };
       auto score = [&](bool ok, int dx, int dy) -> uint32_t {
-        uint32_t part = 0;
+        uint32_t part = 0, odd = 0;
         if (ok) {
-          uint32_t a[4], b[4];
+          const uint32_t o = rb + (uint32_t)(dy * (int)rstride + dx), sh = (o & 3u) * 8u;
+          const bool up = o & 4u;
+          uint2 w[4][2];
 #pragma unroll
-          for (int r = 0; r < 4; ++r) ld8(rb + (ptrdiff_t)(dy + r) * ref.stride + dx, a[r], b[r]);
+          for (int r = 0; r < 4; ++r) {
+            const uint2* p = reinterpret_cast<const uint2*>(ref.plane + (size_t)((o & ~7u) + r * rstride));
+            w[r][0] = __ldg(p);
+            w[r][1] = __ldg(p + 1);
+          }
 #pragma unroll
-          for (int r = 0; r < 4; ++r) part += __vsadu4(s[r].x, a[r]) + __vsadu4(s[r].y, b[r]);
+          for (int r = 0; r < 4; ++r) {
+            const uint32_t a = up ? w[r][0].y : w[r][0].x, b = up ? w[r][1].x : w[r][0].y,
+                           c = up ? w[r][1].y : w[r][1].x;
+            part = sad4(s[r].x, __funnelshift_r(a, b, sh), part);
+            odd = sad4(s[r].y, __funnelshift_r(b, c, sh), odd);
+          }
         }
+        part += odd;
         part += __shfl_xor_sync(kAll, part, 1);
-        return ok ? part + 2u * (uint32_t)min(abs(dx) + abs(dy), 32) : 0xffffffffu;
+        return part + 2u * (uint32_t)min(abs(dx) + abs(dy), 32);
       };
       // Seeds: zero, the left block's vector, the above block's (candidates
       // 0..2); rings around the first neighbour's (candidates 3..14).
       const int ns = 1 + (bx > 0) + (by > 0);
       const uint32_t v1 = bx > 0 ? lv : av;
       const int gx = (int)(int16_t)(v1 & 0xffffu), gy = (int)(int16_t)(v1 >> 16);  // zero with no neighbour
-      int dx, dy;
-      bool ok;
-      if (q < 3) {
-        const uint32_t sv = q == 0 ? 0u : q == 1 ? v1 : av;
-        dx = (int)(int16_t)(sv & 0xffffu);
-        dy = (int)(int16_t)(sv >> 16);
-        ok = q < ns && inplane(dx, dy);
-      } else {
-        dx = gx + ring_x(q - 3);
-        dy = gy + ring_y(q - 3);
-        ok = q < 15 && inplane(dx, dy);
-      }
+      const int hx = (int)(int16_t)(av & 0xffffu), hy = (int)(int16_t)(av >> 16);
+      int dx = q == 0 ? 0 : q == 2 ? hx : q == 1 ? gx : gx + rx0, dy = q == 0 ? 0 : q == 2 ? hy : q == 1 ? gy : gy + ry0;
+      bool ok = (q < 3 ? q < ns : q < 15) && inplane(dx, dy);
       uint32_t cost = score(ok, dx, dy);
-      uint32_t nsad = __popc(__ballot_sync(kAll, ok && q < 3 && half == 0));
-      Pick2 p = argmin(q < 3 ? cost : 0xffffffffu);
-      uint32_t bc = p.cost;
-      int bxm = __shfl_sync(kAll, dx, p.lane), bym = __shfl_sync(kAll, dy, p.lane);
-      if (bc == 0xffffffffu) bxm = bym = 0;  // no seed in the plane
+      uint32_t nsad = ok && q < 3;  // this lane's points scored (two lanes a point)
+      // A cost is below 2^15: 64 differences of at most 255 and a penalty of 64.
+      uint32_t m = __reduce_min_sync(kAll, ok && q < 3 ? cost << 4 | (uint32_t)q : 0xffffffffu);
+      uint32_t bc = m >> 4;
+      const int seed = m == 0xffffffffu ? 0 : (int)(m & 15u);  // none in the plane: zero
+      int bxm = seed == 0 ? 0 : seed == 1 ? gx : hx, bym = seed == 0 ? 0 : seed == 1 ? gy : hy;
       const int cx = bxm, cy = bym;
       int k = q - 3;  // this lane's ring candidate (0..11 where there is one)
       bool known = bxm == gx && bym == gy;
       for (int ring = 0;;) {  // rings `ring`.. of 0, 1, 2 are left around the best
         if (!known) {
           k = q;
-          dx = bxm + ring_x(k);
-          dy = bym + ring_y(k);
-          ok = k < 12 && (k >> 2) >= ring && abs(dx - cx) <= kLowresRange && abs(dy - cy) <= kLowresRange &&
-               inplane(dx, dy);
+          dx = bxm + rx1;
+          dy = bym + ry1;
+          ok = k < 12 && (k >> 2) >= ring && (uint32_t)(dx - cx + kLowresRange) <= 2u * kLowresRange &&
+               (uint32_t)(dy - cy + kLowresRange) <= 2u * kLowresRange && inplane(dx, dy);
           cost = score(ok, dx, dy);
         }
         known = false;
+        // The first ring with a point below the best, its least point, the
+        // first of equal ones; the rings before it and it are the ones scored.
         const bool live = ok && k >= 0;
-        const uint32_t cnt = __ballot_sync(kAll, live && half == 0);
-        const uint32_t low = __ballot_sync(kAll, live && cost < bc);
-        if (low == 0u) {
-          nsad += __popc(cnt);
-          break;
-        }
-        // The first ring with a point below the best; the rings before it
-        // and it are the ones scored.
-        const int at = __shfl_sync(kAll, k, __ffs(low) - 1) >> 2;
-        nsad += __popc(__ballot_sync(kAll, live && half == 0 && (k >> 2) <= at));
-        p = argmin(live && (k >> 2) == at ? cost : 0xffffffffu);
-        bc = p.cost;
-        bxm = __shfl_sync(kAll, dx, p.lane);
-        bym = __shfl_sync(kAll, dy, p.lane);
+        m = __reduce_min_sync(kAll, live && cost < bc ? (uint32_t)(k >> 2) << 24 | cost << 4 | (uint32_t)k : 0xffffffffu);
+        const int at = (int)(m >> 24);  // 255: none
+        nsad += live && (k >> 2) <= at;
+        if (m == 0xffffffffu) break;
+        bc = (m >> 4) & 0xfffffu;
+        bxm += ring_x((int)(m & 15u));
+        bym += ring_y((int)(m & 15u));
         ring = at;
       }
       lv = (uint32_t)(uint16_t)(int16_t)bxm | (uint32_t)(uint16_t)(int16_t)bym << 16;
@@ -300,12 +319,14 @@ __global__ void __launch_bounds__(kLaWarps * 32) lowres_search_kernel(const Lowr
         st_word(words + bx, lv);
         const size_t o = (size_t)pi * n + (size_t)by * bw + bx;
         *reinterpret_cast<uint32_t*>(mv_all + o) = lv;
-        nsad_all[o] = nsad;
+        if (bx > 0) nsad_all[o - 1] = prev_n;
       }
+      prev_n = __reduce_add_sync(kAll, nsad) >> 1;
 #pragma unroll
       for (int r = 0; r < 4; ++r) s[r] = sn[r];
       uw = un;
     }
+    if (lane == 0) nsad_all[(size_t)pi * n + (size_t)(by + 1) * bw - 1] = prev_n;
   }
 }
 
