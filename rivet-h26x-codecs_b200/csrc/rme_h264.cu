@@ -176,8 +176,8 @@ struct RefSearch {
   __device__ __forceinline__ uint32_t sad(int fx, int fy) {
     const S* rp = org + (ptrdiff_t)(fy + sub) * R.stride + fx;
     uint32_t a[WR], b[WR];
-    ldwords<WR>(rp, a);
-    ldwords<WR>(rp + (ptrdiff_t)8 * R.stride, b);
+    ldrow<WR>(rp, a);
+    ldrow<WR>(rp + (ptrdiff_t)8 * R.stride, b);
     return sad2(a, b);
   }
   // Copies rows of 16-byte chunks around whole-sample offset (x, y) into the
@@ -507,6 +507,10 @@ struct RefSearch {
     int bmx = smx, bmy = smy;
     uint32_t bc = kInf;
     bool first = true;
+    // This lane's ring point in the first step (the start is slot 0) and in one
+    // of sixteen lanes a candidate.
+    const int rx0 = ring_x((slot - 1) & 7), ry0 = ring_y((slot - 1) & 7);
+    const int rx1 = ring_x(warp * 2 + (lane >> 4)), ry1 = ring_y(warp * 2 + (lane >> 4));
     // No step leaves the start by more than `far` samples. A walk that went
     // too far for the window has it staged anew.
     const int far = (2 * hpel + qpel + 3) / 4;
@@ -543,10 +547,18 @@ struct RefSearch {
         const bool wide = staged && !first;
         const int sl = wide ? warp * 2 + (lane >> 4) : slot, part = wide ? lane & 15 : sub;
         int mx, my;
-        vec(sl, mx, my);
+        if (wide) {
+          mx = (int)(int16_t)(cmx + rx1 * step);
+          my = (int)(int16_t)(cmy + ry1 * step);
+        } else if (first && slot > 0) {
+          mx = (int)(int16_t)(cmx + rx0 * step);
+          my = (int)(int16_t)(cmy + ry0 * step);
+        } else {
+          vec(sl, mx, my);
+        }
         bool ok = sl < n;
         if (sl >= base)
-          ok = ok && mx >= qlx && mx <= qhx && my >= qly && my <= qhy &&
+          ok = ok && (uint32_t)(mx - qlx) <= (uint32_t)(qhx - qlx) && (uint32_t)(my - qly) <= (uint32_t)(qhy - qly) &&
                !((uint32_t)(mx - prevx + step) <= 2u * step && (uint32_t)(my - prevy + step) <= 2u * step);
         const uint32_t rt = rate(mx, my);
         uint32_t v = kNone;
@@ -613,6 +625,36 @@ __device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSme
     __syncwarp();
   }
   Nb A{false, -1, 0, 0};
+  // What does not change along the row, read once (the frame's description is
+  // in global memory, and the steps' barriers would have it read again).
+  const int gr = min(g, nref - 1), width = F.width, height = F.height, pad = F.pad, vr = F.vr;
+  const int hpel = F.hpel_iters, qpel = F.qpel_iters;
+  const float ratio = F.refine_ratio;
+  const uint32_t ref_cost = F.ref_cost[gr];
+  RefSearch<S> q{sm, sm.src[0], F.ref[gr], F.tab, F.range, F.umh, F.dia, F.qpel_diamond};
+  q.g = g;
+  q.warp = warp;
+  q.lane = lane;
+  q.sub = lane & 7;
+  q.slot = warp * 4 + (lane >> 3);
+  q.height = height;
+  q.win = sm.win[gr];
+  q.B.w = q.B.h = 16;
+  q.B.y = my * 16;
+  q.B.ly = max(4 - pad - q.B.y, -vr);  // search_bounds (h264_hpel.rs:476-488)
+  q.B.hy = min(height + pad - 20 - q.B.y, vr);
+  // A macroblock's result, written a macroblock later, when the counts have
+  // met: only its vector is waited for.
+  int ended = 0;  // its reference
+  auto write = [&](int mx) {
+    const RefResult& w = sm.fin[mx & 1][ended];
+    write_result(&F.out[my * mbw + mx], w.mx, w.my, ended, w.cost, w.satd, w.imx, w.imy, w.icost, sm.nsad[mx & 1],
+                 sm.nsatd[mx & 1], 0);
+    cnt[0] += 1;
+    cnt[1] += sm.nsad[mx & 1];
+    cnt[2] += sm.nsatd[mx & 1];
+    sm.nsad[mx & 1] = sm.nsatd[mx & 1] = 0u;
+  };
   __syncthreads();
   for (int mx = 0; mx < mbw; ++mx) {
     const int par = mx & 1;
@@ -665,34 +707,24 @@ __device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSme
         cx = prx;
         cy = pry;
       }
-      RefSearch<S> q{sm, sm.src[par], F.ref[g], F.tab, F.range, F.umh, F.dia, F.qpel_diamond};
-      q.g = g;
-      q.warp = warp;
-      q.lane = lane;
-      q.sub = lane & 7;
-      q.slot = warp * 4 + (lane >> 3);
-      q.height = F.height;
-      q.win = sm.win[g];
+      q.src = sm.src[par];
 #pragma unroll
       for (int i = 0; i < WR; ++i) {
         q.s0[i] = q.src[q.sub * WR + i];
         q.s1[i] = q.src[(q.sub + 8) * WR + i];
       }
+      q.nsad = q.nsatd = 0;
       H264Blk& B = q.B;
       B.x = mx * 16;
-      B.y = my * 16;
-      B.w = B.h = 16;
       B.px = prx;
       B.py = pry;
-      B.lx = 4 - F.pad - B.x;  // search_bounds (h264_hpel.rs:476-488)
-      B.hx = F.width + F.pad - 20 - B.x;
-      B.ly = max(4 - F.pad - B.y, -F.vr);
-      B.hy = min(F.height + F.pad - 20 - B.y, F.vr);
+      B.lx = 4 - pad - B.x;
+      B.hx = width + pad - 20 - B.x;
       q.org = plane_at<S>(q.R, 0, B.x, B.y);
       RefResult r;
       uint32_t ic0;
       q.whole(nc + (g > 0), cx, cy, r.imx, r.imy, ic0);
-      r.icost = ic0 + F.ref_cost[g];
+      r.icost = ic0 + ref_cost;
       bool gate = false;
       if (nref > 1) {
         // refine_ratio: a further reference whose whole-sample cost is that
@@ -701,17 +733,11 @@ __device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSme
         asm volatile("bar.sync 8, %0;" ::"r"(nref * kRefThreads) : "memory");
         uint32_t before = kInf;
         for (int p = 0; p < g; ++p) before = min(before, sm.icost[par][p]);
-        gate = g > 0 && F.refine_ratio > 0.0f &&
-               __uint2float_rn(r.icost) >= __fmul_rn(F.refine_ratio, __uint2float_rn(before));
+        gate = g > 0 && ratio > 0.0f && __uint2float_rn(r.icost) >= __fmul_rn(ratio, __uint2float_rn(before));
       }
-      q.refine(r.imx, r.imy, gate ? 0 : F.hpel_iters, gate ? 0 : F.qpel_iters, r.mx, r.my, r.satd, r.cost);
-      r.cost += F.ref_cost[g];
+      q.refine(r.imx, r.imy, gate ? 0 : hpel, gate ? 0 : qpel, r.mx, r.my, r.satd, r.cost);
+      r.cost += ref_cost;
       if ((tid & (kRefThreads - 1)) == 0) sm.fin[par][g] = r;
-      const uint32_t nsad = __reduce_add_sync(kFull, q.nsad) / 8, nsatd = __reduce_add_sync(kFull, q.nsatd) / 16;
-      if (lane == 0) {
-        atomicAdd(&sm.nsad[par], nsad);
-        atomicAdd(&sm.nsatd[par], nsatd);
-      }
     }
     if (tid < NSRC) sm.src[par ^ 1][tid] = nsrc;
     __syncthreads();
@@ -726,18 +752,24 @@ __device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSme
     const RefResult& w = sm.fin[par][best];
     A = Nb{true, best, (int)(int16_t)w.mx, (int)(int16_t)w.my};
     if (tid == 0) {
-      const int t = my * mbw + mx;
-      st_relaxed64(F.mvf + t, mv_word(tag | (uint32_t)best, w.mx, w.my));
-      write_result(&F.out[t], w.mx, w.my, best, w.cost, w.satd, w.imx, w.imy, w.icost, sm.nsad[par], sm.nsatd[par], 0);
-      cnt[0] += 1;
-      cnt[1] += sm.nsad[par];
-      cnt[2] += sm.nsatd[par];
-      sm.nsad[par] = sm.nsatd[par] = 0u;
+      st_relaxed64(F.mvf + my * mbw + mx, mv_word(tag | (uint32_t)best, w.mx, w.my));
+      if (mx > 0) write(mx - 1);
+      ended = best;
+    }
+    if (g < nref) {
+      // Both counts in one sum (a lane has a few hundred of each at most).
+      const uint32_t n = __reduce_add_sync(kFull, q.nsad | q.nsatd << 16);
+      if (lane == 0) {
+        atomicAdd(&sm.nsad[par], (n & 0xffffu) / 8);
+        atomicAdd(&sm.nsatd[par], (n >> 16) / 16);
+      }
     }
     wd = wb;
     wb = wc;
     wc = wn;
   }
+  __syncthreads();
+  if (tid == 0) write(mbw - 1);
 }
 
 // Rows are taken in the order the host pushed them (every frame's row 0,
