@@ -307,9 +307,7 @@ def run_ours(args, world, rank, local):
     # Each frame's results go to a buffer the caller keeps (as an encoder
     # keeps its motion field) in pinned memory, which the results' copy
     # fills directly; touched before the timing.
-    # The tuner times its launch shapes (eight for one HEVC frame, each
-    # twice) on the first launches of this size: one frame several times, so
-    # that they are compared on the same content.
+    # Warm-up: the first launches of this size allocate the buffers.
     for _ in range(18):
         ms.search(batch[0][0], batch[0][1], p, stream=sh)
     per_frame = ms.result_count(batch[0][0], batch[0][1], p)
@@ -327,10 +325,8 @@ def run_ours(args, world, rank, local):
     plain_fps = len(batch) / sum(lat)
 
     # ---- batched, device-resident -------------------------------------------
-    # Warm-up: the occupancy tuner times its three variants twice each on
-    # the first six launches of this size, and the winner's CUDA graph is
-    # captured the next time its shape comes; two more steps settle both
-    # before timing.
+    # Warm-up: a launch's CUDA graph is captured the second time its shape
+    # comes; a few more steps settle it before timing.
     warm = max(args.warmup, 3) + 5
     for _ in range(warm):
         outs = step()

@@ -460,9 +460,9 @@ typedef struct {
 
 /* Serving modes. LAUNCHES (0): the frames that arrived since the last launch
  * go into one search launch of their own as soon as one of three launch
- * streams is free, so up to three launches overlap on the device (a launch
- * of one or two frames runs the latency form). RESIDENT (1): one search
- * kernel stays on the GPU and frames join its queue as they arrive. */
+ * streams is free, so up to three launches overlap on the device.
+ * RESIDENT (1): one search kernel stays on the GPU and frames join its queue
+ * as they arrive. */
 #define RME_SERVE_LAUNCHES 0
 #define RME_SERVE_RESIDENT 1
 

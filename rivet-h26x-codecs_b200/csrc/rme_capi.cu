@@ -550,8 +550,8 @@ int make_frame(Ctx* c, const rme_frame* f, const rme_params* p, FrameDesc* fd, r
       fd->nby[l] = src->d.height / sizes[l];
       fd->base[l + 1] = fd->base[l] + fd->nbx[l] * fd->nby[l];
     }
-    // Blocks of 32 or more (the first levels): the tasks a CTA runs in the
-    // latency form.
+    // Blocks of 32 or more (the first levels): the tasks a CTA of the resident
+    // engine runs.
     if (p->predictor_mode == RME_PRED_STANDALONE) {
       int lb = 0;
       while (lb < fd->nlevels && fd->size[lb] >= 32) ++lb;
@@ -720,13 +720,13 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   ++sl.epoch;
   // Pass 2: device pointers and the parts' queues. A part (one sample width
   // and codec) is up to three launches in turn, each over its own queue:
-  //   - its STANDALONE frames' rows (HEVC: their 2Nx2N blocks): against the
-  //     dataflow form that ran one task a warp with dependency counts, H.264
-  //     took 0.53 against 1.60 ms for one CIF frame, 0.86 against 2.49 ms for
-  //     a hundred and 9.6 against 14.7 ms for 64 720p frames of two
-  //     references; HEVC, with the same arithmetic, 1.8 against 6 ms for one
-  //     1080p frame, 8.4 against 10.8 for twelve, 25.0 against 26.2 for 24 of
-  //     10 bits (only forty 8-bit ones 25.3 against 24.2);
+  //   - its STANDALONE frames' rows (HEVC: their 2Nx2N blocks), at every
+  //     launch size: against the dataflow form that ran one task a warp with
+  //     dependency counts, H.264 takes 0.35 against 1.60 ms for one CIF frame
+  //     and 5.9 against 14.5 ms for 64 720p frames of two references; HEVC,
+  //     when both had the same arithmetic, 1.8 against 6 ms for one 1080p
+  //     frame, 8.4 against 10.8 for twelve, 25.0 against 26.2 for 24 of 10
+  //     bits (only forty 8-bit ones 25.3 against 24.2);
   //   - HEVC frames' AMP units, which read those blocks' results;
   //   - GIVEN jobs, largest blocks first.
   std::vector<int64_t> sig;

@@ -233,13 +233,13 @@ __global__ void __maxnreg__(kEngineMaxRegs) engine_kernel(LaunchDesc L, EngineCt
     if (e == 0xffffffffu) continue;
     const int f = (int)(e >> 24), t = (int)(e & 0xffffffu);
     if (F.mvf != nullptr) {  // a row of the frame's 16x16 or 8x8 blocks
-      if (F.bd == 8) hevc_row<uint8_t, true>(L, F, f, (uint32_t)t, sm8, lane);
-      else hevc_row<uint16_t, true>(L, F, f, (uint32_t)t, sm16, lane);
+      if (F.bd == 8) hevc_row<uint8_t>(L, F, f, (uint32_t)t, sm8, lane);
+      else hevc_row<uint16_t>(L, F, f, (uint32_t)t, sm16, lane);
     } else if (t >= F.ntasks || F.mode != RME_PRED_STANDALONE) {
       if (lane == 0) atomicOr(L.status, kStatusBadTask);
       continue;
     } else if (F.codec == RME_CODEC_HEVC) {
-      cont = F.bd == 8 ? hevc_task<uint8_t, true>(L, F, f, t, sm8, lane) : hevc_task<uint16_t, true>(L, F, f, t, sm16, lane);
+      cont = F.bd == 8 ? hevc_task<uint8_t>(L, F, f, t, sm8, lane) : hevc_task<uint16_t>(L, F, f, t, sm16, lane);
     } else {
       cont = F.bd == 8 ? h264_task<uint8_t>(L, F, f, t, sm8, lane) : h264_task<uint16_t>(L, F, f, t, sm16, lane);
     }
@@ -464,12 +464,10 @@ int engine_create(void* ctx, int device, Engine** out) {
   L.status = reinterpret_cast<uint32_t*>(g->d_hdr + kHdrStatus);
   L.counters = g->d_hdr + kHdrCounters;
   L.epoch = reinterpret_cast<const uint32_t*>(g->d_hdr + kHdrEpoch);
-  L.done = nullptr;
   L.ready_big = g->d_ring + (1ull << kRingShift);
   L.head_big = g->d_hdr + kHdrHeadBig;
   L.tail_big = g->d_hdr + kHdrTailBig;
   L.group_ctas = groups;
-  L.patch8 = 1;
   L.ring_shift = kRingShift;
   EngineCtl& E = g->E;
   E.fdone = g->d_fdone;

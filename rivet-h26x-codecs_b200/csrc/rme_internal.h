@@ -70,13 +70,13 @@ struct FrameDesc {
   int32_t ntasks;
   uint32_t gen;  // the resident engine: this frame's generation in its slot
   int32_t big_end;  // HEVC STANDALONE: tasks below big_end * nref are blocks of 32 or more
-  // The row form (HEVC STANDALONE without AMP, latency kernels and the
-  // engine; H.264 STANDALONE, rme_h264.cu): a warp or a CTA owns a row of one
+  // The row form (STANDALONE launches, rme_rows.cu and rme_h264.cu; the
+  // engine's HEVC frames without AMP): a warp or a CTA owns a row of one
   // level and reference (H.264: of macroblocks) and searches its blocks left
   // to right; per task its motion vector is published as one word,
   // (tag << 32) | mv (H.264: the reference in the tag's two low bits), which
-  // the rows below and the next size's rows wait for. Null: the dataflow
-  // form.
+  // the rows below and the next size's rows wait for. Null: a frame of the
+  // engine's tasks.
   unsigned long long* mvf;
   uint32_t tag;     // nonzero, new for every search of the buffer (the launch's epoch, the slot's generation)
   int32_t nrows;    // rows of the frame, both kinds (the engine counts them to completion)
@@ -86,33 +86,28 @@ struct FrameDesc {
 // (20-21), row (0-19).
 constexpr uint32_t row_entry(int l, int r, int row) { return (uint32_t)l << 22 | (uint32_t)r << 20 | (uint32_t)row; }
 
-// A launch's dataflow queue: a task is pushed when its last dependency
-// finishes (the frames' dependency-free tasks are pushed by the host), and
-// warps pop in push order. Slots hold (epoch << 32) | (frame << 24) | task,
-// so a slot of an earlier launch never reads as filled.
+// A launch's queue of rows, AMP units or GIVEN jobs, filled by the host: slots
+// hold (epoch << 32) | (frame << 24) | row or job. The resident engine's
+// queues are rings: a task is pushed when its last dependency finishes (a
+// frame's dependency-free tasks by the engine's publish kernel), and warps
+// pop in push order.
 struct LaunchDesc {
   const FrameDesc* frames;
-  unsigned long long* ready;     // capacity `total`
-  int64_t total;                 // tasks of this launch (= pushes = pops)
+  unsigned long long* ready;     // `total` slots
+  int64_t total;                 // entries of this launch
   unsigned long long* head;      // next slot to pop
-  unsigned long long* tail;      // next slot to push (starts at the host's count)
+  unsigned long long* tail;      // next slot to push (the engine)
   uint32_t* status;
   unsigned long long* counters;  // [tasks, sad, satd, sad_samples, satd_samples]
   const uint32_t* epoch;         // this launch's epoch (device memory: a
                                  // replayed graph keeps its arguments)
-  unsigned long long* done;      // tasks finished, or null: with it a warp
-                                 // runs one task it made ready itself
-                                 // (no queue round trip) and idle warps
-                                 // leave once every task is done
-  // The queue of the tasks a whole CTA runs (32x32 and 64x64 blocks in the
-  // latency form), served by the first `group_ctas` CTAs; 0: none.
+  // The resident engine: the ring of the tasks a whole CTA runs (32x32 and
+  // 64x64 blocks), served by the first `group_ctas` CTAs.
   unsigned long long* ready_big;
   unsigned long long* head_big;
   unsigned long long* tail_big;
   int32_t group_ctas;
-  int32_t patch8;                // the latency form: 8x8 blocks refine from staged phase patches
-  int32_t ring_shift;            // nonzero: the resident engine's ring of
-                                 // 2^ring_shift slots (ring_entry)
+  int32_t ring_shift;            // the engine's rings have 2^ring_shift slots (ring_entry)
 };
 
 // The resident engine (rme_engine.cu): one search kernel that stays on the

@@ -29,9 +29,11 @@
 // Which candidates are scored, in which order they win and how many are
 // counted is the reference's walk (h265_me.rs:3749-3922), as hevc_task runs
 // it with one warp. Search kernel, one B200, before (dataflow or a warp a
-// row, the faster) and now: one 1080p frame of two references 3.8 -> 1.8 ms,
-// 850x478 1.59 -> 0.70 ms, twelve 1080p frames 13.4 -> 8.4 ms, one 2160p
-// 10-bit frame of four references 33 -> 11.7 ms.
+// row, the faster) and now: one 1080p frame of two references 3.8 -> 1.6 ms,
+// 850x478 1.59 -> 0.60 ms, twelve 1080p frames 13.4 -> 7.8 ms, one 2160p
+// 10-bit frame of four references 33 -> 10.4 ms. Rows read by 8-byte loads
+// (fewer passes through L1, more selections) lose 1 to 8 %, the sub-sample
+// planes brought into L1 ahead 0 to 8 %: issue and latency bind, not the loads.
 //
 // A CTA is 256 threads: one row of 64x64 blocks, two of 32x32 or 16x16, four
 // of 8x8. Rows are taken in the order the host pushed them, each after the

@@ -1,6 +1,6 @@
 // The search's device code, shared by the batched kernels (rme_search.cu)
 // and the resident engine (rme_engine.cu): the task functions, the
-// distortion and interpolation-plane reads, the dataflow queue. Each file
+// distortion and interpolation-plane reads, the queues. Each file
 // includes it into its own anonymous namespace. Reads of pictures go
 // through RME_LD32: the read-only cache path in the batched kernels (a
 // launch's pictures do not change while it runs); in the engine, where
@@ -351,7 +351,7 @@ __device__ __forceinline__ const S* plane_at(const DevPlanes& p, int plane, int 
   return (const S*)p.base + (int64_t)plane * p.plane_elems + p.origin + (int64_t)y * p.stride + x;
 }
 
-// ---- dataflow queue ---------------------------------------------------------
+// ---- queues ------------------------------------------------------------------
 
 // A ring slot of the resident engine holds the lap tag of its index (1 to
 // 65535, so that consecutive laps differ and a zeroed slot matches none),
@@ -371,22 +371,17 @@ __device__ __forceinline__ unsigned long long ring_entry(int ring_shift, unsigne
 __device__ __forceinline__ void push_ready(const LaunchDesc& L, int f, int t, bool big = false, uint32_t gen = 0) {
   unsigned long long* const ready = big ? L.ready_big : L.ready;
   const unsigned long long idx = atomicAdd(big ? L.tail_big : L.tail, 1ull);
-  if (L.ring_shift) {  // the engine's ring: the host keeps fewer tasks in flight than it has slots
-    st_release64(ready + (idx & ((1ull << L.ring_shift) - 1ull)), ring_entry(L.ring_shift, idx, gen, f, t));
-  } else if (idx < (unsigned long long)L.total)
-    st_release64(ready + idx, ((unsigned long long)__ldg(L.epoch) << 32) | ((uint32_t)f << 24) | (uint32_t)t);
-  else
-    atomicOr(L.status, kStatusBadTask);
+  // The host keeps fewer tasks in flight than the ring has slots.
+  st_release64(ready + (idx & ((1ull << L.ring_shift) - 1ull)), ring_entry(L.ring_shift, idx, gen, f, t));
 }
 
 __device__ __forceinline__ bool group_task_of(const LaunchDesc& L, const FrameDesc& F, int t);
 
 // A finished task's dependents, task `dtask` in each lane where `rel`
 // (all lanes call): each decrement that reaches zero makes its task ready.
-// Where the launch counts finished tasks, the warp keeps the first task made
-// ready (lowest lane) to run next itself, saving the push, the pop and the
-// hand-over to another warp, unless `cont` already holds one; the others are
-// pushed. Returns `cont`, updated.
+// The warp keeps the first task made ready (lowest lane) to run next itself,
+// saving the push, the pop and the hand-over to another warp, unless `cont`
+// already holds one; the others are pushed. Returns `cont`, updated.
 // Tasks a CTA runs go to their own queue; a warp keeps only a task of its
 // own kind (`group`: the caller is a CTA).
 __device__ __forceinline__ int release_lanes(const LaunchDesc& L, const FrameDesc& F, int f, bool rel, int dtask,
@@ -396,7 +391,7 @@ __device__ __forceinline__ int release_lanes(const LaunchDesc& L, const FrameDes
   const uint32_t m = __ballot_sync(kFull, ready && big == group);
   if (__ballot_sync(kFull, ready) == 0u) return cont;
   int keep = -1;
-  if (m != 0u && cont == -1 && (L.done != nullptr || L.ring_shift)) {
+  if (m != 0u && cont == -1) {
     keep = __ffs(m) - 1;
     cont = (f << 24) | __shfl_sync(kFull, dtask, keep);
   }
@@ -447,17 +442,14 @@ __device__ __forceinline__ unsigned long long mv_word(uint32_t tag, int mvx, int
 
 constexpr uint32_t kPopDone = 0xfffffffeu;  // every task of the launch is done
 
-// The entry in slot `idx` once pushed (lane 0; bounded wait with backoff),
-// kPopDone once every task is done (a slot that will never be filled: the
-// warps that ran tasks they made ready pushed fewer than `total`), or
-// 0xffffffff when the wait runs out (status set).
-__device__ __forceinline__ uint32_t pop_slot(const LaunchDesc& L, unsigned long long idx, uint32_t epoch,
-                                             bool big = false) {
+// The entry in slot `idx` of a launch's queue, which the host filled
+// (lane 0; bounded wait with backoff), or 0xffffffff when the wait runs out
+// (status bit set).
+__device__ __forceinline__ uint32_t pop_slot(const LaunchDesc& L, unsigned long long idx, uint32_t epoch) {
   uint32_t ns = 32, it = 0;
   for (;;) {
-    const unsigned long long v = ld_acquire64((big ? L.ready_big : L.ready) + idx);
+    const unsigned long long v = ld_acquire64(L.ready + idx);
     if ((uint32_t)(v >> 32) == epoch) return (uint32_t)v;
-    if (L.done != nullptr && (it & 3u) == 3u && ld_relaxed64(L.done) >= (unsigned long long)L.total) return kPopDone;
     if (++it >= kSpinLimit) {
       atomicOr(L.status, kStatusWaitTimeout);
       return 0xffffffffu;
@@ -643,7 +635,7 @@ __device__ __forceinline__ uint32_t satd_part(const uint32_t* src, int wr, int t
   return acc;
 }
 
-// ---- 8x8 sub-sample refinement from staged phase patches (latency form) ----
+// ---- 8x8 sub-sample refinement from staged phase patches -----------------
 //
 // refine_subpel around a whole-sample best B only ever reads quarter-sample
 // positions B + (qx, qy) with qx, qy in -3..3 (the half ring at +-2, then the
@@ -805,12 +797,12 @@ __device__ __forceinline__ void prefetch_l1(const void* p) {
   asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
-// Returns a task it made ready to run next (frame << 24 | task), or -1.
-// SPEC: the latency kernels' two-rounds-per-step 8x8 and 16x16 diamond.
+// A STANDALONE frame's task (the resident engine's). Returns a task it made
+// ready to run next (frame << 24 | task), or -1.
 // ROW: the row form (the neighbours' vectors from their published words,
 // this task's published in turn; nothing released), at `rp` in its row,
 // blocks of NB samples (0: the level's size read at run time).
-template <class S, bool SPEC, bool ROW = false, int NB = 0>
+template <class S, bool ROW = false, int NB = 0>
 __device__ int hevc_task(const LaunchDesc& L, const FrameDesc& F, int f, int t, WarpSmem<S>& sm, int lane,
                          RowPos* rp = nullptr) {
   int r, x, y, w, h, ns;
@@ -819,28 +811,7 @@ __device__ int hevc_task(const LaunchDesc& L, const FrameDesc& F, int f, int t, 
   int l = 0, lbx = 0, lby = 0, local = 0;  // STANDALONE: level and block
   bool amp_unit = false;                   // STANDALONE: an AMP unit
   rme_result* out;
-  if (!ROW && F.mode == RME_PRED_GIVEN) {
-    const rme_job* j = &F.jobs[t];
-    if (!given_job_ok(F, j, RME_MAX_SEEDS)) {
-      if (lane == 0) atomicOr(L.status, kStatusBadTask);
-      return -1;
-    }
-    r = j->ref;
-    x = j->x;
-    y = j->y;
-    w = j->w;
-    h = j->h;
-    ns = j->nseeds;
-    p0x = j->mvp[0].x;
-    p0y = j->mvp[0].y;
-    p1x = j->mvp[1].x;
-    p1y = j->mvp[1].y;
-    if (lane < ns) {
-      sx = j->seeds[lane].x;
-      sy = j->seeds[lane].y;
-    }
-    out = &F.out[t];
-  } else if (ROW) {
+  if (ROW) {
     r = rp->r;
   } else {
     r = t % F.nref;
@@ -885,7 +856,7 @@ __device__ int hevc_task(const LaunchDesc& L, const FrameDesc& F, int f, int t, 
     sx = lane == 0 || lane == 1 ? p0x : 0;
     sy = lane == 0 || lane == 1 ? p0y : 0;
     out = &F.out[t];
-  } else if (ROW || F.mode != RME_PRED_GIVEN) {
+  } else {
     if (ROW) {
       l = rp->l;
       lbx = rp->lbx;
@@ -958,19 +929,13 @@ __device__ int hevc_task(const LaunchDesc& L, const FrameDesc& F, int f, int t, 
     out = &F.out[t];
   }
   const DevPlanes& R = F.ref[r];
-  if (!ROW && F.mode == RME_PRED_GIVEN) {
-    if (F.bi_src)  // refine_bi: the target block stands in for the source
-      stage_src<S>(sm.src, (const S*)F.bi_src + (int64_t)t * (kBiBlock * kBiBlock), kBiBlock, w, h, lane);
-    else
-      stage_src<S>(sm.src, plane_at<S>(F.src, 0, x, y), F.src.stride, w, h, lane);
-  }
   const S* org = plane_at<S>(R, 0, x, y);
   const int stride = R.stride;
   constexpr int SPW = 4 / sizeof(S);
   const int wr = w / SPW, tw = w >> 2, th = h >> 2;
   const int padm = F.pad - 4;  // h265_search.rs MARGIN
   const int lox = -padm - x, hix = F.width + padm - w - x, loy = -padm - y, hiy = F.height + padm - h - y;
-  const float lam = F.bi_src ? 2.0f * F.lam : F.lam;  // refine_bi weighs the rate at 2 * lam
+  const float lam = F.lam;
   uint32_t nsad = 0, nsatd = 0;
 
   // Seeds: >> 2, clamp_pos, dedupe (a seed equal to an earlier one is
@@ -998,7 +963,7 @@ __device__ int hevc_task(const LaunchDesc& L, const FrameDesc& F, int f, int t, 
   uint32_t bcost = kInf;
   int state = nk > 0 ? 0 : 1, c0 = 0, it = 0, rings = 0;
   bool moved = false;
-  const bool spec = SPEC && w == h && (w == 8 || w == 16);
+  const bool spec = w == h && (w == 8 || w == 16);
   for (;;) {
     if (state == 1 && it >= 2 * range) {  // the diamond has settled
       if (rings >= F.search_rings) break;
@@ -1010,12 +975,9 @@ __device__ int hevc_task(const LaunchDesc& L, const FrameDesc& F, int f, int t, 
       cyr = by;
     }
     if (spec && state == 1) {
-      // 8x8 and 16x16 in a latency kernel: two diamond rounds per step, fewer
-      // dependent steps on the frame's critical path for more loads per step
-      // (the throughput kernels keep one round per step, and leave this code
-      // out of their text).
-      // Candidates 0..3 (two lanes each)
-      // are the round around the best; 4..15 the next round's points for
+      // 8x8 and 16x16: two diamond rounds per step, fewer dependent steps on
+      // the frame's critical path for more loads per step. Candidates 0..3
+      // (two lanes each) are the round around the best; 4..15 the next round's points for
       // each way the first can move — three new ones each, the fourth being
       // the best itself, whose cost is known and cannot win. The outcome
       // and the count are those of the two rounds taken one after another.
@@ -1129,7 +1091,7 @@ __device__ int hevc_task(const LaunchDesc& L, const FrameDesc& F, int f, int t, 
   const int ntiles = tw * th;
   // Patches need every plane and row a whole number of words apart (true
   // of the library's pictures: 128-byte strides).
-  if (spec && w == 8 && L.patch8 && ((R.stride * (int)sizeof(S)) & 3) == 0 &&
+  if (spec && w == 8 && ((R.stride * (int)sizeof(S)) & 3) == 0 &&
       ((R.plane_elems * (int64_t)sizeof(S)) & 3) == 0) {
     refine8_patched<S>(sm, R, x, y, bx, by, lam, p0x, p0y, p1x, p1y, F.quarter_cross, lane, bmx, bmy, bc, bsatd,
                        nsatd);
@@ -1168,7 +1130,7 @@ __device__ int hevc_task(const LaunchDesc& L, const FrameDesc& F, int f, int t, 
   int cont = -1;
   if (ROW) {
     if (lane == 0) st_relaxed64(F.mvf + t, mv_word(F.tag, bmx, bmy));
-  } else if (!ROW && F.mode != RME_PRED_GIVEN && !amp_unit) {
+  } else if (!amp_unit) {
     // The tasks reading this result: right and lower neighbours of this
     // level, the blocks of the next evaluated size inside this one, this
     // CU's AMP units; each lane releases one of them. Lane 0's result is
@@ -1206,11 +1168,11 @@ __device__ int hevc_task(const LaunchDesc& L, const FrameDesc& F, int f, int t, 
   return cont;
 }
 
-// ---- HEVC, large blocks: one CTA per task (latency form) ----------------------
+// ---- HEVC, large blocks: one CTA per task -------------------------------------
 //
 // A 32x32 or 64x64 block's search is the longest dependent chain of a
 // frame (its level's wavefront has few blocks in flight, each of 1-4 K
-// samples per candidate), so in the latency form a whole CTA runs one: the
+// samples per candidate), so in the resident engine a whole CTA runs one: the
 // 256 threads split every step's candidate rows (SAD, a lane per word of a
 // row: coalesced) or 4x4 tiles (SATD), each warp's sum is added into the
 // candidate's cost in shared memory, and after one barrier every thread
@@ -1691,7 +1653,7 @@ __device__ __forceinline__ bool row_ok(const FrameDesc& F, uint32_t e, int& l, i
          l < F.nlevels && r < F.nref && row < F.nby[l];
 }
 
-template <class S, bool SPEC>
+template <class S>
 __device__ void hevc_row(const LaunchDesc& L, const FrameDesc& F, int f, uint32_t e, WarpSmem<S>& sm, int lane) {
   int l, r, row;
   if (!row_ok(F, e, l, r, row) || (F.size[l] != 8 && F.size[l] != 16)) {
@@ -1703,12 +1665,12 @@ __device__ void hevc_row(const LaunchDesc& L, const FrameDesc& F, int f, uint32_
   if (F.size[l] == 8)
     for (int bx = 0; bx < nbx; ++bx) {
       rp.lbx = bx;
-      hevc_task<S, SPEC, true, 8>(L, F, f, t0 + bx * F.nref, sm, lane, &rp);
+      hevc_task<S, true, 8>(L, F, f, t0 + bx * F.nref, sm, lane, &rp);
     }
   else
     for (int bx = 0; bx < nbx; ++bx) {
       rp.lbx = bx;
-      hevc_task<S, SPEC, true, 16>(L, F, f, t0 + bx * F.nref, sm, lane, &rp);
+      hevc_task<S, true, 16>(L, F, f, t0 + bx * F.nref, sm, lane, &rp);
     }
 }
 

@@ -6,9 +6,7 @@
 //   RME_SERVE_LAUNCHES: the frames admitted since the last launch go into
 //   one search launch of their own as soon as one of kLaunchStreams launch
 //   streams is free, so launches overlap on the device (a frame that
-//   arrives while others are searched starts at once on another stream); a
-//   launch of one or two 1080p frames runs the latency form (the row form
-//   for HEVC), a larger one the throughput form.
+//   arrives while others are searched starts at once on another stream).
 //
 //   RME_SERVE_RESIDENT: frames join the resident engine's running search
 //   (rme_engine.cu) behind their uploads, as soon as a frame slot and ring
