@@ -912,7 +912,7 @@ def run_configs(local: int = 0):
     def measure(name, frames, params, note):
         total = ms.batch_result_count(frames, params)
         dev = torch.empty(total * capi.RESULT_DTYPE.itemsize, dtype=torch.uint8, device=f"cuda:{local}")
-        for _ in range(8):  # the tuner's six trials, the graph's capture, one more
+        for _ in range(8):  # the first calls, the graph's capture, a few more
             outs = ms.search_batch(frames, params, 0, out=dev)
         torch.cuda.synchronize()
         ks = []
@@ -1014,7 +1014,7 @@ def other_configs(local: int = 0) -> dict:
         frames = [(100 + t, [100 + t - 1 - r for r in range(4)]) for t in range(4, 12)]
         total = ms.batch_result_count(frames, p2)
         dev = torch.empty(total * capi.RESULT_DTYPE.itemsize, dtype=torch.uint8, device=f"cuda:{local}")
-        for _ in range(8):  # the tuner's six trials, the graph's capture, one more
+        for _ in range(8):  # the first calls, the graph's capture, a few more
             outs = ms.search_batch(frames, p2, 0, out=dev)
         ks = []
         for _ in range(3):

@@ -140,25 +140,6 @@ __device__ __forceinline__ bool wait_word(const unsigned long long* p, unsigned 
   return true;
 }
 
-// Eight bytes of a row at any byte address (three aligned loads).
-__device__ __forceinline__ void ld8(const uint8_t* p, uint32_t& a, uint32_t& b) {
-  const uintptr_t u = reinterpret_cast<uintptr_t>(p);
-  const uint32_t* q = reinterpret_cast<const uint32_t*>(u & ~uintptr_t(3));
-  const uint32_t sh = (uint32_t)(u & 3) * 8u;
-  const uint32_t w0 = __ldg(q), w1 = __ldg(q + 1), w2 = __ldg(q + 2);
-  a = __funnelshift_r(w0, w1, sh);
-  b = __funnelshift_r(w1, w2, sh);
-}
-
-struct Pick2 {
-  uint32_t cost;
-  int lane;
-};
-__device__ __forceinline__ Pick2 argmin(uint32_t c) {
-  const uint32_t m = __reduce_min_sync(kAll, c);
-  return {m, __ffs(__ballot_sync(kAll, c == m)) - 1};
-}
-
 // |a - b| of four bytes, summed onto acc.
 __device__ __forceinline__ uint32_t sad4(uint32_t a, uint32_t b, uint32_t acc) {
   uint32_t r;
@@ -461,32 +442,53 @@ __global__ void lowres_intra_h264_kernel(LowresDesc L) {
 // four for u16), from aligned loads.
 template <class S>
 struct Row8;
+// By 8-byte loads (as lowres_search_kernel), one more than the row may need:
+// a plane's memory goes on behind its last row. (Left out where the row is
+// aligned, the predicate costs more than the load: 564 us against 491 for
+// eight 8-bit 1080p pairs.)
+template <int N>
+__device__ __forceinline__ void load_words(const void* p, uint32_t (&out)[N]) {
+  const uintptr_t u = reinterpret_cast<uintptr_t>(p);
+  const uint2* q = reinterpret_cast<const uint2*>(u & ~uintptr_t(7));
+  const uint32_t sh = (uint32_t)(u & 3) * 8u;
+  const bool up = u & 4;
+  uint32_t w[N + 2] = {};
+#pragma unroll
+  for (int i = 0; i <= N / 2; ++i) {
+    const uint2 v = __ldg(q + i);
+    w[2 * i] = v.x;
+    w[2 * i + 1] = v.y;
+  }
+  uint32_t t[N + 1];
+#pragma unroll
+  for (int i = 0; i <= N; ++i) t[i] = up ? w[i + 1] : w[i];
+#pragma unroll
+  for (int i = 0; i < N; ++i) out[i] = __funnelshift_r(t[i], t[i + 1], sh);
+}
+// |a - b| of two 16-bit halves, summed onto acc: the larger less the smaller
+// of each and a dot product with ones.
+__device__ __forceinline__ uint32_t sad2(uint32_t a, uint32_t b, uint32_t acc) {
+  uint32_t hi, lo;
+  asm("max.u16x2 %0, %1, %2;" : "=r"(hi) : "r"(a), "r"(b));
+  asm("min.u16x2 %0, %1, %2;" : "=r"(lo) : "r"(a), "r"(b));
+  return __dp2a_lo(hi - lo, 0x0101u, acc);
+}
 template <>
 struct Row8<uint8_t> {
   uint32_t w[2];
-  __device__ __forceinline__ void load(const uint8_t* p) {
-    uint32_t a, b;
-    ld8(p, a, b);
-    w[0] = a;
-    w[1] = b;
+  __device__ __forceinline__ void load(const uint8_t* p) { load_words<2>(p, w); }
+  __device__ __forceinline__ uint32_t sad(const Row8& o, uint32_t acc) const {
+    return sad4(w[1], o.w[1], sad4(w[0], o.w[0], acc));
   }
-  __device__ __forceinline__ uint32_t sad(const Row8& o) const { return __vsadu4(w[0], o.w[0]) + __vsadu4(w[1], o.w[1]); }
 };
 template <>
 struct Row8<uint16_t> {
   uint32_t w[4];
-  __device__ __forceinline__ void load(const uint16_t* p) {
-    const uintptr_t u = reinterpret_cast<uintptr_t>(p);
-    const uint32_t* q = reinterpret_cast<const uint32_t*>(u & ~uintptr_t(3));
-    const uint32_t sh = (uint32_t)(u & 3) * 8u;
-    uint32_t v[5];
+  __device__ __forceinline__ void load(const uint16_t* p) { load_words<4>(p, w); }
+  __device__ __forceinline__ uint32_t sad(const Row8& o, uint32_t acc) const {
 #pragma unroll
-    for (int i = 0; i < 5; ++i) v[i] = __ldg(q + i);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = __funnelshift_r(v[i], v[i + 1], sh);
-  }
-  __device__ __forceinline__ uint32_t sad(const Row8& o) const {
-    return __vsadu2(w[0], o.w[0]) + __vsadu2(w[1], o.w[1]) + __vsadu2(w[2], o.w[2]) + __vsadu2(w[3], o.w[3]);
+    for (int i = 0; i < 4; ++i) acc = sad2(w[i], o.w[i], acc);
+    return acc;
   }
 };
 
@@ -500,7 +502,10 @@ struct Row8<uint16_t> {
 // each point, the first least cost taken when strictly below the best (the
 // reference's in-order scoring). A pass scores a hexagon step (candidates
 // 0..5) together with the square around the same centre (6..13), which is
-// the walk's last step when the hexagon has settled there.
+// the walk's last step when the hexagon has settled there. As
+// lowres_search_kernel a chain of steps: eight 1080p pairs 553 us with rows by
+// words, ballots and shuffles, 491 us with 8-byte loads and decisions by keys;
+// eight 10-bit 720p pairs 505 -> 369 us.
 template <class S>
 __global__ void __launch_bounds__(kLaWarps * 32) lowres_search_h264_kernel(const LowresDesc* pairs, int npairs,
                                                                            unsigned long long* words_all,
@@ -511,9 +516,9 @@ __global__ void __launch_bounds__(kLaWarps * 32) lowres_search_h264_kernel(const
   const int bw = pairs[0].bw, bh = pairs[0].bh, n = bw * bh, lim = kLowresPad - 8;
   // This lane's offset from the centre: a point of the hexagon or of the
   // 3x3 square without its centre.
-  const int sk = q - 6 < 4 ? q - 6 : q - 5;
-  const int ofx = q == 0 ? -2 : q == 1 ? -1 : q == 2 ? 1 : q == 3 ? 2 : q == 4 ? 1 : q == 5 ? -1 : sk % 3 - 1;
-  const int ofy = q == 0 || q == 3 ? 0 : q < 3 ? -2 : q < 6 ? 2 : sk / 3 - 1;
+  auto off_x = [](int k) { return (int)((0x32131321134310ull >> (4 * k)) & 15u) - 2; };
+  auto off_y = [](int k) { return (int)((0x33322111442002ull >> (4 * k)) & 15u) - 2; };
+  const int ofx = off_x(min(q, 13)), ofy = off_y(min(q, 13));
   bool lost = false;
   for (int pi, by; claim_row(counter, npairs, bh, lane, pi, by);) {
     const LowresDesc cur = pairs[2 * pi], ref = pairs[2 * pi + 1];
@@ -541,14 +546,15 @@ __global__ void __launch_bounds__(kLaWarps * 32) lowres_search_h264_kernel(const
       if (by > 0 && bx + 1 < bw) un = ld_word(up + bx + 1);
       const int lx = max(-x - lim, -2 * kLowresRange), hx = min(cur.pw - 8 - x + lim, 2 * kLowresRange);
       auto score = [&](bool ok, int dx, int dy) -> uint32_t {
-        uint32_t part = 0;
+        uint32_t part = 0, odd = 0;
         if (ok) {
           Row8<S> a[4];
 #pragma unroll
           for (int r = 0; r < 4; ++r) a[r].load(rb + (ptrdiff_t)(dy + r) * ref.stride + dx);
 #pragma unroll
-          for (int r = 0; r < 4; ++r) part += s[r].sad(a[r]);
+          for (int r = 0; r < 4; ++r) (r & 1 ? odd : part) = s[r].sad(a[r], r & 1 ? odd : part);
         }
+        part += odd;
         part += __shfl_xor_sync(kAll, part, 1);
         return ok ? part + 2u * (uint32_t)min(abs(dx) + abs(dy), 64) : 0xffffffffu;
       };
@@ -578,31 +584,36 @@ __global__ void __launch_bounds__(kLaWarps * 32) lowres_search_h264_kernel(const
           bym = c1y;
         }
       }
-      uint32_t live = 0x3f;  // the hexagon's new points
+      uint32_t live = 0x3f, lsad = 0;  // the hexagon's new points; this lane's points scored (two lanes a point)
       for (int it = 0;; ++it) {
         dx = bxm + ofx;
         dy = bym + ofy;
         const bool ok = (q < 6 ? it < kLowresRange && ((live >> q) & 1) : q < 14) && inwin(dx, dy);
         const uint32_t cost = score(ok, dx, dy);
-        nsad += __popc(__ballot_sync(kAll, ok && q < 6 && half == 0));
-        Pick2 p = argmin(q < 6 ? cost : 0xffffffffu);
-        const bool step = p.cost < bc;
+        // Keys of cost and place: the minimum is the decision. (A cost is below
+        // 2^19: 64 differences of at most 4095 and a penalty of 128.)
+        const uint32_t key = ok ? cost << 4 | (uint32_t)q : 0xffffffffu;
+        uint32_t m = __reduce_min_sync(kAll, q < 6 ? key : 0xffffffffu);
+        lsad += ok && q < 6;
+        const bool step = m >> 4 < bc;
         if (!step) {  // settled: the square around the hexagon's centre
-          nsad += __popc(__ballot_sync(kAll, ok && q >= 6 && half == 0));
-          p = argmin(q >= 6 ? cost : 0xffffffffu);
+          lsad += ok && q >= 6;
+          m = __reduce_min_sync(kAll, q < 6 ? 0xffffffffu : key);
         }
-        if (p.cost < bc) {
-          bc = p.cost;
-          bxm = __shfl_sync(kAll, dx, p.lane);
-          bym = __shfl_sync(kAll, dy, p.lane);
+        const int k = (int)(m & 15u);
+        if (m >> 4 < bc) {
+          bc = m >> 4;
+          bxm += off_x(k);
+          bym += off_y(k);
         }
         if (!step) break;
-        const uint32_t r = 7u << ((p.lane >> 1) + 5);
+        const uint32_t r = 7u << (k + 5);
         live = (r | r >> 6 | r >> 12) & 0x3f;
       }
       lv = (uint32_t)(uint16_t)(int16_t)bxm | (uint32_t)(uint16_t)(int16_t)bym << 16;
+      if (lane == 0) st_word(words + bx, lv);
+      nsad += __reduce_add_sync(kAll, lsad) >> 1;
       if (lane == 0) {
-        st_word(words + bx, lv);
         const size_t o = (size_t)pi * n + (size_t)by * bw + bx;
         *reinterpret_cast<uint32_t*>(mv_all + o) = lv;
         nsad_all[o] = nsad;

@@ -209,25 +209,22 @@ __device__ __forceinline__ void ldwords(const void* p, uint32_t (&out)[N]) {
 
 // The same by 8-byte loads, for lanes on lines of their own: each load is then
 // up to 32 passes through L1, and a row of eight bytes takes two instead of
-// three, one of sixteen three instead of five. Reads no 8-byte word that holds
-// none of the bytes.
+// three, one of sixteen three instead of five. Reads up to 8 bytes behind the
+// last one: for the library's own pictures, whose memory goes on.
 template <int N>
 __device__ __forceinline__ void ldrow(const void* p, uint32_t (&out)[N]) {
+  static_assert(N % 2 == 0, "whole 8-byte words");
   const uintptr_t a = reinterpret_cast<uintptr_t>(p);
   const uint2* q = reinterpret_cast<const uint2*>(a & ~uintptr_t(7));
   const uint32_t sh = (uint32_t)(a & 3) * 8u;
   const bool up = a & 4;
-  constexpr int M = N / 2 + 1;  // 8-byte words; the last one's second half only where N is odd
-  uint32_t w[2 * M + 1] = {};
+  uint32_t w[N + 2], t[N + 1];
 #pragma unroll
-  for (int i = 0; i < M; ++i) {
-    if (i == M - 1 && N % 2 == 0 && (a & 7) == 0) break;
+  for (int i = 0; i <= N / 2; ++i) {
     const uint2 v = RME_LD64(q + i);
     w[2 * i] = v.x;
     w[2 * i + 1] = v.y;
   }
-  if (N % 2 == 1 && (a & 7) > 4) w[2 * M] = RME_LD32(reinterpret_cast<const uint32_t*>(q + M));
-  uint32_t t[N + 1];
 #pragma unroll
   for (int i = 0; i <= N; ++i) t[i] = up ? w[i + 1] : w[i];
 #pragma unroll
