@@ -23,8 +23,11 @@
 // went a word at a time; AMP units waited in its queue): the 680,160 AMP units
 // of a 2160p 10-bit frame, four references, 7.0 ms, with the frame's 2Nx2N
 // rows 17.5 ms for 45; 6,000 mixed 10-bit GIVEN jobs 0.76 -> 0.27 ms (a warp
-// each: 0.60), 600 of 8 bits 0.06 (0.21), 20,000 of 8 bits 0.48. Five or six
-// CTAs an SM (spills) gain at most 2 % and lose up to 7.
+// each: 0.60), 600 of 8 bits 0.06 (0.21), 20,000 of 8 bits 0.48. Lists of one
+// shape, 8 and 10 bits: 8,040 16x16 jobs 109 -> 91 and 189 -> 115 us, 480 64x64
+// 241 -> 63 and 517 -> 102; 20,000 8x8, whose 16 words leave half of a warp
+// idle, 95 -> 113 and 145 -> 126. Five or six CTAs an SM (spills) gain at most
+// 2 % and lose up to 7.
 #include <algorithm>
 
 #include "rme_search_impl.cuh"
