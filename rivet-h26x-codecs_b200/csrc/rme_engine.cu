@@ -109,9 +109,9 @@ __global__ void reset_heads_kernel(LaunchDesc L, uint32_t* stop) {
 }
 
 // Registers: at most 112 a thread, so that the grid's two blocks per SM
-// (57,344 registers) leave 8,192 on every SM to the kernels that run beside
-// the resident one (plane builds in blocks of 128 threads, frame
-// preparation and publication, each within that share). With 128, the
+// (57,344 registers) leave 8,192 on every SM, 2,048 on each of its four
+// schedulers, to the kernels that run beside the resident one (plane builds,
+// frame preparation and publication): a warp of at most 64 a thread. With 128, the
 // engine would take every register of every SM, those kernels could not
 // start until it left, and it leaves only once no frame is in flight: the
 // frames queued behind them would never arrive.
