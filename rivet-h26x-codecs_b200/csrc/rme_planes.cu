@@ -294,8 +294,8 @@ __device__ __forceinline__ void phase_columns(const S* g, S* planes, int64_t pla
 // it left, and it waits for the planes). Bound by issue: about 5 instructions
 // an output sample, where a multiply-add per tap and the passes' round trip
 // through shared memory took about 50. One 1080p reference 61 -> 21 us, one of
-// 2160p at 10 bits 203 -> 86 us (3.2 TB/s written), one of 360p 13 -> 8 us; up
-// to 94 registers gave the same but at 1080p and 10 bits (26 us against 31).
+// 2160p at 10 bits 203 -> 85 us (3.3 TB/s written), one of 360p 13 -> 8 us; up
+// to 94 registers, with half as many warps an SM, were no faster.
 template <class S>
 __global__ void __launch_bounds__(64, 16) hevc_phase_kernel(const S* g, S* planes, int64_t plane_elems, int stride,
                                                             int prow, int pcol, int bd, int strip) {
@@ -346,13 +346,14 @@ cudaError_t launch_h264_hpel(DevPlanes p, int bd, int cw, int ch, int pad, cudaS
 
 cudaError_t launch_hevc_phases(DevPlanes p, int bd, int w, int h, int pad, cudaStream_t s) {
   int prow = h + 2 * pad, pcol = w + 2 * pad;
-  // Strips as long as one wave of warps allows (16 an SM), 8 to 64 rows: a
+  // Strips as long as one wave of warps allows (32 an SM), 8 to 64 rows: a
   // strip filters seven rows more than it writes, and a second wave that is
-  // nearly empty costs as much as the first.
+  // nearly empty costs as much as the first (strips for half a wave: 1080p at
+  // 10 bits 30.9 us against 26.7, 2160p 58.7 against 57.4).
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int cols = (pcol + kPhaseTX - 1) / kPhaseTX, strips = std::max(1, nsm * 16 / (4 * cols));
+  const int cols = (pcol + kPhaseTX - 1) / kPhaseTX, strips = std::max(1, nsm * 32 / (4 * cols));
   const int strip = std::min(64, std::max(8, (prow + strips - 1) / strips));
   dim3 blk(64), grd(cols, (prow + strip - 1) / strip, 2);
   prefer_max_shared(hevc_phase_kernel<uint8_t>);
