@@ -713,7 +713,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   CK(sl.d_jobs.ensure(std::max<int64_t>(jobs_off[n], 1)));
   if (!dev_out && !pinned_out) CK(sl.h_out.ensure(std::max<int64_t>(total, 1)));
   CK(sl.h_misc.ensure(kMiscWords));
-  if (sl.epoch == 0 || sl.epoch >= 0x3fffffffu) {  // 30 bits: an H.264 word's tag holds a reference beside it
+  if (sl.epoch == 0 || sl.epoch >= 0x3fffffffu) {  // 30 bits: a word's tag holds two more (a reference)
     CK(cudaMemsetAsync(sl.d_mvf.p, 0, sl.d_mvf.n * sizeof(unsigned long long), s));
     sl.epoch = 0;
   }
@@ -760,9 +760,12 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     int rc = 0;
     fdeps[i] = get_deps(c, src->d, &params[i], frames[i].nref, &rc);
     if (!fdeps[i]) return rc;
-    // A search of this buffer tags its published words anew.
+    // A search of this buffer tags its published words anew: the epoch over
+    // two bits, which hold an H.264 word's reference and are zero in HEVC's.
+    // Both codecs' words lie in this buffer and outlive their launch, so a tag
+    // must not be another epoch's of either codec.
     fd.mvf = sl.d_mvf.p + toff[i];
-    fd.tag = fd.codec == RME_CODEC_H264 ? sl.epoch << 2 : sl.epoch;
+    fd.tag = sl.epoch << 2;
     if (fd.amp) {
       const int64_t big = fd.size[0] == 64 ? (int64_t)(fd.amp_base[1] - fd.amp_base[0]) * fd.nref : 0;
       amp_tasks[k][1] += big;

@@ -78,7 +78,7 @@ struct FrameDesc {
   // the rows below and the next size's rows wait for. Null: a frame of the
   // engine's tasks.
   unsigned long long* mvf;
-  uint32_t tag;     // nonzero, new for every search of the buffer (the launch's epoch, the slot's generation)
+  uint32_t tag;     // nonzero, new for every search of the buffer (the launch's epoch << 2, the slot's generation)
   int32_t nrows;    // rows of the frame, both kinds (the engine counts them to completion)
 };
 
