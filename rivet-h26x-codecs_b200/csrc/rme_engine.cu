@@ -440,6 +440,11 @@ int engine_create(void* ctx, int device, Engine** out) {
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g->ctl, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g->kstream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g->ended, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = load_plane_kernels();
+  if (e == cudaSuccess) e = load_kernel(prepare_kernel);
+  if (e == cudaSuccess) e = load_kernel(publish_kernel);
+  if (e == cudaSuccess) e = load_kernel(publish_rows_kernel);
+  if (e == cudaSuccess) e = load_kernel(reset_heads_kernel);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     engine_destroy(g);

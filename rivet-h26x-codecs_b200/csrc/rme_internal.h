@@ -178,6 +178,17 @@ inline cudaError_t prefer_max_shared(K* kernel) {
                               (int)cudaSharedmemCarveoutMaxShared);
 }
 
+// Brings a kernel's code onto the device (by default the runtime does so at
+// its first use, and that may wait for the whole device: for ever, while a
+// resident search runs that itself waits for the kernel). The engine loads
+// every kernel that runs beside it before it starts.
+template <class K>
+inline cudaError_t load_kernel(K* kernel) {
+  cudaFuncAttributes a;
+  return cudaFuncGetAttributes(&a, kernel);
+}
+cudaError_t load_plane_kernels();  // the uploads' (rme_planes.cu)
+
 // Launch wrappers (defined in the .cu files).
 cudaError_t launch_pad_plane(const void* src, int bd, int w, int h, int sstride, DevPlanes dst, int ch, int pad,
                              cudaStream_t s);

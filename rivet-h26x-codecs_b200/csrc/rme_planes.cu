@@ -311,6 +311,16 @@ __global__ void __launch_bounds__(64, 16) hevc_phase_kernel(const S* g, S* plane
 
 }  // namespace
 
+cudaError_t load_plane_kernels() {
+  cudaError_t e = load_kernel(pad_plane_kernel<uint8_t>);
+  if (e == cudaSuccess) e = load_kernel(pad_plane_kernel<uint16_t>);
+  if (e == cudaSuccess) e = load_kernel(h264_hpel_kernel<uint8_t>);
+  if (e == cudaSuccess) e = load_kernel(h264_hpel_kernel<uint16_t>);
+  if (e == cudaSuccess) e = load_kernel(hevc_phase_kernel<uint8_t>);
+  if (e == cudaSuccess) e = load_kernel(hevc_phase_kernel<uint16_t>);
+  return e;
+}
+
 cudaError_t launch_pad_plane(const void* src, int bd, int w, int h, int sstride, DevPlanes dst, int ch, int pad,
                              cudaStream_t s) {
   const int prow = ch + 2 * pad, bps = bd == 8 ? 1 : 2, chunks = dst.stride * bps / 16;
