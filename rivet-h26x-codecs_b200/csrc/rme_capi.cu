@@ -705,11 +705,12 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   for (int i = 0; i < n; ++i)
     if (ntask[i] >= (1 << 24)) return fail(c, RME_EINVAL, "more than 2^24 tasks in one frame");
   if (!dev_out) CK(sl.d_out.ensure(std::max<int64_t>(total, 1)));
-  unsigned long long* old_mvf = sl.d_mvf.p;
+  const size_t old_words = sl.d_mvf.n;
   CK(sl.d_mvf.ensure(std::max<int64_t>(total, 1)));
-  // Fresh slot memory may hold any word, an epoch's among them: zero it
-  // (epochs start at 1).
-  if (sl.d_mvf.p != old_mvf) sl.epoch = 0;
+  // Fresh slot memory may hold any word, an epoch's among them (another
+  // slot's old buffer): zero it (epochs start at 1). A larger buffer may
+  // begin where the old one did, so its size tells that it is new.
+  if (sl.d_mvf.n != old_words) sl.epoch = 0;
   CK(sl.d_jobs.ensure(std::max<int64_t>(jobs_off[n], 1)));
   if (!dev_out && !pinned_out) CK(sl.h_out.ensure(std::max<int64_t>(total, 1)));
   CK(sl.h_misc.ensure(kMiscWords));

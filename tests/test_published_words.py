@@ -67,3 +67,25 @@ def test_frames_of_both_codecs_change_places_from_call_to_call():
             got = ms.search_batch([frames[i] for i in order], [params[i] for i in order])
             for i, g in zip(order, got):
                 assert_results_equal(g, want[i], f"call {call}, frame {i} of {list(order)}")
+
+
+@pytest.mark.gpu
+def test_a_buffer_that_grows_where_it_stood_holds_no_earlier_words():
+    """Two hundred contexts whose launches grow by small steps, the four
+    slots' buffers at different calls: a larger buffer may begin where the old
+    one did and end over another slot's old words."""
+    rng = np.random.default_rng(2)
+    ref = random_picture(rng, 64, 64, 8)
+    src = shifted(ref, -7, 6, rng, 2.0)
+    src[:32] = shifted(ref, 11, 3, rng, 1.0)[:32]
+    p = oracle.params(HEVC, 32)
+    want = oracle.frame_search(HEVC, 8, src, [ref], p)
+    for context in range(200):
+        with host.MotionSearch(0) as ms:
+            ms.upload(0, src, HEVC, 8)
+            ms.upload(1, ref, HEVC, 8)
+            n = 1
+            while (n := int(n * rng.uniform(1.2, 2.0)) + 1) < 100:
+                for _ in range(rng.integers(1, 7)):
+                    for got in ms.search_batch([(0, [1])] * int(n if rng.random() < 0.7 else rng.integers(1, n + 1)), p):
+                        assert_results_equal(got, want, f"context {context}, {n} frames")
