@@ -348,8 +348,10 @@ struct RefSearch {
     }
     const int x0 = max(bx - range, B.lx), x1 = min(bx + range, B.hx), y0 = max(by - range, B.ly),
               y1 = min(by + range, B.hy);
-    const uint32_t xr = (uint32_t)(x1 - x0), yr = (uint32_t)(y1 - y0);  // the start lies between them
-    auto inside = [&](int x, int y) { return (uint32_t)(x - x0) <= xr && (uint32_t)(y - y0) <= yr; };
+    // The box's columns (the start's among them) and rows: none where a
+    // vertical range of -1 leaves the window empty.
+    const uint32_t xn = (uint32_t)(x1 - x0 + 1), yn = (uint32_t)max(y1 - y0 + 1, 0);
+    auto inside = [&](int x, int y) { return (uint32_t)(x - x0) < xn && (uint32_t)(y - y0) < yn; };
     if (umh) {
       const int cx = bx, cy = by, total = umh_points(range);
       uint32_t mc = kInf, mi = 0xffffffffu;  // this lane's least cost, its first point
@@ -503,7 +505,9 @@ struct RefSearch {
   // ring in one step.
   __device__ __forceinline__ void refine(int smx, int smy, int hpel, int qpel, int& omx, int& omy, uint32_t& osatd,
                                          uint32_t& ocost) {
-    const int qlx = B.lx * 4, qhx = B.hx * 4, qly = B.ly * 4, qhy = B.hy * 4;
+    // The window in quarter samples (no row of an empty one).
+    const int qlx = B.lx * 4, qly = B.ly * 4;
+    const uint32_t qnx = (uint32_t)((B.hx - B.lx) * 4 + 1), qny = (uint32_t)max((B.hy - B.ly) * 4 + 1, 0);
     int bmx = smx, bmy = smy;
     uint32_t bc = kInf;
     bool first = true;
@@ -558,7 +562,7 @@ struct RefSearch {
         }
         bool ok = sl < n;
         if (sl >= base)
-          ok = ok && (uint32_t)(mx - qlx) <= (uint32_t)(qhx - qlx) && (uint32_t)(my - qly) <= (uint32_t)(qhy - qly) &&
+          ok = ok && (uint32_t)(mx - qlx) < qnx && (uint32_t)(my - qly) < qny &&
                !((uint32_t)(mx - prevx + step) <= 2u * step && (uint32_t)(my - prevy + step) <= 2u * step);
         const uint32_t rt = rate(mx, my);
         uint32_t v = kNone;

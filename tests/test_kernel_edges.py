@@ -327,3 +327,29 @@ def test_padded_plane_of_packed_and_of_strided_rows(ms, codec, bd, w, h, extra, 
     want = np.pad(rows[:, :w], ((pad, pad + ch - h), (pad, pad + cw - w)), mode="edge")
     np.testing.assert_array_equal(ms.plane(3300, 0), want)
     ms.release(3300)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bd", [8, 10])
+@pytest.mark.parametrize("vr", [-1, 0, 1])
+@pytest.mark.parametrize("kw", [{}, dict(h264_dia=1, h264_pad=8), dict(h264_umh=1, h264_range=24, h264_hpel_iters=5),
+                                dict(h264_umh=1, h264_range=512), dict(h264_range=40, h264_hpel_iters=64)])
+def test_h264_windows_of_no_row_and_of_few(ms, bd, vr, kw):
+    """A vertical range of -1 leaves the window empty: every start is clamped
+    to the row above, nothing else is scored; 0 and 1 leave one row, three."""
+    rng = np.random.default_rng(bd + vr)
+    w, h, nref = 80, 64, 3
+    refs = [random_picture(rng, w, h, bd)]
+    for k in range(1, nref):
+        refs.append(shifted(refs[0], 3 * k, -2 * k, rng, 2.0))
+    src = shifted(refs[-1], -5, 6, rng, 2.0)
+    for i, pic in enumerate(refs + [src]):
+        ms.upload(3400 + i, pic, H264, bd, as_ref=i < nref)
+    p = oracle.params(H264, 28, h264_vertical_range=vr, **kw)
+    got = ms.search(3400 + nref, [3400 + i for i in range(nref)], p)
+    want = oracle.frame_search(H264, bd, src, refs, p)
+    assert_results_equal(got, want, f"vertical range {vr}")
+    if vr < 0:
+        assert set(want["mvy"]) == {-4} and set(want["n_sad"]) <= set(range(nref, 9 * nref + 1))
+    for i in range(nref + 1):
+        ms.release(3400 + i)
