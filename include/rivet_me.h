@@ -600,6 +600,12 @@ int rme_probe_int_peak(int32_t device, double* ops_per_s);
  * device stays usable; `seconds` (may be NULL) is how long the wait took. */
 int rme_probe_wait_timeout(int32_t device, uint32_t polls, uint32_t* status, double* seconds);
 
+/* The same for this context's searches: from now on a STANDALONE launch's
+ * wait for another row's vector gives up after `polls` polls (1..2^22, the
+ * default), so that a launch whose waits run out can be tried: it ends within
+ * about one such wait, with RME_EDEVICE, its results incomplete. */
+int rme_probe_wait_polls(void* ctx, uint32_t polls);
+
 #ifdef __cplusplus
 }
 #endif

@@ -126,4 +126,5 @@ extern "C" {
     pub fn rme_serve_stop(server: *mut c_void) -> i32;
     pub fn rme_probe_int_peak(device: i32, ops_per_s: *mut f64) -> i32;
     pub fn rme_probe_wait_timeout(device: i32, polls: u32, status: *mut u32, seconds: *mut f64) -> i32;
+    pub fn rme_probe_wait_polls(ctx: *mut c_void, polls: u32) -> i32;
 }

@@ -248,6 +248,7 @@ struct Ctx {
   };
   std::map<std::pair<int, int>, Tune> tune;
   bool tune_on = true;
+  uint32_t wait_polls = kSpinLimit;  // LaunchDesc::wait_polls
   cudaStream_t stream = nullptr;
   // The parts of a launch after the first run on streams of their own,
   // forked from and joined back to the caller's stream.
@@ -860,6 +861,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     L.counters = di + kMiscCounters;
     L.status = reinterpret_cast<uint32_t*>(di + kMiscStatus);
     L.epoch = reinterpret_cast<const uint32_t*>(di + kMiscEpoch);
+    L.wait_polls = c->wait_polls;
     Lgiven[k] = L;
     Lgiven[k].ready = di + given_off[k];
     Lgiven[k].total = (int64_t)given[k].size();
@@ -926,6 +928,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   if (use_graph && !has_given) {
     std::vector<int64_t> gsig = sig;
     gsig.push_back(total);
+    gsig.push_back(c->wait_polls);
     gsig.push_back((int64_t)(uintptr_t)s);
     gsig.push_back((int64_t)(&sl - c->slots));
     gsig.push_back((int64_t)g_buffer_generation);
@@ -1499,6 +1502,12 @@ int rme_hevc_decide(const rme_picture_desc* d, const rme_params* p, int32_t nref
     }
   }
   return 0;
+}
+
+int rme_probe_wait_polls(void* ctx, uint32_t polls) {
+  if (!ctx || polls == 0 || polls > kSpinLimit) return RME_EINVAL;
+  ((Ctx*)ctx)->wait_polls = polls;
+  return RME_OK;
 }
 
 int rme_last_stats(void* ctx, rme_stats* s) {

@@ -123,6 +123,7 @@ struct RowSmem {
   uint32_t icost[2][RME_MAX_REFS];    // whole-sample costs, reference cost included
   RefResult fin[2][RME_MAX_REFS];
   uint32_t nsad[2], nsatd[2];
+  volatile uint32_t lost[RME_MAX_REFS];  // a wait of a reference's warps gave up
   uint32_t entry;
 };
 
@@ -131,16 +132,17 @@ struct RowSmem {
 __device__ __forceinline__ bool row_word_ok(unsigned long long w, uint32_t tag) {
   return ((uint32_t)(w >> 32) & ~3u) == tag;
 }
-// Waits (bounded, as wait_word) for a word already loaded once; false once
-// the wait has run out, after which the caller waits no more.
-__device__ __noinline__ bool wait_row_word(const LaunchDesc& L, const unsigned long long* p, uint32_t tag,
-                                           unsigned long long& w, bool lost) {
+// Waits for a word already loaded once: at most L.wait_polls polls, then the
+// status word's timeout bit; fewer once the launch has failed elsewhere. Returns
+// the word, of another tag where it gave up.
+__device__ __noinline__ unsigned long long poll_row_word(const LaunchDesc& L, const unsigned long long* p, uint32_t tag,
+                                                         unsigned long long w) {
   uint32_t ns = 32;
   for (uint32_t it = 0; !row_word_ok(w, tag); ++it) {
-    if (lost || it >= kSpinLimit) {
-      if (!lost) atomicOr(L.status, kStatusWaitTimeout);
-      w = (unsigned long long)tag << 32;
-      return false;
+    const bool out = it >= L.wait_polls;
+    if (out || ((it & 63u) == 63u && ld_relaxed32(L.status) != 0u)) {
+      if (out) atomicOr(L.status, kStatusWaitTimeout);
+      break;
     }
     if (it >= 16) {
       __nanosleep(ns);
@@ -148,7 +150,17 @@ __device__ __noinline__ bool wait_row_word(const LaunchDesc& L, const unsigned l
     }
     w = ld_relaxed64(p);
   }
-  return true;
+  return w;
+}
+// Sets `lost` (shared memory) where the wait gives up. Every warp waits by
+// itself: behind the search's first barrier a reference's warps all see it and
+// drop what they took from words that may differ (they could take different
+// numbers of steps between their barriers); at the macroblock's end the CTA
+// leaves.
+__device__ __forceinline__ void wait_row_word(const LaunchDesc& L, const unsigned long long* p, uint32_t tag,
+                                              unsigned long long& w, volatile uint32_t& lost) {
+  w = poll_row_word(L, p, tag, w);
+  if (!row_word_ok(w, tag)) lost = 1u;
 }
 
 // One reference's search of a macroblock, by the 128 threads of its group.
@@ -167,6 +179,7 @@ struct RefSearch {
   uint32_t* win;      // this reference's window
   int wx = 0, wy = 0, wofs = 0;  // its centre; the centre's first byte in a row
   int buf = 0;
+  uint32_t lost = 0;             // a wait of the group gave up
   uint32_t nsad = 0, nsatd = 0;  // candidates scored: this lane's eighths, sixteenths
   uint32_t s0[WR], s1[WR];       // source rows sub and sub + 8
 
@@ -340,11 +353,17 @@ struct RefSearch {
       const bool ok = (keep >> slot) & 1u;
       const int fx = __shfl_sync(kFull, qx, slot), fy = __shfl_sync(kFull, qy, slot);
       const uint32_t rt = rate(fx * 4, fy * 4);
-      const uint32_t m = __reduce_min_sync(kFull, share<8>(ok ? sad(fx, fy) + (sub == 0 ? rt : 0u) : kNone));
+      const uint32_t c = share<8>(ok ? sad(fx, fy) + (sub == 0 ? rt : 0u) : kNone);
+      lost = sm.lost[g];
+      const uint32_t m = __reduce_min_sync(kFull, c);
       nsad += ok;
       bcost = m >> 4;
       bx = __shfl_sync(kFull, qx, m & 15);
       by = __shfl_sync(kFull, qy, m & 15);
+      if (__builtin_expect(lost != 0u, 0)) {
+        B.px = B.py = bx = 0;
+        by = min(max(0, B.ly), B.hy);
+      }
     }
     const int x0 = max(bx - range, B.lx), x1 = min(bx + range, B.hx), y0 = max(by - range, B.ly),
               y1 = min(by + range, B.hy);
@@ -601,8 +620,9 @@ struct RefSearch {
   }
 };
 
+// False, for the whole CTA, where a wait gave up: the launch has failed.
 template <class S>
-__device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSmem<S>& sm, int tid, bool& lost,
+__device__ bool h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSmem<S>& sm, int tid,
                          unsigned long long (&cnt)[3]) {
   constexpr int WR = RefSearch<S>::WR, NSRC = 16 * WR;
   const int lane = tid & 31, g = tid >> 7, warp = (tid >> 5) & 3;
@@ -625,7 +645,7 @@ __device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSme
   if (my > 0) {
     wb = ld_relaxed64(up);
     if (mbw > 1) wc = ld_relaxed64(up + 1);
-    if (!wait_row_word(L, up, tag, wb, lost)) lost = true;
+    wait_row_word(L, up, tag, wb, sm.lost[g]);
     __syncwarp();
   }
   Nb A{false, -1, 0, 0};
@@ -663,7 +683,7 @@ __device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSme
   for (int mx = 0; mx < mbw; ++mx) {
     const int par = mx & 1;
     const bool has_c = my > 0 && mx + 1 < mbw;
-    if (has_c && !wait_row_word(L, up + mx + 1, tag, wc, lost)) lost = true;
+    if (has_c) wait_row_word(L, up + mx + 1, tag, wc, sm.lost[g]);
     __syncwarp();
     // The next macroblock's C word and source, on their way during the search.
     unsigned long long wn = 0;
@@ -740,19 +760,22 @@ __device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSme
         gate = g > 0 && ratio > 0.0f && __uint2float_rn(r.icost) >= __fmul_rn(ratio, __uint2float_rn(before));
       }
       q.refine(r.imx, r.imy, gate ? 0 : hpel, gate ? 0 : qpel, r.mx, r.my, r.satd, r.cost);
-      r.cost += ref_cost;
+      r.cost = q.lost ? 0xffffffffu : r.cost + ref_cost;  // (above any other)
       if ((tid & (kRefThreads - 1)) == 0) sm.fin[par][g] = r;
     }
     if (tid < NSRC) sm.src[par ^ 1][tid] = nsrc;
     __syncthreads();
     // The reference of least cost, the first reaching it (all threads).
     int best = 0;
-    uint32_t c16 = sm.fin[par][0].cost;
-    for (int r = 1; r < nref; ++r)
-      if (sm.fin[par][r].cost < c16) {
-        c16 = sm.fin[par][r].cost;
+    uint32_t c16 = sm.fin[par][0].cost, most = c16;
+    for (int r = 1; r < nref; ++r) {
+      const uint32_t c = sm.fin[par][r].cost;
+      most = max(most, c);
+      if (c < c16) {
+        c16 = c;
         best = r;
       }
+    }
     const RefResult& w = sm.fin[par][best];
     A = Nb{true, best, (int)(int16_t)w.mx, (int)(int16_t)w.my};
     if (tid == 0) {
@@ -760,6 +783,7 @@ __device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSme
       if (mx > 0) write(mx - 1);
       ended = best;
     }
+    if (most == 0xffffffffu) return false;  // a wait gave up (checked where little is in flight)
     if (g < nref) {
       // Both counts in one sum (a lane has a few hundred of each at most).
       const uint32_t n = __reduce_add_sync(kFull, q.nsad | q.nsatd << 16);
@@ -774,6 +798,7 @@ __device__ void h264_row(const LaunchDesc& L, const FrameDesc& F, int my, RowSme
   }
   __syncthreads();
   if (tid == 0) write(mbw - 1);
+  return true;
 }
 
 // Rows are taken in the order the host pushed them (every frame's row 0,
@@ -784,8 +809,8 @@ __global__ void __launch_bounds__(RME_MAX_REFS * kRefThreads) h264_row_kernel(La
   __shared__ RowSmem<S> sm;
   const int tid = threadIdx.x;
   const uint32_t epoch = __ldg(L.epoch);
-  bool lost = false;
   unsigned long long cnt[3] = {0, 0, 0};
+  if (tid < RME_MAX_REFS) sm.lost[tid] = 0u;
   for (;;) {
     __syncthreads();
     if (tid == 0) {
@@ -803,7 +828,7 @@ __global__ void __launch_bounds__(RME_MAX_REFS * kRefThreads) h264_row_kernel(La
       if (tid == 0) atomicOr(L.status, kStatusBadTask);
       continue;
     }
-    h264_row<S>(L, F, row, sm, tid, lost, cnt);
+    if (!h264_row<S>(L, F, row, sm, tid, cnt)) break;
   }
   if (tid == 0) {
     atomicAdd(&L.counters[0], cnt[0]);

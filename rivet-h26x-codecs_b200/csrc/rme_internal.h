@@ -101,6 +101,7 @@ struct LaunchDesc {
   unsigned long long* counters;  // [tasks, sad, satd, sad_samples, satd_samples]
   const uint32_t* epoch;         // this launch's epoch (device memory: a
                                  // replayed graph keeps its arguments)
+  uint32_t wait_polls;           // batched rows: polls before a wait for another row's vector gives up
   // The resident engine: the ring of the tasks a whole CTA runs (32x32 and
   // 64x64 blocks), served by the first `group_ctas` CTAs.
   unsigned long long* ready_big;

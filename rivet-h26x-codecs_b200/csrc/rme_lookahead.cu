@@ -140,6 +140,15 @@ __device__ __forceinline__ bool wait_word(const unsigned long long* p, unsigned 
   return true;
 }
 
+// The wait of a warp, all of whose lanes hold the word: where one of them gave
+// up, all go on with zero and wait no more (their steps and votes must agree).
+__device__ __forceinline__ bool wait_above(const unsigned long long* p, unsigned long long& w, uint32_t* status,
+                                           bool lost) {
+  lost = __any_sync(kAll, !wait_word(p, w, status, lost));
+  if (lost) w = 0ull;
+  return lost;
+}
+
 // |a - b| of four bytes, summed onto acc.
 __device__ __forceinline__ uint32_t sad4(uint32_t a, uint32_t b, uint32_t acc) {
   uint32_t r;
@@ -218,7 +227,7 @@ __global__ void __launch_bounds__(kLaWarps * 32) lowres_search_kernel(const Lowr
     for (int bx = 0; bx < bw; ++bx) {
       const int x = bx * 8, xlo = -lim - x;
       const uint32_t rb = rrow + x;
-      if (by > 0 && !wait_word(up + bx, uw, status, lost)) lost = true;
+      if (by > 0) lost = wait_above(up + bx, uw, status, lost);
       const uint32_t av = (uint32_t)uw;
       uint2 sn[4] = {};
       unsigned long long un = 0ull;
@@ -536,7 +545,7 @@ __global__ void __launch_bounds__(kLaWarps * 32) lowres_search_h264_kernel(const
     for (int bx = 0; bx < bw; ++bx) {
       const int x = bx * 8;
       const S* rb = rrow + x;
-      if (by > 0 && !wait_word(up + bx, uw, status, lost)) lost = true;
+      if (by > 0) lost = wait_above(up + bx, uw, status, lost);
       const uint32_t av = (uint32_t)uw;
       Row8<S> sn[4];
       unsigned long long un = 0ull;

@@ -9,7 +9,9 @@
 // latency of one block's dependent steps. Hence
 //   - no queue between blocks: a finished block publishes its vector as one
 //     word (tag, vector), and a block waits (bounded) for its upper and
-//     parent words only, loaded a block ahead; its left vector is at hand;
+//     parent words only, loaded a block ahead; its left vector is at hand.
+//     A wait that runs out ends its group's row, its CTA and, by the status
+//     word, soon the launch;
 //   - several warps a block and few steps: an 8x8 block has 64 threads, a
 //     16x16 or 32x32 block 128, a 64x64 block 256, so that a step is a few
 //     loads a thread, a short sum and one barrier. More threads would repeat
@@ -59,6 +61,7 @@ struct SmallSmem {
   uint32_t src[2][N * N * sizeof(S) / 4];
   uint32_t key[2][kSlots];  // cost << 5 | slot (a cost is below 2^26: at most 64 * 64 * 4095 and the largest rate)
   uint32_t satd[2][16];     // half, quarter
+  volatile uint32_t lost;   // a wait of the group gave up
 };
 
 // The points three rounds of the small diamond can reach, in an order in
@@ -86,6 +89,41 @@ __constant__ uint32_t c_third[8] = {
     1u << 15 | 1u << 3 | 1u << 19 | 1u << 1,  1u << 16 | 1u << 4 | 1u << 1 | 1u << 20,
     1u << 3 | 1u << 17 | 1u << 21 | 1u << 2,  1u << 4 | 1u << 18 | 1u << 2 | 1u << 22,
     1u << 19 | 1u << 21 | 1u << 23 | 1u << 3, 1u << 20 | 1u << 22 | 1u << 4 | 1u << 24};
+
+// Waits for another row's published word, already loaded once (`w`): at most
+// L.wait_polls polls, then the status word's timeout bit; fewer once the launch
+// has failed elsewhere. Returns the word, of another tag where it gave up. (The
+// first polls follow one another, later ones back off, as wait_word's.)
+__device__ __noinline__ unsigned long long poll_published(const LaunchDesc& L, const unsigned long long* p, uint32_t tag,
+                                                          unsigned long long w) {
+  uint32_t ns = 32;
+  for (uint32_t it = 0; (uint32_t)(w >> 32) != tag; ++it) {
+    const bool out = it >= L.wait_polls;
+    if (out || ((it & 63u) == 63u && ld_relaxed32(L.status) != 0u)) {
+      if (out) atomicOr(L.status, kStatusWaitTimeout);
+      break;
+    }
+    if (it >= 16) {
+      __nanosleep(ns);
+      if (ns < 256) ns <<= 1;
+    }
+    w = ld_relaxed64(p);
+  }
+  return w;
+}
+// Sets the group's `lost` (shared memory) where it gave up. All of a group must
+// then know before a step whose number the words decide (a walk's): with
+// different words some would wait at a barrier for ever. A small block's warps
+// each wait by themselves, read `lost` behind the first step's barrier and end
+// the row there; a large block's words are waited for by one warp and read from
+// shared memory by all (a barrier more, few registers: there the check cost
+// spills).
+__device__ __forceinline__ void wait_published(const LaunchDesc& L, const unsigned long long* p, uint32_t tag,
+                                               unsigned long long& w, volatile uint32_t& lost) {
+  if ((uint32_t)(w >> 32) == tag) return;
+  w = poll_published(L, p, tag, w);
+  if ((uint32_t)(w >> 32) != tag) lost = 1u;
+}
 
 // What a row's blocks share, read once.
 template <class S>
@@ -116,9 +154,10 @@ struct RowCount {
   uint32_t tasks = 0, sad = 0, satd = 0, area = 0;
 };
 
-// A row of 8x8 or 16x16 blocks by T threads.
+// A row of 8x8 or 16x16 blocks by T threads. False, for the whole group, where
+// a wait gave up (the launch has failed).
 template <class S, int N, int T>
-__device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, int row, SmallSmem<S, N>& sm, int tid,
+__device__ bool small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, int row, SmallSmem<S, N>& sm, int tid,
                           int bar, RowCount& cnt) {
   constexpr int SPW = 4 / (int)sizeof(S), WR = N / SPW, NSRC = N * WR, TW = N / 4, NT = TW * TW, WPT = 4 / SPW;
   constexpr int PS = (NSRC + T - 1) / T;  // source words a thread stages
@@ -149,6 +188,7 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
   uint32_t nsrc[PS];
   load_src(0, nsrc);
   store_src(sm.src[0], nsrc);
+  if (tid == 0) sm.lost = 0u;
   unsigned long long uw = row > 0 ? ld_relaxed64(up) : 0ull, pw = 0ull;
   if (const unsigned long long* p = parent_of(0)) pw = ld_relaxed64(p);
   uint32_t lv = 0;
@@ -162,9 +202,9 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
   for (int bx = 0; bx < I.nbx; ++bx) {
     const int x = bx * N;
     const uint32_t* const src = sm.src[bx & 1];
-    if (row > 0) uw = wait_word(L, up + (ptrdiff_t)bx * I.nref, I.tag, uw);
+    if (row > 0) wait_published(L, up + (ptrdiff_t)bx * I.nref, I.tag, uw, sm.lost);
     const unsigned long long* const pp = parent_of(x);
-    if (pp) pw = wait_word(L, pp, I.tag, pw);
+    if (pp) wait_published(L, pp, I.tag, pw, sm.lost);
     __syncwarp();
     const uint32_t uv = (uint32_t)uw, pv = pp ? (uint32_t)pw : 0u;
     // The next block's words and source, on their way during the search.
@@ -245,6 +285,7 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
       }
       key = score(std::integral_constant<int, T / kSlots>{}, slot, ok, fx, fy);
     }
+    const bool lost = sm.lost != 0u;
     // The best seed, the first in order (slots 0, 1, 14, 16) of least cost.
     uint32_t best = __reduce_min_sync(kFull, (0x14003u >> lane) & 1u ? key : kNoKey);
     const int s0 = (int)(best & 31u);
@@ -253,6 +294,7 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
     uint32_t bcost = best >> 5;
     int base = ox == ux && oy == uy ? 1 : ox == gx && oy == gy ? 16 : -1;  // its points' slots, where scored
     // The diamond, two rounds a step.
+    if (lost) break;
     for (int it = 0, rings = 0;;) {
       while (it < 2 * range) {
         if (base < 0) {
@@ -417,6 +459,7 @@ __device__ void small_row(const LaunchDesc& L, const FrameDesc& F, int l, int r,
   }
   cnt.area = N * N;
   group_sync<T>(bar);  // the last block's keys and source are read: the buffers may be reused
+  return sm.lost == 0u;
 }
 
 // A 32x32 or 64x64 block's window: the reference's integer plane around a
@@ -430,14 +473,17 @@ struct BigSmem {
   uint32_t src[2][N * N * sizeof(S) / 4];
   uint32_t win[ROWS * WRW];
   uint32_t cost[3][32];  // a step's distortions, summed over the warps; in turn, the next one cleared a step ahead
+  uint32_t word[2];        // the upper and the parent block's vectors
+  volatile uint32_t lost;  // a wait gave up
 };
 
 // A row of 32x32 or 64x64 blocks by T threads: a thread has PW words of the
 // block for the SADs (a warp's lanes side by side in a row) and a 4x4 tile
 // for the SATDs, and scores every candidate of a step on them; the warps'
-// sums meet in shared memory, one barrier a step.
+// sums meet in shared memory, one barrier a step. False as small_row (where
+// a wait gave up the row goes on, and its later waits give up at once).
 template <class S, int N, int T>
-__device__ void big_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, int row, BigSmem<S, N>& sm, int tid,
+__device__ bool big_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, int row, BigSmem<S, N>& sm, int tid,
                         int bar, RowCount& cnt) {
   constexpr int B = (int)sizeof(S), SPW = 4 / B, WR = N / SPW, NSRC = N * WR, PW = NSRC / T, NW = B == 1 ? 3 : 4;
   constexpr int TW = N / 4, NT = TW * TW, WPT = 4 / SPW, WRW = BigSmem<S, N>::WRW, ROWS = BigSmem<S, N>::ROWS;
@@ -465,6 +511,7 @@ __device__ void big_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, i
   uint32_t lv = 0;
   int buf = 0;
   if (tid < 32) sm.cost[0][tid] = 0u;
+  if (tid == 0) sm.lost = 0u;
   group_sync<T>(bar);
   // After a step's sums are in `mine` (lane k: candidate k's over this warp):
   // the totals, lane k candidate k's.
@@ -482,15 +529,22 @@ __device__ void big_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, i
     uint32_t* const src = sm.src[bx & 1];
 #pragma unroll
     for (int k = 0; k < PW; ++k) src[(row0 + k) * WR + wd] = sw[k];
-    if (row > 0) uw = wait_word(L, up + (ptrdiff_t)bx * I.nref, I.tag, uw);
     const unsigned long long* const pp = parent_of(x);
-    if (pp) pw = wait_word(L, pp, I.tag, pw);
-    __syncwarp();
-    const uint32_t uv = (uint32_t)uw, pv = pp ? (uint32_t)pw : 0u;
-    if (bx + 1 < I.nbx) {
-      if (row > 0) uw = ld_relaxed64(up + (ptrdiff_t)(bx + 1) * I.nref);
-      if (const unsigned long long* p = parent_of(x + N)) pw = ld_relaxed64(p);
+    if (tid < 32) {
+      if (row > 0) wait_published(L, up + (ptrdiff_t)bx * I.nref, I.tag, uw, sm.lost);
+      if (pp) wait_published(L, pp, I.tag, pw, sm.lost);
+      __syncwarp();
+      if (lane == 0) {
+        sm.word[0] = (uint32_t)uw;
+        sm.word[1] = pp ? (uint32_t)pw : 0u;
+      }
+      if (bx + 1 < I.nbx) {
+        if (row > 0) uw = ld_relaxed64(up + (ptrdiff_t)(bx + 1) * I.nref);
+        if (const unsigned long long* p = parent_of(x + N)) pw = ld_relaxed64(p);
+      }
     }
+    group_sync<T>(bar);
+    const uint32_t uv = sm.word[0], pv = sm.word[1];
     uint32_t m0 = 0, m1 = 0;
     if (bx > 0) {
       m0 = lv;
@@ -748,6 +802,7 @@ __device__ void big_row(const LaunchDesc& L, const FrameDesc& F, int l, int r, i
   }
   cnt.area = N * N;
   group_sync<T>(bar);
+  return sm.lost == 0u;
 }
 
 template <class S>
@@ -764,8 +819,9 @@ __global__ void __launch_bounds__(kRowThreads, 2) hevc_row_kernel(LaunchDesc L) 
   __shared__ uint32_t entry;
   const int tid = threadIdx.x;
   const uint32_t epoch = __ldg(L.epoch);
+  bool lost = false;  // a wait of this thread's group gave up
   for (;;) {
-    __syncthreads();
+    if (__syncthreads_or(lost)) break;  // the launch has failed (status set)
     if (tid == 0) {
       const unsigned long long idx = atomicAdd(L.head, 1ull);
       entry = idx >= (unsigned long long)L.total ? kPopDone : pop_slot(L, idx, epoch);
@@ -786,13 +842,17 @@ __global__ void __launch_bounds__(kRowThreads, 2) hevc_row_kernel(LaunchDesc L) 
     if (mine >= F.nby[l]) continue;
     RowCount cnt;
     if (N == 8)
-      small_row<S, 8, row_group(8)>(L, F, l, r, mine, reinterpret_cast<SmallSmem<S, 8>*>(smem_raw)[g], gt, bar, cnt);
+      lost = !small_row<S, 8, row_group(8)>(L, F, l, r, mine, reinterpret_cast<SmallSmem<S, 8>*>(smem_raw)[g], gt, bar,
+                                            cnt);
     else if (N == 16)
-      small_row<S, 16, row_group(16)>(L, F, l, r, mine, reinterpret_cast<SmallSmem<S, 16>*>(smem_raw)[g], gt, bar, cnt);
+      lost = !small_row<S, 16, row_group(16)>(L, F, l, r, mine, reinterpret_cast<SmallSmem<S, 16>*>(smem_raw)[g], gt, bar,
+                                            cnt);
     else if (N == 32)
-      big_row<S, 32, row_group(32)>(L, F, l, r, mine, reinterpret_cast<BigSmem<S, 32>*>(smem_raw)[g], gt, bar, cnt);
+      lost = !big_row<S, 32, row_group(32)>(L, F, l, r, mine, reinterpret_cast<BigSmem<S, 32>*>(smem_raw)[g], gt, bar,
+                                            cnt);
     else
-      big_row<S, 64, row_group(64)>(L, F, l, r, mine, reinterpret_cast<BigSmem<S, 64>*>(smem_raw)[g], gt, bar, cnt);
+      lost = !big_row<S, 64, row_group(64)>(L, F, l, r, mine, reinterpret_cast<BigSmem<S, 64>*>(smem_raw)[g], gt, bar,
+                                            cnt);
     if (gt == 0) {
       atomicAdd(&L.counters[0], (unsigned long long)cnt.tasks);
       atomicAdd(&L.counters[1], (unsigned long long)cnt.sad);

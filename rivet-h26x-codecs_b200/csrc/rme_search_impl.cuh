@@ -406,6 +406,12 @@ __device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long l
   return v;
 }
 
+__device__ __forceinline__ uint32_t ld_relaxed32(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ void st_relaxed64(unsigned long long* p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
