@@ -613,6 +613,8 @@ int make_frame(Ctx* c, const rme_frame* f, const rme_params* p, FrameDesc* fd, r
 int finish_launch(Ctx* c, Slot& sl, bool wait_planes = true) {
   if (!sl.busy) return 0;
   sl.busy = false;
+  rme_result* const host_out = sl.host_out;  // not a later launch's, however this one went
+  sl.host_out = nullptr;
   CK(cudaEventSynchronize(sl.done));
   const uint32_t status = (uint32_t)(sl.h_misc.p[kMiscStatus] & 0xffffffffu);
   float ms = 0.0f;
@@ -648,11 +650,9 @@ int finish_launch(Ctx* c, Slot& sl, bool wait_planes = true) {
   if (c->last.tasks != (unsigned long long)sl.total)
     return fail(c, RME_EDEVICE, "the launch ran " + std::to_string(c->last.tasks) + " of " + std::to_string(sl.total) +
                                     " tasks");
-  if (sl.host_out) {
+  if (host_out)
     for (size_t i = 0; i < sl.host_off.size(); ++i)
-      std::memcpy(sl.host_out + sl.host_off[i], sl.h_out.p + sl.dev_off[i], sizeof(rme_result) * sl.host_count[i]);
-    sl.host_out = nullptr;
-  }
+      std::memcpy(host_out + sl.host_off[i], sl.h_out.p + sl.dev_off[i], sizeof(rme_result) * sl.host_count[i]);
   return 0;
 }
 

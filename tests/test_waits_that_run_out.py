@@ -87,3 +87,28 @@ def test_a_batch_of_both_codecs_short_of_polls_ends():
         for _ in range(4):
             for g, w_ in zip(ms.search_batch(frames, params), want):
                 assert_results_equal(g, w_, "with every poll again")
+
+
+@pytest.mark.gpu
+def test_a_failed_launchs_buffer_is_not_written_by_a_later_one():
+    """Pageable results of launches that failed, then launches on the same
+    slots that keep theirs on the device."""
+    import torch
+    rng = np.random.default_rng(3)
+    with host.MotionSearch(0) as ms:
+        src, refs, ids = _frame(ms, rng, 10, HEVC, 8, 416, 240, 1)
+        p = oracle.params(HEVC, 30)
+        want = oracle.frame_search(HEVC, 8, src, refs, p)
+        n = ms.batch_result_count([(10, ids)], p)
+        old = [np.zeros(n, capi.RESULT_DTYPE) for _ in range(4)]  # one for each launch slot
+        _limit(ms, 1)
+        for o in old:
+            with pytest.raises(RuntimeError, match="device status 1"):
+                ms.search_batch([(10, ids)], p, out=o)
+            o.view(np.uint8)[:] = 0x5a
+        _limit(ms, POLLS)
+        out = torch.zeros(n * capi.RESULT_DTYPE.itemsize, dtype=torch.uint8, device="cuda")
+        for k in range(8):
+            ms.search_batch([(10, ids)], p, out=out)
+            assert all((o.view(np.uint8) == 0x5a).all() for o in old), f"call {k}"
+        assert_results_equal(out.cpu().numpy().view(capi.RESULT_DTYPE), want, "on the device")
