@@ -794,7 +794,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
   }
   // GIVEN jobs by their block's area, in 4x4 tiles (1..256), largest first:
   // the jobs that run last are short ones.
-  int64_t given_big[kParts] = {0, 0, 0, 0};
+  int64_t given_big[kParts] = {0, 0, 0, 0}, given_larger[kParts] = {0, 0, 0, 0};
   for (int k = 0; k < kParts; ++k) {
     size_t at[257] = {0}, nk = 0;
     auto tiles = [](const rme_job& j) { return 256 - (j.w >> 2) * (j.h >> 2); };
@@ -804,6 +804,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     if (nk == 0) continue;
     for (int q = 0; q < 256; ++q) at[q + 1] += at[q];
     given_big[k] = (int64_t)at[256 - kFlatBigTiles + 1];
+    given_larger[k] = (int64_t)at[256 - kFlatHalfTiles];
     given[k].resize(nk);
     for (int i = 0; i < n; ++i)
       if (!fdeps[i] && part_of(sl.h_frames.p[i]) == k)
@@ -896,7 +897,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     }
     if (e == cudaSuccess && !given[k].empty())
       e = h264 ? launch_h264_given(Lgiven[k], bytes, variant[k], c->nsm * c->bps[k][variant[k]], sk)
-               : launch_hevc_flat(Lgiven[k], bytes, false, true, n, given_big[k], c->nsm, sk);
+               : launch_hevc_flat(Lgiven[k], bytes, false, true, n, given_big[k], c->nsm, sk, given_larger[k] == 0);
     return e;
   };
   auto enqueue = [&](bool capturing) -> cudaError_t {

@@ -25,8 +25,8 @@
 // rows 17.5 ms for 45; 6,000 mixed 10-bit GIVEN jobs 0.76 -> 0.27 ms (a warp
 // each: 0.60), 600 of 8 bits 0.06 (0.21), 20,000 of 8 bits 0.48. Lists of one
 // shape, 8 and 10 bits: 8,040 16x16 jobs 109 -> 91 and 189 -> 115 us, 480 64x64
-// 241 -> 63 and 517 -> 102; 20,000 8x8, whose 16 words leave half of a warp
-// idle, 95 -> 113 and 145 -> 126. Five or six CTAs an SM (spills) gain at most
+// 241 -> 63 and 517 -> 102; 20,000 8x8 106 -> 104 and 178 -> 140 (of 8 bits
+// 125 while their 16 words left half of a warp idle: HALVES). Five or six CTAs an SM (spills) gain at most
 // 2 % and lose up to 7.
 #include <algorithm>
 
@@ -64,7 +64,10 @@ struct FlatBlock {
 // sample); otherwise its reads find their words by themselves.
 // W: the warps that share the search (1, or all of the CTA's, which then
 // exchange their sums through `part`).
-template <class S, bool WORDS, bool SRC, int W>
+// HALVES: blocks of 8-bit samples, at most sixteen words of them (8x8 and
+// smaller): a half of a warp holds the block, a word a lane, and its halves
+// score candidates of their own.
+template <class S, bool WORDS, bool SRC, int W, bool HALVES>
 __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_result* out, uint32_t (*part)[W][32],
                             uint32_t& nsad, uint32_t& nsatd) {
   const int lane = threadIdx.x & 31, warp = W == 1 ? 0 : (int)(threadIdx.x >> 5), tid = warp * 32 + lane;
@@ -94,8 +97,10 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
   // This lane's words: word wd of `rows` rows from row0 (none for the lanes
   // left over). Rows follow one another, so the diamond reads each once.
   constexpr int STEP = 32 * W;
-  const int segs = min(STEP / wr, h), each = (h + segs - 1) / segs;
-  const int seg = tid / wr, wd = tid - seg * wr, row0 = seg * each, rows = seg < segs ? min(each, h - row0) : 0;
+  static_assert(!HALVES || (B == 1 && W == 1), "a lone warp's 8-bit block");
+  const int place = HALVES ? lane & 15 : tid;
+  const int segs = HALVES ? h : min(STEP / wr, h), each = HALVES ? 1 : (h + segs - 1) / segs;
+  const int seg = place / wr, wd = place - seg * wr, row0 = seg * each, rows = seg < segs ? min(each, h - row0) : 0;
   auto source = [&](const S* q) -> uint32_t {
     return SRC ? RME_LD32(reinterpret_cast<const uint32_t*>(q)) : ldw(q);
   };
@@ -112,6 +117,26 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
     for (int k = 0; k < rows; ++k) acc = add(source(sp + (ptrdiff_t)k * K.src_stride), ldw(rp + (ptrdiff_t)k * stride), acc);
     return __reduce_add_sync(kFull, sum_of(acc));
   };
+  // HALVES: this lane's word of the block; the two halves' sums (at most
+  // 64 * 255 each) in one word, the upper half's above; the candidates of
+  // mask `m`, two at a time: lane k has candidate k's point and gets its SAD.
+  uint32_t own = 0;
+  if constexpr (HALVES) own = rows > 0 ? source(K.src + (ptrdiff_t)row0 * K.src_stride + wd * SPW) : 0u;
+  auto both = [&](uint32_t acc) -> uint32_t { return __reduce_add_sync(kFull, acc << (lane & 16)); };
+  auto pairs = [&](uint32_t m, int px, int py) -> uint32_t {
+    uint32_t mine = 0;
+    while (m != 0u) {
+      const int a = __ffs(m) - 1;
+      m &= m - 1u;
+      const int b = m != 0u ? __ffs(m) - 1 : a, k = lane & 16 ? b : a;
+      m &= m - 1u;
+      const int fx = __shfl_sync(kFull, px, k), fy = __shfl_sync(kFull, py, k);
+      const uint32_t v = both(rows > 0 ? add(own, ldw(org + (ptrdiff_t)(fy + row0) * stride + fx + wd * SPW), 0u) : 0u);
+      if (lane == a) mine = v & 0xffffu;
+      if (lane == b) mine = v >> 16;
+    }
+    return mine;
+  };
 
   // Seeds: >> 2, clamp_pos, deduplicated (`tried`), scored in order.
   const int qx = min(max(K.sx >> 2, lox), hix), qy = min(max(K.sy >> 2, loy), hiy);
@@ -124,10 +149,14 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
   nsad = __popc(kept);
   nsatd = 9;
   uint32_t c = 0;
-  for (uint32_t m = kept; m != 0u; m &= m - 1u) {
-    const int s = __ffs(m) - 1;
-    const uint32_t v = sad1(__shfl_sync(kFull, qx, s), __shfl_sync(kFull, qy, s));
-    if (lane == s) c = v;
+  if constexpr (HALVES) {
+    c = pairs(kept, qx, qy);
+  } else {
+    for (uint32_t m = kept; m != 0u; m &= m - 1u) {
+      const int s = __ffs(m) - 1;
+      const uint32_t v = sad1(__shfl_sync(kFull, qx, s), __shfl_sync(kFull, qy, s));
+      if (lane == s) c = v;
+    }
   }
   c = total(c);
   Pick p = warp_min((kept >> lane) & 1u ? c + rate(qx * 4, qy * 4) : kInf);
@@ -150,7 +179,41 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
       const bool ok = lane < 12 && allowed(fx, fy);
       const uint32_t there = __ballot_sync(kFull, ok);
       uint32_t mine = 0;
-      if (WORDS && fbx - 2 >= lox && fbx + 2 <= hix && fby - 2 >= loy && fby + 2 <= hiy) {
+      if (HALVES && WORDS && fbx - 2 >= lox && fbx + 2 <= hix && fby - 2 >= loy && fby + 2 <= hiy) {
+        // The lower half takes the points of even numbers, the upper half
+        // those of odd numbers, which mirror them: three rows and six points
+        // a lane instead of five and twelve.
+        const int d = lane & 16 ? -1 : 1;
+        const uintptr_t a0 = reinterpret_cast<uintptr_t>(org + (ptrdiff_t)fby * stride + fbx - 2);
+        const uint32_t off = (uint32_t)(a0 & 3);
+        const int rs = stride / 4;
+        uint32_t acc[6] = {};
+        if (rows > 0) {
+          const uint32_t* const wp = reinterpret_cast<const uint32_t*>(a0 & ~uintptr_t(3)) + (ptrdiff_t)row0 * rs + wd;
+          uint32_t v[3][3];  // rows 0, d, 2d
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) v[i][j] = RME_LD32(wp + (ptrdiff_t)(i * d) * rs + j);
+          auto at = [&](int dx, const uint32_t (&q)[3]) {
+            const uint32_t o = off + (uint32_t)(dx + 2);
+            return __funnelshift_r(o >> 2 ? q[1] : q[0], o >> 2 ? q[2] : q[1], (o & 3u) * 8u);
+          };
+          acc[0] = add(own, at(d, v[0]), 0u);
+          acc[1] = add(own, at(0, v[1]), 0u);
+          acc[2] = add(own, at(2 * d, v[0]), 0u);
+          acc[3] = add(own, at(1, v[1]), 0u);
+          acc[4] = add(own, at(-1, v[1]), 0u);
+          acc[5] = add(own, at(0, v[2]), 0u);
+        }
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+          const uint32_t v = both(acc[i]);
+          if (lane >> 1 == i) mine = lane & 1 ? v >> 16 : v & 0xffffu;
+        }
+      } else if (HALVES) {
+        mine = pairs(there, fx, fy);
+      } else if (WORDS && fbx - 2 >= lox && fbx + 2 <= hix && fby - 2 >= loy && fby + 2 <= hiy) {
         uint32_t acc[12];
 #pragma unroll
         for (int q = 0; q < 12; ++q) acc[q] = 0u;
@@ -253,10 +316,14 @@ __device__ void flat_search(const FrameDesc& F, const FlatBlock<S>& K, rme_resul
     const bool ok = lane < 24 && allowed(fx, fy);
     const uint32_t there = __ballot_sync(kFull, ok);
     uint32_t mine = 0;
-    for (uint32_t m = there; m != 0u; m &= m - 1u) {
-      const int s = __ffs(m) - 1;
-      const uint32_t v = sad1(__shfl_sync(kFull, fx, s), __shfl_sync(kFull, fy, s));
-      if (lane == s) mine = v;
+    if constexpr (HALVES) {
+      mine = pairs(there, fx, fy);
+    } else {
+      for (uint32_t m = there; m != 0u; m &= m - 1u) {
+        const int s = __ffs(m) - 1;
+        const uint32_t v = sad1(__shfl_sync(kFull, fx, s), __shfl_sync(kFull, fy, s));
+        if (lane == s) mine = v;
+      }
     }
     mine = total(mine);
     nsad += __popc(there);
@@ -431,8 +498,13 @@ __device__ void amp_block(const FrameDesc& F, int t, int lane, FlatBlock<S>& K) 
 // the others by warps, `chunk` consecutive ones at a time. GIVEN: entry i of
 // L's queue. AMP: the frames' AMP units one frame after another; those of a
 // frame's 64x64 CUs are its big ones (their halves of 1024 samples and more),
-// numbered first over all frames.
-template <class S, bool AMP, bool WORDS>
+// numbered first over all frames. HALVES: GIVEN jobs of 8 bits that are all
+// blocks of half a warp. They have a kernel of their own: beside the larger
+// blocks' code theirs costs those 2 to 10 % (registers), and a list of both
+// that takes two loops in turn waits for the second one's instructions (3,000
+// 8x8 and 3,000 16x16 jobs 61 -> 79 us). 20,000 8x8 jobs 125 -> 104 us, 600 of
+// them 26 -> 22, 20,000 of 8x4, 4x8 and 4x4 104 -> 87.
+template <class S, bool AMP, bool WORDS, bool HALVES = false>
 __global__ void __launch_bounds__(kFlatWarps * 32, kFlatBlocks) hevc_flat_kernel(LaunchDesc L, int nframes, int64_t nbig,
                                                                                  int chunk) {
   __shared__ uint32_t part[2][kFlatWarps][32];
@@ -468,10 +540,12 @@ __global__ void __launch_bounds__(kFlatWarps * 32, kFlatBlocks) hevc_flat_kernel
     else if (!given_block<S>(L, F, t, lane, K)) return;
     uint32_t nsad, nsatd;
     auto* const shared = reinterpret_cast<uint32_t(*)[W][32]>(part);
-    if (AMP || ((reinterpret_cast<uintptr_t>(K.src) & 3) == 0 && (K.src_stride * (int)sizeof(S) & 3) == 0))
-      flat_search<S, WORDS, true, W>(F, K, &F.out[t], shared, nsad, nsatd);
+    if constexpr (HALVES && W == 1)
+      flat_search<S, WORDS, false, W, true>(F, K, &F.out[t], shared, nsad, nsatd);
+    else if (AMP || ((reinterpret_cast<uintptr_t>(K.src) & 3) == 0 && (K.src_stride * (int)sizeof(S) & 3) == 0))
+      flat_search<S, WORDS, true, W, false>(F, K, &F.out[t], shared, nsad, nsatd);
     else
-      flat_search<S, WORDS, false, W>(F, K, &F.out[t], shared, nsad, nsatd);
+      flat_search<S, WORDS, false, W, false>(F, K, &F.out[t], shared, nsad, nsatd);
     if (W > 1 && threadIdx.x >= 32) return;
     cnt[0] += 1;
     cnt[1] += nsad;
@@ -479,7 +553,7 @@ __global__ void __launch_bounds__(kFlatWarps * 32, kFlatBlocks) hevc_flat_kernel
     cnt[3] += (unsigned long long)nsad * (K.w * K.h);
     cnt[4] += (unsigned long long)nsatd * (K.w * K.h);
   };
-  while (nbig > 0) {
+  while (!HALVES && nbig > 0) {
     __syncthreads();  // the last search's sums, and its place, are read
     if (threadIdx.x == 0) next = atomicAdd(L.head, 1ull);
     __syncthreads();
@@ -502,7 +576,7 @@ __global__ void __launch_bounds__(kFlatWarps * 32, kFlatBlocks) hevc_flat_kernel
 }  // namespace
 
 cudaError_t launch_hevc_flat(const LaunchDesc& L, int bytes_per_sample, bool amp, bool words, int nframes, int64_t nbig,
-                             int nsm, cudaStream_t s) {
+                             int nsm, cudaStream_t s, bool halves) {
   const int64_t most = (int64_t)nsm * kFlatBlocks, small = L.total - nbig;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nbig + (small + kFlatWarps - 1) / kFlatWarps, most));
   // Few takes from the counter while many searches are left for every warp.
@@ -510,6 +584,7 @@ cudaError_t launch_hevc_flat(const LaunchDesc& L, int bytes_per_sample, bool amp
   constexpr int T = kFlatWarps * 32;
   if (bytes_per_sample == 1) {
     if (amp) hevc_flat_kernel<uint8_t, true, true><<<grid, T, 0, s>>>(L, nframes, nbig, chunk);
+    else if (words && halves) hevc_flat_kernel<uint8_t, false, true, true><<<grid, T, 0, s>>>(L, nframes, nbig, chunk);
     else if (words) hevc_flat_kernel<uint8_t, false, true><<<grid, T, 0, s>>>(L, nframes, nbig, chunk);
     else hevc_flat_kernel<uint8_t, false, false><<<grid, T, 0, s>>>(L, nframes, nbig, chunk);
   } else {

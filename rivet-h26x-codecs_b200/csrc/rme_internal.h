@@ -264,10 +264,11 @@ int h264_given_blocks_per_sm(int bytes_per_sample, int variant);
 // the units of 64x64 CUs, the jobs of kFlatBigTiles 4x4 tiles and more, each
 // searched by a CTA. L.head and L.tail count the big and the other searches
 // taken. `words`: rows, planes and origins of every picture are whole 32-bit
-// words apart (true of the library's own).
-constexpr int kFlatBigTiles = 64;
+// words apart (true of the library's own). `halves`: every job is a block of at
+// most kFlatHalfTiles 4x4 tiles (used with 8 bits and `words`).
+constexpr int kFlatBigTiles = 64, kFlatHalfTiles = 4;
 cudaError_t launch_hevc_flat(const LaunchDesc& L, int bytes_per_sample, bool amp, bool words, int nframes, int64_t nbig,
-                             int nsm, cudaStream_t s);
+                             int nsm, cudaStream_t s, bool halves = false);
 // HEVC STANDALONE frames' 2Nx2N blocks in their row form (rme_rows.cu): L's
 // queue holds row_entry words, each the first of hevc_row_rows(size)
 // consecutive rows, all pushed by the host, each after the rows it reads.

@@ -31,7 +31,8 @@ namespace {
 
 constexpr int kNoAllocMaxJobs = 65536;
 constexpr size_t kOffFrame = 0;     // FrameDesc
-constexpr size_t kOffMisc = 512;    // 16 x u64: queue header, counters, status, epoch
+constexpr size_t kOffMisc = 512;    // queue header, counters, status, epoch
+constexpr size_t kMiscBytes = 128;
 constexpr size_t kOffTab = 1024;    // H.264 MvCostTable (8193 x u16)
 constexpr size_t kOffSlots = 17664; // queue slots (kNoAllocMaxJobs x u64)
 constexpr size_t kScratchBytes = kOffSlots + (size_t)kNoAllocMaxJobs * 8;
@@ -146,15 +147,17 @@ extern "C" int rme_search_given_noalloc(const rme_picture_desc* d, const rme_par
   }
 
   // The queue header starts at zero but for the tail (every job is ready)
-  // and this call's epoch; the slots are written by a kernel.
-  unsigned long long misc[16];
-  std::memset(misc, 0, sizeof(misc));
+  // and this call's epoch; the slots are written by a kernel. It goes up with the
+  // frame descriptor in one copy (two take 2 us more).
+  static_assert(kOffFrame == 0, "the descriptor begins the block");
+  unsigned long long block[(kOffMisc + kMiscBytes) / 8] = {};
+  std::memcpy(block, &fd, sizeof(fd));
+  unsigned long long* const misc = block + kOffMisc / 8;
   misc[1] = (unsigned long long)njobs;
   misc[10] = epoch;
   unsigned long long* d_misc = reinterpret_cast<unsigned long long*>(base + kOffMisc);
   unsigned long long* slots = reinterpret_cast<unsigned long long*>(base + kOffSlots);
-  if (cudaMemcpyAsync(base + kOffFrame, &fd, sizeof(fd), cudaMemcpyHostToDevice, s) != cudaSuccess) return RME_ECUDA;
-  if (cudaMemcpyAsync(d_misc, misc, sizeof(misc), cudaMemcpyHostToDevice, s) != cudaSuccess) return RME_ECUDA;
+  if (cudaMemcpyAsync(base, block, sizeof(block), cudaMemcpyHostToDevice, s) != cudaSuccess) return RME_ECUDA;
   if (h264 && cudaMemcpyAsync(base + kOffTab, tab, sizeof(tab), cudaMemcpyHostToDevice, s) != cudaSuccess)
     return RME_ECUDA;
   fill_ready<<<(njobs + 255) / 256, 256, 0, s>>>(slots, njobs, epoch);
@@ -188,7 +191,7 @@ extern "C" int rme_search_given_noalloc(const rme_picture_desc* d, const rme_par
     L.tail = d_misc + 2;
     if (launch_hevc_flat(L, bytes, false, words, 1, 0, nsm, s) != cudaSuccess) return RME_ECUDA;
   }
-  if (cudaMemcpyAsync(misc, d_misc, sizeof(misc), cudaMemcpyDeviceToHost, s) != cudaSuccess) return RME_ECUDA;
+  if (cudaMemcpyAsync(misc, d_misc, kMiscBytes, cudaMemcpyDeviceToHost, s) != cudaSuccess) return RME_ECUDA;
   if (cudaStreamSynchronize(s) != cudaSuccess) return RME_ECUDA;
   if ((uint32_t)misc[9] != 0 || misc[4] != (unsigned long long)njobs) return RME_EDEVICE;
   return RME_OK;

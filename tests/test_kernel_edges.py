@@ -206,6 +206,50 @@ def test_given_jobs_of_every_shape(ms, bd, kw):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("bd", [8, 10])
+@pytest.mark.parametrize("kw", [{}, dict(hevc_search_rings=3, hevc_quarter_cross=1), dict(hevc_search_range=2)])
+def test_given_jobs_of_half_a_warp(ms, bd, kw):
+    """Blocks of at most sixteen words (8 bits: a warp's halves score
+    candidates of their own) and just above: one seed to ten, several alike,
+    walks through the picture and along its edges."""
+    rng = np.random.default_rng(bd + 17 * len(kw))
+    w, h = 134, 98
+    ref = random_picture(rng, w, h, bd, smooth=6)
+    src = shifted(ref, 6, -5, rng, 2.0)
+    ms.upload(2920, src, HEVC, bd)
+    ms.upload(2921, ref, HEVC, bd)
+    shapes = [(4, 4), (8, 4), (4, 8), (8, 8), (16, 4), (4, 16), (12, 4), (4, 12), (12, 8), (4, 20), (20, 4)]
+    jobs = np.zeros(660, capi.JOB_DTYPE)
+    for i, j in enumerate(jobs):
+        bw, bh = shapes[i % len(shapes)]
+        j["w"], j["h"] = bw, bh
+        j["x"] = rng.choice([0, w - bw, rng.integers(0, w - bw + 1)])
+        j["y"] = rng.choice([0, h - bh, rng.integers(0, h - bh + 1)])
+        j["nseeds"] = i // len(shapes) % 11
+        spread = 30 if i % 5 else 900
+        j["mvp"] = rng.integers(-spread, spread + 1, (2, 2))
+        j["seeds"] = rng.integers(-spread, spread + 1, (capi.RME_MAX_SEEDS, 2))
+        j["seeds"][2] = j["seeds"][0]
+    p = oracle.params(HEVC, 27, predictor_mode=capi.RME_PRED_GIVEN, **kw)
+    want = oracle.frame_search(HEVC, bd, src, [ref], p, jobs)
+    small = jobs["w"] * jobs["h"] <= 64
+    for pick, name in ((slice(None), "with larger ones"), (small, "small ones only"),
+                       (np.nonzero(small)[0][:1], "one"), (np.nonzero(jobs["w"] * jobs["h"] == 64)[0][:41], "16 words")):
+        assert_results_equal(ms.search(2920, [2921], p, jobs[pick]), want[pick], name)
+    bi = np.zeros(300, capi.BI_JOB_DTYPE)  # refine_bi's search, from target blocks of their own
+    for i, j in enumerate(bi):
+        j["w"], j["h"] = shapes[i % 8]
+        j["x"], j["y"] = rng.integers(0, w - j["w"] + 1), rng.integers(0, h - j["h"] + 1)
+        j["ref"], j["list"] = (0, 1), i & 1
+        j["mv"] = rng.integers(-60, 61, (2, 2))
+        j["mvp"] = j["mv"] + rng.integers(-6, 7, (2, 2))
+    got = ms.bi_refine(2920, [2921, 2920], p, bi)
+    assert_results_equal(got, oracle.hevc_bi(bd, src, [ref, src], p, bi, refine=True), "refine_bi of small blocks")
+    ms.release(2920)
+    ms.release(2921)
+
+
+@pytest.mark.gpu
 def test_amp_frames_of_both_depths_with_given_frames(ms):
     """AMP units of several frames of two depths in one launch, frames
     without units and H.264 frames among them: each as by itself."""
