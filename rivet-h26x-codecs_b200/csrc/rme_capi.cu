@@ -1327,8 +1327,14 @@ int rme_picture_download_plane(void* ctx, int32_t pic_id, int32_t plane, void* o
   if (cols) *cols = C;
   if (!out) return 0;
   const uint8_t* src = (const uint8_t*)p->buf + (size_t)plane * p->planes.plane_elems * bps;
-  CK(cudaMemcpy2D(out, (size_t)C * bps, src, (size_t)p->planes.stride * bps, (size_t)C * bps, R,
-                  cudaMemcpyDeviceToHost));
+  // Behind the context's stream and the last upload on any other one
+  // (the default stream waits for neither: both are non-blocking).
+  cudaStream_t s = c->stream;
+  CK(cudaSetDevice(c->device));
+  CK(cudaStreamWaitEvent(s, c->evp1, 0));
+  CK(cudaMemcpy2DAsync(out, (size_t)C * bps, src, (size_t)p->planes.stride * bps, (size_t)C * bps, R,
+                       cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
   return 0;
 }
 

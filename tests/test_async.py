@@ -90,3 +90,31 @@ def test_an_asynchronous_search_refuses_pageable_memory(ms):
                                            C.cast(out.ctypes.data, C.POINTER(capi.Result)), None)
     assert rc == capi.RME_EINVAL
     assert ms.sync() == 0
+
+
+@pytest.mark.parametrize("own_stream", [False, True])
+@pytest.mark.parametrize("codec,bd", [(HEVC, 10), (H264, 8)])
+def test_a_downloaded_plane_is_the_last_upload_s(ms, codec, bd, own_stream):
+    """An upload returns before its planes are built; a plane asked for right
+    behind it is the new picture's, whole."""
+    import torch
+    rng = np.random.default_rng(bd)
+    w, h, pad = 2560, 1440, 32 if codec == H264 else 80
+    pics = [rng.integers(0, 1 << bd, (h, w)).astype(np.uint8 if bd == 8 else np.uint16) for _ in range(2)]
+    want = [np.pad(p, pad, mode="edge") for p in pics]
+    pinned = [torch.from_numpy(p.view(np.uint8)).pin_memory().numpy().view(p.dtype) for p in pics]
+    stream = torch.cuda.Stream() if own_stream else None
+    last = 3 if codec == H264 else 15
+    built = []
+    for k in range(2):
+        ms.upload(3600 + k, pics[k], codec, bd)
+        torch.cuda.synchronize()
+        built.append(ms.plane(3600 + k, last))
+    for turn in range(6):
+        k = turn & 1
+        ms.upload(3602, pinned[k], codec, bd, stream=stream.cuda_stream if stream else 0)
+        np.testing.assert_array_equal(ms.plane(3602, last), built[k])
+        ms.upload(3602, pinned[1 - k], codec, bd, stream=stream.cuda_stream if stream else 0)
+        np.testing.assert_array_equal(ms.plane(3602, 0), want[1 - k])
+    for i in range(3):
+        ms.release(3600 + i)
