@@ -391,6 +391,14 @@ int check_params(Ctx* c, const rme_params* p, const rme_picture_desc& d) {
   return why ? fail(c, RME_EINVAL, why) : 0;
 }
 
+// Host memory to the device, there when this returns: a copy of pageable memory
+// may return with its last transfer under way, and the launches' streams do not
+// wait for the default one.
+cudaError_t copy_in(void* dst, const void* src, size_t bytes) {
+  cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 const Tables* get_tables(Ctx* c, const rme_params* p, int bd, int* rc) {
   uint32_t scale_bits;
   float scale = p->codec == RME_CODEC_HEVC ? p->hevc_lambda_scale : 1.0f;
@@ -405,7 +413,7 @@ const Tables* get_tables(Ctx* c, const rme_params* p, int bd, int* rc) {
     h264_cost_table(lam, tab.data());
     t.lam = lam;
     cudaError_t e = cudaMalloc(&t.tab, kMvTab * sizeof(uint16_t));
-    if (e == cudaSuccess) e = cudaMemcpy(t.tab, tab.data(), kMvTab * sizeof(uint16_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = copy_in(t.tab, tab.data(), kMvTab * sizeof(uint16_t));
     if (e != cudaSuccess) {
       *rc = cuda_fail(c, e, "table upload");
       return nullptr;
@@ -482,17 +490,16 @@ const Deps* get_deps(Ctx* c, const rme_picture_desc& d, const rme_params* p, int
   }
   cudaError_t e = cudaMalloc(&dp.pending, std::max<size_t>(pend.size(), 1) * sizeof(int32_t));
   if (e == cudaSuccess)
-    e = cudaMemcpy(dp.pending, pend.data(), pend.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+    e = copy_in(dp.pending, pend.data(), pend.size() * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaMalloc(&dp.d_ready, std::max<size_t>(dp.ready.size(), 1) * sizeof(uint32_t));
   if (e == cudaSuccess)
-    e = cudaMemcpy(dp.d_ready, dp.ready.data(), dp.ready.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    e = copy_in(dp.d_ready, dp.ready.data(), dp.ready.size() * sizeof(uint32_t));
   const size_t nrows = dp.rows.size() + dp.rows_big.size();
   if (e == cudaSuccess && nrows > 0) e = cudaMalloc(&dp.d_rows, nrows * sizeof(uint32_t));
   if (e == cudaSuccess && !dp.rows.empty())
-    e = cudaMemcpy(dp.d_rows, dp.rows.data(), dp.rows.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    e = copy_in(dp.d_rows, dp.rows.data(), dp.rows.size() * sizeof(uint32_t));
   if (e == cudaSuccess && !dp.rows_big.empty())
-    e = cudaMemcpy(dp.d_rows + dp.rows.size(), dp.rows_big.data(), dp.rows_big.size() * sizeof(uint32_t),
-                   cudaMemcpyHostToDevice);
+    e = copy_in(dp.d_rows + dp.rows.size(), dp.rows_big.data(), dp.rows_big.size() * sizeof(uint32_t));
   if (e != cudaSuccess) {
     if (dp.pending) cudaFree(dp.pending);
     if (dp.d_ready) cudaFree(dp.d_ready);

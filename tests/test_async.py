@@ -118,3 +118,20 @@ def test_a_downloaded_plane_is_the_last_upload_s(ms, codec, bd, own_stream):
         np.testing.assert_array_equal(ms.plane(3602, 0), want[1 - k])
     for i in range(3):
         ms.release(3600 + i)
+
+
+@pytest.mark.parametrize("codec", [HEVC, H264])
+def test_the_first_call_of_a_setting_has_its_tables(codec):
+    """What a context builds on the host for a quantiser and a frame shape is
+    on the device before the first search that reads it."""
+    from _common import random_picture, shifted
+    import rivet_h26x_codecs_b200.host as host
+    rng = np.random.default_rng(9)
+    ref = random_picture(rng, 48, 32, 8)
+    src = shifted(ref, 3, -2, rng, 2.0)
+    for qp in range(2, 52, 3):
+        p = oracle.params(codec, qp, hevc_amp=qp & 1)
+        with host.MotionSearch(0) as ms:
+            ms.upload(1, src, codec, 8)
+            ms.upload(2, ref, codec, 8)
+            assert_results_equal(ms.search(1, [2], p), oracle.frame_search(codec, 8, src, [ref], p), f"qp {qp}")
