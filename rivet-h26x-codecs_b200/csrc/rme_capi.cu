@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -115,8 +116,10 @@ uint32_t hevc_ref_idx_bits(int r, int nref) {
 }
 
 // Buffers that grow on demand. `generation` counts reallocations across all
-// of them, so launch graphs captured over an old buffer are never replayed.
-static uint64_t g_buffer_generation = 0;
+// of them, so launch graphs captured over an old buffer are never replayed
+// (contexts grow theirs from several threads: a count that fell back would
+// name an older graph again).
+static std::atomic<uint64_t> g_buffer_generation{0};
 
 template <class T>
 struct DevBuf {
@@ -939,7 +942,7 @@ int run_launch(Ctx* c, const rme_frame* frames, const rme_params* params, int n,
     gsig.push_back(c->wait_polls);
     gsig.push_back((int64_t)(uintptr_t)s);
     gsig.push_back((int64_t)(&sl - c->slots));
-    gsig.push_back((int64_t)g_buffer_generation);
+    gsig.push_back((int64_t)g_buffer_generation.load());
     Graph& g = c->graphs[gsig];
     // A shape is captured when it comes a second time (a one-off batch,
     // common in serving, is not worth a capture).
