@@ -1,7 +1,9 @@
-// The search's device code, shared by the batched kernels (rme_search.cu)
-// and the resident engine (rme_engine.cu): the task functions, the
-// distortion and interpolation-plane reads, the queues. Each file
-// includes it into its own anonymous namespace. Reads of pictures go
+// Device code of the searches. Shared by all of them (rme_rows.cu, rme_flat.cu,
+// rme_h264.cu, rme_search.cu, rme_engine.cu): the distortion and
+// interpolation-plane reads, the rates, published words and queues. Reached by
+// the resident engine only: HEVC's tasks (hevc_task, hevc_group_task, their rows,
+// refine8_patched) and H.264's STANDALONE task; h264_task's GIVEN path also by
+// rme_search.cu. Each file includes it into its own anonymous namespace. Reads of pictures go
 // through RME_LD32: the read-only cache path in the batched kernels (a
 // launch's pictures do not change while it runs); in the engine, where
 // picture slots are refilled while the kernel runs, ordinary cached loads,
