@@ -603,7 +603,8 @@ int rme_probe_wait_timeout(int32_t device, uint32_t polls, uint32_t* status, dou
 /* The same for this context's searches: from now on a STANDALONE launch's
  * wait for another row's vector gives up after `polls` polls (1..2^22, the
  * default), so that a launch whose waits run out can be tried: it ends within
- * about one such wait, with RME_EDEVICE, its results incomplete. */
+ * about one such wait, with RME_EDEVICE, its results incomplete. A resident
+ * server takes the limit that its context has when it starts. */
 int rme_probe_wait_polls(void* ctx, uint32_t polls);
 
 #ifdef __cplusplus

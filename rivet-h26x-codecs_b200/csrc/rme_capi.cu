@@ -1023,6 +1023,8 @@ int ctx_standalone_frame(void* ctx, const rme_frame* f, const rme_params* p, Fra
   return 0;
 }
 
+uint32_t ctx_wait_polls(void* ctx) { return ((Ctx*)ctx)->wait_polls; }
+
 bool ctx_frame_rows(void* ctx, const rme_frame* f, const rme_params* p, const uint32_t** rows, int* nrows,
                     const uint32_t** rows_big, int* nrows_big) {
   Ctx* c = (Ctx*)ctx;

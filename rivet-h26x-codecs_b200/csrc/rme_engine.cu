@@ -473,6 +473,7 @@ int engine_create(void* ctx, int device, Engine** out) {
   L.head_big = g->d_hdr + kHdrHeadBig;
   L.tail_big = g->d_hdr + kHdrTailBig;
   L.group_ctas = groups;
+  L.wait_polls = ctx_wait_polls(ctx);
   L.ring_shift = kRingShift;
   EngineCtl& E = g->E;
   E.fdone = g->d_fdone;

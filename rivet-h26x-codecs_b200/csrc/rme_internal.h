@@ -101,7 +101,7 @@ struct LaunchDesc {
   unsigned long long* counters;  // [tasks, sad, satd, sad_samples, satd_samples]
   const uint32_t* epoch;         // this launch's epoch (device memory: a
                                  // replayed graph keeps its arguments)
-  uint32_t wait_polls;           // batched rows: polls before a wait for another row's vector gives up
+  uint32_t wait_polls;           // rows: polls before a wait for another row's vector gives up
   // The resident engine: the ring of the tasks a whole CTA runs (32x32 and
   // 64x64 blocks), served by the first `group_ctas` CTAs.
   unsigned long long* ready_big;
@@ -157,6 +157,7 @@ int ctx_picture_upload(void* ctx, int32_t pic_id, const rme_picture_desc* d, con
 // row comes after the rows it reads. False for other frames.
 bool ctx_frame_rows(void* ctx, const rme_frame* f, const rme_params* p, const uint32_t** rows, int* nrows,
                     const uint32_t** rows_big, int* nrows_big);
+uint32_t ctx_wait_polls(void* ctx);  // LaunchDesc::wait_polls of the context's searches
 
 // Host helpers shared by the entry points (rme_capi.cu; f32 arithmetic
 // compiled without contraction, so it rounds as the reference's Rust does).

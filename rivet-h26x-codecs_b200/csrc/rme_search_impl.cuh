@@ -419,9 +419,11 @@ __device__ __forceinline__ void st_relaxed64(unsigned long long* p, unsigned lon
 }
 
 // The row form: the published word of a task another row owns, waited for
-// until it carries this search's tag (bounded: kSpinLimit polls, then the
+// until it carries this search's tag (bounded: L.wait_polls polls, then the
 // status word's timeout bit and a zero vector, so that a lost dependency
-// ends the search with an error instead of hanging it). The caller has
+// ends the search with an error instead of hanging it; fewer once the status
+// word is set, so that what depends on it does not wait its full time again).
+// The caller has
 // loaded the word once already (`w`), while it staged its source. The first
 // polls follow one another (the upper row is usually a block ahead, so the
 // word comes within a few round trips); later ones back off.
@@ -429,8 +431,9 @@ __device__ __noinline__ unsigned long long wait_word(const LaunchDesc& L, const 
                                                      unsigned long long w) {
   uint32_t ns = 32;
   for (uint32_t it = 0; (uint32_t)(w >> 32) != tag; ++it) {
-    if (it >= kSpinLimit) {
-      atomicOr(L.status, kStatusWaitTimeout);
+    const bool out = it >= L.wait_polls;
+    if (out || ((it & 63u) == 63u && ld_relaxed32(L.status) != 0u)) {
+      if (out) atomicOr(L.status, kStatusWaitTimeout);
       return (unsigned long long)tag << 32;
     }
     if (it >= 16) {

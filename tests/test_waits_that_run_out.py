@@ -112,3 +112,39 @@ def test_a_failed_launchs_buffer_is_not_written_by_a_later_one():
             ms.search_batch([(10, ids)], p, out=out)
             assert all((o.view(np.uint8) == 0x5a).all() for o in old), f"call {k}"
         assert_results_equal(out.cpu().numpy().view(capi.RESULT_DTYPE), want, "on the device")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bd", [8, 10])
+def test_a_resident_search_short_of_polls_reports_it_and_ends(bd):
+    """The engine's rows: the frames complete with an error, soon, and another
+    server on the same device is right."""
+    rng = np.random.default_rng(bd)
+    pics = [random_picture(rng, 416, 240, bd)]
+    while len(pics) < 8:
+        pics.append(shifted(pics[-1], 3, -2, rng, 2.0))
+    p = oracle.params(HEVC, 30)
+    for polls in (1, 40, POLLS):
+        with host.MotionSearch(0) as ms:
+            _limit(ms, polls)
+            srv = host.Server(ms, hbm_budget_bytes=4 << 30, max_frames_per_launch=8, resident=True)
+            got, t0 = {}, time.time()
+            try:
+                assert srv.open_stream(1, HEVC, bd, 416, 240, p, 1) == 0
+                ids = {srv.submit(1, pic): k for k, pic in enumerate(pics)}
+                while len(got) < len(ids):
+                    for c in srv.poll():
+                        got[ids[c["id"]]] = c
+                    assert time.time() - t0 < 20, f"{len(got)} frames"
+                    time.sleep(0.001)
+            finally:
+                srv.stop()
+            failed = {c["status"] for c in got.values()} - {0}
+            assert failed <= {capi.RME_EDEVICE}
+            if polls == 1:
+                assert failed
+            if polls == POLLS:
+                assert not failed
+            for k in (1, 7):
+                if got[k]["status"] == 0 and not failed:
+                    assert_results_equal(got[k]["results"], oracle.frame_search(HEVC, bd, pics[k], [pics[k - 1]], p), f"{k}")
