@@ -253,6 +253,7 @@ struct Ctx {
   bool tune_on = true;
   uint32_t wait_polls = kSpinLimit;  // LaunchDesc::wait_polls
   cudaStream_t stream = nullptr;
+  cudaStream_t tables_in = nullptr;  // copy_in's
   // The parts of a launch after the first run on streams of their own,
   // forked from and joined back to the caller's stream.
   cudaStream_t aux[kParts] = {nullptr, nullptr, nullptr, nullptr};
@@ -306,6 +307,7 @@ struct Ctx {
       if (aux[k]) cudaStreamDestroy(aux[k]);
     }
     if (stream) cudaStreamDestroy(stream);
+    if (tables_in) cudaStreamDestroy(tables_in);
   }
 };
 
@@ -394,12 +396,14 @@ int check_params(Ctx* c, const rme_params* p, const rme_picture_desc& d) {
   return why ? fail(c, RME_EINVAL, why) : 0;
 }
 
-// Host memory to the device, there when this returns: a copy of pageable memory
-// may return with its last transfer under way, and the launches' streams do not
-// wait for the default one.
-cudaError_t copy_in(void* dst, const void* src, size_t bytes) {
-  cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
-  return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+// Host memory to the device, there when this returns, on a stream that carries
+// nothing else. The default stream's copy of pageable memory may return with its
+// last transfer under way; and it first waits for what the caller's program has
+// queued there, which may itself wait for the resident search to leave, whose
+// next frame the serving thread is preparing here.
+cudaError_t copy_in(Ctx* c, void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->tables_in);
+  return e == cudaSuccess ? cudaStreamSynchronize(c->tables_in) : e;
 }
 
 const Tables* get_tables(Ctx* c, const rme_params* p, int bd, int* rc) {
@@ -416,7 +420,7 @@ const Tables* get_tables(Ctx* c, const rme_params* p, int bd, int* rc) {
     h264_cost_table(lam, tab.data());
     t.lam = lam;
     cudaError_t e = cudaMalloc(&t.tab, kMvTab * sizeof(uint16_t));
-    if (e == cudaSuccess) e = copy_in(t.tab, tab.data(), kMvTab * sizeof(uint16_t));
+    if (e == cudaSuccess) e = copy_in(c, t.tab, tab.data(), kMvTab * sizeof(uint16_t));
     if (e != cudaSuccess) {
       *rc = cuda_fail(c, e, "table upload");
       return nullptr;
@@ -493,16 +497,16 @@ const Deps* get_deps(Ctx* c, const rme_picture_desc& d, const rme_params* p, int
   }
   cudaError_t e = cudaMalloc(&dp.pending, std::max<size_t>(pend.size(), 1) * sizeof(int32_t));
   if (e == cudaSuccess)
-    e = copy_in(dp.pending, pend.data(), pend.size() * sizeof(int32_t));
+    e = copy_in(c, dp.pending, pend.data(), pend.size() * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaMalloc(&dp.d_ready, std::max<size_t>(dp.ready.size(), 1) * sizeof(uint32_t));
   if (e == cudaSuccess)
-    e = copy_in(dp.d_ready, dp.ready.data(), dp.ready.size() * sizeof(uint32_t));
+    e = copy_in(c, dp.d_ready, dp.ready.data(), dp.ready.size() * sizeof(uint32_t));
   const size_t nrows = dp.rows.size() + dp.rows_big.size();
   if (e == cudaSuccess && nrows > 0) e = cudaMalloc(&dp.d_rows, nrows * sizeof(uint32_t));
   if (e == cudaSuccess && !dp.rows.empty())
-    e = copy_in(dp.d_rows, dp.rows.data(), dp.rows.size() * sizeof(uint32_t));
+    e = copy_in(c, dp.d_rows, dp.rows.data(), dp.rows.size() * sizeof(uint32_t));
   if (e == cudaSuccess && !dp.rows_big.empty())
-    e = copy_in(dp.d_rows + dp.rows.size(), dp.rows_big.data(), dp.rows_big.size() * sizeof(uint32_t));
+    e = copy_in(c, dp.d_rows + dp.rows.size(), dp.rows_big.data(), dp.rows_big.size() * sizeof(uint32_t));
   if (e != cudaSuccess) {
     if (dp.pending) cudaFree(dp.pending);
     if (dp.d_ready) cudaFree(dp.d_ready);
@@ -1075,7 +1079,9 @@ int rme_ctx_create(void** out, int32_t device) {
   int nsm = 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return RME_ECUDA;
   c->nsm = nsm;
-  if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) return RME_ECUDA;
+  if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&c->tables_in, cudaStreamNonBlocking) != cudaSuccess)
+    return RME_ECUDA;
   // RME_TUNE=0 keeps every launch on the default occupancy variant.
   if (const char* t = std::getenv("RME_TUNE")) c->tune_on = t[0] != '0';
   if (cudaEventCreate(&c->evp0) != cudaSuccess || cudaEventCreate(&c->evp1) != cudaSuccess) return RME_ECUDA;

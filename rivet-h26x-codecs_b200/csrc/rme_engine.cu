@@ -438,7 +438,12 @@ int engine_create(void* ctx, int device, Engine** out) {
   if (e == cudaSuccess) e = cudaMallocHost(&g->h_one, 64);
   if (e == cudaSuccess) *g->h_one = 1u;
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g->ctl, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g->kstream, cudaStreamNonBlocking);
+  // The kernel's blocks are placed before any pending one of the caller's: some
+  // of them alone (the first serve one ring, the others the other) would wait
+  // for the rest, and a kernel in between for them.
+  int prio_least = 0, prio_greatest = 0;
+  if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&prio_least, &prio_greatest);
+  if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&g->kstream, cudaStreamNonBlocking, prio_greatest);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g->ended, cudaEventDisableTiming);
   if (e == cudaSuccess) e = load_plane_kernels();
   if (e == cudaSuccess) e = load_kernel(prepare_kernel);

@@ -553,7 +553,10 @@ int rme_serve_start(void* ctx, const rme_serve_opts* o, void** server) {
   bool ok = true;
   // Launch mode: the searches' streams at the greatest priority and the
   // uploads' (whose plane builds run beside a search) at the least, so that
-  // a search's blocks are placed before pending plane-build blocks.
+  // a search's blocks are placed before pending plane-build blocks. The
+  // resident engine waits for its uploads' kernels, which are small enough to
+  // start beside it: they go first, lest they queue behind a kernel of the
+  // caller's that is not and waits for the engine to leave.
   int prio_least = 0, prio_greatest = 0;
   cudaDeviceGetStreamPriorityRange(&prio_least, &prio_greatest);
   if (!s->resident_engine)
@@ -563,8 +566,8 @@ int rme_serve_start(void* ctx, const rme_serve_opts* o, void** server) {
            cudaEventCreateWithFlags(&L.done, cudaEventDisableTiming) == cudaSuccess &&
            cudaEventCreateWithFlags(&L.copied, cudaEventDisableTiming) == cudaSuccess;
   if (!ok || (s->resident_engine && rme::engine_create(ctx, s->device, &s->eng) != 0) ||
-      cudaStreamCreateWithPriority(&s->upload, cudaStreamNonBlocking, s->resident_engine ? 0 : prio_least) !=
-          cudaSuccess ||
+      cudaStreamCreateWithPriority(&s->upload, cudaStreamNonBlocking,
+                                   s->resident_engine ? prio_greatest : prio_least) != cudaSuccess ||
       cudaStreamCreateWithFlags(&s->copy, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMallocHost(&s->h_status, 64) != cudaSuccess) {
     if (s->eng) rme::engine_destroy(s->eng);
