@@ -462,7 +462,13 @@ typedef struct {
  * go into one search launch of their own as soon as one of three launch
  * streams is free, so up to three launches overlap on the device.
  * RESIDENT (1): one search kernel stays on the GPU and frames join its queue
- * as they arrive. */
+ * as they arrive. It takes most of every SM until no frame has been in flight
+ * for 20 ms, and other kernels of the process wait for that unless their blocks
+ * fit beside it. While it runs, the process must not enter a CUDA call that
+ * waits for such a kernel with the driver's lock held: a copy to pageable memory
+ * (to pinned memory is fine), a device free, the first use of a kernel whose
+ * module loads lazily. The serving thread would be locked out and could not let
+ * the search leave. LAUNCHES has no such rule. */
 #define RME_SERVE_LAUNCHES 0
 #define RME_SERVE_RESIDENT 1
 
