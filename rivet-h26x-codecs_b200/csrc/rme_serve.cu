@@ -606,6 +606,14 @@ int rme_serve_open_stream(void* server, int32_t stream_id, const rme_picture_des
   // open at once, and two more, pinned here rather than on its first
   // submits, and before the lock (pinning is slow).
   const size_t fb = (size_t)d->stride * d->height * (d->bit_depth == 8 ? 1 : 2);
+  auto refusal = [&]() -> int {  // the lock held
+    if (s->streams.count(stream_id)) return RME_EINVAL;
+    return (int)s->streams.size() >= s->o.max_streams || s->resident + bytes > s->o.hbm_budget_bytes ? RME_EBUSY : 0;
+  };
+  {
+    std::lock_guard<std::mutex> lk(s->m);
+    if (const int refuse = refusal()) return refuse;
+  }
   std::vector<void*> bufs;
   for (int k = 0; k < kPerStream + 2; ++k) {
     void* b = nullptr;
@@ -613,12 +621,12 @@ int rme_serve_open_stream(void* server, int32_t stream_id, const rme_picture_des
     bufs.push_back(b);
   }
   std::lock_guard<std::mutex> lk(s->m);
-  const int refuse = s->streams.count(stream_id) ? RME_EINVAL
-                     : ((int)s->streams.size() >= s->o.max_streams || s->resident + bytes > s->o.hbm_budget_bytes)
-                         ? RME_EBUSY
-                         : 0;
-  if (refuse) {
-    for (void* b : bufs) cudaFreeHost(b);
+  // Refused after all (another thread's stream came first): the buffers stay
+  // for later streams. Freeing pinned memory waits for every kernel, the resident
+  // search among them, and keeps the serving thread's copies out meanwhile, so
+  // that it could not let the search leave.
+  if (const int refuse = refusal()) {
+    for (void* b : bufs) s->pool[fb].push_back(b);
     return refuse;
   }
   Stream st;

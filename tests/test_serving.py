@@ -173,3 +173,31 @@ def test_many_frames_recycle_the_engine_slots_and_survive_idle_periods(resident)
                     refs.append(101 + r)
                 want = ms.search(100, refs, _params(codec, qp))
                 assert_results_equal(got[(sid, k)], want, f"stream {sid} frame {k}")
+
+
+def test_a_stream_refused_while_the_engine_runs():
+    """A refusal frees nothing (that would wait for the resident search, which
+    waits for the serving thread) and leaves the running streams alone."""
+    pics = synth.make_sequence(HEVC, 192, 128, 8, 12, 77, 32, 32, 2.0).frames
+    p = _params(HEVC, 32)
+    with host.MotionSearch(0) as ms:
+        srv = host.Server(ms, hbm_budget_bytes=64 << 20, max_frames_per_launch=8, max_streams=2, resident=True)
+        try:
+            assert srv.open_stream(1, HEVC, 8, 192, 128, p, 2) == 0
+            ids = {}
+            for t, pic in enumerate(pics):
+                ids[srv.submit(1, pic)] = t
+                assert srv.open_stream(2, HEVC, 8, 1920, 1080, p, 2) == capi.RME_EBUSY  # the budget
+                if t == 0:
+                    assert srv.open_stream(3, HEVC, 8, 64, 64, p, 1) == 0
+                if t > 0:
+                    assert srv.open_stream(4, HEVC, 8, 64, 64, p, 1) == capi.RME_EBUSY  # the streams
+            got = {ids[c["id"]]: c for c in _wait(srv, len(pics), timeout=30.0)}
+        finally:
+            srv.stop()
+        assert all(c["status"] == 0 for c in got.values())
+        for t, pic in enumerate(pics):
+            ms.upload(t, pic, HEVC, 8)
+        for t in range(1, len(pics)):
+            want = ms.search(t, [t - 1 - r for r in range(min(2, t))], p)
+            assert_results_equal(got[t]["results"], want, f"frame {t}")
